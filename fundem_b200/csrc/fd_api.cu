@@ -484,7 +484,7 @@ struct PairList {
     // (node, partner) of the list set_contacts uploaded last, in slot order
     std::vector<int> up_node, up_partner;
     // slot and pair scratch of the current step only
-    DevArray<int> c_pair, c_hit, p_hist_cnt;
+    DevArray<int> c_pair, c_hit, p_hist_cnt, r_next;
     DevArray<float> c_phi0;  // pair cache: slot bounds of the last rebuild
     DevArray<float> p_bound; // pair cache: per-pair drift bound of a carried step
     DevArray<int> carry_n;   // pair cache: carried steps since the layout was built
@@ -510,7 +510,7 @@ struct PairList {
         }
         c_pair.alloc(cap_contacts); c_hit.alloc(cap_contacts, false); c_force.alloc((size_t)cap_contacts * 9);
         c_phi0.alloc(cap_contacts, false);
-        p_aux.alloc(cap_pairs); p_hist_cnt.alloc(cap_pairs); p_bound.alloc(cap_pairs, false);
+        p_aux.alloc(cap_pairs); p_hist_cnt.alloc(cap_pairs); r_next.alloc(cap_pairs, false); p_bound.alloc(cap_pairs, false);
         carry_n.alloc(1);
         c_test.alloc(cap_contacts, false);
         n_test.alloc(1);
@@ -525,6 +525,7 @@ struct PairList {
             }
             p_aux.grow(capp, 0);
             p_hist_cnt.grow(capp, 0);
+            r_next.grow(capp, 0);
             p_bound.grow(capp, 0);
             cap_pairs = capp;
         }
@@ -557,7 +558,7 @@ struct PairList {
         v.c_node = c.c_node.p; v.c_slave = c.c_slave.p; v.c_spring = c.c_spring.p; v.c_point = c.c_point.p;
         v.c_normal = c.c_normal.p; v.c_overlap = c.c_overlap.p; v.c_en = c.c_en.p; v.c_es = c.c_es.p;
         v.n_slots = c.counters.p + 1; v.n_hits = c.counters.p + 2; v.cap_contacts = cap_contacts;
-        v.c_pair = c_pair.p; v.c_hit = c_hit.p; v.c_k = c.c_k.p; v.o_c_k = o.c_k.p; v.c_force = c_force.p; v.p_aux = p_aux.p; v.p_hist_cnt = p_hist_cnt.p;
+        v.c_pair = c_pair.p; v.c_hit = c_hit.p; v.c_k = c.c_k.p; v.o_c_k = o.c_k.p; v.c_force = c_force.p; v.p_aux = p_aux.p; v.p_hist_cnt = p_hist_cnt.p; v.r_next = r_next.p;
         v.o_c_node = o.c_node.p; v.o_c_spring = o.c_spring.p;
         v.c_phi0 = c_phi0.p;
         v.p_bound = p_bound.p;
@@ -575,11 +576,10 @@ constexpr long long DENSE_CELLS = 1ll << 22;
 struct CellTable {
     FdGrid g{};
     bool hashed = false;
-    DevArray<int> count, start, fill, sorted, idx_b, bcount, bscan;
-    DevArray<unsigned long long> skey, key_b, hkey;
-    DevArray<int2> hval;
+    DevArray<int> next;
+    DevArray<unsigned int> build;
+    DevArray<unsigned long long> head, hkey;
     unsigned long long hmask = 0;
-    int cap = 0;
     void alloc(const FdGrid& grid, int nobj)
     {
         g = grid;
@@ -589,37 +589,23 @@ struct CellTable {
             size_t H = 1024;
             while (H < 2 * m) H <<= 1;
             hkey.alloc(H, false);
-            hval.alloc(H, false);
+            head.alloc(H);
             hmask = H - 1;
-            count.release();
-            start.release();
-            fill.release();
         } else {
-            count.alloc((size_t)std::max<long long>(g.num, 1));
-            start.alloc((size_t)std::max<long long>(g.num, 1), false);
-            fill.alloc((size_t)std::max<long long>(g.num, 1), false);
+            head.alloc((size_t)std::max<long long>(g.num, 1));
             hkey.release();
-            hval.release();
             hmask = 0;
         }
-        sorted.alloc(m);
-        skey.alloc(m, false);
-        key_b.alloc(m, false);
-        idx_b.alloc(m, false);
-        size_t bc = 0, bs = 0;
-        fd::radix_sort_scratch((int)m, bc, bs);
-        bcount.alloc(bc, false);
-        bscan.alloc(bs, false);
-        cap = (int)m;
+        next.alloc(m, false);
+        build.alloc(2);  // with the heads: no head holds a number above these
     }
-    CellTableDev view()
+    CellTableDev view(int par)
     {
         CellTableDev v{};
         v.g = g;
         v.hashed = hashed ? 1 : 0;
-        v.count = count.p; v.start = start.p; v.fill = fill.p; v.hkey = hkey.p; v.hval = hval.p; v.hmask = hmask;
-        v.sorted = sorted.p; v.skey = skey.p; v.key_b = key_b.p; v.idx_b = idx_b.p;
-        v.bcount = bcount.p; v.bscan_tmp = bscan.p; v.nobj_cap = cap;
+        v.head = head.p; v.next = next.p; v.build = build.p; v.par = par;
+        v.hkey = hkey.p; v.hmask = hmask;
         return v;
     }
 };
@@ -639,7 +625,7 @@ struct Ghost {
     // live: null unless the pair cache covers this image set
     fd::GhostDev view(bool with_live = false)
     {
-        return fd::GhostDev{pos.p, hash.p, cells.view(), occ.p, searchers.p, nsearch.p, q.p, vel.p, rot.p,
+        return fd::GhostDev{pos.p, hash.p, cells.view(0), occ.p, searchers.p, nsearch.p, q.p, vel.p, rot.p,
                             with_live ? live.p : nullptr};
     }
 };
@@ -743,7 +729,6 @@ struct fundem_sim {
     CellTable ptab;
     PairList lists[FD_NKIND];
     Ghost ghosts[6];  // X, Y, XY, then the sector images R90, R180, R270
-    DevArray<int> scan_tmp;
     DevArray<unsigned int> flags;
     DevArray<unsigned long long> stats;  // narrow-phase work counters (profiling only)
     std::vector<int> node_base;
@@ -904,7 +889,8 @@ struct fundem_sim {
     }
     // reverse index over the particle and ghost lists (capacity: their pair
     // capacities together)
-    DevArray<int> rev_cnt, rev_off, rev_fill, rev_code;
+    DevArray<int> rev_cnt, rev_off, rev_code, rev_total;
+    DevArray<unsigned long long> rev_head;
     // the reverse index holds the pairs of the lists the last step used
     // (a reallocation empties it: the next step builds it whatever the flags)
     bool rev_valid = false;
@@ -912,7 +898,7 @@ struct fundem_sim {
     {
         const int np = std::max(P.n(), 1);
         if (rev_cnt.n < (size_t)np) {
-            rev_cnt.alloc(np); rev_off.alloc(np); rev_fill.alloc(np);
+            rev_cnt.alloc(np); rev_off.alloc(np); rev_head.alloc(np); rev_total.alloc(1);
             rev_valid = false;
         }
         long long cap = 0;
@@ -923,7 +909,8 @@ struct fundem_sim {
             rev_code.alloc((size_t)cap, false);
             rev_valid = false;
         }
-        return fd::RevDev{rev_cnt.p, rev_off.p, rev_fill.p, rev_code.p, (int)rev_code.n};
+        return fd::RevDev{rev_cnt.p, rev_off.p, rev_code.p, (int)rev_code.n, rev_head.p, rev_total.p,
+                          ptab.build.p + lists[FD_PP].cur};
     }
     long long launches = 0;
     long long hook_steps = 0;  // steps of fundem_step and fundem_step_begin, for capacity checks
@@ -1163,8 +1150,6 @@ struct fundem_sim {
             if (!br_join[b]) FD_CUDA(cudaEventCreateWithFlags(&br_join[b], cudaEventDisableTiming));
         }
         if (!br_fork) FD_CUDA(cudaEventCreateWithFlags(&br_fork, cudaEventDisableTiming));
-        size_t st = std::max<size_t>(fd::scan_tmp_size(pgrid.num), fd::scan_tmp_size(np));
-        scan_tmp.alloc(st + 16);
         if (!flags.p) flags.alloc(1);
         if (!stats.p) stats.alloc(8);
         FD_CUDA(cudaStreamSynchronize(stream));
@@ -1178,14 +1163,16 @@ struct fundem_sim {
         GeoSetDev G = pgeo.view(), GW = wgeo.view();
         fd::MatDev M = pmat.view(), MW = wmat.view();
         fd::StepArgs a = step_args(dt, probe);
-        CellTableDev T = ptab.view();
+        if (new_generation)
+            for (int k = 0; k < FD_NKIND; ++k) lists[k].cur ^= 1;
+        CellTableDev T = ptab.view(lists[FD_PP].cur);
         // pair cache: steps only (a detection outside a step lists the exact
         // pairs and slots, and the next cached step rebuilds)
         const bool pc = with_force && probe == 0.0 && pc_active();
         fd::PairCacheDev pcv{};
         if (pc) pcv = pc_view();
         tbegin(FUNDEM_T_HASH);
-        fd::launch_hash(Pv, pgrid, stream);
+        fd::launch_hash(Pv, pgrid, stream, T.build, T.par);
         if (pc) {
             fd::launch_pair_cache_check(Pv, pcv, stream);
             pc_steps += 1;
@@ -1194,14 +1181,12 @@ struct fundem_sim {
         }
         lists_exact = !pc;
         // with the cache, the particle table serves only rebuild steps
-        fd::launch_cell_table(Pv, T, scan_tmp.p, scan_tmp.n, stream, pc ? pcv.ctrl : nullptr);
+        fd::launch_cell_table(Pv, T, stream, pc ? pcv.ctrl : nullptr);
         // wall hash (visibility and cell for the node test)
         if (W.n_dev > 0) fd::launch_hash(Wv, wgrid, stream);
         if (pc && W.n_dev > 0) fd::launch_pair_cache_check_walls(Wv, GW, pcv, stream);
         tend(FUNDEM_T_HASH);
         int active[FD_NKIND] = {1, 1, 0, 0, 0};
-        if (new_generation)
-            for (int k = 0; k < FD_NKIND; ++k) lists[k].cur ^= 1;
         PairListDev Lg[6];
         // the translated image sets share the pair cache (not with sector
         // periodicity): their pairs and slots are kept with the particle
@@ -1231,7 +1216,7 @@ struct fundem_sim {
                 fd::GhostDev gh = ghosts[d].view(pcg);
                 ObjDev ghostobj = Pg;
                 ghostobj.hash = ghosts[d].hash.p;
-                fd::launch_cell_table(ghostobj, gh.cells, scan_tmp.p, scan_tmp.n, gs, pcg ? gctrl + 5 : nullptr);
+                fd::launch_cell_table(ghostobj, gh.cells, gs, pcg ? gctrl + 5 : nullptr);
             }
             if (sector) {
                 fd::launch_sector_wrap(Pg, pgrid, gs);
@@ -1240,7 +1225,7 @@ struct fundem_sim {
                 for (int d = 3; d < 6; ++d) {
                     ObjDev ghostobj = Pg;
                     ghostobj.hash = ghosts[d].hash.p;
-                    fd::launch_cell_table(ghostobj, sv[d - 3].cells, scan_tmp.p, scan_tmp.n, gs);
+                    fd::launch_cell_table(ghostobj, sv[d - 3].cells, gs);
                 }
             }
             for (int d = 0; d < 6; ++d) {
@@ -1402,7 +1387,7 @@ struct fundem_sim {
         // also rebuild with them.
         const bool ghosts_cached = pcg && (ghosts[0].active || ghosts[1].active || ghosts[2].active);
         const int* rev_gate = (pc && !sector && rev_valid) ? (ghosts_cached ? gctrl + 5 : pcv.ctrl) : nullptr;
-        fd::launch_reverse(Pv, views, active, rv, scan_tmp.p, scan_tmp.n, stream, rev_gate);
+        fd::launch_reverse(Pv, views, active, rv, stream, rev_gate);
         rev_valid = true;
         if (bd.n > 0 && !bonds_done) fd::launch_bonds(Pv, bd, mixed(), stream);
         fd::launch_reduce(Pv, views, active, rv, bd, mixed(), stream);

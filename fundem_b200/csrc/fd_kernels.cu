@@ -2,8 +2,7 @@
 //
 // Per step (one CUDA stream, no host synchronisation):
 //   kick + drift (+ wall drift)            particleIntegrationKernel.cu:3-48
-//   hash + counting sort into a dense cell table
-//                                          mySpatialGrid.cu:4-26, buildHashStartEnd.cu:47-137
+//   hash + lists of the objects per cell   mySpatialGrid.cu:4-26, buildHashStartEnd.cu:47-137
 //   broad phase: one thread per particle lists candidate partners (bounding
 //                spheres, or SDF-grid spheres for walls and ghosts), sorted
 //                by partner id, into an A-major pair list
@@ -177,7 +176,7 @@ __global__ void k_kick_drift(ObjDev P, GeoSetDev G, double3 g, double h, double 
 }
 
 // ---------------------------------------------------------------------------
-// hashing and the dense cell table (counting sort)
+// hashing and the cell table
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void quat_matrix(const fd_quat q, double R[9])
 {
@@ -187,10 +186,20 @@ __device__ __forceinline__ void quat_matrix(const fd_quat q, double R[9])
     R[6] = 2.0 * (q1 * q3 - q0 * q2); R[7] = 2.0 * (q2 * q3 + q0 * q1); R[8] = 1.0 - 2.0 * (q1 * q1 + q2 * q2);
 }
 
-__global__ void k_hash(ObjDev O, FdGrid g)
+// new build numbers for a cell table: one for the list generation this step
+// writes, a fresh one for the other
+__device__ __forceinline__ void bump_build(unsigned int* build, int par)
+{
+    const unsigned int m = max(build[0], build[1]);
+    build[par] = m + 1u;
+    build[par ^ 1] = m + 2u;
+}
+
+__global__ void k_hash(ObjDev O, FdGrid g, unsigned int* build, int par)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= O.n) return;
+    if (i == 0 && build) bump_build(build, par);
     const long long h = fd_hash(O.pos[i], g);
     O.hash[i] = h;
     if (O.rot) {
@@ -261,50 +270,13 @@ __global__ void __launch_bounds__(RS_TPB) k_rs_scatter(const unsigned long long*
     }
 }
 
-// dense table: objects per cell (atomic count), slots by an atomic scatter,
-// then each cell's slots put in ascending object index, so the table equals
-// the one a stable sort of the hashes gives
-__global__ void k_clear_cells(int* a, int* b, long long n, const int* gate)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (gate && *gate == 0)) return;
-    a[i] = 0;
-    b[i] = 0;
-}
-__global__ void k_cell_count(const long long* hash, int n, long long num, int* count, const int* gate)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (gate && *gate == 0)) return;
-    const long long h = hash[i];
-    if (h >= 0 && h < num) atomicAdd(&count[h], 1);
-}
-__global__ void k_cell_scatter(const long long* hash, int n, long long num, const int* start, int* fill, int* sorted,
-                               const int* gate)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (gate && *gate == 0)) return;
-    const long long h = hash[i];
-    if (h < 0 || h >= num) return;
-    sorted[start[h] + atomicAdd(&fill[h], 1)] = i;
-}
-__global__ void k_cell_order(long long num, const int* count, const int* start, int* sorted, const int* gate)
-{
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= num || (gate && *gate == 0)) return;
-    const int m = count[c];
-    if (m < 2) return;
-    int* seg = sorted + start[c];
-    for (int a = 1; a < m; ++a) {
-        const int v = seg[a];
-        int b = a - 1;
-        while (b >= 0 && seg[b] > v) {
-            seg[b + 1] = seg[b];
-            --b;
-        }
-        seg[b + 1] = v;
-    }
-}
-
+// Cell table: the objects of a cell form a list, head and next.  A counting
+// sort took seven launches of 2-4 us each (clear, count, scan, scatter, order;
+// 28 with the radix sort of a sparse grid), all waiting on one another; the
+// list is one launch of one atomic per object.  The order inside a cell does
+// not matter: every search sorts the partners it keeps.  A head carries the
+// number of the build that wrote it, so heads of older builds read as empty
+// and a dense table is never cleared.
 __global__ void k_hkey_clear(unsigned long long* hkey, unsigned long long n, const int* gate)
 {
     const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -323,50 +295,54 @@ __device__ __forceinline__ unsigned long long cell_slot_hash(unsigned long long 
     return k;
 }
 
-__global__ void k_cells_hashed(const unsigned long long* key, int n, long long num, unsigned long long* hkey,
-                               int2* hval, unsigned long long hmask, unsigned int* flags, const int* gate)
+// put object i into the list of head slot `slot`
+__device__ __forceinline__ void cell_push(const CellTableDev& T, unsigned long long slot, unsigned int build, int i)
+{
+    const unsigned long long old =
+        atomicExch(&T.head[slot], ((unsigned long long)build << 32) | (unsigned int)i);
+    T.next[i] = (unsigned int)(old >> 32) == build ? (int)(unsigned int)old : -1;
+}
+
+__global__ void k_cell_link(const long long* hash, int n, CellTableDev T, const int* gate)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || (gate && *gate == 0)) return;
-    const unsigned long long k = key[i];
-    if (k >= (unsigned long long)num || (i > 0 && key[i - 1] == k)) return;
-    int e = i + 1;
-    while (e < n && key[e] == k) ++e;
-    unsigned long long slot = cell_slot_hash(k) & hmask;
-    // the table holds at least twice as many slots as there are objects, so
-    // an empty slot is always found; the probe count is bounded all the same
-    for (unsigned long long probe = 0; probe <= hmask; ++probe) {
-        const unsigned long long prev = atomicCAS(&hkey[slot], RS_NONE, k);
-        if (prev == RS_NONE || prev == k) {
-            hval[slot] = make_int2(i, e - i);
-            return;
-        }
-        slot = (slot + 1) & hmask;
-    }
-    set_flag(flags, FD_FLAG_INDEX);
-}
-
-// objects in cell h: their count, and the first of their slots in *first
-__device__ __forceinline__ int cell_lookup(const CellTableDev& T, long long h, int& first)
-{
+    const long long h = hash[i];
+    if (h < 0 || h >= T.g.num) return;
+    const unsigned int build = T.build[T.par];
     if (!T.hashed) {
-        const int c = T.count[h];
-        if (c) first = T.start[h];
-        return c;
+        cell_push(T, (unsigned long long)h, build, i);
+        return;
     }
     const unsigned long long k = (unsigned long long)h;
     unsigned long long slot = cell_slot_hash(k) & T.hmask;
+    // the table holds at least twice as many slots as there are objects, so
+    // an empty slot is always found; the probe count is bounded all the same
     for (unsigned long long probe = 0; probe <= T.hmask; ++probe) {
-        const unsigned long long kk = T.hkey[slot];
-        if (kk == k) {
-            const int2 v = T.hval[slot];
-            first = v.x;
-            return v.y;
+        const unsigned long long prev = atomicCAS(&T.hkey[slot], RS_NONE, k);
+        if (prev == RS_NONE || prev == k) {
+            cell_push(T, slot, build, i);
+            return;
         }
-        if (kk == RS_NONE) return 0;
         slot = (slot + 1) & T.hmask;
     }
-    return 0;
+}
+
+// first object of cell h in the build of that number, -1 when it holds none
+__device__ __forceinline__ int cell_first(const CellTableDev& T, long long h, unsigned int build)
+{
+    unsigned long long slot = (unsigned long long)h;
+    if (T.hashed) {
+        slot = cell_slot_hash((unsigned long long)h) & T.hmask;
+        for (unsigned long long probe = 0;; ++probe) {
+            const unsigned long long kk = T.hkey[slot];
+            if (kk == (unsigned long long)h) break;
+            if (kk == RS_NONE || probe >= T.hmask) return -1;
+            slot = (slot + 1) & T.hmask;
+        }
+    }
+    const unsigned long long e = T.head[slot];
+    return (unsigned int)(e >> 32) == build ? (int)(unsigned int)e : -1;
 }
 
 // ---------------------------------------------------------------------------
@@ -459,6 +435,7 @@ __global__ void k_ghost_build(ObjDev P, GhostDev Gh, int kind, double ext_skin, 
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
+    if (i == 0) bump_build(Gh.cells.build, Gh.cells.par);
     const FdGrid& g = Gh.cells.g;
     const double3 p = P.pos[i];
     const double3 ox = mk3(g.maxb.x - g.minb.x, 0., 0.), oy = mk3(0., g.maxb.y - g.minb.y, 0.);
@@ -632,6 +609,11 @@ __global__ void k_sector_images(ObjDev P, GhostDev R90, GhostDev R180, GhostDev 
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
+    if (i == 0) {
+        bump_build(R90.cells.build, R90.cells.par);
+        bump_build(R180.cells.build, R180.cells.par);
+        bump_build(R270.cells.build, R270.cells.par);
+    }
     const FdGrid& g = R90.cells.g;
     const double3 p = P.pos[i], v = P.vel[i];
     const fd_quat q = P.q[i];
@@ -806,7 +788,6 @@ __device__ __forceinline__ void ghost_search_range(double3 c, double rA, double 
 #define FD_BROAD_LANES 8
 #endif
 constexpr int BROAD_LANES = FD_BROAD_LANES;  // lanes per particle in the cell-table broad phases
-constexpr int BROAD_CAND = 128;              // candidate slots staged per lane group and pass
 
 // d with its periodic components taken to the nearest image
 __device__ __forceinline__ double3 nl_min_image(double3 d, const NlDev& nl, const FdGrid& g)
@@ -822,8 +803,8 @@ __device__ __forceinline__ double3 nl_min_image(double3 d, const NlDev& nl, cons
     return d;
 }
 
-// Cell-table broad phase, BROAD_LANES lanes per particle A: the lanes read
-// the cells around A, share out the objects in them, test each (partner
+// Cell-table broad phase, BROAD_LANES lanes per particle A: each lane walks the
+// lists of its share of the cells around A and tests the objects (partner
 // order B > A for particle pairs, bounding spheres, body-level cull) and
 // emit A's pairs sorted by partner id.  GHOST: partners are the ghost images
 // of a cell table built from ghost positions (no B > A rule; the reach is the
@@ -851,7 +832,6 @@ __global__ void __launch_bounds__(TPB) k_broad_cells(ObjDev P, GeoSetDev G, Cell
     if (noskin && *noskin) skin = 0.0;
     if (NLB && nl.ctrl[0] == 0) return;
     __shared__ int s_list[TPB / BROAD_LANES][MAX_CAND];
-    __shared__ int s_cand[TPB / BROAD_LANES][BROAD_CAND];
     const unsigned int full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int gl = lane & (BROAD_LANES - 1);
@@ -860,6 +840,7 @@ __global__ void __launch_bounds__(TPB) k_broad_cells(ObjDev P, GeoSetDev G, Cell
     constexpr int GPW = 32 / BROAD_LANES;           // lane groups per warp
     constexpr int GPB = TPB / BROAD_LANES;          // lane groups per block
     const int total = LIST ? *acount : P.n;
+    const unsigned int build = T.build[T.par];
     // warp-uniform loop over the warp's groups
     for (int gw = blockIdx.x * GPB + (gb & ~(GPW - 1)); gw < total; gw += gridDim.x * GPB) {
     const int gidx = gw + (gb & (GPW - 1));
@@ -893,48 +874,27 @@ __global__ void __launch_bounds__(TPB) k_broad_cells(ObjDev P, GeoSetDev G, Cell
     const int ncell_max = __reduce_max_sync(full, ncell);
     int cnt = 0;  // partners that passed (uniform over the lane group)
     for (int c0 = 0; c0 < ncell_max; c0 += BROAD_LANES) {
-        int cc = 0, cs = 0;
+        int B = -1;
         const int ci = c0 + gl;
         if (ci < ncell) {
             const int x = lo.x + ci % nx, y = lo.y + (ci / nx) % ny;
             const int z = lo.z + ci / (nx * ny);
-            const long long h = fd_lin3(x, y, z, T.g.size);
-            cc = cell_lookup(T, h, cs);
+            B = cell_first(T, fd_lin3(x, y, z, T.g.size), build);
         }
-        // exclusive scan of the cell counts over the lane group
-        int incl = cc;
-#pragma unroll
-        for (int d = 1; d < BROAD_LANES; d <<= 1) {
-            const int y = __shfl_up_sync(full, incl, d, BROAD_LANES);
-            if (gl >= d) incl += y;
-        }
-        const int ex = incl - cc;
-        const int tot = __shfl_sync(full, incl, BROAD_LANES - 1, BROAD_LANES);
-        const int tot_max = __reduce_max_sync(full, tot);
-        for (int f0 = 0; f0 < tot_max; f0 += BROAD_LANES) {
-            // stage the table slots of the next BROAD_CAND candidates
-            if (f0 % BROAD_CAND == 0) {
-                __syncwarp();
-                for (int t = max(ex, f0); t < min(ex + cc, f0 + BROAD_CAND); ++t) s_cand[gb][t - f0] = cs + (t - ex);
-                __syncwarp();
-            }
-            const int f = f0 + gl;
+        // each lane walks the list of its cell
+        while (__any_sync(full, B >= 0)) {
             bool pass = false;
-            int B = -1;
-            if (valid && f < tot) {
-                B = T.sorted[s_cand[gb][f % BROAD_CAND]];
-                if (GHOST || B > A) {
-                    const FdGeo& GB = G.geo[P.geo[B]];
-                    const double3 cB = GHOST ? gpos[B] : P.pos[B];
-                    if (NLB) {
-                        const double rs = (rA + GB.radius) * (1.0 + 8.0 * BOUND_REL) + nl.skin;
-                        pass = lengthSq3(nl_min_image(cA - cB, nl, T.g)) <= rs * rs;
-                    } else {
-                        const double rs = rA + (GHOST ? GB.grid_radius : GB.radius) + skin;
-                        if (lengthSq3(cA - cB) <= rs * rs * (1.0 + 4.0 * BOUND_REL))
-                            pass = !body_culled32(cA, rA + skin, cB, (GHOST && grot ? grot : P.rot) + 3ll * B,
-                                                  !GHOST, GB, G, probe);
-                    }
+            if (B >= 0 && (GHOST || B > A)) {
+                const FdGeo& GB = G.geo[P.geo[B]];
+                const double3 cB = GHOST ? gpos[B] : P.pos[B];
+                if (NLB) {
+                    const double rs = (rA + GB.radius) * (1.0 + 8.0 * BOUND_REL) + nl.skin;
+                    pass = lengthSq3(nl_min_image(cA - cB, nl, T.g)) <= rs * rs;
+                } else {
+                    const double rs = rA + (GHOST ? GB.grid_radius : GB.radius) + skin;
+                    if (lengthSq3(cA - cB) <= rs * rs * (1.0 + 4.0 * BOUND_REL))
+                        pass = !body_culled32(cA, rA + skin, cB, (GHOST && grot ? grot : P.rot) + 3ll * B, !GHOST,
+                                              GB, G, probe);
                 }
             }
             const unsigned int gm = (__ballot_sync(full, pass) >> gbase) & ((1u << BROAD_LANES) - 1u);
@@ -943,6 +903,7 @@ __global__ void __launch_bounds__(TPB) k_broad_cells(ObjDev P, GeoSetDev G, Cell
                 if (pos < MAX_CAND) s_list[gb][pos] = B;
             }
             cnt += __popc(gm);
+            if (B >= 0) B = T.next[B];
         }
     }
     __syncwarp();
@@ -2408,6 +2369,7 @@ __global__ void k_pair_sum32(PairListDev L, int with_force)
 // (FD_GX .. FD_GR270 are consecutive)
 constexpr int REV_LISTS = 7;
 __host__ __device__ constexpr int rev_kind(int k) { return k == 0 ? FD_PP : FD_GX + k - 1; }
+__host__ __device__ constexpr int rev_list(int kind) { return kind == FD_PP ? 0 : kind - FD_GX + 1; }
 static_assert(FD_GR270 == FD_GX + 5 && FD_NKIND == FD_GR270 + 1, "ghost kinds are consecutive and last");
 static_assert(FD_NKIND <= 8, "a reverse-index code keeps the kind in 3 bits");
 
@@ -2432,50 +2394,49 @@ __device__ __forceinline__ bool rev_locate(const RevArgs& r, int idx, int& k, in
     return false;
 }
 
-__global__ void k_rev_count(RevArgs r)
+// Two launches: every pair with contact slots joins the list of its partner
+// (heads tagged with the step's build number, as the cell table's, so nothing
+// is cleared), then each particle walks its list into a segment of codes and
+// sorts it.  Counting, scanning and filling took five to seven launches.
+__global__ void k_rev_link(RevArgs r)
 {
     if (r.gate && *r.gate == 0) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *r.R.total = 0;
+    const unsigned int build = *r.R.build;
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x;; idx += gridDim.x * blockDim.x) {
         int k, p;
         if (!rev_locate(r, idx, k, p)) return;
         const int B = r.L[k].pairB[p];
         // only pairs with contact slots carry a force to the partner
-        if (B >= 0 && B < r.n_obj && r.L[k].c_cnt[p] > 0) atomicAdd(&r.R.cnt[B], 1);
-    }
-}
-__global__ void k_rev_fill(RevArgs r)
-{
-    if (r.gate && *r.gate == 0) return;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x;; idx += gridDim.x * blockDim.x) {
-        int k, p;
-        if (!rev_locate(r, idx, k, p)) return;
-        const int B = r.L[k].pairB[p];
-        if (B >= 0 && B < r.n_obj && r.L[k].c_cnt[p] > 0) {
-            const int slot = r.R.off[B] + atomicAdd(&r.R.fill[B], 1);
-            if (slot < r.R.cap) r.R.code[slot] = p * 8 + rev_kind(k);  // pair counts stay below 2^28
-        }
+        if (B < 0 || B >= r.n_obj || r.L[k].c_cnt[p] <= 0) continue;
+        const unsigned int code = (unsigned int)(p * 8 + rev_kind(k));  // pair counts stay below 2^28
+        const unsigned long long old = atomicExch(&r.R.head[B], ((unsigned long long)build << 32) | code);
+        r.L[k].r_next[p] = (unsigned int)(old >> 32) == build ? (int)(unsigned int)old : -1;
     }
 }
 // deterministic order: by owner, then kind (an owner has one pair per kind
 // with a given partner)
-__global__ void k_rev_sort(RevArgs r)
+__global__ void k_rev_build(RevArgs r)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= r.n_obj || (r.gate && *r.gate == 0)) return;
-    const int o = r.R.off[i];
-    const int cnt = min(r.R.cnt[i], r.R.cap - o);
+    const unsigned long long h = r.R.head[i];
+    int cnt = 0;
+    if ((unsigned int)(h >> 32) == *r.R.build)
+        for (int code = (int)(unsigned int)h; code >= 0; code = r.L[rev_list(code & 7)].r_next[code >> 3]) ++cnt;
+    const int o = cnt ? atomicAdd(r.R.total, cnt) : 0;
+    cnt = min(cnt, r.R.cap - o);
+    r.R.off[i] = o;
+    r.R.cnt[i] = cnt;
     int* seg = r.R.code + o;
-    auto key = [&](int code) {
-        const int kind = code & 7;
-        const int k = kind == FD_PP ? 0 : kind - FD_GX + 1;
-        return (long long)r.L[k].pairA[code >> 3] * 8 + kind;
-    };
-    for (int a = 1; a < cnt; ++a) {
-        const int v = seg[a];
-        const long long kv = key(v);
+    auto key = [&](int code) { return (long long)r.L[rev_list(code & 7)].pairA[code >> 3] * 8 + (code & 7); };
+    int code = (int)(unsigned int)h;
+    for (int a = 0; a < cnt; ++a) {
+        const long long kv = key(code);
         int b = a - 1;
         while (b >= 0 && key(seg[b]) > kv) { seg[b + 1] = seg[b]; --b; }
-        seg[b + 1] = v;
+        seg[b + 1] = code;
+        code = r.L[rev_list(code & 7)].r_next[code >> 3];
     }
 }
 
@@ -2794,9 +2755,9 @@ void launch_kick_drift(const ObjDev& P, const GeoSetDev& G, double3 gravity, dou
 {
     if (P.n > 0) { k_kick_drift<<<nblocks(P.n), TPB, 0, s>>>(P, G, gravity, h, dt); note_launch(); }
 }
-void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s)
+void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s, unsigned int* build, int par)
 {
-    if (O.n > 0) { k_hash<<<nblocks(O.n), TPB, 0, s>>>(O, g); note_launch(); }
+    if (O.n > 0) { k_hash<<<nblocks(O.n), TPB, 0, s>>>(O, g, build, par); note_launch(); }
 }
 void radix_sort_scratch(int n, size_t& bcount_ints, size_t& bscan_ints)
 {
@@ -2828,34 +2789,14 @@ void radix_sort_keys(const long long* keys, int n, long long num_keys, unsigned 
         src ^= 1;
     }
 }
-void launch_cell_table(ObjDev& O, CellTableDev& T, int* scan_tmp, size_t, cudaStream_t s, const int* gate)
+void launch_cell_table(const ObjDev& O, const CellTableDev& T, cudaStream_t s, const int* gate)
 {
     if (O.n <= 0) return;
     if (T.hashed) {
-        // sparse grids: radix sort of the keys, runs into a hash table
-        radix_sort_keys(O.hash, O.n, T.g.num, T.skey, T.sorted, T.key_b, T.idx_b, T.bcount, T.bscan_tmp, s, gate);
-        if (gate) {
-            k_hkey_clear<<<nblocks((long long)T.hmask + 1), TPB, 0, s>>>(T.hkey, T.hmask + 1, gate); note_launch();
-        } else {
-            cudaMemsetAsync(T.hkey, 0xff, sizeof(unsigned long long) * (T.hmask + 1), s);
-        }
-        k_cells_hashed<<<nblocks(O.n), TPB, 0, s>>>(T.skey, O.n, T.g.num, T.hkey, T.hval, T.hmask, nullptr, gate);
+        k_hkey_clear<<<nblocks((long long)T.hmask + 1), TPB, 0, s>>>(T.hkey, T.hmask + 1, gate);
         note_launch();
-        return;
     }
-    // dense grids: count, scan, scatter, then each cell in object order
-    if (gate) {
-        k_clear_cells<<<nblocks(T.g.num), TPB, 0, s>>>(T.count, T.fill, T.g.num, gate);
-        note_launch();
-    } else {
-        cudaMemsetAsync(T.count, 0, sizeof(int) * T.g.num, s);
-        cudaMemsetAsync(T.fill, 0, sizeof(int) * T.g.num, s);
-    }
-    k_cell_count<<<nblocks(O.n), TPB, 0, s>>>(O.hash, O.n, T.g.num, T.count, gate); note_launch();
-    scan_exclusive(T.count, T.start, T.g.num, scan_tmp, s, gate);
-    k_cell_scatter<<<nblocks(O.n), TPB, 0, s>>>(O.hash, O.n, T.g.num, T.start, T.fill, T.sorted, gate);
-    note_launch();
-    k_cell_order<<<nblocks(T.g.num), TPB, 0, s>>>(T.g.num, T.count, T.start, T.sorted, gate); note_launch();
+    k_cell_link<<<nblocks(O.n), TPB, 0, s>>>(O.hash, O.n, T, gate); note_launch();
 }
 void launch_wrap(ObjDev& P, const FdGrid& g, int dim, cudaStream_t s, int* ctrl, const double3* src)
 {
@@ -3035,8 +2976,8 @@ void launch_narrow(int kind, const ObjDev& P, const GeoSetDev& G, const MatDev& 
     note_launch();
 }
 
-void launch_reverse(const ObjDev& P, PairListDev* lists, const int* active, RevDev& R, int* scan_tmp, size_t,
-                    cudaStream_t s, const int* gate)
+void launch_reverse(const ObjDev& P, PairListDev* lists, const int* active, const RevDev& R, cudaStream_t s,
+                    const int* gate)
 {
     if (P.n <= 0) return;
     RevArgs r;
@@ -3047,17 +2988,8 @@ void launch_reverse(const ObjDev& P, PairListDev* lists, const int* active, RevD
     r.R = R;
     r.n_obj = P.n;
     r.gate = gate;
-    if (gate) {
-        k_clear_cells<<<nblocks(P.n), TPB, 0, s>>>(R.cnt, R.fill, P.n, gate); note_launch();
-    } else {
-        cudaMemsetAsync(R.cnt, 0, sizeof(int) * P.n, s);
-        cudaMemsetAsync(R.fill, 0, sizeof(int) * P.n, s);
-    }
-    const int g = 148 * 8;
-    k_rev_count<<<g, TPB, 0, s>>>(r); note_launch();
-    scan_exclusive(R.cnt, R.off, P.n, scan_tmp, s, gate);
-    k_rev_fill<<<g, TPB, 0, s>>>(r); note_launch();
-    k_rev_sort<<<nblocks(P.n), TPB, 0, s>>>(r); note_launch();
+    k_rev_link<<<148 * 8, TPB, 0, s>>>(r); note_launch();
+    k_rev_build<<<nblocks(P.n), TPB, 0, s>>>(r); note_launch();
 }
 
 void launch_bonds(const ObjDev& P, BondDev& B, bool mixed, cudaStream_t s)

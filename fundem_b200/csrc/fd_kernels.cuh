@@ -52,6 +52,7 @@ struct PairListDev {
     double* c_force;   // 9 per slot: F, torque on A, torque on B (contacts only)
     int4* p_aux;       // per pair: cell of B (x, y, z), first history slot
     int* p_hist_cnt;   // per pair: history slots
+    int* r_next;       // per pair: the next pair (code) of its partner's list
     double* c_spring;  // 3 per contact
     double* c_point;   // 3 per contact (records)
     double* c_normal;  // 3 per contact (records)
@@ -82,9 +83,13 @@ struct PairListDev {
 struct RevDev {
     int* cnt;
     int* off;
-    int* fill;
     int* code;
     int cap;
+    // the build: per particle the head of a list of its pairs (build number
+    // << 32 | code, next in PairListDev::r_next), and the codes placed so far
+    unsigned long long* head;
+    int* total;
+    const unsigned int* build;  // the step's build number (the particle cell table's)
 };
 
 struct ObjDev {
@@ -127,31 +132,22 @@ struct MatDev {
     const double* e;
 };
 
-// Cell table of one object set (hashGrid of buildHashStartEnd.cu:69-137).
-// The objects' 64-bit cell keys are sorted by a stable LSD radix sort (so
-// each cell lists its objects in ascending index, as the reference's stable
-// thrust::sort_by_key does); the runs of equal keys are the cells.  A grid of
-// few cells keeps a dense start/count table over all cells; a grid of many
-// cells (dense would be large next to the object count) keeps an
-// open-addressing hash table of its occupied cells instead.
+// Cell table of one object set (hashGrid of buildHashStartEnd.cu:69-137): a
+// list of the objects in each cell.  A grid of few cells keeps a head per
+// cell; a grid of many cells (dense would be large next to the object count)
+// keeps an open-addressing hash table of its occupied cells instead.  A head
+// holds (build number << 32 | first object): a head of another build is
+// empty.  There is one build number per list generation; each is newer than
+// every number a head can hold when its step begins.
 struct CellTableDev {
     FdGrid g;
-    int hashed;                 // 0: dense table, 1: hash table of occupied cells
-    int* count;                 // dense: objects per cell
-    int* start;                 // dense: first slot of each cell (valid where count > 0)
-    int* fill;                  // dense: scatter counters
+    int hashed;                 // 0: a head per cell, 1: hash table of occupied cells
+    unsigned long long* head;   // per cell, or per table slot
+    int* next;                  // per object: the next one in its cell, -1 for the last
+    unsigned int* build;        // [2] build numbers
+    int par;                    // the list generation of this step: build[par] is its number
     unsigned long long* hkey;   // hashed: cell key per table slot (~0: empty)
-    int2* hval;                 // hashed: (first slot, objects) per table slot
     unsigned long long hmask;   // hashed: table size - 1 (a power of two)
-    int* sorted;                // object index per slot, by cell key
-    unsigned long long* skey;   // cell key per slot (~0 for objects in no cell, last)
-    // sort scratch: the second key/index buffers, per-block digit counts and
-    // their scan's temporary
-    unsigned long long* key_b;
-    int* idx_b;
-    int* bcount;
-    int* bscan_tmp;
-    int nobj_cap;               // objects the scratch holds
 };
 
 struct GhostDev {
@@ -324,12 +320,12 @@ void launch_drift(const ObjDev& O, double dt, cudaStream_t s);
 // pass: the end of one step and the start of the next
 void launch_kick_drift(const ObjDev& P, const GeoSetDev& G, double3 gravity, double h, double dt, cudaStream_t s);
 // cell hash of each object (-1 outside the grid) and its single-precision
-// rotation rows
-void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s);
-// the cell table from the objects' hashes (O.hash); with gate non-null a
-// hash-table build runs only when *gate != 0 (the pair cache's rebuild flag)
-void launch_cell_table(ObjDev& O, CellTableDev& T, int* scan_tmp, size_t scan_tmp_ints, cudaStream_t s,
-                       const int* gate = nullptr);
+// rotation rows; build (non-null): the cell table's build numbers, renewed for
+// a step of list generation par
+void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s, unsigned int* build = nullptr, int par = 0);
+// the cell table from the objects' hashes (O.hash); with gate non-null it is
+// built only when *gate != 0 (the pair cache's rebuild flag)
+void launch_cell_table(const ObjDev& O, const CellTableDev& T, cudaStream_t s, const int* gate = nullptr);
 // stable sort of n 64-bit keys (key 0 .. num_keys - 1, or negative: last) on
 // the stream: out_idx gets the permutation, out_key the sorted keys (~0 for
 // the negative ones).  Scratch: key_b (n), idx_b (n), bcount and bscan_tmp
@@ -397,8 +393,8 @@ void launch_narrow(int kind, const ObjDev& P, const GeoSetDev& G, const MatDev& 
                    const GhostDev* gh, PairListDev& L, const StepArgs& a, int with_force, bool mixed, cudaStream_t s);
 // gate (non-null): the index is rebuilt only when *gate != 0 (a step whose
 // lists keep their pairs keeps the index of the step that built them)
-void launch_reverse(const ObjDev& P, PairListDev* lists, const int* active, RevDev& R, int* scan_tmp,
-                    size_t scan_tmp_ints, cudaStream_t s, const int* gate = nullptr);
+void launch_reverse(const ObjDev& P, PairListDev* lists, const int* active, const RevDev& R, cudaStream_t s,
+                    const int* gate = nullptr);
 // mixed: single-precision contact law, bond law and force sums
 void launch_bonds(const ObjDev& P, BondDev& B, bool mixed, cudaStream_t s);
 void launch_reduce(ObjDev& P, PairListDev* lists, const int* active, const RevDev& R, const BondDev& B, bool mixed,
