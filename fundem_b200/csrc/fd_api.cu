@@ -484,10 +484,9 @@ struct PairList {
     // (node, partner) of the list set_contacts uploaded last, in slot order
     std::vector<int> up_node, up_partner;
     // slot and pair scratch of the current step only
-    DevArray<int> c_pair, c_hit, p_hist_cnt, r_next;
+    DevArray<int> c_pair, c_hit, p_hist_cnt, r_next, p_hit;
     DevArray<float> c_phi0;  // pair cache: slot bounds of the last rebuild
     DevArray<float> p_bound; // pair cache: per-pair drift bound of a carried step
-    DevArray<int> carry_n;   // pair cache: carried steps since the layout was built
     DevArray<int> c_test, n_test;  // pair cache: slots listed for the predicate pass
     DevArray<double> c_force;
     DevArray<int4> p_aux;
@@ -510,8 +509,7 @@ struct PairList {
         }
         c_pair.alloc(cap_contacts); c_hit.alloc(cap_contacts, false); c_force.alloc((size_t)cap_contacts * 9);
         c_phi0.alloc(cap_contacts, false);
-        p_aux.alloc(cap_pairs); p_hist_cnt.alloc(cap_pairs); r_next.alloc(cap_pairs, false); p_bound.alloc(cap_pairs, false);
-        carry_n.alloc(1);
+        p_aux.alloc(cap_pairs); p_hist_cnt.alloc(cap_pairs); r_next.alloc(cap_pairs, false); p_hit.alloc(cap_pairs); p_bound.alloc(cap_pairs, false);
         c_test.alloc(cap_contacts, false);
         n_test.alloc(1);
         allocated = true;
@@ -526,6 +524,7 @@ struct PairList {
             p_aux.grow(capp, 0);
             p_hist_cnt.grow(capp, 0);
             r_next.grow(capp, 0);
+            p_hit.grow(capp, cap_pairs);
             p_bound.grow(capp, 0);
             cap_pairs = capp;
         }
@@ -558,11 +557,10 @@ struct PairList {
         v.c_node = c.c_node.p; v.c_slave = c.c_slave.p; v.c_spring = c.c_spring.p; v.c_point = c.c_point.p;
         v.c_normal = c.c_normal.p; v.c_overlap = c.c_overlap.p; v.c_en = c.c_en.p; v.c_es = c.c_es.p;
         v.n_slots = c.counters.p + 1; v.n_hits = c.counters.p + 2; v.cap_contacts = cap_contacts;
-        v.c_pair = c_pair.p; v.c_hit = c_hit.p; v.c_k = c.c_k.p; v.o_c_k = o.c_k.p; v.c_force = c_force.p; v.p_aux = p_aux.p; v.p_hist_cnt = p_hist_cnt.p; v.r_next = r_next.p;
+        v.c_pair = c_pair.p; v.c_hit = c_hit.p; v.c_k = c.c_k.p; v.o_c_k = o.c_k.p; v.c_force = c_force.p; v.p_aux = p_aux.p; v.p_hist_cnt = p_hist_cnt.p; v.r_next = r_next.p; v.p_hit = p_hit.p;
         v.o_c_node = o.c_node.p; v.o_c_spring = o.c_spring.p;
         v.c_phi0 = c_phi0.p;
         v.p_bound = p_bound.p;
-        v.carry_n = carry_n.p;
         v.c_test = c_test.p;
         v.n_test = n_test.p;
         return v;
@@ -597,7 +595,10 @@ struct CellTable {
             hmask = 0;
         }
         next.alloc(m, false);
-        build.alloc(2);  // with the heads: no head holds a number above these
+        // with the zeroed heads: no head holds a number from these on
+        build.alloc(2, false);
+        const unsigned int first[2] = {1u, 1u};
+        FD_CUDA(after_legacy(cudaMemcpy(build.p, first, sizeof(first), cudaMemcpyHostToDevice)));
     }
     CellTableDev view(int par)
     {
@@ -613,7 +614,7 @@ struct CellTable {
 struct Ghost {
     DevArray<double3> pos;
     DevArray<long long> hash;
-    DevArray<int> occ, searchers, nsearch;
+    DevArray<int> occ;
     CellTable cells;
     // sector images only: orientation, velocity, rotation rows
     DevArray<fd_quat> q;
@@ -625,7 +626,7 @@ struct Ghost {
     // live: null unless the pair cache covers this image set
     fd::GhostDev view(bool with_live = false)
     {
-        return fd::GhostDev{pos.p, hash.p, cells.view(0), occ.p, searchers.p, nsearch.p, q.p, vel.p, rot.p,
+        return fd::GhostDev{pos.p, hash.p, cells.view(0), occ.p, q.p, vel.p, rot.p,
                             with_live ? live.p : nullptr};
     }
 };
@@ -753,7 +754,7 @@ struct fundem_sim {
     }
     fd::NlDev nl_view()
     {
-        return fd::NlDev{nl_ref.p, nl_vis.p, nl_cnt.p, nl_list.p, nl_ctrl.p, NL_SKIN * pgeo.rmax, perX, perY, 0.0};
+        return fd::NlDev{nl_ref.p, nl_vis.p, nl_cnt.p, nl_list.p, nl_ctrl.p, NL_SKIN * pgeo.rmax, perX, perY};
     }
     // contiguous views handed out by fundem_contact_view_get / fundem_bond_view_get
     struct ContactView {
@@ -910,7 +911,79 @@ struct fundem_sim {
             rev_valid = false;
         }
         return fd::RevDev{rev_cnt.p, rev_off.p, rev_code.p, (int)rev_code.n, rev_head.p, rev_total.p,
-                          ptab.build.p + lists[FD_PP].cur};
+                          ptab.build.p + lists[FD_PP].cur, nullptr, nullptr};
+    }
+    // Small sets step with two launches (launch_small_pairs,
+    // launch_small_advance).  The rule: no images, no pair cache or neighbour
+    // list (so fewer particles than either starts at), a dense cell table,
+    // and not under the stage timers, which see the stages one by one.
+    // Measured per step of a pour (graph replay): see k_small_pairs.
+    DevArray<int> small_head;
+    DevArray<double> small_own;
+    bool small_on() const
+    {
+        return P.n_dev > 0 && P.n_dev < NL_MIN_PARTICLES && !use_nl && !pc_active() && !perX && !perY && !sector &&
+               !ptab.hashed && (!profiling || capturing);
+    }
+    // the current step (set by front): small, with the pair cache; whether its
+    // force sums are still to run, and the wrapped positions they take over
+    bool small = false, step_pc = false, sum_pending = false;
+    const double3* step_wrapped = nullptr;
+    int step_active[FD_NKIND] = {};
+    void small_advance(double3 g, double dt, int parts)
+    {
+        PairList &Lp = lists[FD_PP], &Lw = lists[FD_PW];
+        const int next = Lp.cur ^ 1;
+        fd::launch_small_advance(P.view(), pgeo.view(), W.view(), pgrid, wgrid, Lp.view(), bond_view(),
+                                 ptab.view(next), small_head.p, small_own.p, Lp.gen[next].counters.p,
+                                 Lw.gen[next].counters.p, g, dt, mixed(), parts, stream);
+    }
+    fd::StepShared step_shared(bool with_force)
+    {
+        fd::StepShared c{};
+        c.n = P.n_dev;
+        c.G = pgeo.view(); c.GW = wgeo.view();
+        c.M = pmat.view(); c.MW = wmat.view();
+        c.W = W.view();
+        c.pgrid = pgrid; c.wgrid = wgrid;
+        c.T = ptab.view(lists[FD_PP].cur);
+        c.wall_range = wall_groups.empty() ? nullptr : d_wall_groups.p;
+        if (with_force) c.R = rev_view();
+        c.with_force = with_force;
+        c.mixed = mixed();
+        return c;
+    }
+    // what surrounds the detection of a step: parts of launch_advance
+    void advance(double3 g, double dt, int parts)
+    {
+        if (sum_pending) parts |= fd::STEP_SUM;
+        if (small) {
+            if (parts != fd::STEP_BACK) {
+                small_advance(g, dt, parts);
+                sum_pending = false;
+                return;
+            }
+        }
+        const bool sum = sum_pending;
+        sum_pending = false;
+        tbegin((parts & ~fd::STEP_SUM) ? FUNDEM_T_INTEGRATE : FUNDEM_T_REDUCE);
+        PairListDev views[FD_NKIND];
+        for (int k = 0; k < FD_NKIND; ++k) views[k] = lists[k].view();
+        fd::PairCacheDev pcv{};
+        const bool front = (parts & fd::STEP_FRONT) != 0;
+        const bool pc = front && pc_active();
+        if (pc) pcv = pc_view();
+        int* occ[6];
+        for (int d = 0; d < 6; ++d) occ[d] = front && ghosts[d].active ? ghosts[d].occ.p : nullptr;
+        if (front) step_pc = pc;
+        fd::launch_advance(step_shared(sum), P.view(), views, step_active, bond_view(), step_wrapped, g, dt,
+                           pc ? &pcv : nullptr, occ, lists[FD_PP].cur ^ 1, parts, stream);
+        tend((parts & ~fd::STEP_SUM) ? FUNDEM_T_INTEGRATE : FUNDEM_T_REDUCE);
+    }
+    // the force sums of a step whose second half kick is another call's
+    void finish_forces()
+    {
+        if (sum_pending) advance(make_double3(0, 0, 0), 0.0, 0);
     }
     long long launches = 0;
     long long hook_steps = 0;  // steps of fundem_step and fundem_step_begin, for capacity checks
@@ -938,22 +1011,20 @@ struct fundem_sim {
             g.exec = nullptr;
         }
     }
-    // the particle-wall list (branch 1) and, with translated periodicity,
-    // the image lists (branch 0) are detected on streams of their own beside
-    // the particle-particle list.  The image branch works on a copy of the
-    // positions that the periodic wraps change (the other lists are detected
-    // with them unwrapped); the wrapped positions come back at the join.
-    cudaStream_t br_stream[2] = {nullptr, nullptr};
-    cudaEvent_t br_fork = nullptr, br_join[2] = {nullptr, nullptr};
+    // the bonds run on a stream of their own beside the detection, which
+    // shares nothing they write; with translated periodicity the images and
+    // the bonds see the wrapped positions, which stay in a copy until the force
+    // sums (the particle and wall lists are detected with them unwrapped)
+    cudaStream_t br_stream = nullptr;
+    cudaEvent_t br_fork = nullptr, br_join = nullptr;
     DevArray<double3> img_pos;
+    DevArray<unsigned int> end_done;
     ~fundem_sim()
     {
         drop_graph();
         if (cap_stream) cudaStreamDestroy(cap_stream);
-        for (int b = 0; b < 2; ++b) {
-            if (br_stream[b]) cudaStreamDestroy(br_stream[b]);
-            if (br_join[b]) cudaEventDestroy(br_join[b]);
-        }
+        if (br_stream) cudaStreamDestroy(br_stream);
+        if (br_join) cudaEventDestroy(br_join);
         if (br_fork) cudaEventDestroy(br_fork);
     }
     AdjState adj;
@@ -1139,16 +1210,16 @@ struct fundem_sim {
                 ghosts[d].hash.alloc(std::max(np, 1));
                 if (d < 3) ghosts[d].live.alloc(std::max(np, 1));
                 ghosts[d].occ.alloc(6);
-                ghosts[d].searchers.alloc(std::max(np, 1));
-                ghosts[d].nsearch.alloc(1);
                 ghosts[d].cells.alloc(pgrid, np);
             }
         }
+        small_head.alloc(std::max(np, 1), false);
+        small_own.alloc(6 * (size_t)std::max(np, 1));
+        FD_CUDA(after_legacy(cudaMemset(small_head.p, 0xff, sizeof(int) * small_head.n)));
         if ((perX || perY) && !sector) img_pos.alloc(std::max(np, 1), false);
-        for (int b = 0; b < 2; ++b) {
-            if (!br_stream[b]) FD_CUDA(cudaStreamCreateWithFlags(&br_stream[b], cudaStreamNonBlocking));
-            if (!br_join[b]) FD_CUDA(cudaEventCreateWithFlags(&br_join[b], cudaEventDisableTiming));
-        }
+        if (!br_stream) FD_CUDA(cudaStreamCreateWithFlags(&br_stream, cudaStreamNonBlocking));
+        if (!br_join) FD_CUDA(cudaEventCreateWithFlags(&br_join, cudaEventDisableTiming));
+        if (!end_done.p) end_done.alloc(1);
         if (!br_fork) FD_CUDA(cudaEventCreateWithFlags(&br_fork, cudaEventDisableTiming));
         if (!flags.p) flags.alloc(1);
         if (!stats.p) stats.alloc(8);
@@ -1156,244 +1227,199 @@ struct fundem_sim {
         setup_done = true;
     }
 
-    // hash + detection (+ forces) of one step, LSSolver.h:1201-1215
+    void record_slots(int kind)
+    {
+        FD_CUDA(cudaMemcpyAsync(recording->ns(kind, record_step), lists[kind].view().n_slots, sizeof(int),
+                                cudaMemcpyDeviceToDevice, stream));
+    }
+    void record_bonds(fd::BondDev& bd)
+    {
+        bd.rec_active = recording->bond_active.p + (long long)record_step * bd.n;
+        bd.rec_rij = recording->bond_rij.p + 3ll * record_step * bd.n;
+        bd.rec_dn = recording->bond_dn.p + 3ll * record_step * bd.n;
+    }
+
+    // detection (+ forces) of one step, LSSolver.h:1201-1215; the force sums
+    // are left to finish_forces, back or back_front.  A step's bodies are
+    // hashed by its front; a detection outside a step hashes them here.
     void detect_all(bool with_force, double dt, double probe = 0.0, bool new_generation = true)
     {
         ObjDev Pv = P.view(), Wv = W.view();
-        GeoSetDev G = pgeo.view(), GW = wgeo.view();
-        fd::MatDev M = pmat.view(), MW = wmat.view();
-        fd::StepArgs a = step_args(dt, probe);
         if (new_generation)
             for (int k = 0; k < FD_NKIND; ++k) lists[k].cur ^= 1;
-        CellTableDev T = ptab.view(lists[FD_PP].cur);
+        fd::StepArgs a = step_args(dt, probe);
+        fd::BondDev bd = bond_view();
+        if (recording && bd.n > 0) record_bonds(bd);
+        if (with_force && small) {
+            fd::StepShared c = step_shared(false);
+            fd::launch_bonds(Pv, bd, mixed(), stream);
+            fd::AdjRec recw{};
+            if (recording) {
+                a.rec = recording->rec(FD_PP, record_step);
+                recw = recording->rec(FD_PW, record_step);
+            }
+            lists_exact = true;
+            PairListDev Lp = lists[FD_PP].view(), Lw = lists[FD_PW].view();
+            fd::launch_small_pairs(Pv, c.G, c.M, Wv, c.GW, c.MW, pgrid, wgrid, c.T, Lp, Lw, a, recw, c.wall_range,
+                                   small_head.p, small_own.p, mixed(), stream);
+            if (recording)
+                for (int k : {FD_PP, FD_PW}) record_slots(k);
+            sum_pending = true;
+            FD_CUDA(cudaGetLastError());
+            return;
+        }
         // pair cache: steps only (a detection outside a step lists the exact
         // pairs and slots, and the next cached step rebuilds)
-        const bool pc = with_force && probe == 0.0 && pc_active();
+        const bool pc = with_force && step_pc;
         fd::PairCacheDev pcv{};
-        if (pc) pcv = pc_view();
-        tbegin(FUNDEM_T_HASH);
-        fd::launch_hash(Pv, pgrid, stream, T.build, T.par);
         if (pc) {
-            fd::launch_pair_cache_check(Pv, pcv, stream);
+            pcv = pc_view();
             pc_steps += 1;
         } else if (pc_on) {
             pc_force = true;
         }
         lists_exact = !pc;
-        // with the cache, the particle table serves only rebuild steps
-        fd::launch_cell_table(Pv, T, stream, pc ? pcv.ctrl : nullptr);
-        // wall hash (visibility and cell for the node test)
-        if (W.n_dev > 0) fd::launch_hash(Wv, wgrid, stream);
-        if (pc && W.n_dev > 0) fd::launch_pair_cache_check_walls(Wv, GW, pcv, stream);
-        tend(FUNDEM_T_HASH);
-        int active[FD_NKIND] = {1, 1, 0, 0, 0};
-        PairListDev Lg[6];
         // the translated image sets share the pair cache (not with sector
         // periodicity): their pairs and slots are kept with the particle
         // pairs', and a wrap or an image in a clamped cell rebuilds them
         const bool pcg = pc && !sector;
         int* gctrl = pcg ? pcv.ctrl : nullptr;
-        bool img_wrapped = false;
-        // PeriodicBoundaryXY2D then PeriodicBoundarySector::updateGhostSpatialGrid
-        // (LSSolver.h:780-784), then the detection of every image set, on
-        // stream gs with the particle set Pg.  wrap_src non-null: Pg.pos is a
-        // separate array, and the first wrap fills it from wrap_src.
-        auto image_stage = [&](cudaStream_t gs, ObjDev Pg, const double3* wrap_src) {
-            tbegin(FUNDEM_T_GHOST);
-            const int kinds[6] = {FD_GX, FD_GY, FD_GXY, FD_GR90, FD_GR180, FD_GR270};
-            for (int d = 0; d < 3; ++d) {
-                if (!ghosts[d].active) continue;
-                if (d < 2) {
-                    fd::launch_wrap(Pg, pgrid, d, gs, gctrl, img_wrapped ? nullptr : wrap_src);
-                    img_wrapped = true;
-                }
-                fd::GhostDev gh = ghosts[d].view(pcg);
-                fd::launch_ghost_build(Pg, gh, kinds[d], gs, pcg ? pcv.skin : 0.0, gctrl);
+        const bool images = perX || perY;
+        fd::StepShared c = step_shared(with_force);
+        if (with_force) {
+            // the reverse index depends only on the lists' pairs: under the
+            // pair cache (without sector images, whose lists are detected
+            // afresh every step) a step that keeps them keeps the index
+            if (pc && !sector && rev_valid) {
+                c.R.gate = pcv.ctrl;
+                c.R.gate2 = images ? pcv.ctrl + 4 : nullptr;
             }
-            if (pcg) fd::launch_ghost_gate(gctrl, gs);
-            for (int d = 0; d < 3; ++d) {
-                if (!ghosts[d].active) continue;
-                fd::GhostDev gh = ghosts[d].view(pcg);
-                ObjDev ghostobj = Pg;
-                ghostobj.hash = ghosts[d].hash.p;
-                fd::launch_cell_table(ghostobj, gh.cells, gs, pcg ? gctrl + 5 : nullptr);
-            }
-            if (sector) {
-                fd::launch_sector_wrap(Pg, pgrid, gs);
-                fd::GhostDev sv[3] = {ghosts[3].view(), ghosts[4].view(), ghosts[5].view()};
-                fd::launch_sector_images(Pg, sv, gs);
-                for (int d = 3; d < 6; ++d) {
-                    ObjDev ghostobj = Pg;
-                    ghostobj.hash = ghosts[d].hash.p;
-                    fd::launch_cell_table(ghostobj, sv[d - 3].cells, gs);
-                }
-            }
-            for (int d = 0; d < 6; ++d) {
-                if (!ghosts[d].active) continue;
-                const bool cached = pcg && d < 3;
-                fd::GhostDev gh = ghosts[d].view(cached);
-                Lg[d] = lists[kinds[d]].view();
-                fd::StepArgs ag = a;
-                if (cached) {
-                    ag.skin = pcv.skin;
-                    ag.gate = gctrl + 5;
-                    ag.noskin = gctrl + 6;
-                    ag.drift = pcv.drift;
-                    ag.disp = pcv.disp;
-                    fd::launch_broad_ghost(Pg, G, gh, Lg[d], flags.p, probe, gs, pcv.skin, gctrl + 5, gctrl + 6);
-                } else {
-                    fd::launch_broad_ghost(Pg, G, gh, Lg[d], flags.p, probe, gs);
-                }
-                ag.rec = recording ? recording->rec(kinds[d], record_step) : fd::AdjRec{};
-                fd::launch_narrow(kinds[d], Pg, G, M, Wv, GW, MW, pgrid, wgrid, &gh, Lg[d], ag, with_force, mixed(),
-                                  gs);
-                if (recording)
-                    FD_CUDA(cudaMemcpyAsync(recording->ns(kinds[d], record_step), Lg[d].n_slots, sizeof(int),
-                                            cudaMemcpyDeviceToDevice, gs));
-                active[kinds[d]] = 1;
-            }
-            tend(FUNDEM_T_GHOST);
-        };
-        PairListDev Lpw = lists[FD_PW].view();
-        auto wall_stage = [&](cudaStream_t ws) {
-            tbegin(FUNDEM_T_BROAD);
-            fd::launch_broad_pw(Pv, G, Wv, GW, wgrid, Lpw, flags.p, probe, ws,
-                                wall_groups.empty() ? nullptr : d_wall_groups.p, pc ? pcv.skin : 0.0,
-                                pc ? pcv.ctrl : nullptr);
-            tend(FUNDEM_T_BROAD);
-            tbegin(FUNDEM_T_NARROW_PW);
-            // the particle-wall list shares the cache (wall drifts and cells
-            // in its rebuild flag)
-            fd::StepArgs aw = a;
-            aw.rec = recording ? recording->rec(FD_PW, record_step) : fd::AdjRec{};
-            if (pc) {
-                aw.skin = pcv.skin;
-                aw.gate = pcv.ctrl;
-                aw.drift = pcv.drift;
-                aw.disp = pcv.disp;
-                aw.driftB = pcv.wdrift;
-                aw.dispB = pcv.wdisp;
-            }
-            fd::launch_narrow(FD_PW, Pv, G, M, Wv, GW, MW, pgrid, wgrid, nullptr, Lpw, aw, with_force, mixed(), ws);
-            if (pc && W.n_dev > 0) fd::launch_pair_cache_commit_walls(Wv, pcv, ws);
-            if (recording)
-                FD_CUDA(cudaMemcpyAsync(recording->ns(FD_PW, record_step), Lpw.n_slots, sizeof(int),
-                                        cudaMemcpyDeviceToDevice, ws));
-            tend(FUNDEM_T_NARROW_PW);
-        };
-        // outside per-stage timing the wall list and the images (translated
-        // periodicity) run beside the particle-particle list, and the bonds
-        // at the end of one of them.  Each branch reads and writes nothing
-        // another one writes: its own lists, tables and image arrays; the
-        // wall references of the pair cache (branch 1); the wrapped copy of
-        // the positions and the pair cache's words 4-7, which the others do
-        // not read (branch 0); the bond arrays (the branch that runs the
-        // bonds); the flags and counters with atomics.  The pair cache's
-        // rebuild flag (word 0) and drifts are written before the fork.
-        const bool branches = br_stream[0] && br_stream[1] && (!profiling || capturing);
-        const bool img_branch = branches && (perX || perY) && !sector && img_pos.p && img_pos.n >= (size_t)Pv.n;
-        // the bonds read only positions (after the wraps) and orientations:
-        // they run at the end of a branch, off the particle pairs' path
-        fd::BondDev bd = bond_view();
-        if (recording && bd.n > 0) {
-            bd.rec_active = recording->bond_active.p + (long long)record_step * bd.n;
-            bd.rec_rij = recording->bond_rij.p + 3ll * record_step * bd.n;
-            bd.rec_dn = recording->bond_dn.p + 3ll * record_step * bd.n;
-        }
-        bool bonds_done = false;
-        if (branches) FD_CUDA(cudaEventRecord(br_fork, stream));
-        if (img_branch) {
-            FD_CUDA(cudaStreamWaitEvent(br_stream[0], br_fork, 0));
-            ObjDev Pg = Pv;
-            Pg.pos = img_pos.p;
-            image_stage(br_stream[0], Pg, Pv.pos);
-            if (with_force && bd.n > 0) {
-                fd::launch_bonds(Pg, bd, mixed(), br_stream[0]);
-                bonds_done = true;
-            }
-            FD_CUDA(cudaEventRecord(br_join[0], br_stream[0]));
-        }
-        if (branches) {
-            FD_CUDA(cudaStreamWaitEvent(br_stream[1], br_fork, 0));
-            wall_stage(br_stream[1]);
-            if (with_force && bd.n > 0 && !bonds_done && !(perX || perY || sector)) {
-                fd::launch_bonds(Pv, bd, mixed(), br_stream[1]);
-                bonds_done = true;
-            }
-            FD_CUDA(cudaEventRecord(br_join[1], br_stream[1]));
-        }
-        PairListDev Lpp = lists[FD_PP].view();
-        tbegin(FUNDEM_T_BROAD);
-        if (use_nl) {
-            fd::NlDev nl = nl_view();
-            nl.pair_skin = pc ? pcv.skin : 0.0;
-            fd::launch_broad_pp_nl(Pv, G, T, Lpp, nl, flags.p, probe, stream, pc ? pcv.ctrl : nullptr);
+            rev_valid = true;
         } else {
-            fd::launch_broad_pp(Pv, G, T, Lpp, flags.p, probe, stream, pc ? pcv.skin : 0.0, pc ? pcv.ctrl : nullptr);
+            tbegin(FUNDEM_T_HASH);
+            fd::launch_hash(Pv, pgrid, stream, c.T.build, c.T.par);
+            if (W.n_dev > 0) fd::launch_hash(Wv, wgrid, stream);
+            for (int d = 0; d < 6; ++d)
+                if (ghosts[d].active) fd::reset_image_box(ghosts[d].occ.p, stream);
+            tend(FUNDEM_T_HASH);
         }
-        tend(FUNDEM_T_BROAD);
-        tbegin(FUNDEM_T_NARROW_PP);
-        a.rec = recording ? recording->rec(FD_PP, record_step) : fd::AdjRec{};
-        {
-            fd::StepArgs ap = a;
-            if (pc) {
-                ap.skin = pcv.skin;
-                ap.gate = pcv.ctrl;
-                ap.drift = pcv.drift;
-                ap.disp = pcv.disp;
+        // the particles at their wrapped positions: a copy, which replaces the
+        // positions in the force sums; in place with sector periodicity, whose
+        // images are then detected after the particle and wall lists
+        ObjDev Pg = Pv;
+        if (images && !sector) Pg.pos = img_pos.p;
+        int active[FD_NKIND] = {1, 1};
+        fd::ListArgs L[FD_NKIND];
+        int n = 0;
+        auto add = [&](int kind) {
+            fd::ListArgs& l = L[n++];
+            const bool image = kind != FD_PP && kind != FD_PW;
+            l.kind = kind;
+            l.P = image ? Pg : Pv;
+            l.gh = fd::GhostDev{};
+            l.L = lists[kind].view();
+            l.a = a;
+            l.a.rec = recording ? recording->rec(kind, record_step) : fd::AdjRec{};
+            const bool cached = image ? pcg && kind <= FD_GXY : pc;
+            if (image) {
+                l.gh = ghosts[kind - FD_GX].view(cached);
+                active[kind] = 1;
             }
-            fd::launch_narrow(FD_PP, Pv, G, M, Wv, GW, MW, pgrid, wgrid, nullptr, Lpp, ap, with_force, mixed(), stream);
-        }
-        if (pc) {
-            fd::launch_pair_cache_commit(Pv, pcv, Lpp, stream);
-        }
-        if (recording)
-            FD_CUDA(cudaMemcpyAsync(recording->ns(FD_PP, record_step), Lpp.n_slots, sizeof(int),
-                                    cudaMemcpyDeviceToDevice, stream));
-        tend(FUNDEM_T_NARROW_PP);
-        if (branches) FD_CUDA(cudaStreamWaitEvent(stream, br_join[1], 0));
-        else wall_stage(stream);
-        if (img_branch) {
-            // the image detection ran beside; its wrapped positions replace
-            // the ones the particle and wall lists were detected with
-            FD_CUDA(cudaStreamWaitEvent(stream, br_join[0], 0));
-            if (img_wrapped && Pv.n > 0)
-                FD_CUDA(cudaMemcpyAsync(Pv.pos, img_pos.p, sizeof(double3) * Pv.n, cudaMemcpyDeviceToDevice, stream));
-        } else if (perX || perY || sector) {
-            image_stage(stream, Pv, nullptr);
-        }
-        auto pc_end = [&] {
-            if (!pc) return;
-            PairListDev gl[4];
-            int ng = 0;
-            gl[ng++] = Lpw;
-            for (int d = 0; d < 3 && pcg; ++d)
-                if (ghosts[d].active) gl[ng++] = Lg[d];
-            fd::launch_pair_cache_end(pcv, gl, ng, stream);
+            if (!cached) return;
+            l.a.skin = pcv.skin;
+            l.a.gate = pcv.ctrl;
+            l.a.drift = pcv.drift;
+            l.a.disp = pcv.disp;
+            if (kind == FD_PW) {
+                l.a.driftB = pcv.wdrift;
+                l.a.dispB = pcv.wdisp;
+            }
+            if (image) l.a.gate2 = l.a.noskin = pcv.ctrl + 4;
         };
+        // the added lists; under the stage timers each group is a set of its own
+        auto run = [&](int t_broad, int t_narrow) {
+            fd::NlDev nl{};
+            const bool use = use_nl && !pc;  // the cache's rebuilds search the cells
+            if (use) nl = nl_view();
+            tbegin(t_broad);
+            fd::launch_broad(L, n, c, use ? &nl : nullptr, stream);
+            tend(t_broad);
+            tbegin(t_narrow);
+            fd::launch_narrow(L, n, c, stream);
+            tend(t_narrow);
+            if (recording)
+                for (int k = 0; k < n; ++k) record_slots(L[k].kind);
+            n = 0;
+        };
+        auto translated = [&] {
+            if (!images) return;
+            fd::GhostDev gh[3];
+            int on[3];
+            for (int d = 0; d < 3; ++d) {
+                gh[d] = ghosts[d].view(pcg);
+                on[d] = ghosts[d].active;
+            }
+            fd::launch_images(Pv, Pg.pos, gh, on, pcg ? pcv.skin : 0.0, gctrl, stream);
+        };
+        // the bonds read positions after the wraps and orientations, and write
+        // their own arrays: beside the detection, off its path
+        bool forked = false;
+        auto bonds = [&] {
+            if (!with_force || bd.n == 0) return;
+            forked = br_stream && (!profiling || capturing);
+            if (forked) {
+                FD_CUDA(cudaEventRecord(br_fork, stream));
+                FD_CUDA(cudaStreamWaitEvent(br_stream, br_fork, 0));
+            }
+            tbegin(FUNDEM_T_REDUCE);
+            fd::launch_bonds(Pg, bd, mixed(), forked ? br_stream : stream);
+            tend(FUNDEM_T_REDUCE);
+            if (forked) FD_CUDA(cudaEventRecord(br_join, br_stream));
+        };
+        const bool timed = profiling && !capturing;
+        if (!sector) {
+            tbegin(FUNDEM_T_GHOST);
+            translated();
+            tend(FUNDEM_T_GHOST);
+            bonds();
+        }
+        add(FD_PW);
+        if (timed) run(FUNDEM_T_BROAD, FUNDEM_T_NARROW_PW);
+        if (timed || sector) {
+            add(FD_PP);
+            if (timed) run(FUNDEM_T_BROAD, FUNDEM_T_NARROW_PP);
+        }
+        if (sector) {
+            // LSSolver.h:780-784: wraps and images after the other detections
+            if (n) run(FUNDEM_T_BROAD, FUNDEM_T_NARROW_PP);
+            tbegin(FUNDEM_T_GHOST);
+            translated();
+            fd::launch_sector_wrap(Pg, pgrid, stream);
+            fd::GhostDev sv[3] = {ghosts[3].view(), ghosts[4].view(), ghosts[5].view()};
+            fd::launch_sector_images(Pg, sv, stream);
+            tend(FUNDEM_T_GHOST);
+            bonds();
+        }
+        for (int d = 0; d < 6; ++d)
+            if (ghosts[d].active) add(FD_GX + d);
+        if (!timed && !sector) add(FD_PP);
+        if (n) run(FUNDEM_T_GHOST, FUNDEM_T_GHOST);
+        step_wrapped = images && !sector ? img_pos.p : nullptr;
         if (!with_force) {
-            pc_end();
+            if (step_wrapped && Pv.n > 0)
+                FD_CUDA(cudaMemcpyAsync(Pv.pos, img_pos.p, sizeof(double3) * Pv.n, cudaMemcpyDeviceToDevice, stream));
             FD_CUDA(cudaGetLastError());
             return;
         }
         tbegin(FUNDEM_T_REDUCE);
         PairListDev views[FD_NKIND];
         for (int k = 0; k < FD_NKIND; ++k) views[k] = lists[k].view();
-        fd::RevDev rv = rev_view();
-        // the reverse index depends only on the lists' pairs: under the pair
-        // cache (without sector images, whose lists are detected afresh every
-        // step) a step that keeps them keeps the index.  The gate is the
-        // rebuild flag of the particle pairs, or of the image lists, which
-        // also rebuild with them.
-        const bool ghosts_cached = pcg && (ghosts[0].active || ghosts[1].active || ghosts[2].active);
-        const int* rev_gate = (pc && !sector && rev_valid) ? (ghosts_cached ? gctrl + 5 : pcv.ctrl) : nullptr;
-        fd::launch_reverse(Pv, views, active, rv, stream, rev_gate);
-        rev_valid = true;
-        if (bd.n > 0 && !bonds_done) fd::launch_bonds(Pv, bd, mixed(), stream);
-        fd::launch_reduce(Pv, views, active, rv, bd, mixed(), stream);
-        pc_end();
-
+        std::copy(active, active + FD_NKIND, step_active);
+        fd::launch_step_end(Pv, Wv, views, active, c.R, pc ? &pcv : nullptr, pcg, end_done.p, stream);
         tend(FUNDEM_T_REDUCE);
+        if (forked) FD_CUDA(cudaStreamWaitEvent(stream, br_join, 0));
+        sum_pending = true;
+        if (timed) finish_forces();
         FD_CUDA(cudaGetLastError());
     }
 
@@ -1480,28 +1506,14 @@ struct fundem_sim {
 
     void front(double3 g, double dt)
     {
-        ObjDev Pv = P.view(), Wv = W.view();
-        tbegin(FUNDEM_T_INTEGRATE);
-        fd::launch_kick(Pv, pgeo.view(), g, 0.5 * dt, stream);
-        fd::launch_drift(Pv, dt, stream);
-        fd::launch_drift(Wv, dt, stream);
-        tend(FUNDEM_T_INTEGRATE);
+        small = small_on();
+        sum_pending = false;
+        step_wrapped = nullptr;
+        advance(g, dt, fd::STEP_FRONT);
     }
-    void back(double3 g, double dt)
-    {
-        tbegin(FUNDEM_T_INTEGRATE);
-        fd::launch_kick(P.view(), pgeo.view(), g, 0.5 * dt, stream);
-        tend(FUNDEM_T_INTEGRATE);
-    }
-    // back() of one step and front() of the next, the particles in one pass
-    void back_front(double3 g, double dt)
-    {
-        ObjDev Pv = P.view(), Wv = W.view();
-        tbegin(FUNDEM_T_INTEGRATE);
-        fd::launch_kick_drift(Pv, pgeo.view(), g, 0.5 * dt, dt, stream);
-        fd::launch_drift(Wv, dt, stream);
-        tend(FUNDEM_T_INTEGRATE);
-    }
+    void back(double3 g, double dt) { advance(g, dt, fd::STEP_BACK); }
+    // back() of one step and front() of the next, the bodies in one pass
+    void back_front(double3 g, double dt) { advance(g, dt, fd::STEP_BACK | fd::STEP_FRONT); }
 };
 
 namespace {
@@ -2015,6 +2027,7 @@ int fundem_step_begin(fundem_sim* s, const double g[3], double dt)
         s->pc_prepare();
         s->front(d3(g), dt);
         s->detect_all(true, dt);
+        s->finish_forces();
     });
 }
 

@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 #include <mutex>
 
 namespace fd {
@@ -118,61 +119,85 @@ __global__ void k_scan_add(int* out, long long n, const int* tile_off, const int
 // ---------------------------------------------------------------------------
 // integration, particleIntegrationKernel.cu:3-48 and myQua.h:77-93
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void kick_one(ObjDev& P, const GeoSetDev& G, double3 g, double h, int i)
+struct Body {
+    double3 x, v, w;
+    fd_quat q;
+};
+
+// The arithmetic below is written with explicit fused multiply-adds: one
+// kernel runs a half kick alone, another two of them around the step boundary,
+// and what the compiler contracts would differ between them.  The pattern is
+// the compiler's for the expressions written out: in a sum of products the
+// leftmost product is fused first.
+__device__ __forceinline__ double3 fma3(double3 a, double s, double3 b)
 {
-    const int gi = P.geo[i];
-    const FdGeo& geo = G.geo[gi];
-    const double invM = geo.inv_mass;
-    if (fd_is_zero(invM)) return;
-    P.vel[i] = P.vel[i] + (P.force[i] * invM + g) * h;
-    const double3 w = P.angvel[i];
-    const fd_quat q = P.q[i];
-    const double3 Iw = fd_smv(fd_rot_tensor(q, geo.inertia), w);
-    P.angvel[i] = w + fd_smv(fd_rot_tensor(q, geo.inv_inertia), P.torque[i] - cross3(w, Iw)) * h;
+    return mk3(__fma_rn(a.x, s, b.x), __fma_rn(a.y, s, b.y), __fma_rn(a.z, s, b.z));
+}
+__device__ __forceinline__ double dot3f(double ax, double ay, double az, double bx, double by, double bz)
+{
+    return __fma_rn(az, bz, __fma_rn(ax, bx, __dmul_rn(ay, by)));
+}
+__device__ __forceinline__ double3 smv_fma(fd_sym m, double3 v)
+{
+    return mk3(dot3f(m.xx, m.xy, m.xz, v.x, v.y, v.z), dot3f(m.xy, m.yy, m.yz, v.x, v.y, v.z),
+               dot3f(m.xz, m.yz, m.zz, v.x, v.y, v.z));
+}
+__device__ __forceinline__ double3 cross_fma(double3 a, double3 b)
+{
+    return mk3(__fma_rn(a.y, b.z, -__dmul_rn(a.z, b.y)), __fma_rn(a.z, b.x, -__dmul_rn(a.x, b.z)),
+               __fma_rn(a.x, b.y, -__dmul_rn(a.y, b.x)));
+}
+// R(q) I R(q)^T (rotateTensor, myMat.h:75-158)
+__device__ __forceinline__ fd_sym rot_tensor_fma(fd_quat q, fd_sym I)
+{
+    const double x2 = 2.0 * q.q1, y2 = 2.0 * q.q2, z2 = 2.0 * q.q3;
+    const double a = __fma_rn(-y2, q.q2, __fma_rn(-z2, q.q3, 1.0)), b = __fma_rn(x2, q.q2, -__dmul_rn(z2, q.q0)),
+                 c = __fma_rn(x2, q.q3, __dmul_rn(y2, q.q0));
+    const double d = __fma_rn(x2, q.q2, __dmul_rn(z2, q.q0)), e = __fma_rn(-x2, q.q1, __fma_rn(-z2, q.q3, 1.0)),
+                 f = __fma_rn(y2, q.q3, -__dmul_rn(x2, q.q0));
+    const double g = __fma_rn(x2, q.q3, -__dmul_rn(y2, q.q0)), h = __fma_rn(y2, q.q3, __dmul_rn(x2, q.q0)),
+                 i = __fma_rn(-x2, q.q1, __fma_rn(-y2, q.q2, 1.0));
+    const double3 r0 = smv_fma(I, mk3(a, b, c)), r1 = smv_fma(I, mk3(d, e, f)), r2 = smv_fma(I, mk3(g, h, i));
+    fd_sym r;
+    r.xx = dot3f(r0.x, r0.y, r0.z, a, b, c);
+    r.yy = dot3f(r1.x, r1.y, r1.z, d, e, f);
+    r.zz = dot3f(r2.x, r2.y, r2.z, g, h, i);
+    r.xy = dot3f(r0.x, r0.y, r0.z, d, e, f);
+    r.xz = dot3f(r0.x, r0.y, r0.z, g, h, i);
+    r.yz = dot3f(r1.x, r1.y, r1.z, g, h, i);
+    return r;
 }
 
-__global__ void k_kick(ObjDev P, GeoSetDev G, double3 g, double h)
+__device__ __forceinline__ void kick_body(Body& b, const FdGeo& geo, double3 F, double3 T, double3 g, double h)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    kick_one(P, G, g, h, i);
+    const double invM = geo.inv_mass;
+    if (fd_is_zero(invM)) return;
+    b.v = fma3(fma3(F, invM, g), h, b.v);
+    const double3 wxL = cross_fma(b.w, smv_fma(rot_tensor_fma(b.q, geo.inertia), b.w));
+    const double3 r = mk3(__dsub_rn(T.x, wxL.x), __dsub_rn(T.y, wxL.y), __dsub_rn(T.z, wxL.z));
+    b.w = fma3(smv_fma(rot_tensor_fma(b.q, geo.inv_inertia), r), h, b.w);
 }
 
 __device__ __forceinline__ fd_quat quat_integrate(fd_quat q, double3 w, double dt)
 {
-    const double3 v = w * (0.5 * dt);
-    fd_quat d;
-    d.q0 = -q.q1 * v.x - q.q2 * v.y - q.q3 * v.z;
-    d.q1 = q.q0 * v.x + q.q3 * v.y - q.q2 * v.z;
-    d.q2 = -q.q3 * v.x + q.q0 * v.y + q.q1 * v.z;
-    d.q3 = q.q2 * v.x - q.q1 * v.y + q.q0 * v.z;
-    fd_quat s = {q.q0 + d.q0, q.q1 + d.q1, q.q2 + d.q2, q.q3 + d.q3};
-    return fd_normalize_q(s);
+    const double h = 0.5 * dt;
+    const double3 v = mk3(__dmul_rn(w.x, h), __dmul_rn(w.y, h), __dmul_rn(w.z, h));
+    fd_quat s;
+    s.q0 = __dadd_rn(q.q0, -dot3f(q.q1, q.q2, q.q3, v.x, v.y, v.z));
+    s.q1 = __dadd_rn(q.q1, dot3f(q.q0, q.q3, -q.q2, v.x, v.y, v.z));
+    s.q2 = __dadd_rn(q.q2, dot3f(-q.q3, q.q0, q.q1, v.x, v.y, v.z));
+    s.q3 = __dadd_rn(q.q3, dot3f(q.q2, -q.q1, q.q0, v.x, v.y, v.z));
+    const double l2 = __fma_rn(s.q3, s.q3, dot3f(s.q0, s.q1, s.q2, s.q0, s.q1, s.q2));
+    if (fd_is_zero(l2)) return s;
+    const double inv = rsqrt(l2);
+    fd_quat r = {__dmul_rn(s.q0, inv), __dmul_rn(s.q1, inv), __dmul_rn(s.q2, inv), __dmul_rn(s.q3, inv)};
+    return r;
 }
 
-__device__ __forceinline__ void drift_one(ObjDev& O, double dt, int i)
+__device__ __forceinline__ void drift_body(Body& b, double dt)
 {
-    O.pos[i] = O.pos[i] + dt * O.vel[i];
-    O.q[i] = quat_integrate(O.q[i], O.angvel[i], dt);
-}
-
-__global__ void k_drift(ObjDev O, double dt)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= O.n) return;
-    drift_one(O, dt, i);
-}
-
-// the second half kick of one step, then the first half kick and the drift
-// of the next (no force is computed between them): one pass over the state
-// instead of three, each half kick the same arithmetic as k_kick's
-__global__ void k_kick_drift(ObjDev P, GeoSetDev G, double3 g, double h, double dt)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    kick_one(P, G, g, h, i);
-    kick_one(P, G, g, h, i);
-    drift_one(P, dt, i);
+    b.x = fma3(b.v, dt, b.x);
+    b.q = quat_integrate(b.q, b.w, dt);
 }
 
 // ---------------------------------------------------------------------------
@@ -184,6 +209,21 @@ __device__ __forceinline__ void quat_matrix(const fd_quat q, double R[9])
     R[0] = 1.0 - 2.0 * (q2 * q2 + q3 * q3); R[1] = 2.0 * (q1 * q2 - q0 * q3); R[2] = 2.0 * (q1 * q3 + q0 * q2);
     R[3] = 2.0 * (q1 * q2 + q0 * q3); R[4] = 1.0 - 2.0 * (q1 * q1 + q3 * q3); R[5] = 2.0 * (q2 * q3 - q0 * q1);
     R[6] = 2.0 * (q1 * q3 - q0 * q2); R[7] = 2.0 * (q2 * q3 + q0 * q1); R[8] = 1.0 - 2.0 * (q1 * q1 + q2 * q2);
+}
+
+// cell hash and single-precision rotation rows of object i at x, q
+__device__ __forceinline__ long long hash_one(const ObjDev& O, const FdGrid& g, int i, double3 x, fd_quat q)
+{
+    const long long h = fd_hash(x, g);
+    O.hash[i] = h;
+    if (O.rot) {
+        double R[9];
+        quat_matrix(q, R);
+        O.rot[3 * i + 0] = make_float4((float)R[0], (float)R[1], (float)R[2], 0.f);
+        O.rot[3 * i + 1] = make_float4((float)R[3], (float)R[4], (float)R[5], 0.f);
+        O.rot[3 * i + 2] = make_float4((float)R[6], (float)R[7], (float)R[8], 0.f);
+    }
+    return h;
 }
 
 // new build numbers for a cell table: one for the list generation this step
@@ -200,15 +240,7 @@ __global__ void k_hash(ObjDev O, FdGrid g, unsigned int* build, int par)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= O.n) return;
     if (i == 0 && build) bump_build(build, par);
-    const long long h = fd_hash(O.pos[i], g);
-    O.hash[i] = h;
-    if (O.rot) {
-        double R[9];
-        quat_matrix(O.q[i], R);
-        O.rot[3 * i + 0] = make_float4((float)R[0], (float)R[1], (float)R[2], 0.f);
-        O.rot[3 * i + 1] = make_float4((float)R[3], (float)R[4], (float)R[5], 0.f);
-        O.rot[3 * i + 2] = make_float4((float)R[6], (float)R[7], (float)R[8], 0.f);
-    }
+    hash_one(O, g, i, O.pos[i], O.q[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -270,6 +302,13 @@ __global__ void __launch_bounds__(RS_TPB) k_rs_scatter(const unsigned long long*
     }
 }
 
+// the pair cache's gate: the list is built this step, not carried over
+__device__ __forceinline__ bool list_built(const StepArgs& a)
+{
+    return a.gate == nullptr || *a.gate != 0 || (a.gate2 && *a.gate2 != 0);
+}
+__device__ __forceinline__ double list_skin(const StepArgs& a) { return (a.noskin && *a.noskin) ? 0.0 : a.skin; }
+
 // Cell table: the objects of a cell form a list, head and next.  A counting
 // sort took seven launches of 2-4 us each (clear, count, scan, scatter, order;
 // 28 with the radix sort of a sparse grid), all waiting on one another; the
@@ -277,10 +316,10 @@ __global__ void __launch_bounds__(RS_TPB) k_rs_scatter(const unsigned long long*
 // not matter: every search sorts the partners it keeps.  A head carries the
 // number of the build that wrote it, so heads of older builds read as empty
 // and a dense table is never cleared.
-__global__ void k_hkey_clear(unsigned long long* hkey, unsigned long long n, const int* gate)
+__global__ void k_hkey_clear(unsigned long long* hkey, unsigned long long n, StepArgs a)
 {
     const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (gate && *gate == 0)) return;
+    if (i >= n || !list_built(a)) return;
     hkey[i] = RS_NONE;
 }
 
@@ -303,13 +342,10 @@ __device__ __forceinline__ void cell_push(const CellTableDev& T, unsigned long l
     T.next[i] = (unsigned int)(old >> 32) == build ? (int)(unsigned int)old : -1;
 }
 
-__global__ void k_cell_link(const long long* hash, int n, CellTableDev T, const int* gate)
+// object i, of cell hash h, into the table
+__device__ __forceinline__ void cell_link(const CellTableDev& T, long long h, unsigned int build, int i)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (gate && *gate == 0)) return;
-    const long long h = hash[i];
     if (h < 0 || h >= T.g.num) return;
-    const unsigned int build = T.build[T.par];
     if (!T.hashed) {
         cell_push(T, (unsigned long long)h, build, i);
         return;
@@ -373,27 +409,12 @@ __device__ __forceinline__ int wrap_code(double3 cA, double3 ri, double3 cB, dou
            27 * (sh(rj.y - cB.y, Ly) + 1);
 }
 
-__global__ void k_wrap(ObjDev P, FdGrid g, int dim, int* ctrl, const double3* src)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    const double3 p0 = src ? src[i] : P.pos[i];
-    const double3 p1 = dim == 0 ? wrap_x(p0, g) : wrap_y(p0, g);
-    P.pos[i] = p1;
-    // under the pair cache a wrap changes which particles have images: the
-    // ghost lists of this step are built afresh, and every list at the next
-    if (ctrl && (p1.x != p0.x || p1.y != p0.y)) {
-        ctrl[4] = 1;
-        ctrl[7] = 1;
-    }
-}
-
 // calculateGhostHashKernel, including its z test against maxBound.y (:236):
 // an image outside the domain is hashed into the clamped boundary cell, an
 // image inside it is not a ghost
 // Returns the directions (bit 0 x, 1 y, 2 z) in which the image lies
 // outside the domain.
-__device__ __forceinline__ int image_hash(GhostDev& Gh, int i, double3 r)
+__device__ __forceinline__ int image_hash(const GhostDev& Gh, int i, double3 r)
 {
     const FdGrid& g = Gh.cells.g;
     int3 gc = fd_cell_of(r, g);
@@ -431,13 +452,9 @@ __device__ __forceinline__ int image_out_mask(double3 r, const FdGrid& g)
     if (r.z < g.minb.z || r.z >= g.maxb.y) m |= 4;
     return m;
 }
-__global__ void k_ghost_build(ObjDev P, GhostDev Gh, int kind, double ext_skin, int* ctrl)
+__device__ __forceinline__ void image_build(const GhostDev& Gh, int kind, int i, double3 p, double ext_skin, int* ctrl)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    if (i == 0) bump_build(Gh.cells.build, Gh.cells.par);
     const FdGrid& g = Gh.cells.g;
-    const double3 p = P.pos[i];
     const double3 ox = mk3(g.maxb.x - g.minb.x, 0., 0.), oy = mk3(0., g.maxb.y - g.minb.y, 0.);
     const double3 shift = kind == FD_GX ? ox : kind == FD_GY ? oy : ox + oy;
     const int3 c = fd_cell_of(p, g);
@@ -471,31 +488,42 @@ __global__ void k_ghost_build(ObjDev P, GhostDev Gh, int kind, double ext_skin, 
     }
 }
 
-__global__ void k_ghost_gate(int* ctrl)
-{
-    ctrl[5] = (ctrl[0] != 0 || ctrl[4] != 0) ? 1 : 0;
-    ctrl[6] = ctrl[4];
-}
-
-// end of a cached step
-struct CachedCounts {
-    int* n_pairs[4];
-    int* n_slots[4];
-    int cap_pairs[4];
-    int cap_contacts[4];
-    int n;
+// the periodic wraps (into dst, which may be P.pos) and the translated images:
+// x wraps, x images, y wraps, y and xy images (PeriodicBoundaryXY2D,
+// LSSolver.h:780-784).  One pass over the positions in place of five launches.
+struct ImageArgs {
+    ObjDev P;
+    double3* dst;
+    GhostDev gh[3];   // X, Y, XY
+    int on[3];
+    double ext_skin;
+    int* ctrl;        // the pair cache's, or null
 };
-// a build of the particle-wall or ghost lists that overflowed is not kept
-__global__ void k_pc_end(int* ctrl, CachedCounts gc)
+__global__ void k_images(ImageArgs a)
 {
-    for (int k = 0; k < gc.n; ++k)
-        if (*gc.n_pairs[k] > gc.cap_pairs[k] || *gc.n_slots[k] > gc.cap_contacts[k]) ctrl[7] = 1;
-    ctrl[3] = ctrl[7];
-    ctrl[7] = 0;
-    ctrl[0] = 0;
-    ctrl[4] = 0;
-    ctrl[5] = 0;
-    ctrl[6] = 0;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.P.n) return;
+    if (i == 0)
+        for (int d = 0; d < 3; ++d)
+            if (a.on[d]) bump_build(a.gh[d].cells.build, a.gh[d].cells.par);
+    const double3 p0 = a.P.pos[i];
+    double3 p = p0;
+    if (a.on[0]) {
+        p = wrap_x(p, a.gh[0].cells.g);
+        image_build(a.gh[0], FD_GX, i, p, a.ext_skin, a.ctrl);
+    }
+    if (a.on[1]) {
+        p = wrap_y(p, a.gh[1].cells.g);
+        image_build(a.gh[1], FD_GY, i, p, a.ext_skin, a.ctrl);
+    }
+    if (a.on[2]) image_build(a.gh[2], FD_GXY, i, p, a.ext_skin, a.ctrl);
+    a.dst[i] = p;
+    // under the pair cache a wrap changes which particles have images: the
+    // ghost lists of this step are built afresh, and every list at the next
+    if (a.ctrl && (p.x != p0.x || p.y != p0.y)) {
+        a.ctrl[4] = 1;
+        a.ctrl[7] = 1;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -655,12 +683,20 @@ __device__ __forceinline__ void body_search_range(double3 c, double r, const FdG
 
 __device__ __forceinline__ void decode_cell(long long h, int3 s, int3& c)
 {
+    if ((unsigned long long)h < (1ull << 31) && (long long)s.x * s.y < (1ll << 31)) {
+        // grids of fewer than 2^31 cells: 32-bit divisions
+        const unsigned int u = (unsigned int)h, row = u / (unsigned int)s.x;
+        c.x = (int)(u - row * (unsigned int)s.x);
+        c.z = (int)(row / (unsigned int)s.y);
+        c.y = (int)(row - (unsigned int)c.z * (unsigned int)s.y);
+        return;
+    }
     c.x = (int)(h % s.x);
     c.y = (int)((h / s.x) % s.y);
     c.z = (int)(h / ((long long)s.x * s.y));
 }
 
-__device__ void emit_pairs(int A, int* buf, int cnt, int total, PairListDev& L, unsigned int* flags)
+__device__ void emit_pairs(int A, int* buf, int cnt, int total, const PairListDev& L, unsigned int* flags)
 {
     if (total > MAX_CAND) set_flag(flags, FD_FLAG_NEIGHBOR_OVERFLOW);
     // insertion sort by partner id: deterministic pair order
@@ -810,28 +846,19 @@ __device__ __forceinline__ double3 nl_min_image(double3 d, const NlDev& nl, cons
 // of a cell table built from ghost positions (no B > A rule; the reach is the
 // partner's SDF grid radius, since ghost pairs have no radius test).
 //
-// LIST: only the particles in alist[0 .. *acount) search (the ghost phases
-// list the particles whose search box reaches a ghost image; the others
-// were given empty segments by k_ghost_searchers).
-//
 // NLB: build the neighbour list instead of the pairs (only when a rebuild
 // was requested): the sphere test is widened by the skin, the body-level
 // cull is left to the per-step filter, and each particle's partners go to its
 // fixed slice of the list.
 //
 // skin (pair cache): partners within rA + rB + skin are listed and the
-// body-level cull treats A's sphere as skin larger; gate: the kernel runs
-// only when *gate != 0 (null: always).
-template <bool GHOST, bool LIST, bool NLB>
-__global__ void __launch_bounds__(TPB) k_broad_cells(ObjDev P, GeoSetDev G, CellTableDev T, const double3* gpos,
-                                                     const float4* grot, const int* occ, const int* alist, const int* acount,
-                                                     PairListDev L, NlDev nl, unsigned int* flags, double probe,
-                                                     double skin, const int* gate, const int* noskin)
+// body-level cull treats A's sphere as skin larger.
+template <bool GHOST, bool NLB>
+__device__ __forceinline__ void broad_cells(const ObjDev& P, const GeoSetDev& G, const CellTableDev& T,
+                                            const double3* gpos, const float4* grot, const int* occ,
+                                            const PairListDev& L, const NlDev& nl, unsigned int* flags, double probe,
+                                            double skin, int block, int nblocks, int (*s_list)[MAX_CAND])
 {
-    if (gate && *gate == 0) return;
-    if (noskin && *noskin) skin = 0.0;
-    if (NLB && nl.ctrl[0] == 0) return;
-    __shared__ int s_list[TPB / BROAD_LANES][MAX_CAND];
     const unsigned int full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int gl = lane & (BROAD_LANES - 1);
@@ -839,13 +866,13 @@ __global__ void __launch_bounds__(TPB) k_broad_cells(ObjDev P, GeoSetDev G, Cell
     const int gb = threadIdx.x / BROAD_LANES;
     constexpr int GPW = 32 / BROAD_LANES;           // lane groups per warp
     constexpr int GPB = TPB / BROAD_LANES;          // lane groups per block
-    const int total = LIST ? *acount : P.n;
+    const int total = P.n;
     const unsigned int build = T.build[T.par];
     // warp-uniform loop over the warp's groups
-    for (int gw = blockIdx.x * GPB + (gb & ~(GPW - 1)); gw < total; gw += gridDim.x * GPB) {
+    for (int gw = block * GPB + (gb & ~(GPW - 1)); gw < total; gw += nblocks * GPB) {
     const int gidx = gw + (gb & (GPW - 1));
     const bool valid = gidx < total;
-    const int A = valid ? (LIST ? alist[gidx] : gidx) : 0;
+    const int A = valid ? gidx : 0;
     double3 cA = mk3(0., 0., 0.);
     double rA = 0.;
     int3 lo = make_int3(0, 0, 0), hi = make_int3(-1, -1, -1);
@@ -946,15 +973,22 @@ __global__ void __launch_bounds__(TPB) k_broad_cells(ObjDev P, GeoSetDev G, Cell
     }
 }
 
+// the neighbour list, when a rebuild of it was requested
+__global__ void __launch_bounds__(TPB) k_broad_nl(ObjDev P, GeoSetDev G, CellTableDev T, NlDev nl, unsigned int* flags)
+{
+    __shared__ int s_list[TPB / BROAD_LANES][MAX_CAND];
+    if (nl.ctrl[0] == 0) return;
+    broad_cells<false, true>(P, G, T, nullptr, nullptr, nullptr, PairListDev{}, nl, flags, 0.0, 0.0, blockIdx.x,
+                             gridDim.x, s_list);
+}
+
 // neighbour list: request a rebuild when a particle moved more than skin / 2
 // since the last build or changed visibility
-__global__ void k_nl_check(ObjDev P, NlDev nl, FdGrid g, const int* gate)
+__global__ void k_nl_check(ObjDev P, NlDev nl, FdGrid g)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n || (gate && *gate == 0)) return;
-    // with the pair cache, partners within rA + rB + pair_skin must stay
-    // listed: the list is rebuilt before any particle moves (skin - pair_skin) / 2
-    const double h = 0.5 * (nl.skin - nl.pair_skin);
+    if (i >= P.n) return;
+    const double h = 0.5 * nl.skin;
     const bool moved = lengthSq3(nl_min_image(P.pos[i] - nl.ref[i], nl, g)) > h * h;
     const bool vis = P.hash[i] >= 0;
     if (moved || vis != (nl.vis[i] != 0)) nl.ctrl[0] = 1;
@@ -964,9 +998,8 @@ __global__ void k_nl_check(ObjDev P, NlDev nl, FdGrid g, const int* gate)
 // body-level cull of the cell search, on the listed partners (ascending, so
 // each particle's pairs come out in partner order)
 __global__ void __launch_bounds__(TPB) k_nl_filter(ObjDev P, GeoSetDev G, PairListDev L, NlDev nl,
-                                                   unsigned int* flags, double probe, const int* gate)
+                                                   unsigned int* flags, double probe)
 {
-    if (gate && *gate == 0) return;
     constexpr int LN = 8;  // lanes per particle
     const unsigned int full = 0xffffffffu;
     const int lane = threadIdx.x & 31, gl = lane & (LN - 1), gbase = lane & ~(LN - 1);
@@ -991,9 +1024,9 @@ __global__ void __launch_bounds__(TPB) k_nl_filter(ObjDev P, GeoSetDev G, PairLi
             if (P.hash[B] >= 0) {
                 const FdGeo& GB = G.geo[P.geo[B]];
                 const double3 cB = P.pos[B];
-                const double rs = rA + GB.radius + nl.pair_skin;
+                const double rs = rA + GB.radius;
                 if (lengthSq3(cA - cB) <= rs * rs * (1.0 + 4.0 * BOUND_REL))
-                    pass = !body_culled32(cA, rA + nl.pair_skin, cB, P.rot + 3ll * B, true, GB, G, probe);
+                    pass = !body_culled32(cA, rA, cB, P.rot + 3ll * B, true, GB, G, probe);
             }
         }
         const unsigned int gm = (__ballot_sync(full, pass) >> gbase) & ((1u << LN) - 1u);
@@ -1023,20 +1056,21 @@ __global__ void __launch_bounds__(TPB) k_nl_filter(ObjDev P, GeoSetDev G, PairLi
 // ---------------------------------------------------------------------------
 // pair cache of the particle-particle list (see PairCacheDev)
 // ---------------------------------------------------------------------------
-// flag a rebuild when a particle drifted by more than skin / 2 since the last
-// build or changed visibility
-__global__ void k_pc_check(ObjDev P, PairCacheDev c)
+// 2 sin(theta / 2) = 2 |vector part of q conj(r)|: the chord a unit lever arm
+// sweeps under the rotation from r to q
+__device__ __forceinline__ double turn_chord(fd_quat q, fd_quat r)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    const double3 d = P.pos[i] - c.ref_pos[i];
-    // 2 sin(theta / 2) = 2 |vector part of q conj(q0)|: the chord a unit
-    // lever arm sweeps under the rotation since the build
-    const fd_quat q = P.q[i], r = c.ref_q[i];
     const double vx = r.q0 * q.q1 - q.q0 * r.q1 - (q.q2 * r.q3 - q.q3 * r.q2);
     const double vy = r.q0 * q.q2 - q.q0 * r.q2 - (q.q3 * r.q1 - q.q1 * r.q3);
     const double vz = r.q0 * q.q3 - q.q0 * r.q3 - (q.q1 * r.q2 - q.q2 * r.q1);
-    const double chord = 2.0 * sqrt(vx * vx + vy * vy + vz * vz);
+    return 2.0 * sqrt(vx * vx + vy * vy + vz * vz);
+}
+// the drift bound of particle i since the last build, and a rebuild when it
+// exceeds skin / 2 or the particle changed visibility
+__device__ __forceinline__ void cache_check(const PairCacheDev& c, int i, double3 x, fd_quat q, bool vis)
+{
+    const double3 d = x - c.ref_pos[i];
+    const double chord = turn_chord(q, c.ref_q[i]);
     const double drift = sqrt(lengthSq3(d)) + c.reach * chord;
     // every particle's bound, for the slot test of the predicate pass
     c.drift[i] = __double2float_ru(drift);
@@ -1050,157 +1084,54 @@ __global__ void k_pc_check(ObjDev P, PairCacheDev c)
     }
     // a little below skin / 2, so that the two drifts of a pair stay below
     // the single-precision skin the culling stages use
-    const bool vis = P.hash[i] >= 0;
     if (!(drift <= 0.5 * c.skin * (1.0 - 1e-6)) || vis != (c.ref_vis[i] != 0)) c.ctrl[0] = 1;
 }
-
-// a step without a rebuild: this step's pairs and slots are the previous
-// step's, carried over; each pair's history is its own slots of the previous
-// step, and its partner's cell is taken from this step's hash
-__global__ void k_pc_carry(PairListDev L, int n_obj, const long long* hash, FdGrid g, const int* gate,
-                           const float* drift, const float4* disp, const float* driftB, const float4* dispB,
-                           const int* geo_of, const FdGeo* geos, float spacing_margin)
-{
-    if (*gate != 0) return;
-    const int npairs = min(L.o_counters[0], L.cap_pairs);
-    const int nslots = min(L.o_counters[1], L.cap_contacts);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    // the layout (segments, pairs, slot keys) is copied into the other
-    // generation on the first carried step after a build; from the second on
-    // both generations hold it already
-    const bool copy = L.carry_n == nullptr || *L.carry_n == 0;
-    if (t0 == 0) {
-        *L.n_pairs = L.o_counters[0];
-        *L.n_slots = L.o_counters[1];
-    }
-    if (copy)
-        for (long long i = t0; i < n_obj; i += stride) {
-            L.seg_off[i] = L.o_seg_off[i];
-            L.seg_cnt[i] = L.o_seg_cnt[i];
-        }
-    for (long long p = t0; p < npairs; p += stride) {
-        const int A = L.o_pairA[p];
-        const int B = L.o_pairB[p];
-        const int off = L.o_c_off[p], cnt = L.o_c_cnt[p];
-        if (copy) {
-            L.pairA[p] = A;
-            L.pairB[p] = B;
-            L.c_off[p] = off;
-            L.c_cnt[p] = cnt;
-        }
-        if (drift && disp && L.p_bound) {
-            // the slot bound's right-hand side for the pair (see k_contact):
-            // lip_B times how far a node can have moved in B's frame, plus a
-            // margin in units of B's grid spacing (the single-precision
-            // predicate's rounding).  The node's offset from B's centre moved
-            // by at most |dc_A - dc_B| + the two rotation parts (lever arms up
-            // to the reach); the displacements are stored in single
-            // precision, whose rounding (1e-7 of each) the term
-            // 1e-6 (drift_A + drift_B) covers; never more than the sum of
-            // the two drift bounds.
-            const FdGeo& GB = geos[geo_of[B]];
-            const float lip = __double2float_ru(GB.lip);
-            const float4 a = disp[A], b = dispB[B];
-            const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
-            const float dab = __fadd_ru(drift[A], driftB[B]);
-            const float rel = __fadd_ru(__fadd_ru(__fsqrt_ru(__fadd_ru(__fadd_ru(__fmul_ru(dx, dx), __fmul_ru(dy, dy)),
-                                                                       __fmul_ru(dz, dz))),
-                                                  __fadd_ru(a.w, b.w)),
-                                        __fmul_ru(1e-6f, dab));
-            float bound = __fmul_ru(lip, fminf(rel, dab));
-            if (spacing_margin > 0.f)
-                bound = __fadd_ru(__fmul_ru(bound, 1.000001f), __fmul_ru(spacing_margin, __double2float_ru(GB.spacing)));
-            L.p_bound[p] = bound;
-        }
-        if (cnt > 0) {
-            int3 bc;
-            decode_cell(hash[B], g.size, bc);
-            L.p_aux[p] = make_int4(bc.x, bc.y, bc.z, off);
-            L.p_hist_cnt[p] = cnt;
-        }
-    }
-    if (copy)
-        for (long long k = t0; k < nslots; k += stride) L.c_k[k] = L.o_c_k[k];
-}
-
-// after the particle-particle narrow phase of a rebuild step: its state is the
-// new reference; the flag is cleared for the next step
-__global__ void k_pc_commit(ObjDev P, PairCacheDev c, PairListDev L)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n || c.ctrl[0] == 0) return;
-    c.ref_pos[i] = P.pos[i];
-    c.ref_q[i] = P.q[i];
-    c.ref_vis[i] = P.hash[i] >= 0;
-    if (i == 0) {
-        c.ctrl[1] += 1;
-        // a build whose pairs or slots did not fit is not kept: the next
-        // step builds again (the host grows the lists at its next check)
-        c.ctrl[2] = (*L.n_pairs > L.cap_pairs || *L.n_slots > L.cap_contacts) ? 1 : 0;
-    }
-}
-
 // walls: the drift bound of each wall since the last build (rotation lever
 // arm: its SDF-grid radius, the farthest a node inside its grid can be), and
 // a rebuild when it exceeds skin / 2 or the wall's cell changed (the
 // particle-wall candidates follow the wall's cell)
-__global__ void k_pc_check_walls(ObjDev W, GeoSetDev GW, PairCacheDev c)
+__device__ __forceinline__ void cache_check_wall(const PairCacheDev& c, int w, double3 x, fd_quat q, long long hash,
+                                                 double grid_radius)
 {
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= W.n) return;
-    const double3 d = W.pos[w] - c.wref_pos[w];
-    const fd_quat q = W.q[w], r = c.wref_q[w];
-    const double vx = r.q0 * q.q1 - q.q0 * r.q1 - (q.q2 * r.q3 - q.q3 * r.q2);
-    const double vy = r.q0 * q.q2 - q.q0 * r.q2 - (q.q3 * r.q1 - q.q1 * r.q3);
-    const double vz = r.q0 * q.q3 - q.q0 * r.q3 - (q.q1 * r.q2 - q.q2 * r.q1);
-    const double rot = GW.geo[W.geo[w]].grid_radius * 2.0 * sqrt(vx * vx + vy * vy + vz * vz);
+    const double3 d = x - c.wref_pos[w];
+    const double rot = grid_radius * turn_chord(q, c.wref_q[w]);
     const double drift = sqrt(lengthSq3(d)) + rot;
     c.wdrift[w] = __double2float_ru(drift);
     c.wdisp[w] = make_float4((float)d.x, (float)d.y, (float)d.z, __double2float_ru(rot));
     if (c.ctrl[0] != 0) return;
-    if (!(drift <= 0.5 * c.skin * (1.0 - 1e-6)) || W.hash[w] != c.wref_hash[w]) c.ctrl[0] = 1;
-}
-__global__ void k_pc_commit_walls(ObjDev W, PairCacheDev c)
-{
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= W.n || c.ctrl[0] == 0) return;
-    c.wref_pos[w] = W.pos[w];
-    c.wref_q[w] = W.q[w];
-    c.wref_hash[w] = W.hash[w];
+    if (!(drift <= 0.5 * c.skin * (1.0 - 1e-6)) || hash != c.wref_hash[w]) c.ctrl[0] = 1;
 }
 
-// ghost phases: particles whose search box reaches the cells holding ghost
-// images are listed for k_broad_cells<true, true>; the others get empty
-// segments here
-__global__ void k_ghost_searchers(ObjDev P, GeoSetDev G, FdGrid g, const int* occ, PairListDev L, int* alist,
-                                  int* acount, double skin, const int* gate, const int* noskin)
+// The slot bound of a carried pair (see k_slot_filter): lip_B times how far a
+// node can have moved in B's frame since the build, plus a margin in units of
+// B's grid spacing (the single-precision predicate's rounding).  The node's
+// offset from B's centre moved by at most |dc_A - dc_B| + the two rotation
+// parts (lever arms up to the reach); the displacements are stored in single
+// precision, whose rounding (1e-7 of each) the term 1e-6 (drift_A + drift_B)
+// covers; never more than the sum of the two drift bounds.
+__device__ __forceinline__ float pair_bound(float driftA, float4 a, float driftB, float4 b, const FdGeo& GB,
+                                            float spacing_margin)
 {
-    const int A = blockIdx.x * blockDim.x + threadIdx.x;
-    if (A >= P.n || (gate && *gate == 0)) return;
-    if (noskin && *noskin) skin = 0.0;
-    const double rA = G.geo[P.geo[A]].radius;
-    const double reach = (rA + G.grid_rmax) * (1.0 + 8.0 * BOUND_REL) + skin;
-    int3 lo, hi;
-    ghost_search_range(P.pos[A], rA * (1.0 + 8.0 * BOUND_REL) + skin, reach, g, lo, hi);
-    const bool any = max(lo.x, occ[0]) <= min(hi.x, occ[3]) && max(lo.y, occ[1]) <= min(hi.y, occ[4]) &&
-                     max(lo.z, occ[2]) <= min(hi.z, occ[5]);
-    if (any) {
-        alist[atomicAdd(acount, 1)] = A;
-    } else {
-        L.seg_off[A] = 0;
-        L.seg_cnt[A] = 0;
-    }
+    const float lip = __double2float_ru(GB.lip);
+    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    const float dab = __fadd_ru(driftA, driftB);
+    const float rel = __fadd_ru(__fadd_ru(__fsqrt_ru(__fadd_ru(__fadd_ru(__fmul_ru(dx, dx), __fmul_ru(dy, dy)),
+                                                               __fmul_ru(dz, dz))),
+                                          __fadd_ru(a.w, b.w)),
+                                __fmul_ru(1e-6f, dab));
+    float bound = __fmul_ru(lip, fminf(rel, dab));
+    if (spacing_margin > 0.f)
+        bound = __fadd_ru(__fmul_ru(bound, 1.000001f), __fmul_ru(spacing_margin, __double2float_ru(GB.spacing)));
+    return bound;
 }
 
 // wall_range (null: every wall): per particle, the first wall and the number
 // of walls it can meet (the walls of its own simulation in a batch of
 // simulations tiled into one)
-__global__ void k_broad_pw(ObjDev P, GeoSetDev G, ObjDev W, GeoSetDev GW, FdGrid wg, PairListDev L,
-                           unsigned int* flags, double probe, const int2* wall_range, double skin, const int* gate)
+__device__ __forceinline__ void broad_walls(const ObjDev& P, const GeoSetDev& G, const ObjDev& W, const GeoSetDev& GW,
+                                            const FdGrid& wg, const PairListDev& L, unsigned int* flags, double probe,
+                                            const int2* wall_range, double skin, int A)
 {
-    const int A = blockIdx.x * blockDim.x + threadIdx.x;
-    if (A >= P.n || (gate && *gate == 0)) return;
     const double3 cA = P.pos[A];
     const double rA = G.geo[P.geo[A]].radius;
     int3 lo, hi;
@@ -1331,6 +1262,94 @@ struct SlaveGhost {
 template <> struct Slave<FD_GX> : SlaveGhost {};
 template <> struct Slave<FD_GY> : SlaveGhost {};
 template <> struct Slave<FD_GXY> : SlaveGhost {};
+
+// The lists of a step share each stage's launch: every stage of every list was
+// a launch of its own on one of three streams (75 launches a carried step,
+// most of them reading the rebuild flag and returning), and at one or two
+// microseconds each they were a third of the step at 65,000 particles.  Each
+// list has a range of a launch's blocks.
+struct ListSet {
+    NarrowArgs l[FD_NKIND];
+    int kind[FD_NKIND];           // FD_PP .. FD_GR270
+    int block0[FD_NKIND + 1];
+    int n;
+    CellTableDev T;               // the particles' cell table
+    const int2* wall_range;       // see broad_walls
+    int* rev_total;               // zeroed with the lists' counters (null: no index is built)
+    float spacing_margin;         // see pair_bound
+};
+// the list a block works on, and its place among that list's blocks
+__device__ __forceinline__ int list_of(const ListSet& a, int& block, int& nblocks)
+{
+    int k = 0;
+    while (k + 1 < a.n && (int)blockIdx.x >= a.block0[k + 1]) ++k;
+    block = (int)blockIdx.x - a.block0[k];
+    nblocks = a.block0[k + 1] - a.block0[k];
+    return k;
+}
+
+// First stage.  A list that is built: its counters cleared, its partners'
+// cell table.  A carried one: its pairs and slots are those of the build
+// (k_step_end left them in both generations), and each pair gets its slot bound.
+__global__ void __launch_bounds__(TPB) k_begin_lists(ListSet a)
+{
+    int block, nblocks;
+    const int li = list_of(a, block, nblocks);
+    const NarrowArgs& n = a.l[li];
+    const PairListDev& L = n.L;
+    const int kind = a.kind[li];
+    const bool built = list_built(n.a);
+    const int t0 = block * blockDim.x + threadIdx.x, stride = nblocks * blockDim.x;
+    if (t0 == 0) {
+        *L.n_hits = 0;
+        *L.n_test = 0;
+        if (built) {
+            *L.n_pairs = 0;
+            *L.n_slots = 0;
+        }
+        if (li == 0 && a.rev_total) *a.rev_total = 0;
+    }
+    if (built) {
+        if (kind == FD_PW) return;
+        const CellTableDev& T = kind == FD_PP ? a.T : n.gh.cells;
+        const long long* hash = kind == FD_PP ? n.P.hash : n.gh.hash;
+        const unsigned int build = T.build[T.par];
+        for (int i = t0; i < n.P.n; i += stride) cell_link(T, hash[i], build, i);
+        return;
+    }
+    if (!n.a.drift) return;
+    const bool wall = kind == FD_PW;
+    const float* driftB = n.a.driftB ? n.a.driftB : n.a.drift;
+    const float4* dispB = n.a.dispB ? n.a.dispB : n.a.disp;
+    const int npairs = min(*L.n_pairs, L.cap_pairs);
+    for (int p = t0; p < npairs; p += stride) {
+        const int A = L.pairA[p], B = L.pairB[p];
+        const FdGeo& GB = wall ? n.GW.geo[n.W.geo[B]] : n.G.geo[n.P.geo[B]];
+        L.p_hit[p] = 0;
+        L.p_bound[p] = pair_bound(n.a.drift[A], n.a.disp[A], driftB[B], dispB[B], GB, wall ? 0.f : a.spacing_margin);
+    }
+}
+
+// broad phase of every list that is built
+__global__ void __launch_bounds__(TPB) k_broad_lists(ListSet a)
+{
+    __shared__ int s_list[TPB / BROAD_LANES][MAX_CAND];
+    int block, nblocks;
+    const int li = list_of(a, block, nblocks);
+    const NarrowArgs& n = a.l[li];
+    if (!list_built(n.a)) return;
+    const double skin = list_skin(n.a);
+    if (a.kind[li] == FD_PP) {
+        broad_cells<false, false>(n.P, n.G, a.T, nullptr, nullptr, nullptr, n.L, NlDev{}, n.a.flags, n.a.probe, skin,
+                                  block, nblocks, s_list);
+    } else if (a.kind[li] == FD_PW) {
+        for (int A = block * blockDim.x + threadIdx.x; A < n.P.n; A += nblocks * blockDim.x)
+            broad_walls(n.P, n.G, n.W, n.GW, n.wgrid, n.L, n.a.flags, n.a.probe, a.wall_range, skin, A);
+    } else {
+        broad_cells<true, false>(n.P, n.G, n.gh.cells, n.gh.pos, n.gh.rot, n.gh.occ, n.L, NlDev{}, n.a.flags,
+                                 n.a.probe, skin, block, nblocks, s_list);
+    }
+}
 
 // Evaluate node predicate for one node.  Returns true when overlap >= 0 and
 // fills the grid fraction and the eight corner values.
@@ -1486,6 +1505,79 @@ __device__ __forceinline__ bool node_filtered(const float4 p, const CullXf& x, c
     return true;
 }
 
+// The nodes of A that may pass the predicate against B, for one warp:
+// cluster culling with one cluster per lane, then the single-precision filter
+// over the nodes of the surviving clusters.  Their keys go to queue in
+// cluster order; returns how many, and the clusters kept.
+template <int KIND>
+__device__ __forceinline__ int cull_pair(const NarrowArgs& n, int A, int B, double skin, int lane,
+                                         unsigned short* queue, int& kept)
+{
+    const unsigned int lt_mask = (1u << lane) - 1u;
+    const FdGeo& GA = n.G.geo[n.P.geo[A]];
+    const double3 cA = n.P.pos[A];
+    const double3 cB = Slave<KIND>::pos(n, B);
+    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const GeoSetDev& SB = Slave<KIND>::set(n);
+    const double rB = GB.radius;
+    const int ncl = GA.clus_count;
+    if (ncl > MAX_CLUSTERS) set_flag(n.a.flags, FD_FLAG_CLUSTER_OVERFLOW);
+    unsigned long long keep = 0ull;
+    const CullXf xf = cull_transform(n.P.rot + 3ll * A, Slave<KIND>::rot(n, B), cA, cB);
+    for (int c0 = 0; c0 < min(ncl, MAX_CLUSTERS); c0 += 32) {
+        const int c = c0 + lane;
+        bool k = false;
+        if (c < ncl) {
+            float4 cl = n.G.clus_sphere[GA.clus_off + c];
+            cl.w += (float)skin;
+            k = !cluster_culled<KIND>(cl, xf, GB, SB, rB, n.a.probe);
+        }
+        keep |= ((unsigned long long)__ballot_sync(0xffffffffu, k)) << c0;
+    }
+    kept = __popcll(keep);
+    const float perr = 4e-6f * (float)(length3(cA - cB) + GA.radius + rB + GB.spacing) + (float)skin;
+    int ncand = 0;
+    // a cluster's range and nodes are loaded while the one before is filtered:
+    // range, node and cell minimum are three dependent loads a cluster
+    int2 cr = make_int2(0, 0);
+    float4 nd = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto fetch = [&] {
+        const int c = __ffsll((long long)keep) - 1;
+        keep &= keep - 1ull;
+        cr = n.G.clus_range[GA.clus_off + c];
+        if (lane < cr.y) nd = n.G.nodes32[GA.node_off + cr.x + lane];
+    };
+    bool more = keep != 0ull;
+    if (more) fetch();
+    while (more) {
+        const int2 r = cr;
+        const float4 node = nd;
+        more = keep != 0ull;
+        if (more) fetch();
+        const bool cand = lane < r.y && !node_filtered<KIND>(node, xf, GB, SB, (float)rB, perr, n.a.probe);
+        const unsigned int m = __ballot_sync(0xffffffffu, cand);
+        if (cand) queue[ncand + __popc(m & lt_mask)] = (unsigned short)(r.x + lane);
+        ncand += __popc(m);
+    }
+    __syncwarp();
+    return ncand;
+}
+
+// the slots of the pair (A, B) in the previous step's list, for one warp
+__device__ __forceinline__ void find_history(const PairListDev& L, int A, int B, int lane, int& off, int& cnt)
+{
+    off = cnt = 0;
+    const int os = L.o_seg_off[A], on = L.o_seg_cnt[A];
+    int found = -1;
+    for (int k0 = 0; k0 < on && found < 0; k0 += 32) {
+        const int k = k0 + lane;
+        const bool eq = (k < on) && (L.o_pairB[os + k] == B);
+        const unsigned int m = __ballot_sync(0xffffffffu, eq);
+        if (m) found = os + k0 + __ffs(m) - 1;
+    }
+    if (found >= 0) { off = L.o_c_off[found]; cnt = L.o_c_cnt[found]; }
+}
+
 // ---------------------------------------------------------------------------
 // narrow phase, stage 1: one warp per candidate pair.  The clusters of A's
 // surface nodes are culled against B, the nodes of the surviving clusters are
@@ -1495,74 +1587,28 @@ __device__ __forceinline__ bool node_filtered(const float4 p, const CullXf& x, c
 // source of its contacts.
 // ---------------------------------------------------------------------------
 //
-// With the pair cache (n.a.gate non-null) the kernel runs only on rebuild
-// steps, and every culling margin is widened by the skin n.a.skin: a cluster
+// With the pair cache it runs only on rebuild steps, and every culling margin
+// is widened by the skin: a cluster
 // is kept when it may come within reach of B after moves of up to the skin,
 // a node is slotted when it may pass the predicate after such moves.
 template <int KIND>
-__global__ void __launch_bounds__(NARROW_WARPS * 32, FD_SELECT_MIN_BLOCKS) k_select(NarrowArgs n)
+__device__ __forceinline__ void select_list(const NarrowArgs& n, int block, int nblocks,
+                                            unsigned short (*s_node)[MAX_NODE_QUEUE], unsigned long long* s_stats)
 {
-    if (n.a.gate && *n.a.gate == 0) return;
-    // a new layout: the next carried step copies it (k_pc_carry)
-    if (blockIdx.x == 0 && threadIdx.x == 0 && n.L.carry_n) *n.L.carry_n = 0;
-    __shared__ unsigned short s_node[NARROW_WARPS][MAX_NODE_QUEUE];
-    // work counters, summed per block and added to the global ones once
-    __shared__ unsigned long long s_stats[4];
-    if (n.a.stats && threadIdx.x < 4) s_stats[threadIdx.x] = 0ull;
-    __syncthreads();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    const unsigned int lt_mask = (1u << lane) - 1u;
-    PairListDev& L = n.L;
+    const PairListDev& L = n.L;
     const int npairs = min(*L.n_pairs, L.cap_pairs);
-    const int nwarps = gridDim.x * NARROW_WARPS;
-    const double skin = (n.a.noskin && *n.a.noskin) ? 0.0 : n.a.skin;
-    for (int p = blockIdx.x * NARROW_WARPS + wib; p < npairs; p += nwarps) {
+    const int nwarps = nblocks * NARROW_WARPS;
+    const double skin = list_skin(n.a);
+    for (int p = block * NARROW_WARPS + wib; p < npairs; p += nwarps) {
         const int A = L.pairA[p];
         const int B = L.pairB[p];
-        const FdGeo& GA = n.G.geo[n.P.geo[A]];
-        const double3 cA = n.P.pos[A];
-        const double3 cB = Slave<KIND>::pos(n, B);
-        const FdGeo& GB = Slave<KIND>::geo(n, B);
-        const GeoSetDev& SB = Slave<KIND>::set(n);
-        const double rB = GB.radius;
-        const int ncl = GA.clus_count;
-        if (ncl > MAX_CLUSTERS) set_flag(n.a.flags, FD_FLAG_CLUSTER_OVERFLOW);
-        // ---- cluster culling, one cluster per lane
-        unsigned long long keep = 0ull;
-        const CullXf xf = cull_transform(n.P.rot + 3ll * A, Slave<KIND>::rot(n, B), cA, cB);
-        for (int c0 = 0; c0 < min(ncl, MAX_CLUSTERS); c0 += 32) {
-            const int c = c0 + lane;
-            bool k = false;
-            if (c < ncl) {
-                float4 cl = n.G.clus_sphere[GA.clus_off + c];
-                cl.w += (float)skin;
-                k = !cluster_culled<KIND>(cl, xf, GB, SB, rB, n.a.probe);
-            }
-            keep |= ((unsigned long long)__ballot_sync(0xffffffffu, k)) << c0;
-        }
-        const int kept = __popcll(keep);
-        // ---- single-precision filter over the nodes of the surviving
-        // clusters; nodes that may pass the predicate are queued in cluster
-        // order
-        const float perr = 4e-6f * (float)(length3(cA - cB) + GA.radius + rB + GB.spacing) + (float)skin;
-        int ncand = 0;
-        while (keep) {
-            const int c = __ffsll((long long)keep) - 1;
-            keep &= keep - 1ull;
-            const int2 cr = n.G.clus_range[GA.clus_off + c];
-            const int k = cr.x + lane;
-            bool cand = false;
-            if (lane < cr.y)
-                cand = !node_filtered<KIND>(n.G.nodes32[GA.node_off + k], xf, GB, SB, (float)rB, perr, n.a.probe);
-            const unsigned int m = __ballot_sync(0xffffffffu, cand);
-            if (cand) s_node[wib][ncand + __popc(m & lt_mask)] = (unsigned short)k;
-            ncand += __popc(m);
-        }
-        __syncwarp();
+        int kept;
+        int ncand = cull_pair<KIND>(n, A, B, skin, lane, s_node[wib], kept);
         if (n.a.stats && lane == 0) {
             atomicAdd(&s_stats[0], 1ull);
-            atomicAdd(&s_stats[1], (unsigned long long)min(ncl, MAX_CLUSTERS));
+            atomicAdd(&s_stats[1], (unsigned long long)min(n.G.geo[n.P.geo[A]].clus_count, MAX_CLUSTERS));
             atomicAdd(&s_stats[2], (unsigned long long)kept);
             atomicAdd(&s_stats[3], (unsigned long long)ncand);
         }
@@ -1579,18 +1625,8 @@ __global__ void __launch_bounds__(NARROW_WARPS * 32, FD_SELECT_MIN_BLOCKS) k_sel
         }
         if (ncand > 0) {
             // history: the same pair in the previous step's list
-            int oc_off = 0, oc_cnt = 0;
-            {
-                const int os = L.o_seg_off[A], on = L.o_seg_cnt[A];
-                int found = -1;
-                for (int k0 = 0; k0 < on && found < 0; k0 += 32) {
-                    const int k = k0 + lane;
-                    const bool eq = (k < on) && (L.o_pairB[os + k] == B);
-                    const unsigned int m = __ballot_sync(0xffffffffu, eq);
-                    if (m) found = os + k0 + __ffs(m) - 1;
-                }
-                if (found >= 0) { oc_off = L.o_c_off[found]; oc_cnt = L.o_c_cnt[found]; }
-            }
+            int oc_off, oc_cnt;
+            find_history(L, A, B, lane, oc_off, oc_cnt);
             for (int i = lane; i < ncand; i += 32) {
                 L.c_pair[base + i] = p;
                 L.c_k[base + i] = s_node[wib][i];
@@ -1605,9 +1641,28 @@ __global__ void __launch_bounds__(NARROW_WARPS * 32, FD_SELECT_MIN_BLOCKS) k_sel
         if (lane == 0) {
             L.c_off[p] = base;
             L.c_cnt[p] = ncand;
+            L.p_hit[p] = 0;
         }
         __syncwarp();
     }
+}
+
+__global__ void __launch_bounds__(NARROW_WARPS * 32, FD_SELECT_MIN_BLOCKS) k_select_lists(ListSet a)
+{
+    __shared__ unsigned short s_node[NARROW_WARPS][MAX_NODE_QUEUE];
+    // work counters, summed per block and added to the global ones once
+    __shared__ unsigned long long s_stats[4];
+    int block, nblocks;
+    const int li = list_of(a, block, nblocks);
+    const NarrowArgs& n = a.l[li];
+    if (!list_built(n.a)) return;
+    if (n.a.stats && threadIdx.x < 4) s_stats[threadIdx.x] = 0ull;
+    __syncthreads();
+    // the sector images differ from the translated ones only in the state the
+    // ghost traits read: one instance serves every image list
+    if (a.kind[li] == FD_PP) select_list<FD_PP>(n, block, nblocks, s_node, s_stats);
+    else if (a.kind[li] == FD_PW) select_list<FD_PW>(n, block, nblocks, s_node, s_stats);
+    else select_list<FD_GX>(n, block, nblocks, s_node, s_stats);
     if (n.a.stats) {
         __syncthreads();
         if (threadIdx.x < 4 && s_stats[threadIdx.x]) {
@@ -1631,15 +1686,15 @@ __global__ void __launch_bounds__(NARROW_WARPS * 32, FD_SELECT_MIN_BLOCKS) k_sel
 // pair cache, particle-particle list, carried steps: the slots the predicate
 // pass must test.  A slot is skipped when its node was outside B at the
 // rebuild by more than the SDF can change under the pair's relative motion
-// since (|grad phi| <= lip, the trilinear bound; k_pc_carry stored the pair's
-// bound); the others are listed, so that the predicate pass runs full warps.
+// since (|grad phi| <= lip, the trilinear bound; k_begin_lists stored the
+// pair's bound); the others are listed, so that the predicate pass runs full warps.
 // The wall and image lists are short: there the extra pass cost more than
 // the idle lanes, and the predicate pass tests the bound itself.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(TPB) k_slot_filter(NarrowArgs n)
 {
-    PairListDev& L = n.L;
-    if (n.a.gate == nullptr || *n.a.gate != 0 || L.c_test == nullptr) return;
+    const PairListDev& L = n.L;
+    if (list_built(n.a)) return;
     const int nitems = min(*L.n_slots, L.cap_contacts);
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -1701,34 +1756,209 @@ __global__ void __launch_bounds__(TPB) k_slot_filter(NarrowArgs n)
     }
 }
 
-template <int KIND, int PASS>
-__global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONTACT_MIN_BLOCKS) k_contact(NarrowArgs n)
+// one slot's node against its partner
+struct SlotEval {
+    double3 cA, cB, r, gp;  // centres, node offset from A's centre, node
+    fd_quat qB;
+    int pool;               // the node in the node pools
+    double ov, fx, fy, fz, pv[8];
+};
+
+// the exact predicate of node k (relative to the geometry) of A against B;
+// e.ov keeps ov0 when the predicate stops before the distance
+template <int KIND>
+__device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, int A, int B, int k, int3 bcell, double ov0,
+                                               SlotEval& e)
 {
-    PairListDev& L = n.L;
+    const FdGeo& GA = n.G.geo[n.P.geo[A]];
+    e.cA = n.P.pos[A];
+    const fd_quat qA = n.P.q[A];
+    e.cB = Slave<KIND>::pos(n, B);
+    e.qB = Slave<KIND>::q(n, B);
+    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const GeoSetDev& SB = Slave<KIND>::set(n);
+    const FdGrid& sg = Slave<KIND>::grid(n);
+    const double rB2 = GB.radius * GB.radius;
+    e.pool = GA.node_off + k;
+    const double3 node = n.G.nodes[e.pool];
+    e.r = xm_rot(qA, node);
+    e.gp = mk3(e.r.x + e.cA.x, e.r.y + e.cA.y, e.r.z + e.cA.z);
+    e.ov = ov0;
+    return node_predicate<KIND>(e.gp, bcell, sg, e.cB, e.qB, GB, SB.sdf, rB2, n.a.probe, e.ov, e.fx, e.fy, e.fz, e.pv);
+}
+
+// Slot s of list L, a contact by the predicate e: normal, contact point,
+// history (the pair's previous slots are oc_off .. oc_off + oc_cnt - 1),
+// records, and with forces the contact law, whose force and torques on A and B
+// go to o.  Returns the global boundary-node id.
+template <int KIND>
+__device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int s, int A,
+                                           int B, int k, int oc_off, int oc_cnt, const SlotEval& e, double o[9])
+{
+    const bool periodic = (KIND == FD_PP || KIND == FD_PW) && (n.a.periodic_x || n.a.periodic_y);
+    const FdGeo& GA = n.G.geo[n.P.geo[A]];
+    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const double3 cA = e.cA, cB = e.cB, r = e.r, gp = e.gp;
+    const fd_quat qB = e.qB;
+    const double ov = e.ov;
+    const int pool = e.pool;
+    double3 nrm = fd_gradient_q(e.fx, e.fy, e.fz, e.pv);
+    nrm = fd_rot(qB, nrm);
+    nrm = fd_normalize(nrm);
+    const double3 pt = gp + (0.5 * ov) * nrm;
+    const int nid = n.P.node_base[A] + n.G.node_lid[pool];
+    double3 spring = mk3(0., 0., 0.);
+    int hist = -1;
+    {
+        // the previous slots of the pair are ascending in node
+        // key; a node appears at most once per pair.  A carried
+        // layout keeps each slot's previous self at its index.
+        const int oc_end = oc_off + oc_cnt;
+        int lo = oc_off, hi = oc_end;
+        if (s >= oc_off && s < oc_end && L.o_c_k[s] == k) lo = hi = s;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (L.o_c_k[mid] < k) lo = mid + 1; else hi = mid;
+        }
+        if (lo < oc_end && L.o_c_k[lo] == k && L.o_c_node[lo] == nid) {
+            const double* sp = L.o_c_spring + 3ll * lo;
+            spring = mk3(sp[0], sp[1], sp[2]);
+            hist = lo;
+        }
+    }
+    if (R.hit && s < R.cap) {
+        R.A[s] = A;
+        R.B[s] = B;
+        R.Bp[s] = KIND == FD_PW ? -1 : B;
+        R.geoB[s] = KIND == FD_PW ? n.W.geo[B] : n.P.geo[B];
+        R.matB[s] = KIND == FD_PW ? n.W.mat[B] : n.P.mat[B];
+        R.nid[s] = nid;
+        R.hist[s] = hist;
+        R.rel[3 * s + 0] = gp.x - cB.x;
+        R.rel[3 * s + 1] = gp.y - cB.y;
+        R.rel[3 * s + 2] = gp.z - cB.z;
+        R.sprev[3 * s + 0] = spring.x;
+        R.sprev[3 * s + 1] = spring.y;
+        R.sprev[3 * s + 2] = spring.z;
+        R.qB[4 * s + 0] = qB.q0;
+        R.qB[4 * s + 1] = qB.q1;
+        R.qB[4 * s + 2] = qB.q2;
+        R.qB[4 * s + 3] = qB.q3;
+        R.arm[3 * s + 0] = r.x;
+        R.arm[3 * s + 1] = r.y;
+        R.arm[3 * s + 2] = r.z;
+        R.wrap[s] = 13 + 27;  // no shift unless the force side records one
+    }
+    double kn = 0., ks = 0.;
+    if (n.with_force) {
+        // force-side state (positions after the periodic wrap,
+        // LSSolver.h:1175-1190)
+        double3 ri = cA, rj = cB;
+        if (periodic) {
+            if (n.a.periodic_x) { ri = wrap_x(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_x(rj, n.pgrid); }
+            if (n.a.periodic_y) { ri = wrap_y(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_y(rj, n.pgrid); }
+        }
+        double3 vi = n.P.vel[A], vjs = Slave<KIND>::vel(n, B);
+        const double3 wi = n.P.angvel[A];
+        if ((KIND == FD_PP || KIND == FD_PW) && n.a.sector) {
+            sector_fold(ri, vi, n.pgrid.minb);
+            if (KIND == FD_PP) sector_fold(rj, vjs, n.pgrid.minb);
+        }
+        const int mi = n.P.mat[A];
+        const double invMi = GA.inv_mass;
+        const double kni = n.M.kn[mi], ksi = n.M.ks[mi], mui = n.M.mu[mi], ei = n.M.e[mi];
+        double3 vj, wj;
+        double effM = 0., mu, res;
+        if (KIND == FD_PW) {
+            vj = vjs;
+            wj = n.W.angvel[B];
+            const int mj = n.W.mat[B];
+            mu = fmin(mui, n.MW.mu[mj]);
+            res = fmin(ei, n.MW.e[mj]);
+            if (invMi > 0.) effM = 1. / invMi;
+            kn = kni;
+            ks = ksi;
+        } else {
+            vj = vjs;
+            wj = n.P.angvel[B];
+            const double invMj = GB.inv_mass;
+            const int mj = n.P.mat[B];
+            const double knj = n.M.kn[mj], ksj = n.M.ks[mj];
+            if (kni > 0. && knj > 0.) kn = kni * knj / (kni + knj);
+            if (ksi > 0. && ksj > 0.) ks = ksi * ksj / (ksi + ksj);
+            if (invMi > 0. || invMj > 0.) effM = 1. / (invMi + invMj);
+            res = fmin(ei, n.M.e[mj]);
+            mu = fmin(mui, n.M.mu[mj]);
+        }
+        const double3 vc = (vi + cross3(wi, pt - ri)) - (vj + cross3(wj, pt - rj));
+        if (R.hit && s < R.cap) {
+            R.vc[3 * s + 0] = vc.x;
+            R.vc[3 * s + 1] = vc.y;
+            R.vc[3 * s + 2] = vc.z;
+            R.wrap[s] = wrap_code(cA, ri, cB, rj, n.pgrid);
+        }
+        double3 F = mk3(0., 0., 0.);
+        linear_contact(F, spring, vc, nrm, ov, n.a.dt, kn, ks, mu, res, effM);
+        const double3 TA = cross3(pt - ri, F);
+        const double3 TB = cross3(pt - rj, -F);
+                            o[0] = F.x; o[1] = F.y; o[2] = F.z;
+        o[3] = TA.x; o[4] = TA.y; o[5] = TA.z;
+        o[6] = TB.x; o[7] = TB.y; o[8] = TB.z;
+    }
+    L.c_slave[s] = B;
+    L.c_spring[3 * s + 0] = spring.x;
+    L.c_spring[3 * s + 1] = spring.y;
+    L.c_spring[3 * s + 2] = spring.z;
+    if (n.a.records) {
+        if (!n.with_force) {
+            const int mi = n.P.mat[A];
+            kn = n.M.kn[mi];
+            ks = n.M.ks[mi];
+            if (KIND != FD_PW) {
+                const int mj = n.P.mat[B];
+                const double knj = n.M.kn[mj], ksj = n.M.ks[mj];
+                kn = (kn > 0. && knj > 0.) ? kn * knj / (kn + knj) : 0.;
+                ks = (ks > 0. && ksj > 0.) ? ks * ksj / (ks + ksj) : 0.;
+            }
+        }
+        L.c_point[3 * s + 0] = pt.x;
+        L.c_point[3 * s + 1] = pt.y;
+        L.c_point[3 * s + 2] = pt.z;
+        L.c_normal[3 * s + 0] = nrm.x;
+        L.c_normal[3 * s + 1] = nrm.y;
+        L.c_normal[3 * s + 2] = nrm.z;
+        L.c_overlap[s] = ov;
+        L.c_en[s] = 0.5 * ov * ov * kn;
+        L.c_es[s] = 0.5 * lengthSq3(spring) * ks;
+    }
+    return nid;
+}
+
+template <int KIND, int PASS>
+__device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int nblocks)
+{
+    const PairListDev& L = n.L;
     // pair cache (particle-particle, particle-wall and translated image
     // lists, predicate pass): a rebuild step tests every slot and stores its
     // bound; a carried step tests the slots k_slot_filter listed (the
     // particle-particle list) or tests the slot bound here (the others).  An
     // image list under the cache also holds the pairs of particles that have
     // no image entry this step: their slots hold no contact.
-    constexpr bool TRANSLATED = KIND == FD_GX || KIND == FD_GY || KIND == FD_GXY;
-    const bool cache = (KIND == FD_PP || KIND == FD_PW || TRANSLATED) && PASS == 0 && n.a.gate != nullptr &&
-                       L.c_phi0 != nullptr && n.a.drift != nullptr;
-    const bool carried = cache && *n.a.gate == 0;
-    const bool listed = KIND == FD_PP && carried && L.c_test != nullptr;
-    const bool slot_test = carried && !listed;
-    const bool phi0_store = cache && !carried;
-    const bool live_test = TRANSLATED && PASS == 0 && n.gh.live != nullptr;
+    constexpr bool IMAGE = KIND != FD_PP && KIND != FD_PW;
+    const bool cache = n.a.gate != nullptr;
+    const bool carried = !list_built(n.a);
+    const bool listed = KIND == FD_PP && PASS == 0 && carried;
+    const bool slot_test = PASS == 0 && carried && !listed;
+    const bool phi0_store = PASS == 0 && cache && !carried;
+    const bool live_test = IMAGE && PASS == 0 && n.gh.live != nullptr;
     // pass 0: every slot (or the listed ones); pass 1: the slots pass 0
     // listed as contacts
     const int nitems = PASS == 0 ? min(listed ? *L.n_test : *L.n_slots, L.cap_contacts)
                                  : min(*L.n_hits, L.cap_contacts);
     const int lane = threadIdx.x & 31;
-    const bool periodic = (KIND == FD_PP || KIND == FD_PW) && (n.a.periodic_x || n.a.periodic_y);
-    const int stride = gridDim.x * blockDim.x;
-    if (carried && blockIdx.x == 0 && threadIdx.x == 0 && L.carry_n) atomicAdd(L.carry_n, 1);
+    const int stride = nblocks * blockDim.x;
     int hits = 0;
-    for (int s0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); s0 < nitems; s0 += stride) {
+    for (int s0 = block * blockDim.x + (threadIdx.x & ~31); s0 < nitems; s0 += stride) {
         const int t = s0 + lane;
         bool continue_slot = false;
         const int s = t < nitems ? (PASS == 1 ? L.c_hit[t] : listed ? L.c_test[t] : t) : t;
@@ -1750,168 +1980,36 @@ __global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONT
             const int k = L.c_k[s];
             const int A = L.pairA[p];
             const int B = L.pairB[p];
-            const int4 aux = L.p_aux[p];
-            const int3 bcell = make_int3(aux.x, aux.y, aux.z);
-            const FdGeo& GA = n.G.geo[n.P.geo[A]];
-            const double3 cA = n.P.pos[A];
-            const fd_quat qA = n.P.q[A];
-            const double3 cB = Slave<KIND>::pos(n, B);
-            const fd_quat qB = Slave<KIND>::q(n, B);
-            const FdGeo& GB = Slave<KIND>::geo(n, B);
-            const GeoSetDev& SB = Slave<KIND>::set(n);
-            const FdGrid& sg = Slave<KIND>::grid(n);
-            const double rB2 = GB.radius * GB.radius;
-            const int pool = GA.node_off + k;
-            const double3 node = n.G.nodes[pool];
-            const double3 r = xm_rot(qA, node);
-            const double3 gp = mk3(r.x + cA.x, r.y + cA.y, r.z + cA.z);
+            // a carried slot's history is its previous self, and its partner's
+            // cell this step's
+            int4 aux = make_int4(0, 0, 0, s);
+            int hist = 1;
+            if (carried) {
+                int3 bc;
+                decode_cell(Slave<KIND>::hash(n, B), Slave<KIND>::grid(n).size, bc);
+                aux.x = bc.x; aux.y = bc.y; aux.z = bc.z;
+            } else {
+                aux = L.p_aux[p];
+                hist = L.p_hist_cnt[p];
+            }
+            SlotEval e;
             // an overlap the predicate did not reach stays +inf (a slot that
             // is never skipped)
-            double ov = PASS == 0 ? __longlong_as_double(0x7ff0000000000000ll) : 0., fx = 0., fy = 0., fz = 0., pv[8];
-            hit = node_predicate<KIND>(gp, bcell, sg, cB, qB, GB, SB.sdf, rB2, n.a.probe, ov, fx, fy, fz, pv);
-            if (phi0_store) L.c_phi0[s] = __double2float_rd(-ov);
+            hit = slot_predicate<KIND>(n, A, B, k, make_int3(aux.x, aux.y, aux.z),
+                                       PASS == 0 ? __longlong_as_double(0x7ff0000000000000ll) : 0., e);
+            if (phi0_store) L.c_phi0[s] = __double2float_rd(-e.ov);
             int nid = -1;
-            if (PASS == 1 && hit) {
-                double3 nrm = fd_gradient_q(fx, fy, fz, pv);
-                nrm = fd_rot(qB, nrm);
-                nrm = fd_normalize(nrm);
-                const double3 pt = gp + (0.5 * ov) * nrm;
-                nid = n.P.node_base[A] + n.G.node_lid[pool];
-                double3 spring = mk3(0., 0., 0.);
-                int hist = -1;
-                {
-                    // the previous slots of the pair are ascending in node
-                    // key; a node appears at most once per pair.  A carried
-                    // layout keeps each slot's previous self at its index.
-                    const int oc_off = aux.w, oc_end = aux.w + L.p_hist_cnt[p];
-                    int lo = oc_off, hi = oc_end;
-                    if (s >= oc_off && s < oc_end && L.o_c_k[s] == k) lo = hi = s;
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1;
-                        if (L.o_c_k[mid] < k) lo = mid + 1; else hi = mid;
-                    }
-                    if (lo < oc_end && L.o_c_k[lo] == k && L.o_c_node[lo] == nid) {
-                        const double* sp = L.o_c_spring + 3ll * lo;
-                        spring = mk3(sp[0], sp[1], sp[2]);
-                        hist = lo;
-                    }
-                }
-                const AdjRec& R = n.a.rec;
-                if (R.hit && s < R.cap) {
-                    R.A[s] = A;
-                    R.B[s] = B;
-                    R.Bp[s] = KIND == FD_PW ? -1 : B;
-                    R.geoB[s] = KIND == FD_PW ? n.W.geo[B] : n.P.geo[B];
-                    R.matB[s] = KIND == FD_PW ? n.W.mat[B] : n.P.mat[B];
-                    R.nid[s] = nid;
-                    R.hist[s] = hist;
-                    R.rel[3 * s + 0] = gp.x - cB.x;
-                    R.rel[3 * s + 1] = gp.y - cB.y;
-                    R.rel[3 * s + 2] = gp.z - cB.z;
-                    R.sprev[3 * s + 0] = spring.x;
-                    R.sprev[3 * s + 1] = spring.y;
-                    R.sprev[3 * s + 2] = spring.z;
-                    R.qB[4 * s + 0] = qB.q0;
-                    R.qB[4 * s + 1] = qB.q1;
-                    R.qB[4 * s + 2] = qB.q2;
-                    R.qB[4 * s + 3] = qB.q3;
-                    R.arm[3 * s + 0] = r.x;
-                    R.arm[3 * s + 1] = r.y;
-                    R.arm[3 * s + 2] = r.z;
-                    R.wrap[s] = 13 + 27;  // no shift unless the force side records one
-                }
-                double kn = 0., ks = 0.;
-                if (n.with_force) {
-                    // force-side state (positions after the periodic wrap,
-                    // LSSolver.h:1175-1190)
-                    double3 ri = cA, rj = cB;
-                    if (periodic) {
-                        if (n.a.periodic_x) { ri = wrap_x(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_x(rj, n.pgrid); }
-                        if (n.a.periodic_y) { ri = wrap_y(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_y(rj, n.pgrid); }
-                    }
-                    double3 vi = n.P.vel[A], vjs = Slave<KIND>::vel(n, B);
-                    const double3 wi = n.P.angvel[A];
-                    if ((KIND == FD_PP || KIND == FD_PW) && n.a.sector) {
-                        sector_fold(ri, vi, n.pgrid.minb);
-                        if (KIND == FD_PP) sector_fold(rj, vjs, n.pgrid.minb);
-                    }
-                    const int mi = n.P.mat[A];
-                    const double invMi = GA.inv_mass;
-                    const double kni = n.M.kn[mi], ksi = n.M.ks[mi], mui = n.M.mu[mi], ei = n.M.e[mi];
-                    double3 vj, wj;
-                    double effM = 0., mu, res;
-                    if (KIND == FD_PW) {
-                        vj = vjs;
-                        wj = n.W.angvel[B];
-                        const int mj = n.W.mat[B];
-                        mu = fmin(mui, n.MW.mu[mj]);
-                        res = fmin(ei, n.MW.e[mj]);
-                        if (invMi > 0.) effM = 1. / invMi;
-                        kn = kni;
-                        ks = ksi;
-                    } else {
-                        vj = vjs;
-                        wj = n.P.angvel[B];
-                        const double invMj = GB.inv_mass;
-                        const int mj = n.P.mat[B];
-                        const double knj = n.M.kn[mj], ksj = n.M.ks[mj];
-                        if (kni > 0. && knj > 0.) kn = kni * knj / (kni + knj);
-                        if (ksi > 0. && ksj > 0.) ks = ksi * ksj / (ksi + ksj);
-                        if (invMi > 0. || invMj > 0.) effM = 1. / (invMi + invMj);
-                        res = fmin(ei, n.M.e[mj]);
-                        mu = fmin(mui, n.M.mu[mj]);
-                    }
-                    const double3 vc = (vi + cross3(wi, pt - ri)) - (vj + cross3(wj, pt - rj));
-                    if (R.hit && s < R.cap) {
-                        R.vc[3 * s + 0] = vc.x;
-                        R.vc[3 * s + 1] = vc.y;
-                        R.vc[3 * s + 2] = vc.z;
-                        R.wrap[s] = wrap_code(cA, ri, cB, rj, n.pgrid);
-                    }
-                    double3 F = mk3(0., 0., 0.);
-                    linear_contact(F, spring, vc, nrm, ov, n.a.dt, kn, ks, mu, res, effM);
-                    const double3 TA = cross3(pt - ri, F);
-                    const double3 TB = cross3(pt - rj, -F);
-                    double* o = L.c_force + 9ll * s;
-                    o[0] = F.x; o[1] = F.y; o[2] = F.z;
-                    o[3] = TA.x; o[4] = TA.y; o[5] = TA.z;
-                    o[6] = TB.x; o[7] = TB.y; o[8] = TB.z;
-                }
-                L.c_slave[s] = B;
-                L.c_spring[3 * s + 0] = spring.x;
-                L.c_spring[3 * s + 1] = spring.y;
-                L.c_spring[3 * s + 2] = spring.z;
-                if (n.a.records) {
-                    if (!n.with_force) {
-                        const int mi = n.P.mat[A];
-                        kn = n.M.kn[mi];
-                        ks = n.M.ks[mi];
-                        if (KIND != FD_PW) {
-                            const int mj = n.P.mat[B];
-                            const double knj = n.M.kn[mj], ksj = n.M.ks[mj];
-                            kn = (kn > 0. && knj > 0.) ? kn * knj / (kn + knj) : 0.;
-                            ks = (ks > 0. && ksj > 0.) ? ks * ksj / (ks + ksj) : 0.;
-                        }
-                    }
-                    L.c_point[3 * s + 0] = pt.x;
-                    L.c_point[3 * s + 1] = pt.y;
-                    L.c_point[3 * s + 2] = pt.z;
-                    L.c_normal[3 * s + 0] = nrm.x;
-                    L.c_normal[3 * s + 1] = nrm.y;
-                    L.c_normal[3 * s + 2] = nrm.z;
-                    L.c_overlap[s] = ov;
-                    L.c_en[s] = 0.5 * ov * ov * kn;
-                    L.c_es[s] = 0.5 * lengthSq3(spring) * ks;
-                }
-            }
+            if (PASS == 1 && hit)
+                nid = contact_law<KIND>(n, L, n.a.rec, s, A, B, k, aux.w, hist, e, L.c_force + 9ll * s);
             if (PASS == 1) {
                 L.c_node[s] = nid;
             } else {
-                if (!hit) L.c_node[s] = -1;
+                if (hit) L.p_hit[p] = 1;
+                else L.c_node[s] = -1;
                 if (n.a.rec.hit && s < n.a.rec.cap) n.a.rec.hit[s] = hit ? 1 : 0;
             }
         }
-        if (cache && !listed && n.a.stats) {
+        if (PASS == 0 && cache && !listed && n.a.stats) {
             // slots given the exact predicate, slots skipped (k_slot_filter
             // counts the listed steps)
             const unsigned int tested = __ballot_sync(0xffffffffu, t < nitems && !continue_slot);
@@ -1940,20 +2038,43 @@ __global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONT
 // a fixed butterfly combines the lanes, so the result does not depend on
 // where the pair's slots lie.
 // ---------------------------------------------------------------------------
-__global__ void k_pair_sum(PairListDev L, int with_force)
+template <typename Real>
+__device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int block, int nblocks, bool link,
+                                         const RevDev& R, int n_obj)
 {
+    const Real* cf = reinterpret_cast<const Real*>(L.c_force);
+    Real* pf = reinterpret_cast<Real*>(L.pf);
     const int npairs = min(*L.n_pairs, L.cap_pairs);
     const int lane = threadIdx.x & 31, grp = lane >> 3, l = lane & 7;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int warp = (block * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (nblocks * blockDim.x) >> 5;
+    const unsigned int build = link ? *R.build : 0u;
     for (int p0 = warp * 4; p0 < npairs; p0 += nwarps * 4) {
         const int p = p0 + grp;
-        double acc[9] = {0., 0., 0., 0., 0., 0., 0., 0., 0.};
+        Real acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         int o = 0, c = 0;
-        if (p < npairs && with_force) {
-            o = L.c_off[p];
+        bool hit = false;
+        if (p < npairs) {
             c = L.c_cnt[p];
+            hit = L.p_hit[p] != 0;
+            if (hit) o = L.c_off[p];
         }
+        // a list that is built: the pair joins its partner's list of the
+        // reverse index (only pairs with contact slots carry a force)
+        if (link && l == 0 && c > 0) {
+            const int B = L.pairB[p];
+            if (B >= 0 && B < n_obj) {
+                const unsigned int code = (unsigned int)(p * 8 + kind);  // pair counts stay below 2^28
+                const unsigned long long old =
+                    atomicExch(&R.head[B], ((unsigned long long)build << 32) | code);
+                L.r_next[p] = (unsigned int)(old >> 32) == build ? (int)(unsigned int)old : -1;
+            }
+        }
+        // three pairs in four hold no contact (settled beds: 8 slots and a
+        // quarter of a contact per pair): their slots are not looked at, and
+        // the force sums skip them by the same flag.  With every pair's slots
+        // read the sums took 118 us for 262,144 particles.
+        if (!hit) c = 0;
         // slots l, l + 8, l + 16, ... in order; four node ids loaded ahead
         for (int j0 = l; j0 < c; j0 += 32) {
             int nd[4];
@@ -1962,13 +2083,11 @@ __global__ void k_pair_sum(PairListDev L, int with_force)
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 if (nd[u] < 0) continue;
-                const double* f = L.c_force + 9ll * (o + j0 + 8 * u);
+                const Real* f = cf + 9ll * (o + j0 + 8 * u);
 #pragma unroll
                 for (int t = 0; t < 9; ++t) acc[t] += f[t];
             }
         }
-        // pairs without contact slots keep no sum: k_reduce skips them by
-        // their slot count
         if (__any_sync(0xffffffffu, c > 0)) {
 #pragma unroll
             for (int t = 0; t < 9; ++t) {
@@ -1978,7 +2097,7 @@ __global__ void k_pair_sum(PairListDev L, int with_force)
             }
         }
         if (p < npairs && c > 0) {
-            double* out = L.pf + 9ll * p;
+            Real* out = pf + 9ll * p;
 #pragma unroll
             for (int t = 0; t < 8; ++t)
                 if (l == t) out[t] = acc[t];
@@ -2057,31 +2176,247 @@ __device__ __forceinline__ v3f linear_contact32(double3& spring, v3f vc, v3f n, 
     return fn + (-ks * tof(spring) - cs * vs);
 }
 
-template <int KIND, int PASS>
-__global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONTACT_MIN_BLOCKS) k_contact32(NarrowArgs n)
+// one slot's node against its partner, single-precision SDF
+struct SlotEval32 {
+    double3 cA, cB, rd, gp;  // centres, node offset from A's centre, node
+    int pool;
+    float ov, phi0, fx, fy, fz, pv[8];
+};
+
+// as slot_predicate
+template <int KIND>
+__device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int B, int k, int3 bcell, float ov0,
+                                                 SlotEval32& e)
 {
-    PairListDev& L = n.L;
+    const FdGeo& GA = n.G.geo[n.P.geo[A]];
+    const double3 cA = n.P.pos[A];
+    const double3 cB = Slave<KIND>::pos(n, B);
+    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const GeoSetDev& SB = Slave<KIND>::set(n);
+    const FdGrid& sg = Slave<KIND>::grid(n);
+    // the rigid transforms in double precision (as in FP64 mode), the
+    // position inside the cell and the SDF interpolation in single
+    e.cA = cA;
+    e.cB = cB;
+    e.pool = GA.node_off + k;
+    e.rd = xm_rot(n.P.q[A], n.G.nodes[e.pool]);
+    const double3 gp = mk3(e.rd.x + cA.x, e.rd.y + cA.y, e.rd.z + cA.z);
+    e.gp = gp;
+    int3 lo, hi;
+    fd_node_range(gp, sg, lo, hi);
+    float fx = 0.f, fy = 0.f, fz = 0.f;
+    float* pv = e.pv;
+    bool hit = false;
+    e.ov = ov0;
+    e.phi0 = __int_as_float(0xff800000);  // the slot bound to store (-inf: never skipped)
+    if (bcell.x >= lo.x && bcell.x <= hi.x && bcell.y >= lo.y && bcell.y <= hi.y && bcell.z >= lo.z && bcell.z <= hi.z) {
+        const double3 rel = mk3(gp.x - cB.x, gp.y - cB.y, gp.z - cB.z);
+        if (!Slave<KIND>::radius_test || xm_len2(rel) <= GB.radius * GB.radius) {
+            const double3 lp = xm_rrot(rel, Slave<KIND>::q(n, B));
+            const double gx = (lp.x - GB.origin.x) * GB.inv_spacing;
+            const double gy = (lp.y - GB.origin.y) * GB.inv_spacing;
+            const double gz = (lp.z - GB.origin.z) * GB.inv_spacing;
+            const int i0 = (int)floor(gx), j0 = (int)floor(gy), k0 = (int)floor(gz);
+            if (i0 >= 0 && j0 >= 0 && k0 >= 0 && i0 < GB.size.x - 1 && j0 < GB.size.y - 1 &&
+                k0 < GB.size.z - 1) {
+                fx = (float)(gx - (double)i0);
+                fy = (float)(gy - (double)j0);
+                fz = (float)(gz - (double)k0);
+                const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
+                const long long c0 = GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
+                if (KIND == FD_PW) {
+                    // wall grids are coarse (a plane wall is one cell
+                    // the size of the domain, corner values of tenths
+                    // of a metre): single-precision interpolation
+                    // there would carry errors of 1e-8 m, so the
+                    // (few) wall contacts interpolate in double
+                    const double* S = SB.sdf + c0;
+                    double pd[8] = {__ldg(S), __ldg(S + 1), __ldg(S + sx), __ldg(S + sx + 1), __ldg(S + sxy),
+                                    __ldg(S + sxy + 1), __ldg(S + sxy + sx), __ldg(S + sxy + sx + 1)};
+                    const double ovd = -xm_trilinear(gx - (double)i0, gy - (double)j0, gz - (double)k0, pd);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) pv[c] = (float)pd[c];
+                    e.ov = (float)ovd;
+                    e.phi0 = __double2float_rd(-ovd);
+                    hit = ovd >= -n.a.probe;
+                } else {
+                    const float* S = SB.sdf32 + c0;
+                    pv[0] = __ldg(S); pv[1] = __ldg(S + 1); pv[2] = __ldg(S + sx); pv[3] = __ldg(S + sx + 1);
+                    pv[4] = __ldg(S + sxy); pv[5] = __ldg(S + sxy + 1); pv[6] = __ldg(S + sxy + sx);
+                    pv[7] = __ldg(S + sxy + sx + 1);
+                    const float c00 = pv[0] * (1.f - fx) + pv[1] * fx, c10 = pv[2] * (1.f - fx) + pv[3] * fx;
+                    const float c01 = pv[4] * (1.f - fx) + pv[5] * fx, c11 = pv[6] * (1.f - fx) + pv[7] * fx;
+                    e.ov = -((c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz);
+                    e.phi0 = -e.ov;
+                    hit = e.ov >= -(float)n.a.probe;
+                }
+            }
+        }
+    }
+    e.fx = fx;
+    e.fy = fy;
+    e.fz = fz;
+    return hit;
+}
+
+// as contact_law
+template <int KIND>
+__device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int s, int A,
+                                             int B, int k, int oc_off, int oc_cnt, const SlotEval32& e, float o[9])
+{
+    const bool periodic = (KIND == FD_PP || KIND == FD_PW) && (n.a.periodic_x || n.a.periodic_y);
+    const FdGeo& GA = n.G.geo[n.P.geo[A]];
+    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const float4* RB = Slave<KIND>::rot(n, B);
+    const float4 b0 = RB[0], b1 = RB[1], b2 = RB[2];
+    const double3 cA = e.cA, cB = e.cB, rd = e.rd, gp = e.gp;
+    const v3f r = tof(rd);  // node offset from A's centre
+    const float ov = e.ov, fy = e.fy, fz = e.fz;
+    const float* pv = e.pv;
+    const int pool = e.pool;
+    // gradient with the x weight truncated as the reference does
+    // (LSParticleContactDetectionKernel.cuh:34)
+    const float wy0 = 1.f - fy, wy1 = fy, wz0 = 1.f - fz, wz1 = fz;
+    const v3f gB = mkf((pv[1] - pv[0]) * wy0 * wz0 + (pv[3] - pv[2]) * wy1 * wz0 +
+                           (pv[5] - pv[4]) * wy0 * wz1 + (pv[7] - pv[6]) * wy1 * wz1,
+                       (pv[2] - pv[0]) * wz0 + (pv[6] - pv[4]) * wz1,
+                       (pv[4] - pv[0]) * wy0 + (pv[6] - pv[2]) * wy1);
+    v3f nrm = rowsf(b0, b1, b2, gB);
+    const float l2 = dotf(nrm, nrm);
+    nrm = l2 > 1e-20f ? rsqrtf(l2) * nrm : mkf(0.f, 0.f, 0.f);
+    const v3f arm = r + (0.5f * ov) * nrm;  // contact point relative to A's centre
+    const int nid = n.P.node_base[A] + n.G.node_lid[pool];
+    double3 spring = mk3(0., 0., 0.);
+    int hist = -1;
+    {
+        const int oc_end = oc_off + oc_cnt;
+        int lo2 = oc_off, hi2 = oc_end;
+        if (s >= oc_off && s < oc_end && L.o_c_k[s] == k) lo2 = hi2 = s;
+        while (lo2 < hi2) {
+            const int mid = (lo2 + hi2) >> 1;
+            if (L.o_c_k[mid] < k) lo2 = mid + 1; else hi2 = mid;
+        }
+        if (lo2 < oc_end && L.o_c_k[lo2] == k && L.o_c_node[lo2] == nid) {
+            const double* sp = L.o_c_spring + 3ll * lo2;
+            spring = mk3(sp[0], sp[1], sp[2]);
+            hist = lo2;
+        }
+    }
+    if (R.hit && s < R.cap) {
+        const fd_quat qB = Slave<KIND>::q(n, B);
+        R.A[s] = A;
+        R.B[s] = B;
+        R.Bp[s] = KIND == FD_PW ? -1 : B;
+        R.geoB[s] = KIND == FD_PW ? n.W.geo[B] : n.P.geo[B];
+        R.matB[s] = KIND == FD_PW ? n.W.mat[B] : n.P.mat[B];
+        R.nid[s] = nid;
+        R.hist[s] = hist;
+        R.rel[3 * s + 0] = gp.x - cB.x;
+        R.rel[3 * s + 1] = gp.y - cB.y;
+        R.rel[3 * s + 2] = gp.z - cB.z;
+        R.sprev[3 * s + 0] = spring.x;
+        R.sprev[3 * s + 1] = spring.y;
+        R.sprev[3 * s + 2] = spring.z;
+        R.qB[4 * s + 0] = qB.q0;
+        R.qB[4 * s + 1] = qB.q1;
+        R.qB[4 * s + 2] = qB.q2;
+        R.qB[4 * s + 3] = qB.q3;
+        R.arm[3 * s + 0] = rd.x;
+        R.arm[3 * s + 1] = rd.y;
+        R.arm[3 * s + 2] = rd.z;
+        R.wrap[s] = 13 + 27;  // no shift unless the force side records one
+    }
+    const int mi = n.P.mat[A];
+    float kn = 0.f, ks = 0.f;
+    float mu, res, effM = 0.f;
+    const double kni = n.M.kn[mi], ksi = n.M.ks[mi];
+    const double invMi = GA.inv_mass;
+    if (KIND == FD_PW) {
+        const int mj = n.W.mat[B];
+        mu = (float)fmin(n.M.mu[mi], n.MW.mu[mj]);
+        res = (float)fmin(n.M.e[mi], n.MW.e[mj]);
+        if (invMi > 0.) effM = (float)(1. / invMi);
+        kn = (float)kni;
+        ks = (float)ksi;
+    } else {
+        const int mj = n.P.mat[B];
+        const double knj = n.M.kn[mj], ksj = n.M.ks[mj], invMj = GB.inv_mass;
+        if (kni > 0. && knj > 0.) kn = (float)(kni * knj / (kni + knj));
+        if (ksi > 0. && ksj > 0.) ks = (float)(ksi * ksj / (ksi + ksj));
+        if (invMi > 0. || invMj > 0.) effM = (float)(1. / (invMi + invMj));
+        res = (float)fmin(n.M.e[mi], n.M.e[mj]);
+        mu = (float)fmin(n.M.mu[mi], n.M.mu[mj]);
+    }
+    if (n.with_force) {
+        double3 ri = cA, rj = cB;
+        if (periodic) {
+            if (n.a.periodic_x) { ri = wrap_x(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_x(rj, n.pgrid); }
+            if (n.a.periodic_y) { ri = wrap_y(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_y(rj, n.pgrid); }
+        }
+        double3 vid = n.P.vel[A], vjd = Slave<KIND>::vel(n, B);
+        if ((KIND == FD_PP || KIND == FD_PW) && n.a.sector) {
+            sector_fold(ri, vid, n.pgrid.minb);
+            if (KIND == FD_PP) sector_fold(rj, vjd, n.pgrid.minb);
+        }
+        const v3f armA = tof(cA - ri) + arm;
+        const v3f armB = tof(cA - rj) + arm;
+        const v3f vi = tof(vid), wi = tof(n.P.angvel[A]);
+        const v3f vj = tof(vjd);
+        const v3f wj = tof(KIND == FD_PW ? n.W.angvel[B] : n.P.angvel[B]);
+        const v3f vc = (vi + crossf(wi, armA)) - (vj + crossf(wj, armB));
+        if (R.hit && s < R.cap) {
+            R.vc[3 * s + 0] = vc.x;
+            R.vc[3 * s + 1] = vc.y;
+            R.vc[3 * s + 2] = vc.z;
+            R.wrap[s] = wrap_code(cA, ri, cB, rj, n.pgrid);
+        }
+        const v3f F = linear_contact32(spring, vc, nrm, ov, (float)n.a.dt, kn, ks, mu, res, effM);
+        const v3f TA = crossf(armA, F);
+        const v3f TB = crossf(armB, -F);
+        o[0] = F.x; o[1] = F.y; o[2] = F.z;
+        o[3] = TA.x; o[4] = TA.y; o[5] = TA.z;
+        o[6] = TB.x; o[7] = TB.y; o[8] = TB.z;
+    }
+    L.c_slave[s] = B;
+    L.c_spring[3 * s + 0] = spring.x;
+    L.c_spring[3 * s + 1] = spring.y;
+    L.c_spring[3 * s + 2] = spring.z;
+    if (n.a.records) {
+        L.c_point[3 * s + 0] = cA.x + arm.x;
+        L.c_point[3 * s + 1] = cA.y + arm.y;
+        L.c_point[3 * s + 2] = cA.z + arm.z;
+        L.c_normal[3 * s + 0] = nrm.x;
+        L.c_normal[3 * s + 1] = nrm.y;
+        L.c_normal[3 * s + 2] = nrm.z;
+        L.c_overlap[s] = ov;
+        L.c_en[s] = 0.5 * (double)ov * (double)ov * (double)kn;
+        L.c_es[s] = 0.5 * lengthSq3(spring) * (double)ks;
+    }
+    return nid;
+}
+
+template <int KIND, int PASS>
+__device__ __forceinline__ void contact_list32(const NarrowArgs& n, int block, int nblocks)
+{
+    const PairListDev& L = n.L;
     float* cf = reinterpret_cast<float*>(L.c_force);
     // pass 0: every slot; pass 1: the slots pass 0 listed as contacts
     const int nitems = PASS == 0 ? min(*L.n_slots, L.cap_contacts) : min(*L.n_hits, L.cap_contacts);
     const int lane = threadIdx.x & 31;
-    const bool periodic = (KIND == FD_PP || KIND == FD_PW) && (n.a.periodic_x || n.a.periodic_y);
-    const int stride = gridDim.x * blockDim.x;
+    const int stride = nblocks * blockDim.x;
     // pair cache, as in k_contact; the single-precision predicate's own
     // rounding (a few 1e-7 of the SDF values) is covered by a margin of
     // 1e-4 of B's grid spacing in the pair bound
-    constexpr bool TRANSLATED = KIND == FD_GX || KIND == FD_GY || KIND == FD_GXY;
-    const bool cache = (KIND == FD_PP || KIND == FD_PW || TRANSLATED) && PASS == 0 && n.a.gate != nullptr &&
-                       L.c_phi0 != nullptr && n.a.drift != nullptr;
-    const bool carried = cache && *n.a.gate == 0;
-    const bool listed = KIND == FD_PP && carried && L.c_test != nullptr;
-    const bool slot_test = carried && !listed;
-    const bool phi0_store = cache && !carried;
-    const bool live_test = TRANSLATED && PASS == 0 && n.gh.live != nullptr;
+    constexpr bool IMAGE = KIND != FD_PP && KIND != FD_PW;
+    const bool cache = n.a.gate != nullptr;
+    const bool carried = !list_built(n.a);
+    const bool listed = KIND == FD_PP && PASS == 0 && carried;
+    const bool slot_test = PASS == 0 && carried && !listed;
+    const bool phi0_store = PASS == 0 && cache && !carried;
+    const bool live_test = IMAGE && PASS == 0 && n.gh.live != nullptr;
     const int nitems_c = PASS == 0 && listed ? min(*L.n_test, L.cap_contacts) : nitems;
-    if (carried && blockIdx.x == 0 && threadIdx.x == 0 && L.carry_n) atomicAdd(L.carry_n, 1);
     int hits = 0;
-    for (int s0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); s0 < nitems_c; s0 += stride) {
+    for (int s0 = block * blockDim.x + (threadIdx.x & ~31); s0 < nitems_c; s0 += stride) {
         const int t = s0 + lane;
         const int s = t < nitems_c ? (PASS == 1 ? L.c_hit[t] : listed ? L.c_test[t] : t) : t;
         bool hit = false;
@@ -2093,8 +2428,8 @@ __global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONT
                 if (phi0_store) L.c_phi0[s] = __int_as_float(0xff800000);  // -inf: never skipped
                 continue_slot = true;
             } else if (slot_test && L.c_phi0[s] > __fadd_ru(L.p_bound[p], 1e-12f)) {
-                // k_pc_carry's pair bound carries the margin of 1e-4 of B's
-                // grid spacing in this precision
+                // pair_bound carries the margin of 1e-4 of B's grid spacing in
+                // this precision
                 L.c_node[s] = -1;
                 continue_slot = true;
             }
@@ -2104,199 +2439,32 @@ __global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONT
             const int k = L.c_k[s];
             const int A = L.pairA[p];
             const int B = L.pairB[p];
-            const int4 aux = L.p_aux[p];
-            const FdGeo& GA = n.G.geo[n.P.geo[A]];
-            const double3 cA = n.P.pos[A];
-            const double3 cB = Slave<KIND>::pos(n, B);
-            const FdGeo& GB = Slave<KIND>::geo(n, B);
-            const GeoSetDev& SB = Slave<KIND>::set(n);
-            const FdGrid& sg = Slave<KIND>::grid(n);
-            const float4* RB = Slave<KIND>::rot(n, B);
-            const float4 b0 = RB[0], b1 = RB[1], b2 = RB[2];
-            // the rigid transforms in double precision (as in FP64 mode), the
-            // position inside the cell and the SDF interpolation in single
-            const int pool = GA.node_off + k;
-            const double3 rd = xm_rot(n.P.q[A], n.G.nodes[pool]);
-            const double3 gp = mk3(rd.x + cA.x, rd.y + cA.y, rd.z + cA.z);
-            const v3f r = tof(rd);  // node offset from A's centre
-            int3 lo, hi;
-            fd_node_range(gp, sg, lo, hi);
+            // a carried slot's history is its previous self, and its partner's
+            // cell this step's
+            int4 aux = make_int4(0, 0, 0, s);
+            int hist = 1;
+            if (carried) {
+                int3 bc;
+                decode_cell(Slave<KIND>::hash(n, B), Slave<KIND>::grid(n).size, bc);
+                aux.x = bc.x; aux.y = bc.y; aux.z = bc.z;
+            } else {
+                aux = L.p_aux[p];
+                hist = L.p_hist_cnt[p];
+            }
+            SlotEval32 e;
             // an overlap the predicate did not reach stays +inf (a slot that
             // is never skipped)
-            float ov = PASS == 0 ? __int_as_float(0x7f800000) : 0.f, fx = 0.f, fy = 0.f, fz = 0.f, pv[8];
-            float phi0v = __int_as_float(0xff800000);  // the slot bound to store (-inf: never skipped)
-            if (aux.x >= lo.x && aux.x <= hi.x && aux.y >= lo.y && aux.y <= hi.y && aux.z >= lo.z && aux.z <= hi.z) {
-                const double3 rel = mk3(gp.x - cB.x, gp.y - cB.y, gp.z - cB.z);
-                if (!Slave<KIND>::radius_test || xm_len2(rel) <= GB.radius * GB.radius) {
-                    const double3 lp = xm_rrot(rel, Slave<KIND>::q(n, B));
-                    const double gx = (lp.x - GB.origin.x) * GB.inv_spacing;
-                    const double gy = (lp.y - GB.origin.y) * GB.inv_spacing;
-                    const double gz = (lp.z - GB.origin.z) * GB.inv_spacing;
-                    const int i0 = (int)floor(gx), j0 = (int)floor(gy), k0 = (int)floor(gz);
-                    if (i0 >= 0 && j0 >= 0 && k0 >= 0 && i0 < GB.size.x - 1 && j0 < GB.size.y - 1 &&
-                        k0 < GB.size.z - 1) {
-                        fx = (float)(gx - (double)i0);
-                        fy = (float)(gy - (double)j0);
-                        fz = (float)(gz - (double)k0);
-                        const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
-                        const long long c0 = GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
-                        if (KIND == FD_PW) {
-                            // wall grids are coarse (a plane wall is one cell
-                            // the size of the domain, corner values of tenths
-                            // of a metre): single-precision interpolation
-                            // there would carry errors of 1e-8 m, so the
-                            // (few) wall contacts interpolate in double
-                            const double* S = SB.sdf + c0;
-                            double pd[8] = {__ldg(S), __ldg(S + 1), __ldg(S + sx), __ldg(S + sx + 1), __ldg(S + sxy),
-                                            __ldg(S + sxy + 1), __ldg(S + sxy + sx), __ldg(S + sxy + sx + 1)};
-                            const double ovd = -xm_trilinear(gx - (double)i0, gy - (double)j0, gz - (double)k0, pd);
-#pragma unroll
-                            for (int c = 0; c < 8; ++c) pv[c] = (float)pd[c];
-                            ov = (float)ovd;
-                            phi0v = __double2float_rd(-ovd);
-                            hit = ovd >= -n.a.probe;
-                        } else {
-                            const float* S = SB.sdf32 + c0;
-                            pv[0] = __ldg(S); pv[1] = __ldg(S + 1); pv[2] = __ldg(S + sx); pv[3] = __ldg(S + sx + 1);
-                            pv[4] = __ldg(S + sxy); pv[5] = __ldg(S + sxy + 1); pv[6] = __ldg(S + sxy + sx);
-                            pv[7] = __ldg(S + sxy + sx + 1);
-                            const float c00 = pv[0] * (1.f - fx) + pv[1] * fx, c10 = pv[2] * (1.f - fx) + pv[3] * fx;
-                            const float c01 = pv[4] * (1.f - fx) + pv[5] * fx, c11 = pv[6] * (1.f - fx) + pv[7] * fx;
-                            ov = -((c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz);
-                            phi0v = -ov;
-                            hit = ov >= -(float)n.a.probe;
-                        }
-                    }
-                }
-            }
-            if (phi0_store) L.c_phi0[s] = phi0v;
+            hit = slot_predicate32<KIND>(n, A, B, k, make_int3(aux.x, aux.y, aux.z),
+                                         PASS == 0 ? __int_as_float(0x7f800000) : 0.f, e);
+            if (phi0_store) L.c_phi0[s] = e.phi0;
             int nid = -1;
-            if (PASS == 1 && hit) {
-                // gradient with the x weight truncated as the reference does
-                // (LSParticleContactDetectionKernel.cuh:34)
-                const float wy0 = 1.f - fy, wy1 = fy, wz0 = 1.f - fz, wz1 = fz;
-                const v3f gB = mkf((pv[1] - pv[0]) * wy0 * wz0 + (pv[3] - pv[2]) * wy1 * wz0 +
-                                       (pv[5] - pv[4]) * wy0 * wz1 + (pv[7] - pv[6]) * wy1 * wz1,
-                                   (pv[2] - pv[0]) * wz0 + (pv[6] - pv[4]) * wz1,
-                                   (pv[4] - pv[0]) * wy0 + (pv[6] - pv[2]) * wy1);
-                v3f nrm = rowsf(b0, b1, b2, gB);
-                const float l2 = dotf(nrm, nrm);
-                nrm = l2 > 1e-20f ? rsqrtf(l2) * nrm : mkf(0.f, 0.f, 0.f);
-                const v3f arm = r + (0.5f * ov) * nrm;  // contact point relative to A's centre
-                nid = n.P.node_base[A] + n.G.node_lid[pool];
-                double3 spring = mk3(0., 0., 0.);
-                int hist = -1;
-                {
-                    const int oc_off = aux.w, oc_end = aux.w + L.p_hist_cnt[p];
-                    int lo2 = oc_off, hi2 = oc_end;
-                    if (s >= oc_off && s < oc_end && L.o_c_k[s] == k) lo2 = hi2 = s;
-                    while (lo2 < hi2) {
-                        const int mid = (lo2 + hi2) >> 1;
-                        if (L.o_c_k[mid] < k) lo2 = mid + 1; else hi2 = mid;
-                    }
-                    if (lo2 < oc_end && L.o_c_k[lo2] == k && L.o_c_node[lo2] == nid) {
-                        const double* sp = L.o_c_spring + 3ll * lo2;
-                        spring = mk3(sp[0], sp[1], sp[2]);
-                        hist = lo2;
-                    }
-                }
-                const AdjRec& R = n.a.rec;
-                if (R.hit && s < R.cap) {
-                    const fd_quat qB = Slave<KIND>::q(n, B);
-                    R.A[s] = A;
-                    R.B[s] = B;
-                    R.Bp[s] = KIND == FD_PW ? -1 : B;
-                    R.geoB[s] = KIND == FD_PW ? n.W.geo[B] : n.P.geo[B];
-                    R.matB[s] = KIND == FD_PW ? n.W.mat[B] : n.P.mat[B];
-                    R.nid[s] = nid;
-                    R.hist[s] = hist;
-                    R.rel[3 * s + 0] = gp.x - cB.x;
-                    R.rel[3 * s + 1] = gp.y - cB.y;
-                    R.rel[3 * s + 2] = gp.z - cB.z;
-                    R.sprev[3 * s + 0] = spring.x;
-                    R.sprev[3 * s + 1] = spring.y;
-                    R.sprev[3 * s + 2] = spring.z;
-                    R.qB[4 * s + 0] = qB.q0;
-                    R.qB[4 * s + 1] = qB.q1;
-                    R.qB[4 * s + 2] = qB.q2;
-                    R.qB[4 * s + 3] = qB.q3;
-                    R.arm[3 * s + 0] = rd.x;
-                    R.arm[3 * s + 1] = rd.y;
-                    R.arm[3 * s + 2] = rd.z;
-                    R.wrap[s] = 13 + 27;  // no shift unless the force side records one
-                }
-                const int mi = n.P.mat[A];
-                float kn = 0.f, ks = 0.f;
-                float mu, res, effM = 0.f;
-                const double kni = n.M.kn[mi], ksi = n.M.ks[mi];
-                const double invMi = GA.inv_mass;
-                if (KIND == FD_PW) {
-                    const int mj = n.W.mat[B];
-                    mu = (float)fmin(n.M.mu[mi], n.MW.mu[mj]);
-                    res = (float)fmin(n.M.e[mi], n.MW.e[mj]);
-                    if (invMi > 0.) effM = (float)(1. / invMi);
-                    kn = (float)kni;
-                    ks = (float)ksi;
-                } else {
-                    const int mj = n.P.mat[B];
-                    const double knj = n.M.kn[mj], ksj = n.M.ks[mj], invMj = GB.inv_mass;
-                    if (kni > 0. && knj > 0.) kn = (float)(kni * knj / (kni + knj));
-                    if (ksi > 0. && ksj > 0.) ks = (float)(ksi * ksj / (ksi + ksj));
-                    if (invMi > 0. || invMj > 0.) effM = (float)(1. / (invMi + invMj));
-                    res = (float)fmin(n.M.e[mi], n.M.e[mj]);
-                    mu = (float)fmin(n.M.mu[mi], n.M.mu[mj]);
-                }
-                if (n.with_force) {
-                    double3 ri = cA, rj = cB;
-                    if (periodic) {
-                        if (n.a.periodic_x) { ri = wrap_x(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_x(rj, n.pgrid); }
-                        if (n.a.periodic_y) { ri = wrap_y(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_y(rj, n.pgrid); }
-                    }
-                    double3 vid = n.P.vel[A], vjd = Slave<KIND>::vel(n, B);
-                    if ((KIND == FD_PP || KIND == FD_PW) && n.a.sector) {
-                        sector_fold(ri, vid, n.pgrid.minb);
-                        if (KIND == FD_PP) sector_fold(rj, vjd, n.pgrid.minb);
-                    }
-                    const v3f armA = tof(cA - ri) + arm;
-                    const v3f armB = tof(cA - rj) + arm;
-                    const v3f vi = tof(vid), wi = tof(n.P.angvel[A]);
-                    const v3f vj = tof(vjd);
-                    const v3f wj = tof(KIND == FD_PW ? n.W.angvel[B] : n.P.angvel[B]);
-                    const v3f vc = (vi + crossf(wi, armA)) - (vj + crossf(wj, armB));
-                    if (R.hit && s < R.cap) {
-                        R.vc[3 * s + 0] = vc.x;
-                        R.vc[3 * s + 1] = vc.y;
-                        R.vc[3 * s + 2] = vc.z;
-                        R.wrap[s] = wrap_code(cA, ri, cB, rj, n.pgrid);
-                    }
-                    const v3f F = linear_contact32(spring, vc, nrm, ov, (float)n.a.dt, kn, ks, mu, res, effM);
-                    const v3f TA = crossf(armA, F);
-                    const v3f TB = crossf(armB, -F);
-                    float* o = cf + 9ll * s;
-                    o[0] = F.x; o[1] = F.y; o[2] = F.z;
-                    o[3] = TA.x; o[4] = TA.y; o[5] = TA.z;
-                    o[6] = TB.x; o[7] = TB.y; o[8] = TB.z;
-                }
-                L.c_slave[s] = B;
-                L.c_spring[3 * s + 0] = spring.x;
-                L.c_spring[3 * s + 1] = spring.y;
-                L.c_spring[3 * s + 2] = spring.z;
-                if (n.a.records) {
-                    L.c_point[3 * s + 0] = cA.x + arm.x;
-                    L.c_point[3 * s + 1] = cA.y + arm.y;
-                    L.c_point[3 * s + 2] = cA.z + arm.z;
-                    L.c_normal[3 * s + 0] = nrm.x;
-                    L.c_normal[3 * s + 1] = nrm.y;
-                    L.c_normal[3 * s + 2] = nrm.z;
-                    L.c_overlap[s] = ov;
-                    L.c_en[s] = 0.5 * (double)ov * (double)ov * (double)kn;
-                    L.c_es[s] = 0.5 * lengthSq3(spring) * (double)ks;
-                }
-            }
+            if (PASS == 1 && hit)
+                nid = contact_law32<KIND>(n, L, n.a.rec, s, A, B, k, aux.w, hist, e, cf + 9ll * s);
             if (PASS == 1) {
                 L.c_node[s] = nid;
             } else {
-                if (!hit) L.c_node[s] = -1;
+                if (hit) L.p_hit[p] = 1;
+                else L.c_node[s] = -1;
                 if (n.a.rec.hit && s < n.a.rec.cap) n.a.rec.hit[s] = hit ? 1 : 0;
             }
         }
@@ -2315,129 +2483,148 @@ __global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONT
     if (PASS == 0 && n.a.stats && lane == 0 && hits) atomicAdd(&n.a.stats[3], (unsigned long long)hits);
 }
 
-// stage 3 in single precision: eight lanes per pair, as k_pair_sum
-__global__ void k_pair_sum32(PairListDev L, int with_force)
+// the two contact passes and the pair sums of every list
+template <bool MIXED, int PASS>
+__global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONTACT_MIN_BLOCKS) k_contact_lists(ListSet a)
 {
-    const float* cf = reinterpret_cast<const float*>(L.c_force);
-    float* pf = reinterpret_cast<float*>(L.pf);
-    const int npairs = min(*L.n_pairs, L.cap_pairs);
-    const int lane = threadIdx.x & 31, grp = lane >> 3, l = lane & 7;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int p0 = warp * 4; p0 < npairs; p0 += nwarps * 4) {
-        const int p = p0 + grp;
-        float acc[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        int o = 0, c = 0;
-        if (p < npairs && with_force) {
-            o = L.c_off[p];
-            c = L.c_cnt[p];
-        }
-        for (int j0 = l; j0 < c; j0 += 32) {
-            int nd[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) nd[u] = j0 + 8 * u < c ? L.c_node[o + j0 + 8 * u] : -1;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (nd[u] < 0) continue;
-                const float* f = cf + 9ll * (o + j0 + 8 * u);
-#pragma unroll
-                for (int t = 0; t < 9; ++t) acc[t] += f[t];
-            }
-        }
-        if (__any_sync(0xffffffffu, c > 0)) {
-#pragma unroll
-            for (int t = 0; t < 9; ++t) {
-                acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 4);
-                acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 2);
-                acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 1);
-            }
-        }
-        if (p < npairs && c > 0) {
-            float* out = pf + 9ll * p;
-#pragma unroll
-            for (int t = 0; t < 8; ++t)
-                if (l == t) out[t] = acc[t];
-            if (l == 0) out[8] = acc[8];
-        }
+    int block, nblocks;
+    const int li = list_of(a, block, nblocks);
+    const NarrowArgs& n = a.l[li];
+    if (MIXED) {
+        if (a.kind[li] == FD_PP) contact_list32<FD_PP, PASS>(n, block, nblocks);
+        else if (a.kind[li] == FD_PW) contact_list32<FD_PW, PASS>(n, block, nblocks);
+        else contact_list32<FD_GX, PASS>(n, block, nblocks);
+    } else {
+        if (a.kind[li] == FD_PP) contact_list<FD_PP, PASS>(n, block, nblocks);
+        else if (a.kind[li] == FD_PW) contact_list<FD_PW, PASS>(n, block, nblocks);
+        else contact_list<FD_GX, PASS>(n, block, nblocks);
     }
 }
 
 // ---------------------------------------------------------------------------
 // reverse index: pairs grouped by partner B, sorted by A
 // ---------------------------------------------------------------------------
-// kinds that have a partner side: particle pairs and the six ghost lists
-// (FD_GX .. FD_GR270 are consecutive)
-constexpr int REV_LISTS = 7;
-__host__ __device__ constexpr int rev_kind(int k) { return k == 0 ? FD_PP : FD_GX + k - 1; }
-__host__ __device__ constexpr int rev_list(int kind) { return kind == FD_PP ? 0 : kind - FD_GX + 1; }
-static_assert(FD_GR270 == FD_GX + 5 && FD_NKIND == FD_GR270 + 1, "ghost kinds are consecutive and last");
+// (with the image lists): every pair with contact slots joins the list of its
+// partner in the pair sums (heads tagged with the step's build number, as the
+// cell table's, so nothing is cleared), and at the step's end each particle
+// walks its list into a segment of codes and sorts it.  Counting, scanning,
+// filling and sorting were seven launches.
 static_assert(FD_NKIND <= 8, "a reverse-index code keeps the kind in 3 bits");
 
-struct RevArgs {
-    PairListDev L[REV_LISTS];
-    int active[REV_LISTS];
+// the index is built: always (gate null), or on the steps that build a list
+__device__ __forceinline__ bool rev_built(const RevDev& R)
+{
+    return R.gate == nullptr || *R.gate != 0 || (R.gate2 && *R.gate2 != 0);
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(TPB) k_sum_lists(ListSet a, RevDev R)
+{
+    int block, nblocks;
+    const int li = list_of(a, block, nblocks);
+    const NarrowArgs& n = a.l[li];
+    sum_list<Real>(n.L, a.kind[li], block, nblocks, a.kind[li] != FD_PW && rev_built(R), R, n.P.n);
+}
+
+// End of a step.  The reverse index, where a list was built; under the pair
+// cache the layout of each list that was built goes to the other generation
+// too (a carried step then finds it in place), the bodies' state becomes the
+// new reference, and the last block renews the flags: a list that overflowed
+// asks for a rebuild, this step's requests become the next step's.
+struct EndArgs {
+    ObjDev P, W;
+    PairListDev L[FD_NKIND];  // by kind
+    int active[FD_NKIND];
     RevDev R;
-    int n_obj;
-    const int* gate;  // non-null: build only when *gate != 0
+    PairCacheDev pc;
+    int cached;               // the pair cache is on; ghosts: so are the translated image lists
+    int cached_ghosts;
+    unsigned int* done;       // blocks finished (returns to 0)
 };
-
-// the pair behind a flat index over the active lists
-__device__ __forceinline__ bool rev_locate(const RevArgs& r, int idx, int& k, int& p)
+__global__ void __launch_bounds__(TPB) k_step_end(EndArgs a)
 {
-#pragma unroll
-    for (k = 0; k < REV_LISTS; ++k) {
-        if (!r.active[k]) continue;
-        const int np = min(*r.L[k].n_pairs, r.L[k].cap_pairs);
-        if (idx < np) { p = idx; return true; }
-        idx -= np;
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (rev_built(a.R)) {
+        const unsigned int build = *a.R.build;
+        for (int i = i0; i < a.P.n; i += stride) {
+            const unsigned long long h = a.R.head[i];
+            int cnt = 0;
+            if ((unsigned int)(h >> 32) == build)
+                for (int code = (int)(unsigned int)h; code >= 0; code = a.L[code & 7].r_next[code >> 3]) ++cnt;
+            const int o = cnt ? atomicAdd(a.R.total, cnt) : 0;
+            cnt = min(cnt, a.R.cap - o);
+            a.R.off[i] = o;
+            a.R.cnt[i] = cnt;
+            // by owner, then kind (an owner has one pair per kind with a given
+            // partner)
+            int* seg = a.R.code + o;
+            auto key = [&](int code) { return (long long)a.L[code & 7].pairA[code >> 3] * 8 + (code & 7); };
+            int code = (int)(unsigned int)h;
+            for (int n = 0; n < cnt; ++n) {
+                const long long kv = key(code);
+                int b = n - 1;
+                while (b >= 0 && key(seg[b]) > kv) { seg[b + 1] = seg[b]; --b; }
+                seg[b + 1] = code;
+                code = a.L[code & 7].r_next[code >> 3];
+            }
+        }
     }
-    return false;
-}
-
-// Two launches: every pair with contact slots joins the list of its partner
-// (heads tagged with the step's build number, as the cell table's, so nothing
-// is cleared), then each particle walks its list into a segment of codes and
-// sorts it.  Counting, scanning and filling took five to seven launches.
-__global__ void k_rev_link(RevArgs r)
-{
-    if (r.gate && *r.gate == 0) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *r.R.total = 0;
-    const unsigned int build = *r.R.build;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x;; idx += gridDim.x * blockDim.x) {
-        int k, p;
-        if (!rev_locate(r, idx, k, p)) return;
-        const int B = r.L[k].pairB[p];
-        // only pairs with contact slots carry a force to the partner
-        if (B < 0 || B >= r.n_obj || r.L[k].c_cnt[p] <= 0) continue;
-        const unsigned int code = (unsigned int)(p * 8 + rev_kind(k));  // pair counts stay below 2^28
-        const unsigned long long old = atomicExch(&r.R.head[B], ((unsigned long long)build << 32) | code);
-        r.L[k].r_next[p] = (unsigned int)(old >> 32) == build ? (int)(unsigned int)old : -1;
+    if (!a.cached) return;
+    const bool built = a.pc.ctrl[0] != 0, ghosts_built = built || a.pc.ctrl[4] != 0;
+    for (int k = 0; k < FD_NKIND; ++k) {
+        if (!a.active[k] || !(k <= FD_PW ? built : ghosts_built && a.cached_ghosts)) continue;
+        const PairListDev& L = a.L[k];
+        const int np = min(*L.n_pairs, L.cap_pairs), ns = min(*L.n_slots, L.cap_contacts);
+        if (i0 == 0) {
+            L.o_counters[0] = *L.n_pairs;
+            L.o_counters[1] = *L.n_slots;
+        }
+        for (int i = i0; i < a.P.n; i += stride) {
+            L.o_seg_off[i] = L.seg_off[i];
+            L.o_seg_cnt[i] = L.seg_cnt[i];
+        }
+        for (int p = i0; p < np; p += stride) {
+            L.o_pairA[p] = L.pairA[p];
+            L.o_pairB[p] = L.pairB[p];
+            L.o_c_off[p] = L.c_off[p];
+            L.o_c_cnt[p] = L.c_cnt[p];
+        }
+        for (int s = i0; s < ns; s += stride) L.o_c_k[s] = L.c_k[s];
     }
-}
-// deterministic order: by owner, then kind (an owner has one pair per kind
-// with a given partner)
-__global__ void k_rev_build(RevArgs r)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= r.n_obj || (r.gate && *r.gate == 0)) return;
-    const unsigned long long h = r.R.head[i];
-    int cnt = 0;
-    if ((unsigned int)(h >> 32) == *r.R.build)
-        for (int code = (int)(unsigned int)h; code >= 0; code = r.L[rev_list(code & 7)].r_next[code >> 3]) ++cnt;
-    const int o = cnt ? atomicAdd(r.R.total, cnt) : 0;
-    cnt = min(cnt, r.R.cap - o);
-    r.R.off[i] = o;
-    r.R.cnt[i] = cnt;
-    int* seg = r.R.code + o;
-    auto key = [&](int code) { return (long long)r.L[rev_list(code & 7)].pairA[code >> 3] * 8 + (code & 7); };
-    int code = (int)(unsigned int)h;
-    for (int a = 0; a < cnt; ++a) {
-        const long long kv = key(code);
-        int b = a - 1;
-        while (b >= 0 && key(seg[b]) > kv) { seg[b + 1] = seg[b]; --b; }
-        seg[b + 1] = code;
-        code = r.L[rev_list(code & 7)].r_next[code >> 3];
+    if (built) {
+        for (int i = i0; i < a.P.n; i += stride) {
+            a.pc.ref_pos[i] = a.P.pos[i];
+            a.pc.ref_q[i] = a.P.q[i];
+            a.pc.ref_vis[i] = a.P.hash[i] >= 0;
+        }
+        for (int w = i0; w < a.W.n; w += stride) {
+            a.pc.wref_pos[w] = a.W.pos[w];
+            a.pc.wref_q[w] = a.W.q[w];
+            a.pc.wref_hash[w] = a.W.hash[w];
+        }
     }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicInc(a.done, gridDim.x - 1) != gridDim.x - 1) return;
+    // the last block: every other one has read the flags
+    int* ctrl = a.pc.ctrl;
+    auto overflowed = [&](int k) {
+        return *a.L[k].n_pairs > a.L[k].cap_pairs || *a.L[k].n_slots > a.L[k].cap_contacts;
+    };
+    if (built) {
+        ctrl[1] += 1;
+        // a build whose pairs or slots did not fit is not kept: the next step
+        // builds again (the host grows the lists at its next check)
+        ctrl[2] = overflowed(FD_PP) ? 1 : 0;
+    }
+    int request = ctrl[7];
+    for (int k = FD_PW; k < FD_NKIND; ++k)
+        if (a.active[k] && (k == FD_PW || a.cached_ghosts) && overflowed(k)) request = 1;
+    ctrl[3] = request;
+    ctrl[7] = 0;
+    ctrl[0] = 0;
+    ctrl[4] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -2449,10 +2636,10 @@ __global__ void k_bonds(ObjDev P, BondDev Bd)
     if (k >= Bd.n) return;
     double* E = Bd.energy + 6ll * k;
     double* O = Bd.out + 9ll * k;
-    for (int t = 0; t < 9; ++t) O[t] = 0.;
     if (Bd.rec_active) Bd.rec_active[k] = Bd.active[k] != 0;
     if (Bd.active[k] == 0) {
         for (int t = 0; t < 6; ++t) E[t] = 0.;
+        for (int t = 0; t < 9; ++t) O[t] = 0;
         return;
     }
     const int i = Bd.master[k], j = Bd.slave[k];
@@ -2519,10 +2706,10 @@ __global__ void k_bonds32(ObjDev P, BondDev Bd)
     if (k >= Bd.n) return;
     double* E = Bd.energy + 6ll * k;
     float* O = reinterpret_cast<float*>(Bd.out) + 9ll * k;
-    for (int t = 0; t < 9; ++t) O[t] = 0.f;
     if (Bd.rec_active) Bd.rec_active[k] = Bd.active[k] != 0;
     if (Bd.active[k] == 0) {
         for (int t = 0; t < 6; ++t) E[t] = 0.;
+        for (int t = 0; t < 9; ++t) O[t] = 0;
         return;
     }
     const int i = Bd.master[k], j = Bd.slave[k];
@@ -2597,56 +2784,517 @@ struct ReduceArgs {
 
 // Real = double: FP64 mode; Real = float: mixed mode (pair and bond results
 // stored and summed in single precision)
-template <typename Real>
-__global__ void k_reduce(ReduceArgs r)
+template <typename Real> struct ForceSum {
+    Real F[3] = {0, 0, 0}, T[3] = {0, 0, 0};
+    // one pair or bond result, as the body's own (F, torque) or as the partner's
+    __device__ __forceinline__ void add(const Real* pf, Real sgn, int torque)
+    {
+        F[0] += sgn * pf[0];
+        F[1] += sgn * pf[1];
+        F[2] += sgn * pf[2];
+        T[0] += pf[torque];
+        T[1] += pf[torque + 1];
+        T[2] += pf[torque + 2];
+    }
+    // the pairs the particle owns in one list
+    __device__ __forceinline__ void own(const PairListDev& L, int i)
+    {
+        const int s = L.seg_off[i], c = L.seg_cnt[i];
+        for (int k = s; k < s + c; ++k)
+            if (L.p_hit[k]) add(reinterpret_cast<const Real*>(L.pf) + 9ll * k, Real(1), 3);  // no contact, no sum kept
+    }
+    __device__ __forceinline__ void bonds(const BondDev& B, int i)
+    {
+        const Real* out = reinterpret_cast<const Real*>(B.out);
+        for (int e = B.plist_off[i]; e < B.plist_off[i + 1]; ++e) {
+            const int code = B.plist[e];
+            const Real* o = out + 9ll * (code >> 1);
+            if ((code & 1) == 0) add(o, Real(1), 3);
+            else add(o, Real(-1), 6);
+        }
+    }
+};
+
+// What surrounds a step's detection: the force sums of one step (SUM), its
+// second half kick (BACK), and the next step's first half kick, drift, hash
+// and pair-cache check, walls too (FRONT).  Between two steps all of it is one
+// pass over the bodies; the sums, the copy of the wrapped positions, two
+// kicks, two drifts, two hashes and two checks were a launch each.
+struct AdvanceArgs {
+    ObjDev P, W;
+    GeoSetDev G, GW;
+    FdGrid pgrid, wgrid;
+    ReduceArgs r;             // SUM
+    const double3* wrapped;   // the positions after the periodic wraps (null: P.pos)
+    double3 gravity;
+    double h, dt;
+    unsigned int* build;      // FRONT: the cell table's build numbers, renewed for
+    int par;                  // a step of this list generation
+    PairCacheDev pc;
+    int cached;
+    int* occ[6];              // occupied-cell boxes of the image tables, reset
+};
+template <typename Real, bool SUM, bool BACK, bool FRONT>
+__global__ void __launch_bounds__(128) k_advance(AdvanceArgs a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= r.P.n) return;
-    Real F[3] = {0, 0, 0}, T[3] = {0, 0, 0};
-    auto add = [](Real* acc, const Real* v, Real sgn) {
-        acc[0] += sgn * v[0];
-        acc[1] += sgn * v[1];
-        acc[2] += sgn * v[2];
-    };
-    // pairs the particle owns, kind by kind
-    for (int kind = 0; kind < FD_NKIND; ++kind) {
-        if (!r.active[kind]) continue;
-        const PairListDev& L = r.L[kind];
-        const Real* pfa = reinterpret_cast<const Real*>(L.pf);
-        const int s = L.seg_off[i], c = L.seg_cnt[i];
-        for (int k = s; k < s + c; ++k) {
-            if (L.c_cnt[k] == 0) continue;  // no contact slot, no sum kept
-            const Real* pf = pfa + 9ll * k;
-            add(F, pf, Real(1));
-            add(T, pf + 3, Real(1));
+    if (FRONT && i < 36 && a.occ[i / 6]) a.occ[i / 6][i % 6] = i % 6 < 3 ? 0x7f7f7f7f : -1;
+    if (FRONT && i == 0) bump_build(a.build, a.par);
+    if (i < a.P.n) {
+        double3 F, T;
+        if (SUM) {
+            const ReduceArgs& r = a.r;
+            ForceSum<Real> f;
+            // pairs the particle owns, kind by kind
+            for (int kind = 0; kind < FD_NKIND; ++kind)
+                if (r.active[kind]) f.own(r.L[kind], i);
+            // pairs in which it is the partner, by owner
+            const int rs = r.R.off[i], rc = min(r.R.cnt[i], r.R.cap - rs);
+            for (int e = rs; e < rs + rc; ++e) {
+                const int code = r.R.code[e];
+                const int kind = code & 7, k = code >> 3;
+                const PairListDev& L = r.L[kind];
+                if (!L.p_hit[k]) continue;
+                if (kind != FD_PP && L.pairA[k] == i) continue;  // a particle against its own ghost
+                f.add(reinterpret_cast<const Real*>(L.pf) + 9ll * k, Real(-1), 6);
+            }
+            if (r.B.n > 0) f.bonds(r.B, i);
+            F = mk3((double)f.F[0], (double)f.F[1], (double)f.F[2]);
+            T = mk3((double)f.T[0], (double)f.T[1], (double)f.T[2]);
+            a.P.force[i] = F;
+            a.P.torque[i] = T;
+            if (!FRONT && a.wrapped) a.P.pos[i] = a.wrapped[i];
+        } else {
+            F = a.P.force[i];
+            T = a.P.torque[i];
+        }
+        if (!BACK && !FRONT) return;
+        Body b;
+        b.v = a.P.vel[i];
+        b.w = a.P.angvel[i];
+        b.q = a.P.q[i];
+        const FdGeo& geo = a.G.geo[a.P.geo[i]];
+        if (BACK) kick_body(b, geo, F, T, a.gravity, a.h);
+        if (FRONT) {
+            b.x = SUM && a.wrapped ? a.wrapped[i] : a.P.pos[i];
+            kick_body(b, geo, F, T, a.gravity, a.h);
+            drift_body(b, a.dt);
+            a.P.pos[i] = b.x;
+            a.P.q[i] = b.q;
+            const long long hash = hash_one(a.P, a.pgrid, i, b.x, b.q);
+            if (a.cached) cache_check(a.pc, i, b.x, b.q, hash >= 0);
+        }
+        a.P.vel[i] = b.v;
+        a.P.angvel[i] = b.w;
+    } else if (FRONT && i - a.P.n < a.W.n) {
+        const int w = i - a.P.n;
+        Body b{a.W.pos[w], a.W.vel[w], a.W.angvel[w], a.W.q[w]};
+        drift_body(b, a.dt);
+        a.W.pos[w] = b.x;
+        a.W.q[w] = b.q;
+        const long long hash = hash_one(a.W, a.wgrid, w, b.x, b.q);
+        if (a.cached) cache_check_wall(a.pc, w, b.x, b.q, hash, a.GW.geo[a.W.geo[w]].grid_radius);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Small sets (no neighbour list, no pair cache, no images).  A step of the
+// staged kernels is 24 dependent launches, each a few microseconds of latency
+// and next to no work at these sizes: 102 us a step for 1,000 particles in a
+// graph replay.  Here a step is two launches.  k_small_pairs takes each
+// particle's partners and walls from the cell lists, and each candidate pair
+// through culling, predicate, contact law and pair sum in one warp;
+// k_small_advance sums each particle's pairs and runs the half kicks, the drift, the hash
+// and the cell lists of the next step.  The sums run in the staged kernels'
+// order, so the results are theirs.  A warp keeps only its pair's few slots
+// busy in the contact law, so large sets stay with the staged kernels.
+// ---------------------------------------------------------------------------
+constexpr int SMALL_BODIES = 4;               // particles per block
+constexpr int SMALL_WARPS = 2 * SMALL_BODIES;  // a warp for each one's partners, one for its walls
+constexpr int MAX_FOUND = 512;                // objects of the cells around a particle, staged for the test
+
+struct SmallArgs {
+    NarrowArgs n;          // n.L, n.a.rec: the particle-particle list
+    PairListDev Lw;        // the particle-wall list
+    AdjRec recw;
+    CellTableDev T;
+    const int2* wall_range;
+    int* r_head;           // per particle: the last pair with a contact it is the partner of
+    void* own;             // per particle: force and torque of its own pairs (6 Real)
+};
+
+// one pair of list L, one warp: slots, predicate, law, pair sum; returns its
+// contacts
+template <int KIND, bool MIXED>
+__device__ __forceinline__ int small_pair(const SmallArgs& a, const PairListDev& L, const AdjRec& R, int p, int A,
+                                          int B, int lane, unsigned short* queue, unsigned long long* stats)
+{
+    using Real = typename std::conditional<MIXED, float, double>::type;
+    const NarrowArgs& n = a.n;
+    const unsigned int full = 0xffffffffu;
+    int kept;
+    int ncand = cull_pair<KIND>(n, A, B, 0.0, lane, queue, kept);
+    if (n.a.stats && lane == 0) {
+        atomicAdd(&stats[0], 1ull);
+        atomicAdd(&stats[1], (unsigned long long)min(n.G.geo[n.P.geo[A]].clus_count, MAX_CLUSTERS));
+        atomicAdd(&stats[2], (unsigned long long)kept);
+        atomicAdd(&stats[4], (unsigned long long)ncand);
+    }
+    if (ncand == 0) {
+        if (lane == 0) {
+            L.c_off[p] = 0;
+            L.c_cnt[p] = 0;
+        }
+        return 0;
+    }
+    int base = 0;
+    if (lane == 0) base = atomicAdd(L.n_slots, ncand);
+    int oc_off, oc_cnt;
+    find_history(L, A, B, lane, oc_off, oc_cnt);
+    base = __shfl_sync(full, base, 0);
+    if (base + ncand > L.cap_contacts) {
+        if (lane == 0) set_flag(n.a.flags, FD_FLAG_CONTACT_OVERFLOW);
+        base = 0;
+        ncand = 0;
+    }
+    if (lane == 0) {
+        L.c_off[p] = base;
+        L.c_cnt[p] = ncand;
+    }
+    int3 bcell;
+    decode_cell(Slave<KIND>::hash(n, B), Slave<KIND>::grid(n).size, bcell);
+    Real acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    int hits = 0;
+    for (int i0 = 0; i0 < ncand; i0 += 32) {
+        const int i = i0 + lane, s = base + i;
+        Real o[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        bool hit = false;
+        if (i < ncand) {
+            const int k = queue[i];
+            int nid = -1;
+            if (MIXED) {
+                SlotEval32 e;
+                hit = slot_predicate32<KIND>(n, A, B, k, bcell, 0.f, e);
+                if (hit)
+                    nid = contact_law32<KIND>(n, L, R, s, A, B, k, oc_off, oc_cnt, e, reinterpret_cast<float*>(o));
+            } else {
+                SlotEval e;
+                hit = slot_predicate<KIND>(n, A, B, k, bcell, 0., e);
+                if (hit)
+                    nid = contact_law<KIND>(n, L, R, s, A, B, k, oc_off, oc_cnt, e, reinterpret_cast<double*>(o));
+            }
+            L.c_k[s] = k;
+            L.c_node[s] = nid;
+            if (R.hit && s < R.cap) R.hit[s] = hit ? 1 : 0;
+        }
+        const unsigned int m = __ballot_sync(full, hit);
+        hits += __popc(m);
+        if (m == 0) continue;
+        // k_pair_sum's order: lane l of eight adds slots l, l + 8, ... in turn
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int src = (lane & 7) + 8 * u;
+            const bool on = (m >> src) & 1u;
+#pragma unroll
+            for (int t = 0; t < 9; ++t) {
+                const Real v = __shfl_sync(full, o[t], src);
+                if (on) acc[t] += v;
+            }
         }
     }
-    // pairs in which it is the partner, by owner
-    {
-        const int rs = r.R.off[i], rc = min(r.R.cnt[i], r.R.cap - rs);
-        for (int e = rs; e < rs + rc; ++e) {
-            const int code = r.R.code[e];
-            const int kind = code & 7, k = code >> 3;
-            const PairListDev& L = r.L[kind];
-            if (kind != FD_PP && L.pairA[k] == i) continue;  // a particle against its own ghost
-            if (L.c_cnt[k] == 0) continue;
-            const Real* pf = reinterpret_cast<const Real*>(L.pf) + 9ll * k;
-            add(F, pf, Real(-1));
-            add(T, pf + 6, Real(1));
+    // a pair without a contact sums to zero: nobody reads it
+    if (hits == 0) return 0;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+        acc[t] += __shfl_xor_sync(full, acc[t], 4);
+        acc[t] += __shfl_xor_sync(full, acc[t], 2);
+        acc[t] += __shfl_xor_sync(full, acc[t], 1);
+    }
+    Real* out = reinterpret_cast<Real*>(L.pf) + 9ll * p;
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+        if (lane == t) out[t] = acc[t];
+    if (lane == 0) {
+        atomicAdd(L.n_hits, hits);
+        if (KIND == FD_PP) L.r_next[p] = atomicExch(&a.r_head[B], p);
+        if (n.a.stats) atomicAdd(&stats[3], (unsigned long long)hits);
+    }
+    return hits;
+}
+
+// the pairs of particle A with the partners in list[0 .. cnt - 1], one warp:
+// ascending partners, and a task for each; range: the tasks' first and count
+__device__ __forceinline__ void small_emit(const PairListDev& L, unsigned int* flags, int A, const int* list, int cnt,
+                                           int kind, int lane, int4* task, int* ntask, int2* range)
+{
+    const unsigned int full = 0xffffffffu;
+    if (cnt > MAX_CAND && lane == 0) set_flag(flags, FD_FLAG_NEIGHBOR_OVERFLOW);
+    int n = min(cnt, MAX_CAND);
+    int base = 0, t0 = 0;
+    if (lane == 0 && n > 0) {
+        base = atomicAdd(L.n_pairs, n);
+        if (base + n > L.cap_pairs) {
+            set_flag(flags, FD_FLAG_PAIR_OVERFLOW);
+            n = 0;
+        } else {
+            t0 = atomicAdd(ntask, n);
         }
     }
-    if (r.B.n > 0) {
-        const Real* out = reinterpret_cast<const Real*>(r.B.out);
-        for (int e = r.B.plist_off[i]; e < r.B.plist_off[i + 1]; ++e) {
-            const int code = r.B.plist[e];
-            const int b = code >> 1, side = code & 1;
-            const Real* o = out + 9ll * b;
-            if (side == 0) { add(F, o, Real(1)); add(T, o + 3, Real(1)); }
-            else { add(F, o, Real(-1)); add(T, o + 6, Real(1)); }
+    n = __shfl_sync(full, n, 0);
+    base = __shfl_sync(full, base, 0);
+    t0 = __shfl_sync(full, t0, 0);
+    if (lane == 0) {
+        L.seg_off[A] = n > 0 ? base : 0;
+        L.seg_cnt[A] = n;
+        *range = make_int2(t0, n);
+    }
+    for (int e = lane; e < n; e += 32) {
+        const int v = list[e];
+        int r = 0;
+        for (int j = 0; j < n; ++j) r += (list[j] < v);
+        L.pairA[base + r] = A;
+        L.pairB[base + r] = v;
+        task[t0 + r] = make_int4(A, v, base + r, kind);
+    }
+    __syncwarp();
+}
+
+template <bool MIXED>
+__global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small_pairs(SmallArgs a)
+{
+    using Real = typename std::conditional<MIXED, float, double>::type;
+    // the candidate lists and the node queues are not in use together
+    __shared__ union {
+        unsigned short queue[SMALL_WARPS][MAX_NODE_QUEUE];
+        int found[SMALL_BODIES][MAX_FOUND];
+    } u;
+    __shared__ int s_list[SMALL_WARPS][MAX_CAND];
+    __shared__ int4 s_task[SMALL_WARPS * MAX_CAND];
+    __shared__ unsigned char s_hit[SMALL_WARPS * MAX_CAND];
+    __shared__ int2 s_range[SMALL_WARPS];
+    __shared__ int s_ntask;
+    __shared__ unsigned long long s_stats[5];
+    const NarrowArgs& n = a.n;
+    const unsigned int full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int body = wib % SMALL_BODIES;
+    if (threadIdx.x == 0) s_ntask = 0;
+    if (threadIdx.x < 5) s_stats[threadIdx.x] = 0ull;
+    if (threadIdx.x < SMALL_WARPS) s_range[threadIdx.x] = make_int2(0, 0);
+    __syncthreads();
+    const CellTableDev& T = a.T;
+    const unsigned int build = T.build[T.par];
+    // the other generation's step needs a number no head can hold
+    if (blockIdx.x == 0 && threadIdx.x == 0) T.build[T.par ^ 1] = build + 1u;
+    const int A = blockIdx.x * SMALL_BODIES + body;
+    if (A < n.P.n) {
+        const double3 cA = n.P.pos[A];
+        const double rA = n.G.geo[n.P.geo[A]].radius;
+        int* list = s_list[wib];
+        int cnt = 0;
+        int3 lo, hi;
+        if (wib < SMALL_BODIES) {
+            // partners: each lane walks the list of a cell, and the objects
+            // found are tested side by side (a test is a chain of five loads)
+            int* found = u.found[body];
+            partner_search_range(cA, (rA + n.G.rmax) * (1.0 + 8.0 * BOUND_REL), T.g, lo, hi);
+            const int nx = hi.x - lo.x + 1, ny = hi.y - lo.y + 1, nz = hi.z - lo.z + 1;
+            const int ncell = nx * ny * nz;
+            int nf = 0;
+            auto test = [&] {
+                __syncwarp();
+                for (int f0 = 0; f0 < nf; f0 += 32) {
+                    bool pass = false;
+                    int B = -1;
+                    if (f0 + lane < nf) {
+                        B = found[f0 + lane];
+                        const FdGeo& GB = n.G.geo[n.P.geo[B]];
+                        const double3 cB = n.P.pos[B];
+                        const double rs = rA + GB.radius;
+                        if (lengthSq3(cA - cB) <= rs * rs * (1.0 + 4.0 * BOUND_REL))
+                            pass = !body_culled32(cA, rA, cB, n.P.rot + 3ll * B, true, GB, n.G, n.a.probe);
+                    }
+                    const unsigned int m = __ballot_sync(full, pass);
+                    if (pass) {
+                        const int at = cnt + __popc(m & ((1u << lane) - 1u));
+                        if (at < MAX_CAND) list[at] = B;
+                    }
+                    cnt += __popc(m);
+                }
+                nf = 0;
+                __syncwarp();
+            };
+            for (int c0 = 0; c0 < ncell; c0 += 32) {
+                const int ci = c0 + lane;
+                int B = -1;
+                if (ci < ncell)
+                    B = cell_first(T, fd_lin3(lo.x + ci % nx, lo.y + (ci / nx) % ny, lo.z + ci / (nx * ny), T.g.size),
+                                   build);
+                while (__any_sync(full, B >= 0)) {
+                    const unsigned int m = __ballot_sync(full, B > A);
+                    if (nf + __popc(m) > MAX_FOUND) test();
+                    if (B > A) found[nf + __popc(m & ((1u << lane) - 1u))] = B;
+                    nf += __popc(m);
+                    if (B >= 0) B = T.next[B];
+                }
+            }
+            test();
+            small_emit(n.L, n.a.flags, A, list, cnt, FD_PP, lane, s_task, &s_ntask, &s_range[wib]);
+        } else {
+            body_search_range(cA, rA * (1.0 + BOUND_REL), n.wgrid, lo, hi);
+            const int2 wr = a.wall_range ? a.wall_range[A] : make_int2(0, n.W.n);
+            const int wend = min(wr.x + wr.y, n.W.n);
+            for (int w0 = max(wr.x, 0); w0 < wend; w0 += 32) {
+                const int w = w0 + lane;
+                bool pass = false;
+                const long long h = w < wend ? n.W.hash[w] : -1;
+                if (h >= 0 && h < n.wgrid.num) {
+                    int3 c;
+                    decode_cell(h, n.wgrid.size, c);
+                    if (c.x >= lo.x && c.x <= hi.x && c.y >= lo.y && c.y <= hi.y && c.z >= lo.z && c.z <= hi.z) {
+                        const FdGeo& GB = n.GW.geo[n.W.geo[w]];
+                        const double rs = rA + GB.grid_radius;
+                        const double3 cW = n.W.pos[w];
+                        pass = lengthSq3(cA - cW) <= rs * rs * (1.0 + 4.0 * BOUND_REL) &&
+                               !body_culled32(cA, rA, cW, n.W.rot + 3ll * w, false, GB, n.GW, n.a.probe);
+                    }
+                }
+                const unsigned int m = __ballot_sync(full, pass);
+                if (pass) {
+                    const int at = cnt + __popc(m & ((1u << lane) - 1u));
+                    if (at < MAX_CAND) list[at] = w;
+                }
+                cnt += __popc(m);
+            }
+            __syncwarp();
+            small_emit(a.Lw, n.a.flags, A, list, cnt, FD_PW, lane, s_task, &s_ntask, &s_range[wib]);
         }
     }
-    r.P.force[i] = mk3((double)F[0], (double)F[1], (double)F[2]);
-    r.P.torque[i] = mk3((double)T[0], (double)T[1], (double)T[2]);
+    __syncthreads();
+    // the block's pairs, shared out over its warps
+    for (int t = wib; t < s_ntask; t += SMALL_WARPS) {
+        const int4 k = s_task[t];
+        const int hits =
+            k.w == FD_PP ? small_pair<FD_PP, MIXED>(a, n.L, n.a.rec, k.z, k.x, k.y, lane, u.queue[wib], s_stats)
+                         : small_pair<FD_PW, MIXED>(a, a.Lw, a.recw, k.z, k.x, k.y, lane, u.queue[wib], s_stats);
+        if (lane == 0) s_hit[t] = hits > 0;
+        __syncwarp();
+    }
+    __syncthreads();
+    // each particle's own pairs, partners then walls, in order: lane t < 3 sums
+    // the force, lane 3 <= t < 6 the torque
+    if (wib < SMALL_BODIES && A < n.P.n && lane < 6) {
+        Real acc = 0;
+        for (int w = 0; w < 2; ++w) {
+            const int2 r = s_range[body + w * SMALL_BODIES];
+            const Real* pf = reinterpret_cast<const Real*>(w ? a.Lw.pf : n.L.pf);
+            for (int t = r.x; t < r.x + r.y; ++t)
+                if (s_hit[t]) acc += pf[9ll * s_task[t].z + lane];
+        }
+        reinterpret_cast<Real*>(a.own)[6ll * A + lane] = acc;
+    }
+    if (n.a.stats && threadIdx.x < 5 && s_stats[threadIdx.x])
+        atomicAdd(&n.a.stats[threadIdx.x], s_stats[threadIdx.x]);
+}
+
+struct SmallAdvanceArgs {
+    ObjDev P, W;
+    GeoSetDev G;
+    FdGrid pgrid, wgrid;
+    PairListDev Lp;        // the step's particle-particle list
+    BondDev B;
+    CellTableDev T;        // the next step's table
+    int* r_head;           // see SmallArgs
+    const void* own;
+    int* zero[2];          // counters of the next step's lists (three each)
+    double3 gravity;
+    double h, dt;
+};
+
+// the particle's pairs as a partner, by owner; its list is emptied
+template <typename Real>
+__device__ __forceinline__ void small_partner_sum(const SmallAdvanceArgs& a, int i, ForceSum<Real>& f)
+{
+    constexpr int LOCAL = 16;
+    const PairListDev& L = a.Lp;
+    const int head = a.r_head[i];
+    if (head < 0) return;
+    a.r_head[i] = -1;
+    int pair[LOCAL], owner[LOCAL], cnt = 0;
+    for (int p = head; p >= 0; p = L.r_next[p], ++cnt) {
+        if (cnt >= LOCAL) continue;
+        const int own = L.pairA[p];
+        int b = cnt - 1;
+        while (b >= 0 && owner[b] > own) { owner[b + 1] = owner[b]; pair[b + 1] = pair[b]; --b; }
+        owner[b + 1] = own;
+        pair[b + 1] = p;
+    }
+    const Real* pf = reinterpret_cast<const Real*>(L.pf);
+    if (cnt <= LOCAL) {
+        for (int e = 0; e < cnt; ++e) f.add(pf + 9ll * pair[e], Real(-1), 6);
+        return;
+    }
+    // a body with many owners: the next owner in order by a pass over the list
+    int last = -1;
+    for (int e = 0; e < cnt; ++e) {
+        int best = 0x7fffffff, at = head;
+        for (int p = head; p >= 0; p = L.r_next[p]) {
+            const int own = L.pairA[p];
+            if (own > last && own < best) { best = own; at = p; }
+        }
+        last = best;
+        f.add(pf + 9ll * at, Real(-1), 6);
+    }
+}
+
+// SUM: the step's forces; BACK: its second half kick; FRONT: the next step's
+// first half kick, drift, hash and cell lists
+template <typename Real, bool SUM, bool BACK, bool FRONT>
+__global__ void __launch_bounds__(64) k_small_advance(SmallAdvanceArgs a)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (FRONT && i < 6) a.zero[i / 3][i % 3] = 0;
+    if (i < a.P.n) {
+        double3 F, T;
+        if (SUM) {
+            ForceSum<Real> f;
+            const Real* own = reinterpret_cast<const Real*>(a.own) + 6ll * i;
+            for (int t = 0; t < 3; ++t) {
+                f.F[t] = own[t];
+                f.T[t] = own[3 + t];
+            }
+            small_partner_sum(a, i, f);
+            if (a.B.n > 0) f.bonds(a.B, i);
+            F = mk3((double)f.F[0], (double)f.F[1], (double)f.F[2]);
+            T = mk3((double)f.T[0], (double)f.T[1], (double)f.T[2]);
+            a.P.force[i] = F;
+            a.P.torque[i] = T;
+        } else {
+            F = a.P.force[i];
+            T = a.P.torque[i];
+        }
+        if (!BACK && !FRONT) return;
+        Body b{a.P.pos[i], a.P.vel[i], a.P.angvel[i], a.P.q[i]};
+        const FdGeo& geo = a.G.geo[a.P.geo[i]];
+        if (BACK) kick_body(b, geo, F, T, a.gravity, a.h);
+        if (FRONT) {
+            kick_body(b, geo, F, T, a.gravity, a.h);
+            drift_body(b, a.dt);
+            a.P.pos[i] = b.x;
+            a.P.q[i] = b.q;
+            const long long h = hash_one(a.P, a.pgrid, i, b.x, b.q);
+            if (h >= 0 && h < a.T.g.num) cell_push(a.T, (unsigned long long)h, a.T.build[a.T.par], i);
+        }
+        a.P.vel[i] = b.v;
+        a.P.angvel[i] = b.w;
+    } else if (FRONT && i - a.P.n < a.W.n) {
+        const int w = i - a.P.n;
+        Body b{a.W.pos[w], a.W.vel[w], a.W.angvel[w], a.W.q[w]};
+        drift_body(b, a.dt);
+        a.W.pos[w] = b.x;
+        a.W.q[w] = b.q;
+        hash_one(a.W, a.wgrid, w, b.x, b.q);
+    }
 }
 
 }  // namespace
@@ -2743,18 +3391,6 @@ void scan_inclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t
     k_scan_add<<<(unsigned)tiles, SCAN_TPB, 0, s>>>(out, n, sums, nullptr); note_launch();
 }
 
-void launch_kick(const ObjDev& P, const GeoSetDev& G, double3 gravity, double h, cudaStream_t s)
-{
-    if (P.n > 0) { k_kick<<<nblocks(P.n), TPB, 0, s>>>(P, G, gravity, h); note_launch(); }
-}
-void launch_drift(const ObjDev& O, double dt, cudaStream_t s)
-{
-    if (O.n > 0) { k_drift<<<nblocks(O.n), TPB, 0, s>>>(O, dt); note_launch(); }
-}
-void launch_kick_drift(const ObjDev& P, const GeoSetDev& G, double3 gravity, double h, double dt, cudaStream_t s)
-{
-    if (P.n > 0) { k_kick_drift<<<nblocks(P.n), TPB, 0, s>>>(P, G, gravity, h, dt); note_launch(); }
-}
 void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s, unsigned int* build, int par)
 {
     if (O.n > 0) { k_hash<<<nblocks(O.n), TPB, 0, s>>>(O, g, build, par); note_launch(); }
@@ -2789,30 +3425,17 @@ void radix_sort_keys(const long long* keys, int n, long long num_keys, unsigned 
         src ^= 1;
     }
 }
-void launch_cell_table(const ObjDev& O, const CellTableDev& T, cudaStream_t s, const int* gate)
+void launch_images(const ObjDev& P, double3* dst, const GhostDev* gh, const int* on, double ext_skin, int* ctrl,
+                   cudaStream_t s)
 {
-    if (O.n <= 0) return;
-    if (T.hashed) {
-        k_hkey_clear<<<nblocks((long long)T.hmask + 1), TPB, 0, s>>>(T.hkey, T.hmask + 1, gate);
-        note_launch();
-    }
-    k_cell_link<<<nblocks(O.n), TPB, 0, s>>>(O.hash, O.n, T, gate); note_launch();
+    if (P.n <= 0) return;
+    ImageArgs a{P, dst, {gh[0], gh[1], gh[2]}, {on[0], on[1], on[2]}, ext_skin, ctrl};
+    k_images<<<nblocks(P.n), TPB, 0, s>>>(a); note_launch();
 }
-void launch_wrap(ObjDev& P, const FdGrid& g, int dim, cudaStream_t s, int* ctrl, const double3* src)
+void reset_image_box(int* occ, cudaStream_t s)
 {
-    if (P.n > 0) { k_wrap<<<nblocks(P.n), TPB, 0, s>>>(P, g, dim, ctrl, src); note_launch(); }
-}
-void launch_ghost_build(const ObjDev& P, GhostDev& Gh, int kind, cudaStream_t s, double ext_skin, int* ctrl)
-{
-    // occupied-cell box of the ghost images: empty until the build fills it
-    cudaMemsetAsync(Gh.occ, 0x7f, 3 * sizeof(int), s);
-    cudaMemsetAsync(Gh.occ + 3, 0xff, 3 * sizeof(int), s);
-    if (P.n > 0) { k_ghost_build<<<nblocks(P.n), TPB, 0, s>>>(P, Gh, kind, ext_skin, ctrl); note_launch(); }
-}
-void launch_ghost_gate(int* ctrl, cudaStream_t s)
-{
-    k_ghost_gate<<<1, 1, 0, s>>>(ctrl);
-    note_launch();
+    cudaMemsetAsync(occ, 0x7f, 3 * sizeof(int), s);
+    cudaMemsetAsync(occ + 3, 0xff, 3 * sizeof(int), s);
 }
 void launch_sector_wrap(ObjDev& P, const FdGrid& g, cudaStream_t s)
 {
@@ -2820,176 +3443,213 @@ void launch_sector_wrap(ObjDev& P, const FdGrid& g, cudaStream_t s)
 }
 void launch_sector_images(const ObjDev& P, GhostDev* R, cudaStream_t s)
 {
-    for (int d = 0; d < 3; ++d) {
-        cudaMemsetAsync(R[d].occ, 0x7f, 3 * sizeof(int), s);
-        cudaMemsetAsync(R[d].occ + 3, 0xff, 3 * sizeof(int), s);
-    }
     if (P.n > 0) { k_sector_images<<<nblocks(P.n), TPB, 0, s>>>(P, R[0], R[1], R[2]); note_launch(); }
 }
 
-void launch_broad_pp(const ObjDev& P, const GeoSetDev& G, const CellTableDev& T, PairListDev& L,
-                     unsigned int* flags, double probe, cudaStream_t s, double skin, const int* gate)
+namespace {
+// kernel arguments of a set of lists, with blocks[k] blocks for list k
+ListSet list_set(const ListArgs* lists, int n, const StepShared& c, const int* blocks)
 {
-    cudaMemsetAsync(L.n_pairs, 0, sizeof(int), s);
-    if (P.n > 0) {
-        k_broad_cells<false, false, false><<<nblocks((long long)P.n * BROAD_LANES), TPB, 0, s>>>(
-            P, G, T, nullptr, nullptr, nullptr, nullptr, nullptr, L, NlDev{}, flags, probe, skin, gate, nullptr);
+    ListSet a;
+    a.n = n;
+    a.T = c.T;
+    a.wall_range = c.wall_range;
+    a.rev_total = c.with_force ? c.R.total : nullptr;
+    a.spacing_margin = c.mixed ? 1e-4f : 0.f;
+    int b = 0;
+    for (int k = 0; k < n; ++k) {
+        NarrowArgs& m = a.l[k];
+        m.P = lists[k].P; m.G = c.G; m.M = c.M; m.W = c.W; m.GW = c.GW; m.MW = c.MW;
+        m.pgrid = c.pgrid; m.wgrid = c.wgrid; m.gh = lists[k].gh; m.L = lists[k].L; m.a = lists[k].a;
+        m.with_force = c.with_force;
+        a.kind[k] = lists[k].kind;
+        a.block0[k] = b;
+        b += blocks[k];
+    }
+    a.block0[n] = b;
+    return a;
+}
+}  // namespace
+
+void launch_broad(const ListArgs* lists, int n, const StepShared& c, NlDev* nl, cudaStream_t s)
+{
+    if (n <= 0 || c.n <= 0) return;
+    int blocks[FD_NKIND];
+    // sparse tables: the keys of the lists that are built are cleared first
+    for (int k = 0; k < n; ++k) {
+        if (lists[k].kind == FD_PW) continue;
+        const CellTableDev& T = lists[k].kind == FD_PP ? c.T : lists[k].gh.cells;
+        if (!T.hashed) continue;
+        k_hkey_clear<<<nblocks((long long)T.hmask + 1), TPB, 0, s>>>(T.hkey, T.hmask + 1, lists[k].a);
         note_launch();
     }
-}
-void launch_broad_pp_nl(const ObjDev& P, const GeoSetDev& G, const CellTableDev& T, PairListDev& L, NlDev& nl,
-                        unsigned int* flags, double probe, cudaStream_t s, const int* gate)
-{
-    cudaMemsetAsync(L.n_pairs, 0, sizeof(int), s);
-    if (P.n <= 0) return;
-    k_nl_check<<<nblocks(P.n), TPB, 0, s>>>(P, nl, T.g, gate); note_launch();
-    k_broad_cells<false, false, true><<<nblocks((long long)P.n * BROAD_LANES), TPB, 0, s>>>(
-        P, G, T, nullptr, nullptr, nullptr, nullptr, nullptr, L, nl, flags, probe, 0.0, gate, nullptr);
-    note_launch();
-    k_nl_filter<<<nblocks((long long)P.n * 8), TPB, 0, s>>>(P, G, L, nl, flags, probe, gate); note_launch();
-}
-void launch_pair_cache_check(const ObjDev& P, const PairCacheDev& c, cudaStream_t s)
-{
-    if (P.n > 0) { k_pc_check<<<nblocks(P.n), TPB, 0, s>>>(P, c); note_launch(); }
-}
-void launch_pair_cache_commit(const ObjDev& P, const PairCacheDev& c, const PairListDev& L, cudaStream_t s)
-{
-    if (P.n > 0) { k_pc_commit<<<nblocks(P.n), TPB, 0, s>>>(P, c, L); note_launch(); }
-}
-void launch_pair_cache_end(const PairCacheDev& c, const PairListDev* lists, int n_lists, cudaStream_t s)
-{
-    CachedCounts gc{};
-    gc.n = std::min(n_lists, 4);
-    for (int k = 0; k < gc.n; ++k) {
-        gc.n_pairs[k] = lists[k].n_pairs;
-        gc.n_slots[k] = lists[k].n_slots;
-        gc.cap_pairs[k] = lists[k].cap_pairs;
-        gc.cap_contacts[k] = lists[k].cap_contacts;
-    }
-    k_pc_end<<<1, 1, 0, s>>>(c.ctrl, gc);
-    note_launch();
-}
-
-void launch_broad_pw(const ObjDev& P, const GeoSetDev& G, const ObjDev& W, const GeoSetDev& GW,
-                     const FdGrid& wg, PairListDev& L, unsigned int* flags, double probe, cudaStream_t s,
-                     const int2* wall_range, double skin, const int* gate)
-{
-    cudaMemsetAsync(L.n_pairs, 0, sizeof(int), s);
-    if (P.n > 0) {
-        k_broad_pw<<<nblocks(P.n), TPB, 0, s>>>(P, G, W, GW, wg, L, flags, probe, wall_range, skin, gate);
-        note_launch();
-    }
-}
-void launch_pair_cache_check_walls(const ObjDev& W, const GeoSetDev& GW, const PairCacheDev& c, cudaStream_t s)
-{
-    if (W.n > 0) { k_pc_check_walls<<<nblocks(W.n), TPB, 0, s>>>(W, GW, c); note_launch(); }
-}
-void launch_pair_cache_commit_walls(const ObjDev& W, const PairCacheDev& c, cudaStream_t s)
-{
-    if (W.n > 0) { k_pc_commit_walls<<<nblocks(W.n), TPB, 0, s>>>(W, c); note_launch(); }
-}
-void launch_broad_ghost(const ObjDev& P, const GeoSetDev& G, const GhostDev& Gh, PairListDev& L,
-                        unsigned int* flags, double probe, cudaStream_t s, double skin, const int* gate,
-                        const int* noskin)
-{
-    cudaMemsetAsync(L.n_pairs, 0, sizeof(int), s);
-    if (P.n <= 0) return;
-    cudaMemsetAsync(Gh.nsearch, 0, sizeof(int), s);
-    k_ghost_searchers<<<nblocks(P.n), TPB, 0, s>>>(P, G, Gh.cells.g, Gh.occ, L, Gh.searchers, Gh.nsearch, skin,
-                                                    gate, noskin);
-    note_launch();
-    const long long groups = std::min<long long>(P.n, 148ll * 8 * (TPB / BROAD_LANES));
-    k_broad_cells<true, true, false><<<nblocks(groups * BROAD_LANES), TPB, 0, s>>>(
-        P, G, Gh.cells, Gh.pos, Gh.rot, Gh.occ, Gh.searchers, Gh.nsearch, L, NlDev{}, flags, probe, skin, gate,
-        noskin);
-    note_launch();
-}
-
-void launch_narrow(int kind, const ObjDev& P, const GeoSetDev& G, const MatDev& M, const ObjDev& W,
-                   const GeoSetDev& GW, const MatDev& MW, const FdGrid& pgrid, const FdGrid& wgrid,
-                   const GhostDev* gh, PairListDev& L, const StepArgs& a, int with_force, bool mixed, cudaStream_t s)
-{
-    cudaMemsetAsync(L.n_slots, 0, 2 * sizeof(int), s);  // slots and contacts
-    NarrowArgs n;
-    n.P = P; n.G = G; n.M = M; n.W = W; n.GW = GW; n.MW = MW; n.pgrid = pgrid; n.wgrid = wgrid;
-    if (gh) n.gh = *gh; else memset(&n.gh, 0, sizeof(n.gh));
-    n.L = L; n.a = a; n.with_force = with_force;
-    const long long need = ((long long)L.cap_pairs + NARROW_WARPS - 1) / NARROW_WARPS;
-    // grid-stride kernels sized in blocks per SM (the pair and slot counts
-    // are known only on the device): the defaults fill one resident wave
-    const int sel_bps = a.shape[0] > 0 ? a.shape[0] : FD_SELECT_MIN_BLOCKS;
-    const int grid = (int)std::max(1ll, std::min(need, 148ll * sel_bps));
-    const int pgrid0 = 148 * (a.shape[1] > 0 ? a.shape[1] : FD_PROBE_MIN_BLOCKS);
-    const int cgrid = 148 * (a.shape[2] > 0 ? a.shape[2] : 4);
-    const int sgrid = 148 * (a.shape[3] > 0 ? a.shape[3] : 4);
-#define FD_NARROW_CASE(K)                                                              \
-    case K:                                                                            \
-        k_select<K><<<grid, NARROW_WARPS * 32, 0, s>>>(n); note_launch();                             \
-        if (a.gate) {                                                                  \
-            const bool wall = K == FD_PW;                                              \
-            k_pc_carry<<<148 * 8, TPB, 0, s>>>(                                        \
-                L, P.n, wall ? W.hash : gh ? gh->hash : P.hash, wall ? wgrid : pgrid, a.gate, a.drift, \
-                a.disp, a.driftB ? a.driftB : a.drift, a.dispB ? a.dispB : a.disp,      \
-                wall ? W.geo : P.geo, wall ? GW.geo : G.geo, (mixed && !wall) ? 1e-4f : 0.f);          \
-            note_launch();                                                             \
-            if (K == FD_PP) {                                                          \
-                cudaMemsetAsync(L.n_test, 0, sizeof(int), s);                          \
-                k_slot_filter<<<pgrid0, TPB, 0, s>>>(n);                               \
-                note_launch();                                                         \
-            }                                                                          \
-        }                                                                              \
-        if (mixed) {                                                                   \
-            k_contact32<K, 0><<<pgrid0, TPB, 0, s>>>(n); note_launch();                               \
-            k_contact32<K, 1><<<cgrid, TPB, 0, s>>>(n); note_launch();                                \
-        } else {                                                                       \
-            k_contact<K, 0><<<pgrid0, TPB, 0, s>>>(n); note_launch();                                 \
-            k_contact<K, 1><<<cgrid, TPB, 0, s>>>(n); note_launch();                                  \
-        }                                                                              \
-        break;
-    switch (kind) {
-        FD_NARROW_CASE(FD_PP)
-        FD_NARROW_CASE(FD_PW)
-        FD_NARROW_CASE(FD_GX)
-        FD_NARROW_CASE(FD_GY)
-        FD_NARROW_CASE(FD_GXY)
-    case FD_GR90:
-    case FD_GR180:
-    case FD_GR270:
-        // the sector images differ from the translated ones only in the state
-        // the ghost traits read, so they share the ghost kernels
-        k_select<FD_GX><<<grid, NARROW_WARPS * 32, 0, s>>>(n); note_launch();
-        if (mixed) {
-            k_contact32<FD_GX, 0><<<pgrid0, TPB, 0, s>>>(n); note_launch();
-            k_contact32<FD_GX, 1><<<cgrid, TPB, 0, s>>>(n); note_launch();
-        } else {
-            k_contact<FD_GX, 0><<<pgrid0, TPB, 0, s>>>(n); note_launch();
-            k_contact<FD_GX, 1><<<cgrid, TPB, 0, s>>>(n); note_launch();
+    for (int k = 0; k < n; ++k) blocks[k] = std::min(nblocks(c.n), 148 * 8);
+    ListSet a = list_set(lists, n, c, blocks);
+    k_begin_lists<<<a.block0[n], TPB, 0, s>>>(a); note_launch();
+    if (nl) {
+        // the particle-particle list comes from the neighbour list
+        for (int k = 0; k < n; ++k) {
+            if (lists[k].kind != FD_PP) continue;
+            k_nl_check<<<nblocks(c.n), TPB, 0, s>>>(lists[k].P, *nl, c.T.g); note_launch();
+            k_broad_nl<<<nblocks((long long)c.n * BROAD_LANES), TPB, 0, s>>>(lists[k].P, c.G, c.T, *nl, lists[k].a.flags);
+            note_launch();
+            k_nl_filter<<<nblocks((long long)c.n * 8), TPB, 0, s>>>(lists[k].P, c.G, lists[k].L, *nl, lists[k].a.flags,
+                                                                   lists[k].a.probe);
+            note_launch();
         }
-        break;
     }
-#undef FD_NARROW_CASE
-    if (mixed) {
-        k_pair_sum32<<<sgrid, TPB, 0, s>>>(L, with_force);
-    } else {
-        k_pair_sum<<<sgrid, TPB, 0, s>>>(L, with_force);
+    int total = 0;
+    for (int k = 0; k < n; ++k) {
+        const bool pp = lists[k].kind == FD_PP;
+        blocks[k] = pp && nl ? 0
+                    : lists[k].kind == FD_PW ? std::min(nblocks(c.n), 148 * 4)
+                                             : std::min(nblocks((long long)c.n * BROAD_LANES), 148 * 4);
+        total += blocks[k];
     }
+    if (total == 0) return;
+    a = list_set(lists, n, c, blocks);
+    k_broad_lists<<<total, TPB, 0, s>>>(a); note_launch();
+}
+
+void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream_t s)
+{
+    if (n <= 0 || c.n <= 0) return;
+    // grid-stride kernels sized in blocks per SM (the pair and slot counts are
+    // known only on the device): the particle-particle list's defaults fill
+    // one resident wave; the short wall and image lists come first and get a
+    // quarter of it each, so that they end before the long list does
+    const int* shape = lists[0].a.shape;
+    auto share = [&](int* blocks, int per_sm) {
+        for (int k = 0; k < n; ++k) {
+            const long long need = ((long long)lists[k].L.cap_pairs + NARROW_WARPS - 1) / NARROW_WARPS;
+            const long long most = lists[k].kind == FD_PP || n == 1 ? 148ll * per_sm : 148ll * std::max(per_sm / 4, 1);
+            blocks[k] = (int)std::max(1ll, std::min(need, most));
+        }
+    };
+    int blocks[FD_NKIND];
+    share(blocks, shape[0] > 0 ? shape[0] : FD_SELECT_MIN_BLOCKS);
+    ListSet a = list_set(lists, n, c, blocks);
+    k_select_lists<<<a.block0[n], NARROW_WARPS * 32, 0, s>>>(a); note_launch();
+    const int probe = shape[1] > 0 ? shape[1] : FD_PROBE_MIN_BLOCKS;
+    for (int k = 0; k < n; ++k) {
+        if (lists[k].kind != FD_PP || !lists[k].a.gate) continue;
+        k_slot_filter<<<148 * probe, TPB, 0, s>>>(a.l[k]); note_launch();
+    }
+    share(blocks, probe);
+    a = list_set(lists, n, c, blocks);
+    if (c.mixed) k_contact_lists<true, 0><<<a.block0[n], TPB, 0, s>>>(a);
+    else k_contact_lists<false, 0><<<a.block0[n], TPB, 0, s>>>(a);
+    note_launch();
+    share(blocks, shape[2] > 0 ? shape[2] : 4);
+    a = list_set(lists, n, c, blocks);
+    if (c.mixed) k_contact_lists<true, 1><<<a.block0[n], TPB, 0, s>>>(a);
+    else k_contact_lists<false, 1><<<a.block0[n], TPB, 0, s>>>(a);
+    note_launch();
+    if (!c.with_force) return;
+    share(blocks, shape[3] > 0 ? shape[3] : 4);
+    a = list_set(lists, n, c, blocks);
+    if (c.mixed) k_sum_lists<float><<<a.block0[n], TPB, 0, s>>>(a, c.R);
+    else k_sum_lists<double><<<a.block0[n], TPB, 0, s>>>(a, c.R);
     note_launch();
 }
 
-void launch_reverse(const ObjDev& P, PairListDev* lists, const int* active, const RevDev& R, cudaStream_t s,
-                    const int* gate)
+void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists, const int* active, const RevDev& R,
+                     const PairCacheDev* pc, bool cached_ghosts, unsigned int* done, cudaStream_t s)
 {
     if (P.n <= 0) return;
-    RevArgs r;
-    for (int k = 0; k < REV_LISTS; ++k) {
-        r.L[k] = lists[rev_kind(k)];
-        r.active[k] = active[rev_kind(k)];
+    EndArgs a;
+    a.P = P;
+    a.W = W;
+    for (int k = 0; k < FD_NKIND; ++k) { a.L[k] = lists[k]; a.active[k] = active[k]; }
+    a.R = R;
+    a.cached = pc != nullptr;
+    a.cached_ghosts = cached_ghosts;
+    if (pc) a.pc = *pc; else memset(&a.pc, 0, sizeof(a.pc));
+    a.done = done;
+    k_step_end<<<std::min(nblocks(P.n), 148 * 8), TPB, 0, s>>>(a); note_launch();
+}
+
+void launch_advance(const StepShared& c, const ObjDev& P, const PairListDev* lists, const int* active, const BondDev& B,
+                    const double3* wrapped, double3 gravity, double dt, const PairCacheDev* pc, int* const* occ,
+                    int par, int parts, cudaStream_t s)
+{
+    if (P.n <= 0) return;
+    AdvanceArgs a;
+    a.P = P; a.W = c.W; a.G = c.G; a.GW = c.GW; a.pgrid = c.pgrid; a.wgrid = c.wgrid;
+    a.r.R = c.R;
+    a.r.B = B;
+    for (int k = 0; k < FD_NKIND; ++k) { a.r.L[k] = lists[k]; a.r.active[k] = active[k]; }
+    a.wrapped = wrapped;
+    a.gravity = gravity;
+    a.h = 0.5 * dt;
+    a.dt = dt;
+    a.build = c.T.build;
+    a.par = par;
+    a.cached = pc != nullptr;
+    if (pc) a.pc = *pc; else memset(&a.pc, 0, sizeof(a.pc));
+    for (int d = 0; d < 6; ++d) a.occ[d] = occ[d];
+    const int tpb = 128;
+    const int blocks = std::max(1, nblocks(P.n + ((parts & STEP_FRONT) ? c.W.n : 0), tpb));
+#define FD_ADVANCE(S, K, F)                                                                  \
+    case (S ? STEP_SUM : 0) | (K ? STEP_BACK : 0) | (F ? STEP_FRONT : 0):                    \
+        if (c.mixed) k_advance<float, S, K, F><<<blocks, tpb, 0, s>>>(a);                    \
+        else k_advance<double, S, K, F><<<blocks, tpb, 0, s>>>(a);                           \
+        note_launch();                                                                       \
+        break;
+    switch (parts) {
+        FD_ADVANCE(false, false, true)
+        FD_ADVANCE(false, true, false)
+        FD_ADVANCE(false, true, true)
+        FD_ADVANCE(true, false, false)
+        FD_ADVANCE(true, true, false)
+        FD_ADVANCE(true, true, true)
     }
-    r.R = R;
-    r.n_obj = P.n;
-    r.gate = gate;
-    k_rev_link<<<148 * 8, TPB, 0, s>>>(r); note_launch();
-    k_rev_build<<<nblocks(P.n), TPB, 0, s>>>(r); note_launch();
+#undef FD_ADVANCE
+}
+
+void launch_small_pairs(const ObjDev& P, const GeoSetDev& G, const MatDev& M, const ObjDev& W, const GeoSetDev& GW,
+                        const MatDev& MW, const FdGrid& pgrid, const FdGrid& wgrid, const CellTableDev& T,
+                        const PairListDev& Lp, const PairListDev& Lw, const StepArgs& a, const AdjRec& recw,
+                        const int2* wall_range, int* r_head, void* own, bool mixed, cudaStream_t s)
+{
+    if (P.n <= 0) return;
+    SmallArgs k;
+    NarrowArgs& n = k.n;
+    n.P = P; n.G = G; n.M = M; n.W = W; n.GW = GW; n.MW = MW; n.pgrid = pgrid; n.wgrid = wgrid;
+    memset(&n.gh, 0, sizeof(n.gh));
+    n.L = Lp; n.a = a; n.with_force = 1;
+    k.Lw = Lw; k.recw = recw; k.T = T; k.wall_range = wall_range; k.r_head = r_head;
+    k.own = own;
+    const int blocks = (P.n + SMALL_BODIES - 1) / SMALL_BODIES;
+    if (mixed) k_small_pairs<true><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
+    else k_small_pairs<false><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
+    note_launch();
+}
+
+void launch_small_advance(const ObjDev& P, const GeoSetDev& G, const ObjDev& W, const FdGrid& pgrid,
+                          const FdGrid& wgrid, const PairListDev& Lp, const BondDev& B, const CellTableDev& T,
+                          int* r_head, const void* own, int* zero_p, int* zero_w, double3 gravity, double dt,
+                          bool mixed, int parts, cudaStream_t s)
+{
+    if (P.n <= 0) return;
+    SmallAdvanceArgs a{P, W, G, pgrid, wgrid, Lp, B, T, r_head, own, {zero_p, zero_w}, gravity, 0.5 * dt, dt};
+    // small blocks: the work is a chain of dependent loads per particle, so it
+    // goes to as many SMs as there are
+    const int tpb = 64;
+    const int blocks = std::max(1, (P.n + ((parts & STEP_FRONT) ? W.n : 0) + tpb - 1) / tpb);
+#define FD_ADVANCE(S, K, F)                                                                                    \
+    case (S ? STEP_SUM : 0) | (K ? STEP_BACK : 0) | (F ? STEP_FRONT : 0):                                   \
+        if (mixed) k_small_advance<float, S, K, F><<<blocks, tpb, 0, s>>>(a);                                  \
+        else k_small_advance<double, S, K, F><<<blocks, tpb, 0, s>>>(a);                                       \
+        note_launch();                                                                                         \
+        break;
+    switch (parts) {
+        FD_ADVANCE(false, false, true)
+        FD_ADVANCE(true, false, false)
+        FD_ADVANCE(true, true, false)
+        FD_ADVANCE(true, true, true)
+    }
+#undef FD_ADVANCE
 }
 
 void launch_bonds(const ObjDev& P, BondDev& B, bool mixed, cudaStream_t s)
@@ -3015,23 +3675,6 @@ void launch_contact_view(const PairListDev& L, long long* keys, int* order, unsi
 void launch_bond_view(const BondDev& B, const BondViewDev& v, cudaStream_t s)
 {
     if (B.n > 0) { k_bond_view<<<nblocks(B.n), TPB, 0, s>>>(B, v); note_launch(); }
-}
-
-void launch_reduce(ObjDev& P, PairListDev* lists, const int* active, const RevDev& R, const BondDev& B, bool mixed,
-                   cudaStream_t s)
-{
-    if (P.n <= 0) return;
-    ReduceArgs r;
-    r.P = P;
-    for (int k = 0; k < FD_NKIND; ++k) { r.L[k] = lists[k]; r.active[k] = active[k]; }
-    r.R = R;
-    r.B = B;
-    if (mixed) {
-        k_reduce<float><<<nblocks(P.n), TPB, 0, s>>>(r);
-    } else {
-        k_reduce<double><<<nblocks(P.n), TPB, 0, s>>>(r);
-    }
-    note_launch();
 }
 
 }  // namespace fd

@@ -16,6 +16,10 @@
 #define FD_PROBE_MIN_BLOCKS 4
 #endif
 
+#ifndef FD_SMALL_MIN_BLOCKS
+#define FD_SMALL_MIN_BLOCKS 2
+#endif
+
 namespace fd {
 
 // Everything one simulation keeps on the device.  Plain pointers; ownership
@@ -53,6 +57,7 @@ struct PairListDev {
     int4* p_aux;       // per pair: cell of B (x, y, z), first history slot
     int* p_hist_cnt;   // per pair: history slots
     int* r_next;       // per pair: the next pair (code) of its partner's list
+    int* p_hit;        // per pair: 1 when a slot of it holds a contact
     double* c_spring;  // 3 per contact
     double* c_point;   // 3 per contact (records)
     double* c_normal;  // 3 per contact (records)
@@ -62,12 +67,11 @@ struct PairListDev {
     int* n_slots;      // device counter: slots used
     int* n_hits;       // device counter: contacts (n_slots + 1)
     int cap_contacts;  // slot capacity
-    int* carry_n;      // pair cache: carried steps since the layout was built
     int* c_test;       // pair cache, carried steps: the slots the bound does not
                        // skip, listed for the predicate pass (n_test of them)
     int* n_test;
     float* p_bound;    // pair cache, carried steps: per pair, how far the SDF can
-                       // have moved at a node since the rebuild (k_pc_carry)
+                       // have moved at a node since the rebuild (pair_bound)
     float* c_phi0;     // pair cache: per slot, the node's signed distance to the
                        // partner at the last rebuild (rounded down; -inf when
                        // the predicate stopped before the distance)
@@ -90,6 +94,10 @@ struct RevDev {
     unsigned long long* head;
     int* total;
     const unsigned int* build;  // the step's build number (the particle cell table's)
+    // the index is built when gate is null, or when *gate or *gate2 (may be
+    // null) is not 0: a step whose lists keep their pairs keeps their index
+    const int* gate;
+    const int* gate2;
 };
 
 struct ObjDev {
@@ -155,8 +163,6 @@ struct GhostDev {
     long long* hash;
     CellTableDev cells;
     int* occ;  // box of the cells holding ghost images: min x, y, z, max x, y, z
-    int* searchers;  // particles whose search box reaches a ghost image
-    int* nsearch;    // their count
     // sector images only (null for the translated X/Y images, which share the
     // particle's orientation and velocity): orientation, velocity and the
     // single-precision rotation rows of each image
@@ -229,8 +235,6 @@ struct NlDev {
     int* ctrl;      // [0]: rebuild requested
     double skin;
     int periodic_x, periodic_y;  // distances and displacements by minimum image
-    double pair_skin;   // positional skin of the pair cache (0 without it): the
-                        // list is rebuilt once a particle moved (skin - pair_skin) / 2
 };
 
 // Pair cache of the particle-particle list.  The candidate pairs and the
@@ -251,11 +255,10 @@ struct PairCacheDev {
     int* ref_vis;       // visibility (hashed) at the last build
     // ctrl: [0] rebuild this step, [1] rebuilds so far, [2] the last build
     // overflowed the particle-particle lists, [3] rebuild at the next step,
-    // [4] the translated ghost lists of this step are built without the
-    // cache (a particle wrapped, or an image outside the domain's other
-    // directions), [5] the ghost lists' gate this step ([0] or [4]), [6]
-    // [4] again, as the ghost kernels' skin switch, [7] rebuild requests of
-    // this step, moved to [3] at its end
+    // [4] the translated ghost lists of this step are built, and without the
+    // cache's skin (a particle wrapped, or an image outside the domain's
+    // other directions), [7] rebuild requests of this step, moved to [3] at
+    // its end
     int* ctrl;
     float* drift;       // per particle: the drift bound since the last build (rounded up)
     float4* disp;       // per particle: displacement since the last build (x, y, z) and
@@ -282,7 +285,8 @@ struct StepArgs {
     int sector;      // sector periodicity (the force side of particle and wall contacts folds bodies)
     int records;
     double skin;       // positional skin of the culling stages (the pair cache; 0 without it)
-    const int* gate;   // pair cache: the selection runs only when *gate != 0 (null: always)
+    const int* gate;   // pair cache: the list is built only when *gate or *gate2 (may be
+    const int* gate2;  // null) is not 0, and carried otherwise (gate null: always built)
     const float* drift;  // pair cache: per-particle drift bounds (see PairCacheDev)
     const float4* disp;  // pair cache: per-particle displacements (see PairCacheDev)
     const float* driftB; // the partners' drift bounds and displacements when they
@@ -313,19 +317,10 @@ struct BondViewDev {
     double3* frames[8]; // master n1 n2 n3 point, slave n1 n2 n3 point (body frames)
 };
 
-// integration and hashing
-void launch_kick(const ObjDev& P, const GeoSetDev& G, double3 gravity, double h, cudaStream_t s);
-void launch_drift(const ObjDev& O, double dt, cudaStream_t s);
-// launch_kick(h), launch_kick(h) and launch_drift(dt) of the particles in one
-// pass: the end of one step and the start of the next
-void launch_kick_drift(const ObjDev& P, const GeoSetDev& G, double3 gravity, double h, double dt, cudaStream_t s);
 // cell hash of each object (-1 outside the grid) and its single-precision
 // rotation rows; build (non-null): the cell table's build numbers, renewed for
 // a step of list generation par
 void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s, unsigned int* build = nullptr, int par = 0);
-// the cell table from the objects' hashes (O.hash); with gate non-null it is
-// built only when *gate != 0 (the pair cache's rebuild flag)
-void launch_cell_table(const ObjDev& O, const CellTableDev& T, cudaStream_t s, const int* gate = nullptr);
 // stable sort of n 64-bit keys (key 0 .. num_keys - 1, or negative: last) on
 // the stream: out_idx gets the permutation, out_key the sorted keys (~0 for
 // the negative ones).  Scratch: key_b (n), idx_b (n), bcount and bscan_tmp
@@ -335,70 +330,83 @@ void radix_sort_keys(const long long* keys, int n, long long num_keys, unsigned 
                      const int* gate = nullptr);
 // ints needed for bcount and bscan_tmp for n keys
 void radix_sort_scratch(int n, size_t& bcount_ints, size_t& bscan_ints);
-// ctrl (the pair cache's, or null): a wrap requests the uncached ghost
-// stage this step and a rebuild at the next
-// src: positions to wrap into P.pos (null: P.pos in place)
-void launch_wrap(ObjDev& P, const FdGrid& g, int dim, cudaStream_t s, int* ctrl = nullptr,
-                 const double3* src = nullptr);
-// ext_skin > 0 (the pair cache, ctrl non-null): particles within ext_skin of
-// the image band get images too (Gh.live marks the true ones); an image
-// outside the domain in a direction it is not translated along (the
-// reference hashes it into a clamped cell) makes this step's ghost stage
-// uncached
-void launch_ghost_build(const ObjDev& P, GhostDev& Gh, int kind, cudaStream_t s, double ext_skin = 0.0,
-                        int* ctrl = nullptr);
-// the ghost lists' gate and skin switch of this step (ctrl[5], ctrl[6])
-void launch_ghost_gate(int* ctrl, cudaStream_t s);
+// The periodic wraps (positions into dst, which may be P.pos) and the
+// translated images gh[d] with on[d] (X, Y, XY).  Under the pair cache (ctrl
+// non-null) a wrap requests the uncached ghost stage this step and a rebuild
+// at the next; particles within ext_skin of the image band get images too
+// (GhostDev::live marks the true ones); an image outside the domain in a
+// direction it is not translated along (the reference hashes it into a clamped
+// cell) makes this step's ghost stage uncached.
+void launch_images(const ObjDev& P, double3* dst, const GhostDev* gh, const int* on, double ext_skin, int* ctrl,
+                   cudaStream_t s);
+// empty occupied-cell box of an image table (before the images are built)
+void reset_image_box(int* occ, cudaStream_t s);
 // sector periodicity: turn bodies that left the quarter sector back in, then
 // build the three turned image sets (R90, R180, R270)
 void launch_sector_wrap(ObjDev& P, const FdGrid& g, cudaStream_t s);
 void launch_sector_images(const ObjDev& P, GhostDev* R, cudaStream_t s);
 
-// pair lists.  skin widens the sphere tests and the body-level cull (the pair
-// cache); with gate non-null the kernels run only when *gate != 0
-void launch_broad_pp(const ObjDev& P, const GeoSetDev& G, const CellTableDev& T, PairListDev& L,
-                     unsigned int* flags, double probe, cudaStream_t s, double skin = 0.0,
-                     const int* gate = nullptr);
-// the same pairs through the neighbour list (check, conditional rebuild, filter)
-void launch_broad_pp_nl(const ObjDev& P, const GeoSetDev& G, const CellTableDev& T, PairListDev& L, NlDev& nl,
-                        unsigned int* flags, double probe, cudaStream_t s, const int* gate = nullptr);
-// pair cache: flag a rebuild when a particle drifted by more than skin / 2
-// (or changed visibility); after the particle-particle narrow phase, keep
-// the state of a rebuild step as the new reference and clear the flag
-void launch_pair_cache_check(const ObjDev& P, const PairCacheDev& c, cudaStream_t s);
-void launch_pair_cache_commit(const ObjDev& P, const PairCacheDev& c, const PairListDev& L, cudaStream_t s);
-// walls: flag a rebuild when a wall drifted by more than skin / 2 or changed
-// cell; after the particle-wall narrow phase of a rebuild, keep their state
-void launch_pair_cache_check_walls(const ObjDev& W, const GeoSetDev& GW, const PairCacheDev& c, cudaStream_t s);
-void launch_pair_cache_commit_walls(const ObjDev& W, const PairCacheDev& c, cudaStream_t s);
-// end of a cached step: a list (particle-wall, ghosts) that overflowed asks
-// for a rebuild, this step's requests become the next step's rebuild, the
-// flags clear
-void launch_pair_cache_end(const PairCacheDev& c, const PairListDev* lists, int n_lists, cudaStream_t s);
-// wall_range (null: every wall): per particle, the first wall and the wall
-// count it may meet (a batch of simulations tiled into one)
-void launch_broad_pw(const ObjDev& P, const GeoSetDev& G, const ObjDev& W, const GeoSetDev& GW,
-                     const FdGrid& wg, PairListDev& L, unsigned int* flags, double probe, cudaStream_t s,
-                     const int2* wall_range = nullptr, double skin = 0.0, const int* gate = nullptr);
-// skin, gate and noskin: the pair cache (ctrl[5], ctrl[6]), as for the
-// particle-particle list
-void launch_broad_ghost(const ObjDev& P, const GeoSetDev& G, const GhostDev& Gh, PairListDev& L,
-                        unsigned int* flags, double probe, cudaStream_t s, double skin = 0.0,
-                        const int* gate = nullptr, const int* noskin = nullptr);
-// a.gate non-null (particle-particle and translated ghost lists under the
-// pair cache): on steps without a rebuild the selection is skipped and the
-// previous step's pairs and slots are carried into this step's list
-void launch_narrow(int kind, const ObjDev& P, const GeoSetDev& G, const MatDev& M, const ObjDev& W,
-                   const GeoSetDev& GW, const MatDev& MW, const FdGrid& pgrid, const FdGrid& wgrid,
-                   const GhostDev* gh, PairListDev& L, const StepArgs& a, int with_force, bool mixed, cudaStream_t s);
-// gate (non-null): the index is rebuilt only when *gate != 0 (a step whose
-// lists keep their pairs keeps the index of the step that built them)
-void launch_reverse(const ObjDev& P, PairListDev* lists, const int* active, const RevDev& R, cudaStream_t s,
-                    const int* gate = nullptr);
+// What the lists of a step share, and one list of it
+struct StepShared {
+    int n;                   // particles
+    GeoSetDev G, GW;
+    MatDev M, MW;
+    ObjDev W;
+    FdGrid pgrid, wgrid;
+    CellTableDev T;          // the particles' cell table
+    // null: every wall; else per particle the first wall and the wall count it
+    // may meet (a batch of simulations tiled into one)
+    const int2* wall_range;
+    RevDev R;
+    int with_force;
+    bool mixed;              // single-precision contact law, bond law and force sums
+};
+struct ListArgs {
+    int kind;
+    ObjDev P;                // the particles (image lists: at their wrapped positions)
+    GhostDev gh;
+    PairListDev L;
+    StepArgs a;
+};
+// The stages of n lists, each stage one launch for all of them.  broad: cell
+// tables and candidate pairs (nl non-null: the particle-particle list's come
+// from the neighbour list; both give the same pairs).  narrow: contact slots,
+// predicate, contact law, pair sums.  Under the pair cache (a.gate) a list
+// that is not built this step keeps the pairs and slots of its last build.
+void launch_broad(const ListArgs* lists, int n, const StepShared& c, NlDev* nl, cudaStream_t s);
+void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream_t s);
+// end of a step's detection: the reverse index, and the pair cache's (pc
+// non-null) layouts, references and flags; done: a zeroed counter
+void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists, const int* active, const RevDev& R,
+                     const PairCacheDev* pc, bool cached_ghosts, unsigned int* done, cudaStream_t s);
+// parts of launch_advance and launch_small_advance: a step's force sums over
+// its lists and bonds; its second half kick; the next step's first half kick,
+// drift (walls too), hashes and, with pc, pair-cache checks, for a step of list
+// generation par.  wrapped (may be null): the positions after the periodic
+// wraps, which replace P.pos.  occ: the image tables' boxes to reset.
+enum { STEP_SUM = 1, STEP_BACK = 2, STEP_FRONT = 4 };
+void launch_advance(const StepShared& c, const ObjDev& P, const PairListDev* lists, const int* active, const BondDev& B,
+                    const double3* wrapped, double3 gravity, double dt, const PairCacheDev* pc, int* const* occ,
+                    int par, int parts, cudaStream_t s);
+// Small sets (dense cell table, no neighbour list, pair cache or images): a
+// step's detection, contact forces and pair sums of the particle-particle and
+// particle-wall lists in one launch.  The cell table and both lists' counters
+// (zero) are those launch_small_advance left; r_head (-1 per particle)
+// collects each partner's pairs for its sum, own (6 per particle) the sums of
+// each particle's own pairs.  a.rec: the record of the
+// particle-particle list, recw of the particle-wall list.
+void launch_small_pairs(const ObjDev& P, const GeoSetDev& G, const MatDev& M, const ObjDev& W, const GeoSetDev& GW,
+                        const MatDev& MW, const FdGrid& pgrid, const FdGrid& wgrid, const CellTableDev& T,
+                        const PairListDev& Lp, const PairListDev& Lw, const StepArgs& a, const AdjRec& recw,
+                        const int2* wall_range, int* r_head, void* own, bool mixed, cudaStream_t s);
+// launch_advance for a small set; its front also fills the cell lists T and
+// zeroes the next lists' counters
+void launch_small_advance(const ObjDev& P, const GeoSetDev& G, const ObjDev& W, const FdGrid& pgrid,
+                          const FdGrid& wgrid, const PairListDev& Lp, const BondDev& B, const CellTableDev& T,
+                          int* r_head, const void* own, int* zero_p, int* zero_w, double3 gravity, double dt,
+                          bool mixed, int parts, cudaStream_t s);
 // mixed: single-precision contact law, bond law and force sums
 void launch_bonds(const ObjDev& P, BondDev& B, bool mixed, cudaStream_t s);
-void launch_reduce(ObjDev& P, PairListDev* lists, const int* active, const RevDev& R, const BondDev& B, bool mixed,
-                   cudaStream_t s);
 // the n contacts of a list (keys and sort scratch of the list's slot
 // capacity; max_key bounds node << 32 | partner) into the view
 void launch_contact_view(const PairListDev& L, long long* keys, int* order, unsigned long long* skey,
