@@ -212,44 +212,194 @@ __device__ __forceinline__ double solid_angle(Vec p, Vec a, Vec b, Vec c)
     return 2.0 * atan2(num, den);
 }
 
-constexpr int MESH_BLOCK = 128;
+// A triangle for the screening passes, in single precision about the grid's
+// centre and in units of the whole extent (so that no length over- or
+// underflows): corners, centroid, and the radius of its corners about the centroid
+// (infinite for slivers, whose exact closest point may be badly rounded:
+// those are always evaluated).
+struct MeshTri {
+    float4 sphere;
+    float ax, ay, az, bx, by, bz, cx, cy, cz, pad[3];
+};
 
-// one thread per grid node; the triangles stream through shared memory in
-// tiles of MESH_BLOCK, every thread of the block reading the same triangle
-// (a broadcast).  The solid angles are summed in triangle order.
-__global__ void __launch_bounds__(MESH_BLOCK) k_levelset_mesh(const double* __restrict__ tri, int ntri, int flip,
-                                                              double3 o, double h, int3 n, long long total,
+__global__ void k_mesh_prepare(const double* __restrict__ tri, int ntri, double3 centre, double unit,
+                               MeshTri* __restrict__ out)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ntri) return;
+    const double* T = tri + 9ll * t;
+    const Vec o = mk(centre.x, centre.y, centre.z);
+    const Vec a = unit * (mk(T[0], T[1], T[2]) - o), b = unit * (mk(T[3], T[4], T[5]) - o),
+              c = unit * (mk(T[6], T[7], T[8]) - o);
+    const Vec g = (1.0 / 3.0) * (a + b + c);
+    const double edge2 = fmax(dot(b - a, b - a), fmax(dot(c - a, c - a), dot(c - b, c - b)));
+    const Vec n = cross(b - a, c - a);
+    const double r = sqrt(fmax(dot(a - g, a - g), fmax(dot(b - g, b - g), dot(c - g, c - g))));
+    const bool sliver = !(dot(n, n) > 1e-10 * edge2 * edge2);
+    MeshTri m;
+    m.sphere = make_float4((float)g.x, (float)g.y, (float)g.z,
+                           sliver ? __int_as_float(0x7f800000) : __double2float_ru(r));
+    m.ax = (float)a.x; m.ay = (float)a.y; m.az = (float)a.z;
+    m.bx = (float)b.x; m.by = (float)b.y; m.bz = (float)b.z;
+    m.cx = (float)c.x; m.cy = (float)c.y; m.cz = (float)c.z;
+    m.pad[0] = m.pad[1] = m.pad[2] = 0.f;
+    out[t] = m;
+}
+
+// half the solid angle in single precision; exact (double precision) where
+// the point lies near the triangle's plane inside it, or near its edges or
+// corners, where the angle jumps or is ill-conditioned
+__device__ __forceinline__ float half_angle32(float px, float py, float pz, const MeshTri& t, Vec x,
+                                              const double* __restrict__ T)
+{
+    const float ax = t.ax - px, ay = t.ay - py, az = t.az - pz;
+    const float bx = t.bx - px, by = t.by - py, bz = t.bz - pz;
+    const float cx = t.cx - px, cy = t.cy - py, cz = t.cz - pz;
+    const float la = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
+    const float lb = sqrtf(fmaf(bx, bx, fmaf(by, by, bz * bz)));
+    const float lc = sqrtf(fmaf(cx, cx, fmaf(cy, cy, cz * cz)));
+    const float num = fmaf(ax, fmaf(by, cz, -bz * cy), fmaf(ay, fmaf(bz, cx, -bx * cz), az * fmaf(bx, cy, -by * cx)));
+    const float lll = la * lb * lc;
+    const float den = lll + fmaf(fmaf(ax, bx, fmaf(ay, by, az * bz)), lc,
+                                 fmaf(fmaf(bx, cx, fmaf(by, cy, bz * cz)), la,
+                                      fmaf(cx, ax, fmaf(cy, ay, cz * az)) * lb));
+    // lengths are in units of the extent, whose roundings are 6e-8: within 1e-4
+    // of a corner the directions to it are too rough
+    const float lim = 0.02f * lll;
+    if (!(fminf(la, fminf(lb, lc)) > 1e-4f && (fabsf(num) > lim || den > lim)))
+        return (float)(0.5 * solid_angle(x, mk(T[0], T[1], T[2]), mk(T[3], T[4], T[5]), mk(T[6], T[7], T[8])));
+    return atan2f(num, den);
+}
+
+constexpr int MESH_WARPS = 4;
+constexpr int MESH_BLOCK = 32 * MESH_WARPS;  // also the triangles staged at a time
+
+// 32 grid nodes (8 x 4 x 1) per block, its warps sharing out the triangles.
+//
+// The distance is the minimum over all triangles and the sign the winding
+// number's (a sum of solid angles), in double precision that was three square
+// roots, an arc tangent and a closest point for every node and triangle: 4.6
+// ms for 48^3 nodes and 2,304 triangles, bound by the double-precision pipe.
+// Here single precision screens both, and double precision decides:
+//   * pass 1 sums the solid angles in single precision (half_angle32) and finds
+//     the triangle of the nearest centroid; its exact distance bounds the
+//     minimum;
+//   * pass 2 takes the exact closest point of the triangles whose sphere comes
+//     within that bound, ties to the first triangle as in a scan in order;
+//   * a winding number within a quarter of the 0.5 it is compared with (no
+//     closed mesh gives one) is summed again in double precision, in
+//     triangle order.
+// So every value is the one the double-precision scan gives.
+__global__ void __launch_bounds__(MESH_BLOCK) k_levelset_mesh(const double* __restrict__ tri,
+                                                              const MeshTri* __restrict__ mesh, int ntri, int flip,
+                                                              double3 o, double h, int3 n, double3 centre, double unit,
                                                               double* __restrict__ out)
 {
-    __shared__ double s_tri[MESH_BLOCK * 9];
-    const long long id = blockIdx.x * (long long)MESH_BLOCK + threadIdx.x;
-    const bool live = id < total;
-    const Vec x = live ? node_point(o, h, id, n) : mk(0.0, 0.0, 0.0);
-    double best = DBL_MAX;
-    Vec near = x;
-    double wsum = 0.0;
-    for (int t0 = 0; t0 < ntri; t0 += MESH_BLOCK) {
+    __shared__ MeshTri s_tri[MESH_BLOCK];
+    __shared__ double s_sum[MESH_WARPS][32], s_d2[MESH_WARPS][32];
+    __shared__ float s_near[MESH_WARPS][32];
+    __shared__ int s_at[MESH_WARPS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long bx = (n.x + 7) / 8, by = (n.y + 3) / 4;
+    const long long blk = blockIdx.x;
+    const int i = (int)(blk % bx) * 8 + (lane & 7), j = (int)((blk / bx) % by) * 4 + (lane >> 3);
+    const int k = (int)(blk / (bx * by));
+    const bool live = i < n.x && j < n.y;
+    const Vec x = mk(o.x + double(i) * h, o.y + double(j) * h, o.z + double(k) * h);
+    const float px = (float)(unit * (x.x - centre.x)), py = (float)(unit * (x.y - centre.y)),
+                pz = (float)(unit * (x.z - centre.z));
+    // what the screening's single precision can be off by in a length: a few
+    // roundings of coordinates of at most one
+    const float slack = 2e-6f;
+    auto stage = [&](int t0) {
+        __syncthreads();
         const int nt = min(MESH_BLOCK, ntri - t0);
+        const float4* src = reinterpret_cast<const float4*>(mesh + t0);
+        float4* dst = reinterpret_cast<float4*>(s_tri);
+        for (int q = threadIdx.x; q < nt * (int)(sizeof(MeshTri) / sizeof(float4)); q += MESH_BLOCK) dst[q] = src[q];
         __syncthreads();
-        for (int k = threadIdx.x; k < nt * 9; k += MESH_BLOCK) s_tri[k] = tri[(long long)t0 * 9 + k];
-        __syncthreads();
-        if (!live) continue;
-        for (int t = 0; t < nt; ++t) {
-            const double* T = s_tri + t * 9;
-            const Vec a = mk(T[0], T[1], T[2]), b = mk(T[3], T[4], T[5]), c = mk(T[6], T[7], T[8]);
-            const Vec q = closest_on_triangle(x, a, b, c);
-            const Vec dq = x - q;
-            const double d2 = dot(dq, dq);
-            if (d2 < best) {
-                best = d2;
-                near = q;
+        return nt;
+    };
+    // pass 1
+    double wsum = 0.0;
+    float near2 = __int_as_float(0x7f800000);
+    int at = 0;
+    for (int t0 = 0; t0 < ntri; t0 += MESH_BLOCK) {
+        const int nt = stage(t0);
+        float part = 0.f;
+        for (int t = 32 * w; t < min(32 * w + 32, nt); ++t) {
+            const MeshTri& m = s_tri[t];
+            const float dx = m.sphere.x - px, dy = m.sphere.y - py, dz = m.sphere.z - pz;
+            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            if (d2 < near2) {
+                near2 = d2;
+                at = t0 + t;
             }
-            wsum += solid_angle(x, a, b, c);
+            part += half_angle32(px, py, pz, m, x, tri + 9ll * (t0 + t));
+        }
+        wsum += (double)part;
+    }
+    s_sum[w][lane] = wsum;
+    s_near[w][lane] = near2;
+    s_at[w][lane] = at;
+    __syncthreads();
+    wsum = 0.0;
+    for (int v = 0; v < MESH_WARPS; ++v) {
+        wsum += s_sum[v][lane];
+        if (s_near[v][lane] < near2 || (s_near[v][lane] == near2 && s_at[v][lane] < at)) {
+            near2 = s_near[v][lane];
+            at = s_at[v][lane];
         }
     }
-    if (!live) return;
+    // pass 2
+    double best = DBL_MAX;
+    int best_at = 0x7fffffff;
+    Vec near = x;
+    float reach = __int_as_float(0x7f800000);
+    auto exact = [&](int t) {
+        const double* T = tri + 9ll * t;
+        const Vec q = closest_on_triangle(x, mk(T[0], T[1], T[2]), mk(T[3], T[4], T[5]), mk(T[6], T[7], T[8]));
+        const Vec dq = x - q;
+        const double d2 = dot(dq, dq);
+        if (d2 < best || (d2 == best && t < best_at)) {
+            best = d2;
+            best_at = t;
+            near = q;
+            reach = __double2float_ru(unit * sqrt(d2)) + slack;
+        }
+    };
+    exact(at);
+    for (int t0 = 0; t0 < ntri; t0 += MESH_BLOCK) {
+        const int nt = stage(t0);
+        for (int t = 32 * w; t < min(32 * w + 32, nt); ++t) {
+            const float4 c = s_tri[t].sphere;
+            const float dx = c.x - px, dy = c.y - py, dz = c.z - pz;
+            const float far = (reach + c.w) * 1.00001f;
+            if (!(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > far * far) && t0 + t != at) exact(t0 + t);
+        }
+    }
+    s_d2[w][lane] = best;
+    s_at[w][lane] = best_at;
+    __syncthreads();
+    int owner = 0;
+    for (int v = 1; v < MESH_WARPS; ++v)
+        if (s_d2[v][lane] < s_d2[owner][lane] ||
+            (s_d2[v][lane] == s_d2[owner][lane] && s_at[v][lane] < s_at[owner][lane]))
+            owner = v;
+    // the warp that holds a node's nearest point finishes it
+    if (!live || owner != w) return;
+    wsum *= 2.0;
+    const double turns = fabs(wsum / (4.0 * 3.14159265358979323846));
+    bool inside = turns > 0.5;
+    if (!(turns < 0.25 || turns > 0.75)) {
+        wsum = 0.0;
+        for (int t = 0; t < ntri; ++t) {
+            const double* T = tri + 9ll * t;
+            wsum += solid_angle(x, mk(T[0], T[1], T[2]), mk(T[3], T[4], T[5]), mk(T[6], T[7], T[8]));
+        }
+        inside = fabs(wsum / (4.0 * 3.14159265358979323846)) > 0.5;
+    }
     const double d = len(x - near);
-    const bool inside = fabs(wsum / (4.0 * 3.14159265358979323846)) > 0.5;
     double f = inside ? -d : d;
     Vec g = mk(0.0, 0.0, 0.0);
     if (d > 1e-30) {
@@ -257,7 +407,7 @@ __global__ void __launch_bounds__(MESH_BLOCK) k_levelset_mesh(const double* __re
         g = inside ? -u : u;
     }
     if (flip) { f = -f; g = -g; }
-    out[id] = grid_value(f, g, h);
+    out[((long long)k * n.y + j) * n.x + i] = grid_value(f, g, h);
 }
 
 }  // namespace
@@ -307,6 +457,9 @@ extern "C" int fundem_levelset_grid(int device, void* stream, const fundem_shape
     const int3 n = make_int3(size[0], size[1], size[2]);
     double* d_out = nullptr;
     double* d_tri = nullptr;
+    MeshTri* d_mesh = nullptr;
+    double3 centre = make_double3(0.0, 0.0, 0.0);
+    double unit = 1.0;
     int status = FUNDEM_OK;
     cudaError_t e = cudaMallocAsync((void**)&d_out, total * sizeof(double), s);
     if (e == cudaSuccess && kind == FUNDEM_SHAPE_MESH) {
@@ -316,16 +469,28 @@ extern "C" int fundem_levelset_grid(int device, void* stream, const fundem_shape
         for (int t = 0; t < nt; ++t)
             for (int k = 0; k < 3; ++k)
                 for (int c = 0; c < 3; ++c) h_tri[t * 9 + k * 3 + c] = shape->vertices[3 * shape->triangles[3 * t + k] + c];
+        // the screening passes' frame
+        centre = make_double3(o.x + 0.5 * (n.x - 1) * spacing, o.y + 0.5 * (n.y - 1) * spacing,
+                              o.z + 0.5 * (n.z - 1) * spacing);
+        double scale = 0.5 * spacing * (n.x + n.y + n.z);
+        for (int v = 0; v < shape->n_vertices; ++v) {
+            const double* q = shape->vertices + 3 * v;
+            scale = std::fmax(scale, std::fabs(q[0] - centre.x) + std::fabs(q[1] - centre.y) + std::fabs(q[2] - centre.z));
+        }
+        unit = 1.0 / scale;
         e = cudaMallocAsync((void**)&d_tri, (size_t)nt * 9 * sizeof(double), s);
+        if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_mesh, (size_t)nt * sizeof(MeshTri), s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_tri, h_tri, (size_t)nt * 9 * sizeof(double), cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         delete[] h_tri;
     }
     if (e == cudaSuccess) {
         if (kind == FUNDEM_SHAPE_MESH) {
-            const long long blocks = (total + MESH_BLOCK - 1) / MESH_BLOCK;
-            k_levelset_mesh<<<(unsigned)blocks, MESH_BLOCK, 0, s>>>(d_tri, shape->n_triangles, shape->positive_inside != 0,
-                                                                    o, spacing, n, total, d_out);
+            const int nt = shape->n_triangles;
+            k_mesh_prepare<<<(nt + 127) / 128, 128, 0, s>>>(d_tri, nt, centre, unit, d_mesh);
+            const long long blocks = (long long)((n.x + 7) / 8) * ((n.y + 3) / 4) * n.z;
+            k_levelset_mesh<<<(unsigned)blocks, MESH_BLOCK, 0, s>>>(d_tri, d_mesh, nt, shape->positive_inside != 0, o,
+                                                                    spacing, n, centre, unit, d_out);
         } else {
             Shape sh;
             sh.kind = kind;
@@ -343,6 +508,7 @@ extern "C" int fundem_levelset_grid(int device, void* stream, const fundem_shape
     if (e == cudaSuccess) e = cudaMemcpyAsync(sdf, d_out, total * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (d_out) cudaFreeAsync(d_out, s);
     if (d_tri) cudaFreeAsync(d_tri, s);
+    if (d_mesh) cudaFreeAsync(d_mesh, s);
     const cudaError_t e2 = cudaStreamSynchronize(s);
     if (e != cudaSuccess || e2 != cudaSuccess) status = FUNDEM_ERR_CUDA;
     if (device >= 0 && device != prev) cudaSetDevice(prev);
