@@ -1019,6 +1019,12 @@ struct fundem_sim {
     cudaEvent_t br_fork = nullptr, br_join = nullptr;
     DevArray<double3> img_pos;
     DevArray<unsigned int> end_done;
+    // read-back of contacts (fundem_get_contacts), and the state a detection
+    // outside a step starts again from (detect_fit)
+    DevArray<double> pack_buf;
+    DevArray<int> pack_at;
+    DevArray<double3> keep_pos, keep_vel;
+    DevArray<fd_quat> keep_q;
     ~fundem_sim()
     {
         drop_graph();
@@ -1472,12 +1478,12 @@ struct fundem_sim {
         FD_CUDA(cudaMemcpy(&f0, flags.p, sizeof(f0), cudaMemcpyDeviceToHost));
         const size_t np = (size_t)P.n();
         const bool wraps = (perX || perY || sector) && np > 0 && P.n_dev == (int)np;
-        DevArray<double3> keep_pos, keep_vel;
-        DevArray<fd_quat> keep_q;
         if (wraps) {
-            keep_pos.alloc(np);
-            keep_vel.alloc(np);
-            keep_q.alloc(np);
+            if (keep_pos.n < np) {
+                keep_pos.alloc(np, false);
+                keep_vel.alloc(np, false);
+                keep_q.alloc(np, false);
+            }
             FD_CUDA(cudaMemcpyAsync(keep_pos.p, P.d_pos.p, np * sizeof(double3), cudaMemcpyDeviceToDevice, stream));
             FD_CUDA(cudaMemcpyAsync(keep_vel.p, P.d_vel.p, np * sizeof(double3), cudaMemcpyDeviceToDevice, stream));
             FD_CUDA(cudaMemcpyAsync(keep_q.p, P.d_q.p, np * sizeof(fd_quat), cudaMemcpyDeviceToDevice, stream));
@@ -2293,43 +2299,53 @@ int fundem_get_contacts(fundem_sim* s, int kind, int* node, int* partner, double
         PairGen& g = L.gen[L.cur];
         FD_CUDA(cudaMemcpy(c, g.counters.p, sizeof(c), cudaMemcpyDeviceToHost));
         // an overflowed list holds no valid contacts (fundem_num_contacts gives 0)
-        const size_t n = (size_t)(c[1] <= L.cap_contacts ? c[1] : 0);
-        std::vector<int> hn(n), hs(n);
-        std::vector<double> hsp(3 * n), hpt(3 * n), hnm(3 * n), hov(n), hen(n), hes(n);
-        if (n) {
-            FD_CUDA(cudaMemcpy(hn.data(), g.c_node.p, sizeof(int) * n, cudaMemcpyDeviceToHost));
-            FD_CUDA(cudaMemcpy(hs.data(), g.c_slave.p, sizeof(int) * n, cudaMemcpyDeviceToHost));
-            FD_CUDA(cudaMemcpy(hsp.data(), g.c_spring.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost));
-            FD_CUDA(cudaMemcpy(hpt.data(), g.c_point.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost));
-            FD_CUDA(cudaMemcpy(hnm.data(), g.c_normal.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost));
-            FD_CUDA(cudaMemcpy(hov.data(), g.c_overlap.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
-            FD_CUDA(cudaMemcpy(hen.data(), g.c_en.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
-            FD_CUDA(cudaMemcpy(hes.data(), g.c_es.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
+        const size_t n = (size_t)(c[1] <= L.cap_contacts ? c[2] : 0);
+        if (n == 0) return;
+        // the contacts are packed on the device, ids and the wanted fields, and
+        // put in order here
+        double* dst[6] = {point, normal, overlap, spring, en, es};
+        const size_t width[6] = {3, 3, 1, 3, 1, 1};
+        size_t words = n;  // ids: one word each
+        for (int f = 0; f < 6; ++f)
+            if (dst[f]) words += width[f] * n;
+        if (s->pack_buf.n < words) {
+            // no captured step reads these: its graphs stay valid
+            const unsigned long long epoch = s->alloc_epoch;
+            s->pack_buf.alloc(words + words / 2, false);
+            if (!s->pack_at.p) s->pack_at.alloc(1);
+            s->alloc_epoch = epoch;
         }
-        // slots that hold no contact carry node id -1
-        std::vector<size_t> order;
-        order.reserve(n);
-        for (size_t k = 0; k < n; ++k)
-            if (hn[k] >= 0) order.push_back(k);
+        size_t off[6] = {0, 0, 0, 0, 0, 0}, at = n;
+        double* dev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+        for (int f = 0; f < 6; ++f) {
+            if (!dst[f]) continue;
+            off[f] = at;
+            dev[f] = s->pack_buf.p + at;
+            at += width[f] * n;
+        }
+        const fd::ContactPackDev v{reinterpret_cast<int2*>(s->pack_buf.p), dev[0], dev[1], dev[2], dev[3], dev[4], dev[5]};
+        fd::launch_pack_contacts(L.view(), v, s->pack_at.p, (int)n, s->stream);
+        int found = 0;
+        std::vector<double> h(words);
+        FD_CUDA(cudaMemcpyAsync(&found, s->pack_at.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+        FD_CUDA(cudaMemcpyAsync(h.data(), s->pack_buf.p, sizeof(double) * words, cudaMemcpyDeviceToHost, s->stream));
+        FD_CUDA(cudaStreamSynchronize(s->stream));
         // the caller sized its arrays with fundem_num_contacts
-        if (order.size() != (size_t)c[2])
-            throw std::runtime_error("contact list inconsistent: " + std::to_string(order.size()) + " contacts in " +
-                                     std::to_string(n) + " slots, counter " + std::to_string(c[2]));
-        std::sort(order.begin(), order.end(), [&](size_t a, size_t b) {
-            return hn[a] != hn[b] ? hn[a] < hn[b] : hs[a] < hs[b];
-        });
-        for (size_t k = 0; k < order.size(); ++k) {
-            const size_t j = order[k];
-            if (node) node[k] = hn[j];
-            if (partner) partner[k] = hs[j];
-            for (int d = 0; d < 3; ++d) {
-                if (spring) spring[3 * k + d] = hsp[3 * j + d];
-                if (point) point[3 * k + d] = hpt[3 * j + d];
-                if (normal) normal[3 * k + d] = hnm[3 * j + d];
-            }
-            if (overlap) overlap[k] = hov[j];
-            if (en) en[k] = hen[j];
-            if (es) es[k] = hes[j];
+        if ((size_t)found != n)
+            throw std::runtime_error("contact list inconsistent: " + std::to_string(found) + " contacts, counter " +
+                                     std::to_string(n));
+        const int2* id = reinterpret_cast<const int2*>(h.data());
+        std::vector<std::pair<uint64_t, uint32_t>> order(n);
+        for (size_t k = 0; k < n; ++k)
+            order[k] = {(uint64_t)(uint32_t)id[k].x << 32 | (uint32_t)id[k].y, (uint32_t)k};
+        std::sort(order.begin(), order.end());
+        for (size_t k = 0; k < n; ++k) {
+            const size_t j = order[k].second;
+            if (node) node[k] = id[j].x;
+            if (partner) partner[k] = id[j].y;
+            for (int f = 0; f < 6; ++f)
+                if (dst[f])
+                    for (size_t d = 0; d < width[f]; ++d) dst[f][width[f] * k + d] = h[off[f] + width[f] * j + d];
         }
     });
 }
@@ -2762,8 +2778,8 @@ int fundem_adjoint_backward_rot(fundem_sim* s, const double* dl_dpos, const doub
         for (int k = 0; k < FD_NKIND; ++k) {
             T.cap[k] = (used[k] && s->lists[k].allocated) ? s->lists[k].cap_contacts : 0;
             const size_t c = (size_t)std::max(T.cap[k], 1);
-            T.ints[k].alloc(9 * c * K, false);
-            T.dbl[k].alloc(16 * c * K, false);
+            if (T.ints[k].n < 9 * c * K) T.ints[k].alloc(9 * c * K, false);
+            if (T.dbl[k].n < 16 * c * K) T.dbl[k].alloc(16 * c * K, false);
         }
         T.nslots.alloc((size_t)K * FD_NKIND);
         fd::BondDev bd = s->bond_view();

@@ -3340,6 +3340,27 @@ __global__ void k_view_gather(PairListDev L, const int* order, long long n, Cont
         v.es[i] = L.c_es[s];
     }
 }
+// the contacts of a list packed field by field (count of them, in no order):
+// the host reads those back instead of every slot, most of which hold none
+__global__ void k_pack_contacts(PairListDev L, ContactPackDev v, int* at, int count)
+{
+    const int nslots = min(*L.n_slots, L.cap_contacts);
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nslots; s += gridDim.x * blockDim.x) {
+        const int node = L.c_node[s];
+        if (node < 0) continue;
+        const int i = atomicAdd(at, 1);
+        if (i >= count) continue;
+        v.id[i] = make_int2(node, L.c_slave[s]);
+        for (int d = 0; d < 3; ++d) {
+            if (v.point) v.point[3 * i + d] = L.c_point[3 * s + d];
+            if (v.normal) v.normal[3 * i + d] = L.c_normal[3 * s + d];
+            if (v.spring) v.spring[3 * i + d] = L.c_spring[3 * s + d];
+        }
+        if (v.overlap) v.overlap[i] = L.c_overlap[s];
+        if (v.en) v.en[i] = L.c_en[s];
+        if (v.es) v.es[i] = L.c_es[s];
+    }
+}
 __global__ void k_bond_view(BondDev B, BondViewDev v)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3671,6 +3692,11 @@ void launch_contact_view(const PairListDev& L, long long* keys, int* order, unsi
     k_view_keys<<<148 * 4, TPB, 0, s>>>(L, keys); note_launch();
     radix_sort_keys(keys, L.cap_contacts, max_key, skey, order, key_b, idx_b, bcount, bscan, s);
     if (n > 0) { k_view_gather<<<148 * 4, TPB, 0, s>>>(L, order, n, v); note_launch(); }
+}
+void launch_pack_contacts(const PairListDev& L, const ContactPackDev& v, int* at, int count, cudaStream_t s)
+{
+    cudaMemsetAsync(at, 0, sizeof(int), s);
+    k_pack_contacts<<<148 * 4, TPB, 0, s>>>(L, v, at, count); note_launch();
 }
 void launch_bond_view(const BondDev& B, const BondViewDev& v, cudaStream_t s)
 {

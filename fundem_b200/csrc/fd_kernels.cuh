@@ -310,6 +310,12 @@ struct ContactViewDev {
     int* master;       // global boundary node
     int* slave;        // partner
 };
+// a list's contacts packed for the host: ids (node, partner) and the wanted
+// fields (null: not wanted)
+struct ContactPackDev {
+    int2* id;
+    double *point, *normal, *overlap, *spring, *en, *es;
+};
 // the bonds' interleaved per-bond parameters and state as one array per field
 struct BondViewDev {
     double* B[4];       // B1 .. B4
@@ -413,6 +419,8 @@ void launch_contact_view(const PairListDev& L, long long* keys, int* order, unsi
                          unsigned long long* key_b, int* idx_b, int* bcount, int* bscan, long long n,
                          long long max_key, const ContactViewDev& v, cudaStream_t s);
 void launch_bond_view(const BondDev& B, const BondViewDev& v, cudaStream_t s);
+// the contacts of a list, at most count, in no order; at: how many there are
+void launch_pack_contacts(const PairListDev& L, const ContactPackDev& v, int* at, int count, cudaStream_t s);
 
 // Kernel launches of the calling thread are counted into *c (null: not
 // counted); the library points it at the calling simulation's counter for
