@@ -259,6 +259,8 @@ struct GeoSetHost {
     DevArray<FdGeo> d_geo;
     DevArray<double> d_sdf;
     DevArray<float> d_sdf32;
+    DevArray<double4> d_sdf_quad;
+    DevArray<float4> d_sdf32_quad;
     DevArray<float> d_dist;
     DevArray<float> d_cellmin;
     DevArray<double3> d_nodes;
@@ -370,6 +372,10 @@ struct GeoSetHost {
         d_sdf.upload(sdf.data(), sdf.size(), s);
         d_sdf32.alloc(std::max<size_t>(sdf32.size(), 1));
         d_sdf32.upload(sdf32.data(), sdf32.size(), s);
+        d_sdf_quad.alloc(std::max<size_t>(sdf.size(), 1), false);
+        d_sdf32_quad.alloc(std::max<size_t>(sdf.size(), 1), false);
+        for (const FdGeo& t : table)
+            fd::launch_sdf_quads(d_sdf.p, d_sdf32.p, d_sdf_quad.p, d_sdf32_quad.p, t.sdf_off, t.size, s);
         d_dist.alloc(std::max<size_t>(dist.size(), 1));
         d_dist.upload(dist.data(), dist.size(), s);
         d_cellmin.alloc(std::max<size_t>(cellmin.size(), 1));
@@ -407,6 +413,8 @@ struct GeoSetHost {
         v.geo = d_geo.p;
         v.sdf = d_sdf.p;
         v.sdf32 = d_sdf32.p;
+        v.sdf_quad = d_sdf_quad.p;
+        v.sdf32_quad = d_sdf32_quad.p;
         v.dist = d_dist.p;
         v.cellmin = d_cellmin.p;
         v.nodes = d_nodes.p;
@@ -473,7 +481,7 @@ struct ObjHost {
 
 struct PairGen {
     DevArray<int> pairA, pairB, seg_off, seg_cnt, c_off, c_cnt, c_node, c_slave, c_k, counters;
-    DevArray<double> pf, c_spring, c_point, c_normal, c_overlap, c_en, c_es;
+    DevArray<double> pf, c_spring;
 };
 
 struct PairList {
@@ -488,7 +496,7 @@ struct PairList {
     DevArray<float> c_phi0;  // pair cache: slot bounds of the last rebuild
     DevArray<float> p_bound; // pair cache: per-pair drift bound of a carried step
     DevArray<int> c_test, n_test;  // pair cache: slots listed for the predicate pass
-    DevArray<double> c_force;
+    DevArray<double> c_rec;
     DevArray<int4> p_aux;
     bool allocated = false;
 
@@ -503,11 +511,9 @@ struct PairList {
             g.c_off.alloc(cap_pairs); g.c_cnt.alloc(cap_pairs); g.pf.alloc((size_t)cap_pairs * 9);
             g.c_node.alloc(cap_contacts); g.c_slave.alloc(cap_contacts); g.c_k.alloc(cap_contacts);
             g.c_spring.alloc((size_t)cap_contacts * 3);
-            g.c_point.alloc((size_t)cap_contacts * 3); g.c_normal.alloc((size_t)cap_contacts * 3);
-            g.c_overlap.alloc(cap_contacts); g.c_en.alloc(cap_contacts); g.c_es.alloc(cap_contacts);
             g.counters.alloc(3);
         }
-        c_pair.alloc(cap_contacts); c_hit.alloc(cap_contacts, false); c_force.alloc((size_t)cap_contacts * 9);
+        c_pair.alloc(cap_contacts); c_hit.alloc(cap_contacts, false); c_rec.alloc((size_t)cap_contacts * fd::CONTACT_REC);
         c_phi0.alloc(cap_contacts, false);
         p_aux.alloc(cap_pairs); p_hist_cnt.alloc(cap_pairs); r_next.alloc(cap_pairs, false); p_hit.alloc(cap_pairs); p_bound.alloc(cap_pairs, false);
         c_test.alloc(cap_contacts, false);
@@ -532,15 +538,12 @@ struct PairList {
             for (PairGen& g : gen) {
                 g.c_node.grow(capc, cap_contacts); g.c_slave.grow(capc, cap_contacts); g.c_k.grow(capc, cap_contacts);
                 g.c_spring.grow((size_t)capc * 3, (size_t)cap_contacts * 3);
-                g.c_point.grow((size_t)capc * 3, (size_t)cap_contacts * 3);
-                g.c_normal.grow((size_t)capc * 3, (size_t)cap_contacts * 3);
-                g.c_overlap.grow(capc, cap_contacts); g.c_en.grow(capc, cap_contacts); g.c_es.grow(capc, cap_contacts);
             }
             c_pair.grow(capc, 0);
             c_hit.grow(capc, 0);
             c_phi0.grow(capc, 0);  // rewritten by the rebuild a grow forces
             c_test.grow(capc, 0);
-            c_force.grow((size_t)capc * 9, 0);
+            c_rec.grow((size_t)capc * fd::CONTACT_REC, (size_t)cap_contacts * fd::CONTACT_REC);
             cap_contacts = capc;
         }
     }
@@ -554,10 +557,9 @@ struct PairList {
         v.o_pairA = o.pairA.p; v.o_counters = o.counters.p;
         v.o_pairB = o.pairB.p; v.o_seg_off = o.seg_off.p; v.o_seg_cnt = o.seg_cnt.p; v.o_c_off = o.c_off.p;
         v.o_c_cnt = o.c_cnt.p;
-        v.c_node = c.c_node.p; v.c_slave = c.c_slave.p; v.c_spring = c.c_spring.p; v.c_point = c.c_point.p;
-        v.c_normal = c.c_normal.p; v.c_overlap = c.c_overlap.p; v.c_en = c.c_en.p; v.c_es = c.c_es.p;
+        v.c_node = c.c_node.p; v.c_slave = c.c_slave.p; v.c_spring = c.c_spring.p;
         v.n_slots = c.counters.p + 1; v.n_hits = c.counters.p + 2; v.cap_contacts = cap_contacts;
-        v.c_pair = c_pair.p; v.c_hit = c_hit.p; v.c_k = c.c_k.p; v.o_c_k = o.c_k.p; v.c_force = c_force.p; v.p_aux = p_aux.p; v.p_hist_cnt = p_hist_cnt.p; v.r_next = r_next.p; v.p_hit = p_hit.p;
+        v.c_pair = c_pair.p; v.c_hit = c_hit.p; v.c_k = c.c_k.p; v.o_c_k = o.c_k.p; v.c_rec = c_rec.p; v.p_aux = p_aux.p; v.p_hist_cnt = p_hist_cnt.p; v.r_next = r_next.p; v.p_hit = p_hit.p;
         v.o_c_node = o.c_node.p; v.o_c_spring = o.c_spring.p;
         v.c_phi0 = c_phi0.p;
         v.p_bound = p_bound.p;

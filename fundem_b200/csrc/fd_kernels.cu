@@ -764,12 +764,13 @@ __device__ __forceinline__ bool sphere_culled(float px, float py, float pz, floa
         gz < GB.size.z - 1) {
         const int i0 = (int)gx, j0 = (int)gy, k0 = (int)gz;
         const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
-        const float* S = SB.sdf32 + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
+        const float4* S = SB.sdf32_quad + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
+        const float4 s0 = __ldg(S), s1 = __ldg(S + sxy);
         const float fx = gx - i0, fy = gy - j0, fz = gz - k0;
-        const float c00 = __ldg(S) * (1.f - fx) + __ldg(S + 1) * fx;
-        const float c10 = __ldg(S + sx) * (1.f - fx) + __ldg(S + sx + 1) * fx;
-        const float c01 = __ldg(S + sxy) * (1.f - fx) + __ldg(S + sxy + 1) * fx;
-        const float c11 = __ldg(S + sxy + sx) * (1.f - fx) + __ldg(S + sxy + sx + 1) * fx;
+        const float c00 = s0.x * (1.f - fx) + s0.y * fx;
+        const float c10 = s0.z * (1.f - fx) + s0.w * fx;
+        const float c01 = s1.x * (1.f - fx) + s1.y * fx;
+        const float c11 = s1.z * (1.f - fx) + s1.w * fx;
         const float phi = (c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz;
         const float bound = (float)GB.lip * rho + (float)probe;
         if (phi - bound > 1e-5f * (fabsf(phi) + bound + (float)GB.spacing)) return true;
@@ -1222,7 +1223,7 @@ template <int KIND> struct Slave;
 template <> struct Slave<FD_PP> {
     __device__ static double3 pos(const NarrowArgs& n, int j) { return n.P.pos[j]; }
     __device__ static double3 vel(const NarrowArgs& n, int j) { return n.P.vel[j]; }
-    __device__ static fd_quat q(const NarrowArgs& n, int j) { return n.P.q[j]; }
+    __device__ static const fd_quat* q(const NarrowArgs& n, int j) { return n.P.q + j; }
     __device__ static const float4* rot(const NarrowArgs& n, int j) { return n.P.rot + 3ll * j; }
     __device__ static const FdGeo& geo(const NarrowArgs& n, int j) { return n.G.geo[n.P.geo[j]]; }
     __device__ static const GeoSetDev& set(const NarrowArgs& n) { return n.G; }
@@ -1233,7 +1234,7 @@ template <> struct Slave<FD_PP> {
 template <> struct Slave<FD_PW> {
     __device__ static double3 pos(const NarrowArgs& n, int j) { return n.W.pos[j]; }
     __device__ static double3 vel(const NarrowArgs& n, int j) { return n.W.vel[j]; }
-    __device__ static fd_quat q(const NarrowArgs& n, int j) { return n.W.q[j]; }
+    __device__ static const fd_quat* q(const NarrowArgs& n, int j) { return n.W.q + j; }
     __device__ static const float4* rot(const NarrowArgs& n, int j) { return n.W.rot + 3ll * j; }
     __device__ static const FdGeo& geo(const NarrowArgs& n, int j) { return n.GW.geo[n.W.geo[j]]; }
     __device__ static const GeoSetDev& set(const NarrowArgs& n) { return n.GW; }
@@ -1248,7 +1249,7 @@ template <> struct Slave<FD_PW> {
 struct SlaveGhost {
     __device__ static double3 pos(const NarrowArgs& n, int j) { return n.gh.pos[j]; }
     __device__ static double3 vel(const NarrowArgs& n, int j) { return n.gh.vel ? n.gh.vel[j] : n.P.vel[j]; }
-    __device__ static fd_quat q(const NarrowArgs& n, int j) { return n.gh.q ? n.gh.q[j] : n.P.q[j]; }
+    __device__ static const fd_quat* q(const NarrowArgs& n, int j) { return (n.gh.q ? n.gh.q : n.P.q) + j; }
     __device__ static const float4* rot(const NarrowArgs& n, int j)
     {
         return (n.gh.rot ? n.gh.rot : n.P.rot) + 3ll * j;
@@ -1351,11 +1352,29 @@ __global__ void __launch_bounds__(TPB) k_broad_lists(ListSet a)
     }
 }
 
+// The predicate and contact passes read about 27 numbers a slot at addresses
+// that differ from lane to lane, and the L1 serves a warp's addresses one line
+// at a time: 79% of its rate at 65,003 particles.  Orientations and the
+// interpolation's corners come in 32-byte loads instead (4 to 1 and 8 to 2).
+__device__ __forceinline__ double4 load_quad(const double4* p)
+{
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+// (of arrays the kernel does not write)
+__device__ __forceinline__ fd_quat load_q(const fd_quat* p)
+{
+    fd_quat v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.q0), "=d"(v.q1), "=d"(v.q2), "=d"(v.q3) : "l"(p));
+    return v;
+}
+
 // Evaluate node predicate for one node.  Returns true when overlap >= 0 and
 // fills the grid fraction and the eight corner values.
 template <int KIND>
 __device__ __forceinline__ bool node_predicate(const double3 gp, const int3 bcell, const FdGrid& sg, const double3 cB,
-                                               const fd_quat qB, const FdGeo& GB, const double* sdf, double rB2,
+                                               const fd_quat qB, const FdGeo& GB, const double4* quads, double rB2,
                                                double probe, double& overlap, double& fx, double& fy, double& fz,
                                                double p[8])
 {
@@ -1378,15 +1397,10 @@ __device__ __forceinline__ bool node_predicate(const double3 gp, const int3 bcel
     fy = gy - (double)j0;
     fz = gz - (double)k0;
     const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
-    const double* S = sdf + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
-    p[0] = __ldg(S);
-    p[1] = __ldg(S + 1);
-    p[2] = __ldg(S + sx);
-    p[3] = __ldg(S + sx + 1);
-    p[4] = __ldg(S + sxy);
-    p[5] = __ldg(S + sxy + 1);
-    p[6] = __ldg(S + sxy + sx);
-    p[7] = __ldg(S + sxy + sx + 1);
+    const double4* S = quads + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
+    const double4 s0 = load_quad(S), s1 = load_quad(S + sxy);
+    p[0] = s0.x; p[1] = s0.y; p[2] = s0.z; p[3] = s0.w;
+    p[4] = s1.x; p[5] = s1.y; p[6] = s1.z; p[7] = s1.w;
     overlap = -xm_trilinear(fx, fy, fz, p);
     return overlap >= -probe;
 }
@@ -1479,11 +1493,12 @@ __device__ __forceinline__ bool node_filtered(const float4 p, const CullXf& x, c
     const float fx = gx - i0, fy = gy - j0, fz = gz - k0;
     if (GB.lip < 4.0) {
         const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
-        const float* S = SB.sdf32 + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
-        const float c00 = __ldg(S) * (1.f - fx) + __ldg(S + 1) * fx;
-        const float c10 = __ldg(S + sx) * (1.f - fx) + __ldg(S + sx + 1) * fx;
-        const float c01 = __ldg(S + sxy) * (1.f - fx) + __ldg(S + sxy + 1) * fx;
-        const float c11 = __ldg(S + sxy + sx) * (1.f - fx) + __ldg(S + sxy + sx + 1) * fx;
+        const float4* S = SB.sdf32_quad + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
+        const float4 s0 = __ldg(S), s1 = __ldg(S + sxy);
+        const float c00 = s0.x * (1.f - fx) + s0.y * fx;
+        const float c10 = s0.z * (1.f - fx) + s0.w * fx;
+        const float c01 = s1.x * (1.f - fx) + s1.y * fx;
+        const float c11 = s1.z * (1.f - fx) + s1.w * fx;
         const float phi = (c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz;
         const float slack = (float)GB.lip * perr + 1e-5f * (fabsf(phi) + (float)GB.spacing);
         return phi - (float)probe > slack;
@@ -1772,9 +1787,9 @@ __device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, int A, int B
 {
     const FdGeo& GA = n.G.geo[n.P.geo[A]];
     e.cA = n.P.pos[A];
-    const fd_quat qA = n.P.q[A];
+    const fd_quat qA = load_q(n.P.q + A);
     e.cB = Slave<KIND>::pos(n, B);
-    e.qB = Slave<KIND>::q(n, B);
+    e.qB = load_q(Slave<KIND>::q(n, B));
     const FdGeo& GB = Slave<KIND>::geo(n, B);
     const GeoSetDev& SB = Slave<KIND>::set(n);
     const FdGrid& sg = Slave<KIND>::grid(n);
@@ -1784,7 +1799,35 @@ __device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, int A, int B
     e.r = xm_rot(qA, node);
     e.gp = mk3(e.r.x + e.cA.x, e.r.y + e.cA.y, e.r.z + e.cA.z);
     e.ov = ov0;
-    return node_predicate<KIND>(e.gp, bcell, sg, e.cB, e.qB, GB, SB.sdf, rB2, n.a.probe, e.ov, e.fx, e.fy, e.fz, e.pv);
+    return node_predicate<KIND>(e.gp, bcell, sg, e.cB, e.qB, GB, SB.sdf_quad, rB2, n.a.probe, e.ov, e.fx, e.fy, e.fz, e.pv);
+}
+
+// A contact's results go out in 16-byte stores to five whole sectors.  As seven
+// arrays (force, point, normal, overlap, energies) they were 18 stores to
+// about eleven part-written sectors at as many places.
+__device__ __forceinline__ void store_record(const PairListDev& L, int s, double3 pt, double3 nrm, double ov,
+                                             double en, double es)
+{
+    double2* o = reinterpret_cast<double2*>(L.c_rec + (long long)CONTACT_REC * s + CONTACT_POINT);
+    o[0] = make_double2(pt.x, pt.y);
+    o[1] = make_double2(pt.z, nrm.x);
+    o[2] = make_double2(nrm.y, nrm.z);
+    o[3] = make_double2(ov, en);
+    reinterpret_cast<double*>(o)[8] = es;
+}
+__device__ __forceinline__ void store_force(const PairListDev& L, int s, const double f[9])
+{
+    double2* o = reinterpret_cast<double2*>(L.c_rec + (long long)CONTACT_REC * s);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) o[t] = make_double2(f[2 * t], f[2 * t + 1]);
+    reinterpret_cast<double*>(o)[8] = f[8];
+}
+__device__ __forceinline__ void store_force(const PairListDev& L, int s, const float f[9])
+{
+    float4* o = reinterpret_cast<float4*>(L.c_rec + (long long)CONTACT_REC * s);
+    o[0] = make_float4(f[0], f[1], f[2], f[3]);
+    o[1] = make_float4(f[4], f[5], f[6], f[7]);
+    reinterpret_cast<float*>(o)[8] = f[8];
 }
 
 // Slot s of list L, a contact by the predicate e: normal, contact point,
@@ -1921,15 +1964,7 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
                 ks = (ks > 0. && ksj > 0.) ? ks * ksj / (ks + ksj) : 0.;
             }
         }
-        L.c_point[3 * s + 0] = pt.x;
-        L.c_point[3 * s + 1] = pt.y;
-        L.c_point[3 * s + 2] = pt.z;
-        L.c_normal[3 * s + 0] = nrm.x;
-        L.c_normal[3 * s + 1] = nrm.y;
-        L.c_normal[3 * s + 2] = nrm.z;
-        L.c_overlap[s] = ov;
-        L.c_en[s] = 0.5 * ov * ov * kn;
-        L.c_es[s] = 0.5 * lengthSq3(spring) * ks;
+        store_record(L, s, pt, nrm, ov, 0.5 * ov * ov * kn, 0.5 * lengthSq3(spring) * ks);
     }
     return nid;
 }
@@ -1999,8 +2034,11 @@ __device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int
                                        PASS == 0 ? __longlong_as_double(0x7ff0000000000000ll) : 0., e);
             if (phi0_store) L.c_phi0[s] = __double2float_rd(-e.ov);
             int nid = -1;
-            if (PASS == 1 && hit)
-                nid = contact_law<KIND>(n, L, n.a.rec, s, A, B, k, aux.w, hist, e, L.c_force + 9ll * s);
+            if (PASS == 1 && hit) {
+                double o[9];
+                nid = contact_law<KIND>(n, L, n.a.rec, s, A, B, k, aux.w, hist, e, o);
+                if (n.with_force) store_force(L, s, o);
+            }
             if (PASS == 1) {
                 L.c_node[s] = nid;
             } else {
@@ -2033,76 +2071,75 @@ __device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int
 }
 
 // ---------------------------------------------------------------------------
-// narrow phase, stage 3: the pair's force and torques summed over its contact
-// slots.  Eight lanes per pair: lane l sums slots l, l + 8, ... in order, then
-// a fixed butterfly combines the lanes, so the result does not depend on
-// where the pair's slots lie.
+// narrow phase, stage 3: the force and torques of each pair that holds a
+// contact, summed over its contacts in slot order (ascending node keys), eight
+// lanes per pair.  The order is the contacts' own: slots without one, of which
+// a cached list holds more, do not change the sum.
+//
+// Bound by the latency of pair, slots, node ids and forces, four loads that
+// wait for one another.  Three pairs in four hold no contact (a settled bed: 8
+// slots and a quarter of a contact per pair), so a warp takes 32 pairs' flags
+// in one load, the next ones' meanwhile, and passes on to those that hold one;
+// with eight lanes looking at each pair the sums took
+// 105 us for 262,144 particles, this way 65.
 // ---------------------------------------------------------------------------
 template <typename Real>
 __device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int block, int nblocks, bool link,
-                                         const RevDev& R, int n_obj)
+                                         const RevDev& R, int n_obj, int3* list)
 {
-    const Real* cf = reinterpret_cast<const Real*>(L.c_force);
     Real* pf = reinterpret_cast<Real*>(L.pf);
-    const int npairs = min(*L.n_pairs, L.cap_pairs);
+    const unsigned int full = 0xffffffffu;
     const int lane = threadIdx.x & 31, grp = lane >> 3, l = lane & 7;
-    const int warp = (block * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (nblocks * blockDim.x) >> 5;
-    const unsigned int build = link ? *R.build : 0u;
-    for (int p0 = warp * 4; p0 < npairs; p0 += nwarps * 4) {
-        const int p = p0 + grp;
-        Real acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        int o = 0, c = 0;
-        bool hit = false;
-        if (p < npairs) {
-            c = L.c_cnt[p];
-            hit = L.p_hit[p] != 0;
-            if (hit) o = L.c_off[p];
-        }
-        // a list that is built: the pair joins its partner's list of the
+    const int thread = block * blockDim.x + threadIdx.x, nthreads = nblocks * blockDim.x;
+    const int npairs = min(*L.n_pairs, L.cap_pairs);
+    if (link) {
+        // a list that is built: each pair joins its partner's list of the
         // reverse index (only pairs with contact slots carry a force)
-        if (link && l == 0 && c > 0) {
+        const unsigned int build = *R.build;
+        for (int p = thread; p < npairs; p += nthreads) {
+            if (L.c_cnt[p] <= 0) continue;
             const int B = L.pairB[p];
-            if (B >= 0 && B < n_obj) {
-                const unsigned int code = (unsigned int)(p * 8 + kind);  // pair counts stay below 2^28
-                const unsigned long long old =
-                    atomicExch(&R.head[B], ((unsigned long long)build << 32) | code);
-                L.r_next[p] = (unsigned int)(old >> 32) == build ? (int)(unsigned int)old : -1;
+            if (B < 0 || B >= n_obj) continue;
+            const unsigned int code = (unsigned int)(p * 8 + kind);  // pair counts stay below 2^28
+            const unsigned long long old = atomicExch(&R.head[B], ((unsigned long long)build << 32) | code);
+            L.r_next[p] = (unsigned int)(old >> 32) == build ? (int)(unsigned int)old : -1;
+        }
+    }
+    const int stride = nthreads >> 5 << 5;
+    int p = thread;
+    bool next = p < npairs && L.p_hit[p] != 0;
+    for (int p0 = thread & ~31; p0 < npairs; p0 += stride) {
+        const bool hit = next;
+        const unsigned int m = __ballot_sync(full, hit);
+        if (hit) list[__popc(m & ((1u << lane) - 1u))] = make_int3(p, L.c_off[p], L.c_cnt[p]);
+        const int count = __popc(m);
+        p += stride;
+        next = p < npairs && L.p_hit[p] != 0;  // the next pairs' flags, meanwhile
+        __syncwarp();
+        for (int i0 = 0; i0 < count; i0 += 4) {
+            const bool on = i0 + grp < count;
+            const int3 q = on ? list[i0 + grp] : make_int3(0, 0, 0);
+            const int o = q.y, c = q.z;
+            Real acc = 0, acc8 = 0;
+            // eight slots at a time: lane l looks at slot l, then adds component
+            // l (lane 0 also the ninth) of the contacts among them in turn
+            const int cmax = __reduce_max_sync(full, c);
+            for (int j0 = 0; j0 < cmax; j0 += 8) {
+                const bool contact = j0 + l < c && L.c_node[o + j0 + l] >= 0;
+                unsigned int m = (__ballot_sync(full, contact) >> (8 * grp)) & 0xffu;
+                for (; m; m &= m - 1u) {
+                    const Real* f =
+                        reinterpret_cast<const Real*>(L.c_rec + (long long)CONTACT_REC * (o + j0 + __ffs(m) - 1));
+                    acc += f[l];
+                    if (l == 0) acc8 += f[8];
+                }
+            }
+            if (on) {
+                pf[9ll * q.x + l] = acc;
+                if (l == 0) pf[9ll * q.x + 8] = acc8;
             }
         }
-        // three pairs in four hold no contact (settled beds: 8 slots and a
-        // quarter of a contact per pair): their slots are not looked at, and
-        // the force sums skip them by the same flag.  With every pair's slots
-        // read the sums took 118 us for 262,144 particles.
-        if (!hit) c = 0;
-        // slots l, l + 8, l + 16, ... in order; four node ids loaded ahead
-        for (int j0 = l; j0 < c; j0 += 32) {
-            int nd[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) nd[u] = j0 + 8 * u < c ? L.c_node[o + j0 + 8 * u] : -1;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (nd[u] < 0) continue;
-                const Real* f = cf + 9ll * (o + j0 + 8 * u);
-#pragma unroll
-                for (int t = 0; t < 9; ++t) acc[t] += f[t];
-            }
-        }
-        if (__any_sync(0xffffffffu, c > 0)) {
-#pragma unroll
-            for (int t = 0; t < 9; ++t) {
-                acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 4);
-                acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 2);
-                acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 1);
-            }
-        }
-        if (p < npairs && c > 0) {
-            Real* out = pf + 9ll * p;
-#pragma unroll
-            for (int t = 0; t < 8; ++t)
-                if (l == t) out[t] = acc[t];
-            if (l == 0) out[8] = acc[8];
-        }
+        __syncwarp();
     }
 }
 
@@ -2199,7 +2236,7 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int
     e.cA = cA;
     e.cB = cB;
     e.pool = GA.node_off + k;
-    e.rd = xm_rot(n.P.q[A], n.G.nodes[e.pool]);
+    e.rd = xm_rot(load_q(n.P.q + A), n.G.nodes[e.pool]);
     const double3 gp = mk3(e.rd.x + cA.x, e.rd.y + cA.y, e.rd.z + cA.z);
     e.gp = gp;
     int3 lo, hi;
@@ -2212,7 +2249,7 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int
     if (bcell.x >= lo.x && bcell.x <= hi.x && bcell.y >= lo.y && bcell.y <= hi.y && bcell.z >= lo.z && bcell.z <= hi.z) {
         const double3 rel = mk3(gp.x - cB.x, gp.y - cB.y, gp.z - cB.z);
         if (!Slave<KIND>::radius_test || xm_len2(rel) <= GB.radius * GB.radius) {
-            const double3 lp = xm_rrot(rel, Slave<KIND>::q(n, B));
+            const double3 lp = xm_rrot(rel, load_q(Slave<KIND>::q(n, B)));
             const double gx = (lp.x - GB.origin.x) * GB.inv_spacing;
             const double gy = (lp.y - GB.origin.y) * GB.inv_spacing;
             const double gz = (lp.z - GB.origin.z) * GB.inv_spacing;
@@ -2230,9 +2267,8 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int
                     // of a metre): single-precision interpolation
                     // there would carry errors of 1e-8 m, so the
                     // (few) wall contacts interpolate in double
-                    const double* S = SB.sdf + c0;
-                    double pd[8] = {__ldg(S), __ldg(S + 1), __ldg(S + sx), __ldg(S + sx + 1), __ldg(S + sxy),
-                                    __ldg(S + sxy + 1), __ldg(S + sxy + sx), __ldg(S + sxy + sx + 1)};
+                    const double4 s0 = load_quad(SB.sdf_quad + c0), s1 = load_quad(SB.sdf_quad + c0 + sxy);
+                    double pd[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
                     const double ovd = -xm_trilinear(gx - (double)i0, gy - (double)j0, gz - (double)k0, pd);
 #pragma unroll
                     for (int c = 0; c < 8; ++c) pv[c] = (float)pd[c];
@@ -2240,10 +2276,9 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int
                     e.phi0 = __double2float_rd(-ovd);
                     hit = ovd >= -n.a.probe;
                 } else {
-                    const float* S = SB.sdf32 + c0;
-                    pv[0] = __ldg(S); pv[1] = __ldg(S + 1); pv[2] = __ldg(S + sx); pv[3] = __ldg(S + sx + 1);
-                    pv[4] = __ldg(S + sxy); pv[5] = __ldg(S + sxy + 1); pv[6] = __ldg(S + sxy + sx);
-                    pv[7] = __ldg(S + sxy + sx + 1);
+                    const float4 s0 = __ldg(SB.sdf32_quad + c0), s1 = __ldg(SB.sdf32_quad + c0 + sxy);
+                    pv[0] = s0.x; pv[1] = s0.y; pv[2] = s0.z; pv[3] = s0.w;
+                    pv[4] = s1.x; pv[5] = s1.y; pv[6] = s1.z; pv[7] = s1.w;
                     const float c00 = pv[0] * (1.f - fx) + pv[1] * fx, c10 = pv[2] * (1.f - fx) + pv[3] * fx;
                     const float c01 = pv[4] * (1.f - fx) + pv[5] * fx, c11 = pv[6] * (1.f - fx) + pv[7] * fx;
                     e.ov = -((c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz);
@@ -2303,7 +2338,7 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
         }
     }
     if (R.hit && s < R.cap) {
-        const fd_quat qB = Slave<KIND>::q(n, B);
+        const fd_quat qB = load_q(Slave<KIND>::q(n, B));
         R.A[s] = A;
         R.B[s] = B;
         R.Bp[s] = KIND == FD_PW ? -1 : B;
@@ -2382,15 +2417,8 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
     L.c_spring[3 * s + 1] = spring.y;
     L.c_spring[3 * s + 2] = spring.z;
     if (n.a.records) {
-        L.c_point[3 * s + 0] = cA.x + arm.x;
-        L.c_point[3 * s + 1] = cA.y + arm.y;
-        L.c_point[3 * s + 2] = cA.z + arm.z;
-        L.c_normal[3 * s + 0] = nrm.x;
-        L.c_normal[3 * s + 1] = nrm.y;
-        L.c_normal[3 * s + 2] = nrm.z;
-        L.c_overlap[s] = ov;
-        L.c_en[s] = 0.5 * (double)ov * (double)ov * (double)kn;
-        L.c_es[s] = 0.5 * lengthSq3(spring) * (double)ks;
+        store_record(L, s, mk3(cA.x + arm.x, cA.y + arm.y, cA.z + arm.z), mk3(nrm.x, nrm.y, nrm.z), ov,
+                     0.5 * (double)ov * (double)ov * (double)kn, 0.5 * lengthSq3(spring) * (double)ks);
     }
     return nid;
 }
@@ -2399,7 +2427,6 @@ template <int KIND, int PASS>
 __device__ __forceinline__ void contact_list32(const NarrowArgs& n, int block, int nblocks)
 {
     const PairListDev& L = n.L;
-    float* cf = reinterpret_cast<float*>(L.c_force);
     // pass 0: every slot; pass 1: the slots pass 0 listed as contacts
     const int nitems = PASS == 0 ? min(*L.n_slots, L.cap_contacts) : min(*L.n_hits, L.cap_contacts);
     const int lane = threadIdx.x & 31;
@@ -2458,8 +2485,11 @@ __device__ __forceinline__ void contact_list32(const NarrowArgs& n, int block, i
                                          PASS == 0 ? __int_as_float(0x7f800000) : 0.f, e);
             if (phi0_store) L.c_phi0[s] = e.phi0;
             int nid = -1;
-            if (PASS == 1 && hit)
-                nid = contact_law32<KIND>(n, L, n.a.rec, s, A, B, k, aux.w, hist, e, cf + 9ll * s);
+            if (PASS == 1 && hit) {
+                float o[9];
+                nid = contact_law32<KIND>(n, L, n.a.rec, s, A, B, k, aux.w, hist, e, o);
+                if (n.with_force) store_force(L, s, o);
+            }
             if (PASS == 1) {
                 L.c_node[s] = nid;
             } else {
@@ -2523,7 +2553,9 @@ __global__ void __launch_bounds__(TPB) k_sum_lists(ListSet a, RevDev R)
     int block, nblocks;
     const int li = list_of(a, block, nblocks);
     const NarrowArgs& n = a.l[li];
-    sum_list<Real>(n.L, a.kind[li], block, nblocks, a.kind[li] != FD_PW && rev_built(R), R, n.P.n);
+    __shared__ int3 s_list[TPB / 32][32];
+    sum_list<Real>(n.L, a.kind[li], block, nblocks, a.kind[li] != FD_PW && rev_built(R), R, n.P.n,
+                   s_list[threadIdx.x >> 5]);
 }
 
 // End of a step.  The reverse index, where a list was built; under the pair
@@ -2796,12 +2828,18 @@ template <typename Real> struct ForceSum {
         T[1] += pf[torque + 1];
         T[2] += pf[torque + 2];
     }
-    // the pairs the particle owns in one list
-    __device__ __forceinline__ void own(const PairListDev& L, int i)
+    // the pairs the particle owns in one list (s: first, c: count; no contact,
+    // no sum kept), four hit flags loaded ahead
+    __device__ __forceinline__ void own(const PairListDev& L, int s, int c)
     {
-        const int s = L.seg_off[i], c = L.seg_cnt[i];
-        for (int k = s; k < s + c; ++k)
-            if (L.p_hit[k]) add(reinterpret_cast<const Real*>(L.pf) + 9ll * k, Real(1), 3);  // no contact, no sum kept
+        for (int k = s; k < s + c; k += 4) {
+            int h[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) h[u] = k + u < s + c ? L.p_hit[k + u] : 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (h[u]) add(reinterpret_cast<const Real*>(L.pf) + 9ll * (k + u), Real(1), 3);
+        }
     }
     __device__ __forceinline__ void bonds(const BondDev& B, int i)
     {
@@ -2845,18 +2883,33 @@ __global__ void __launch_bounds__(128) k_advance(AdvanceArgs a)
         if (SUM) {
             const ReduceArgs& r = a.r;
             ForceSum<Real> f;
-            // pairs the particle owns, kind by kind
-            for (int kind = 0; kind < FD_NKIND; ++kind)
-                if (r.active[kind]) f.own(r.L[kind], i);
-            // pairs in which it is the partner, by owner
-            const int rs = r.R.off[i], rc = min(r.R.cnt[i], r.R.cap - rs);
-            for (int e = rs; e < rs + rc; ++e) {
-                const int code = r.R.code[e];
-                const int kind = code & 7, k = code >> 3;
-                const PairListDev& L = r.L[kind];
-                if (!L.p_hit[k]) continue;
-                if (kind != FD_PP && L.pairA[k] == i) continue;  // a particle against its own ghost
-                f.add(reinterpret_cast<const Real*>(L.pf) + 9ll * k, Real(-1), 6);
+            // pairs the particle owns, kind by kind, then those in which it is
+            // the partner, by owner.  Ranges, codes, flags and sums are loads
+            // that wait for one another: those of all kinds, and of four
+            // codes, are under way together
+            int so[FD_NKIND], sc[FD_NKIND];
+#pragma unroll
+            for (int kind = 0; kind < FD_NKIND; ++kind) {
+                so[kind] = r.active[kind] ? r.L[kind].seg_off[i] : 0;
+                sc[kind] = r.active[kind] ? r.L[kind].seg_cnt[i] : 0;
+            }
+            const int rs = r.R.off[i], re = rs + min(r.R.cnt[i], r.R.cap - rs);
+#pragma unroll
+            for (int kind = 0; kind < FD_NKIND; ++kind) f.own(r.L[kind], so[kind], sc[kind]);
+            for (int e = rs; e < re; e += 4) {
+                int code[4], h[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) code[u] = e + u < re ? r.R.code[e + u] : -1;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) h[u] = code[u] >= 0 ? r.L[code[u] & 7].p_hit[code[u] >> 3] : 0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (!h[u]) continue;
+                    const int kind = code[u] & 7, k = code[u] >> 3;
+                    const PairListDev& L = r.L[kind];
+                    if (kind != FD_PP && L.pairA[k] == i) continue;  // a particle against its own ghost
+                    f.add(reinterpret_cast<const Real*>(L.pf) + 9ll * k, Real(-1), 6);
+                }
             }
             if (r.B.n > 0) f.bonds(r.B, i);
             F = mk3((double)f.F[0], (double)f.F[1], (double)f.F[2]);
@@ -2902,15 +2955,17 @@ __global__ void __launch_bounds__(128) k_advance(AdvanceArgs a)
 // staged kernels is 24 dependent launches, each a few microseconds of latency
 // and next to no work at these sizes: 102 us a step for 1,000 particles in a
 // graph replay.  Here a step is two launches.  k_small_pairs takes each
-// particle's partners and walls from the cell lists, and each candidate pair
-// through culling, predicate, contact law and pair sum in one warp;
-// k_small_advance sums each particle's pairs and runs the half kicks, the drift, the hash
-// and the cell lists of the next step.  The sums run in the staged kernels'
-// order, so the results are theirs.  A warp keeps only its pair's few slots
-// busy in the contact law, so large sets stay with the staged kernels.
+// particle's partners and walls from the cell lists, culls each candidate pair
+// in one warp, takes the block's slots through predicate and contact law one
+// thread each, and sums its pairs with eight lanes each; k_small_advance sums
+// each particle's pairs and runs the half kicks, the drift, the hash and the
+// cell lists of the next step.  The sums run in the staged kernels' order, so
+// the results are theirs.  A block's few slots leave most of its threads idle
+// in the contact law, so large sets stay with the staged kernels.
 // ---------------------------------------------------------------------------
 constexpr int SMALL_BODIES = 4;               // particles per block
 constexpr int SMALL_WARPS = 2 * SMALL_BODIES;  // a warp for each one's partners, one for its walls
+constexpr int SMALL_TASKS = SMALL_BODIES * MAX_CAND;  // pairs of a block, per kind
 constexpr int MAX_FOUND = 512;                // objects of the cells around a particle, staged for the test
 
 struct SmallArgs {
@@ -2923,15 +2978,12 @@ struct SmallArgs {
     void* own;             // per particle: force and torque of its own pairs (6 Real)
 };
 
-// one pair of list L, one warp: slots, predicate, law, pair sum; returns its
-// contacts
-template <int KIND, bool MIXED>
-__device__ __forceinline__ int small_pair(const SmallArgs& a, const PairListDev& L, const AdjRec& R, int p, int A,
-                                          int B, int lane, unsigned short* queue, unsigned long long* stats)
+// one pair of list L, one warp: its slots, written to L.c_k.  Returns the first
+// slot, their count, and the slots of the pair's history.
+template <int KIND>
+__device__ __forceinline__ int4 small_slots(const NarrowArgs& n, const PairListDev& L, int p, int A, int B, int lane,
+                                            unsigned short* queue, unsigned long long* stats)
 {
-    using Real = typename std::conditional<MIXED, float, double>::type;
-    const NarrowArgs& n = a.n;
-    const unsigned int full = 0xffffffffu;
     int kept;
     int ncand = cull_pair<KIND>(n, A, B, 0.0, lane, queue, kept);
     if (n.a.stats && lane == 0) {
@@ -2940,92 +2992,56 @@ __device__ __forceinline__ int small_pair(const SmallArgs& a, const PairListDev&
         atomicAdd(&stats[2], (unsigned long long)kept);
         atomicAdd(&stats[4], (unsigned long long)ncand);
     }
-    if (ncand == 0) {
-        if (lane == 0) {
-            L.c_off[p] = 0;
-            L.c_cnt[p] = 0;
+    int4 slot = make_int4(0, 0, 0, 0);
+    if (ncand > 0) {
+        if (lane == 0) slot.x = atomicAdd(L.n_slots, ncand);
+        find_history(L, A, B, lane, slot.z, slot.w);
+        slot.x = __shfl_sync(0xffffffffu, slot.x, 0);
+        slot.y = ncand;
+        if (slot.x + ncand > L.cap_contacts) {
+            if (lane == 0) set_flag(n.a.flags, FD_FLAG_CONTACT_OVERFLOW);
+            slot.x = slot.y = 0;
         }
-        return 0;
-    }
-    int base = 0;
-    if (lane == 0) base = atomicAdd(L.n_slots, ncand);
-    int oc_off, oc_cnt;
-    find_history(L, A, B, lane, oc_off, oc_cnt);
-    base = __shfl_sync(full, base, 0);
-    if (base + ncand > L.cap_contacts) {
-        if (lane == 0) set_flag(n.a.flags, FD_FLAG_CONTACT_OVERFLOW);
-        base = 0;
-        ncand = 0;
     }
     if (lane == 0) {
-        L.c_off[p] = base;
-        L.c_cnt[p] = ncand;
+        L.c_off[p] = slot.x;
+        L.c_cnt[p] = slot.y;
     }
+    for (int i = lane; i < slot.y; i += 32) L.c_k[slot.x + i] = queue[i];
+    return slot;
+}
+
+// one slot of pair (A, B) of list L: predicate and contact law; true for a contact
+template <int KIND, bool MIXED>
+__device__ __forceinline__ bool small_contact(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int A, int B,
+                                              int s, int oc_off, int oc_cnt)
+{
+    using Real = typename std::conditional<MIXED, float, double>::type;
     int3 bcell;
     decode_cell(Slave<KIND>::hash(n, B), Slave<KIND>::grid(n).size, bcell);
-    Real acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    int hits = 0;
-    for (int i0 = 0; i0 < ncand; i0 += 32) {
-        const int i = i0 + lane, s = base + i;
-        Real o[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        bool hit = false;
-        if (i < ncand) {
-            const int k = queue[i];
-            int nid = -1;
-            if (MIXED) {
-                SlotEval32 e;
-                hit = slot_predicate32<KIND>(n, A, B, k, bcell, 0.f, e);
-                if (hit)
-                    nid = contact_law32<KIND>(n, L, R, s, A, B, k, oc_off, oc_cnt, e, reinterpret_cast<float*>(o));
-            } else {
-                SlotEval e;
-                hit = slot_predicate<KIND>(n, A, B, k, bcell, 0., e);
-                if (hit)
-                    nid = contact_law<KIND>(n, L, R, s, A, B, k, oc_off, oc_cnt, e, reinterpret_cast<double*>(o));
-            }
-            L.c_k[s] = k;
-            L.c_node[s] = nid;
-            if (R.hit && s < R.cap) R.hit[s] = hit ? 1 : 0;
-        }
-        const unsigned int m = __ballot_sync(full, hit);
-        hits += __popc(m);
-        if (m == 0) continue;
-        // k_pair_sum's order: lane l of eight adds slots l, l + 8, ... in turn
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int src = (lane & 7) + 8 * u;
-            const bool on = (m >> src) & 1u;
-#pragma unroll
-            for (int t = 0; t < 9; ++t) {
-                const Real v = __shfl_sync(full, o[t], src);
-                if (on) acc[t] += v;
-            }
-        }
+    const int k = L.c_k[s];
+    int nid = -1;
+    bool hit;
+    Real o[9];
+    if constexpr (MIXED) {
+        SlotEval32 e;
+        hit = slot_predicate32<KIND>(n, A, B, k, bcell, 0.f, e);
+        if (hit) nid = contact_law32<KIND>(n, L, R, s, A, B, k, oc_off, oc_cnt, e, o);
+    } else {
+        SlotEval e;
+        hit = slot_predicate<KIND>(n, A, B, k, bcell, 0., e);
+        if (hit) nid = contact_law<KIND>(n, L, R, s, A, B, k, oc_off, oc_cnt, e, o);
     }
-    // a pair without a contact sums to zero: nobody reads it
-    if (hits == 0) return 0;
-#pragma unroll
-    for (int t = 0; t < 9; ++t) {
-        acc[t] += __shfl_xor_sync(full, acc[t], 4);
-        acc[t] += __shfl_xor_sync(full, acc[t], 2);
-        acc[t] += __shfl_xor_sync(full, acc[t], 1);
-    }
-    Real* out = reinterpret_cast<Real*>(L.pf) + 9ll * p;
-#pragma unroll
-    for (int t = 0; t < 9; ++t)
-        if (lane == t) out[t] = acc[t];
-    if (lane == 0) {
-        atomicAdd(L.n_hits, hits);
-        if (KIND == FD_PP) L.r_next[p] = atomicExch(&a.r_head[B], p);
-        if (n.a.stats) atomicAdd(&stats[3], (unsigned long long)hits);
-    }
-    return hits;
+    if (hit) store_force(L, s, o);
+    L.c_node[s] = nid;
+    if (R.hit && s < R.cap) R.hit[s] = hit ? 1 : 0;
+    return hit;
 }
 
 // the pairs of particle A with the partners in list[0 .. cnt - 1], one warp:
 // ascending partners, and a task for each; range: the tasks' first and count
 __device__ __forceinline__ void small_emit(const PairListDev& L, unsigned int* flags, int A, const int* list, int cnt,
-                                           int kind, int lane, int4* task, int* ntask, int2* range)
+                                           int lane, int2* task, int* ntask, int2* range)
 {
     const unsigned int full = 0xffffffffu;
     if (cnt > MAX_CAND && lane == 0) set_flag(flags, FD_FLAG_NEIGHBOR_OVERFLOW);
@@ -3054,7 +3070,7 @@ __device__ __forceinline__ void small_emit(const PairListDev& L, unsigned int* f
         for (int j = 0; j < n; ++j) r += (list[j] < v);
         L.pairA[base + r] = A;
         L.pairB[base + r] = v;
-        task[t0 + r] = make_int4(A, v, base + r, kind);
+        task[t0 + r] = make_int2(v, SMALL_BODIES * (base + r) + A % SMALL_BODIES);
     }
     __syncwarp();
 }
@@ -3066,19 +3082,29 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
     // the candidate lists and the node queues are not in use together
     __shared__ union {
         unsigned short queue[SMALL_WARPS][MAX_NODE_QUEUE];
-        int found[SMALL_BODIES][MAX_FOUND];
-    } u;
-    __shared__ int s_list[SMALL_WARPS][MAX_CAND];
-    __shared__ int4 s_task[SMALL_WARPS * MAX_CAND];
-    __shared__ unsigned char s_hit[SMALL_WARPS * MAX_CAND];
+        struct {
+            int found[SMALL_BODIES][MAX_FOUND];
+            int list[SMALL_WARPS][MAX_CAND];
+        } c;
+    } q;
+    // the block's pairs (partner, SMALL_BODIES * pair + body), partners in the
+    // first half, walls in the second; their first slots and those of their
+    // histories, and the counts of both; the first slot of each in the block's
+    // order, partners then walls, the walls' from a multiple of 32; contacts
+    __shared__ int2 s_task[2 * SMALL_TASKS];
+    __shared__ int2 s_slot[2 * SMALL_TASKS];
+    __shared__ ushort2 s_cnt[2 * SMALL_TASKS];
+    __shared__ int s_first[2 * SMALL_TASKS + 1];
+    __shared__ int s_hits[2 * SMALL_TASKS];
     __shared__ int2 s_range[SMALL_WARPS];
-    __shared__ int s_ntask;
+    __shared__ int s_ntask[2], s_pw;
     __shared__ unsigned long long s_stats[5];
     const NarrowArgs& n = a.n;
     const unsigned int full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int body = wib % SMALL_BODIES;
-    if (threadIdx.x == 0) s_ntask = 0;
+    if (threadIdx.x < 2) s_ntask[threadIdx.x] = 0;
+    for (int t = threadIdx.x; t < 2 * SMALL_TASKS; t += blockDim.x) s_hits[t] = 0;
     if (threadIdx.x < 5) s_stats[threadIdx.x] = 0ull;
     if (threadIdx.x < SMALL_WARPS) s_range[threadIdx.x] = make_int2(0, 0);
     __syncthreads();
@@ -3086,17 +3112,17 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
     const unsigned int build = T.build[T.par];
     // the other generation's step needs a number no head can hold
     if (blockIdx.x == 0 && threadIdx.x == 0) T.build[T.par ^ 1] = build + 1u;
-    const int A = blockIdx.x * SMALL_BODIES + body;
+    const int A0 = blockIdx.x * SMALL_BODIES, A = A0 + body;
     if (A < n.P.n) {
         const double3 cA = n.P.pos[A];
         const double rA = n.G.geo[n.P.geo[A]].radius;
-        int* list = s_list[wib];
+        int* list = q.c.list[wib];
         int cnt = 0;
         int3 lo, hi;
         if (wib < SMALL_BODIES) {
             // partners: each lane walks the list of a cell, and the objects
             // found are tested side by side (a test is a chain of five loads)
-            int* found = u.found[body];
+            int* found = q.c.found[body];
             partner_search_range(cA, (rA + n.G.rmax) * (1.0 + 8.0 * BOUND_REL), T.g, lo, hi);
             const int nx = hi.x - lo.x + 1, ny = hi.y - lo.y + 1, nz = hi.z - lo.z + 1;
             const int ncell = nx * ny * nz;
@@ -3139,7 +3165,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
                 }
             }
             test();
-            small_emit(n.L, n.a.flags, A, list, cnt, FD_PP, lane, s_task, &s_ntask, &s_range[wib]);
+            small_emit(n.L, n.a.flags, A, list, cnt, lane, s_task, &s_ntask[0], &s_range[wib]);
         } else {
             body_search_range(cA, rA * (1.0 + BOUND_REL), n.wgrid, lo, hi);
             const int2 wr = a.wall_range ? a.wall_range[A] : make_int2(0, n.W.n);
@@ -3167,18 +3193,102 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
                 cnt += __popc(m);
             }
             __syncwarp();
-            small_emit(a.Lw, n.a.flags, A, list, cnt, FD_PW, lane, s_task, &s_ntask, &s_range[wib]);
+            small_emit(a.Lw, n.a.flags, A, list, cnt, lane, s_task + SMALL_TASKS, &s_ntask[1], &s_range[wib]);
         }
     }
     __syncthreads();
     // the block's pairs, shared out over its warps
-    for (int t = wib; t < s_ntask; t += SMALL_WARPS) {
-        const int4 k = s_task[t];
-        const int hits =
-            k.w == FD_PP ? small_pair<FD_PP, MIXED>(a, n.L, n.a.rec, k.z, k.x, k.y, lane, u.queue[wib], s_stats)
-                         : small_pair<FD_PW, MIXED>(a, a.Lw, a.recw, k.z, k.x, k.y, lane, u.queue[wib], s_stats);
-        if (lane == 0) s_hit[t] = hits > 0;
+    const int npp = s_ntask[0], ntask = npp + s_ntask[1];
+    for (int u = wib; u < ntask; u += SMALL_WARPS) {
+        const bool wall = u >= npp;
+        const int t = wall ? SMALL_TASKS + u - npp : u;
+        const int2 k = s_task[t];
+        const int At = A0 + k.y % SMALL_BODIES, p = k.y / SMALL_BODIES;
+        const int4 slot = wall ? small_slots<FD_PW>(n, a.Lw, p, At, k.x, lane, q.queue[wib], s_stats)
+                               : small_slots<FD_PP>(n, n.L, p, At, k.x, lane, q.queue[wib], s_stats);
+        if (lane == 0) {
+            s_slot[t] = make_int2(slot.x, slot.z);
+            s_cnt[t] = make_ushort2((unsigned short)slot.y, (unsigned short)slot.w);
+        }
         __syncwarp();
+    }
+    __syncthreads();
+    if (wib == 0) {
+        int sum = 0;
+        for (int u0 = 0; u0 < ntask; u0 += 32) {
+            const int u = u0 + lane;
+            const int c = u < ntask ? s_cnt[u >= npp ? SMALL_TASKS + u - npp : u].x : 0;
+            int x = c;
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(full, x, d);
+                if (lane >= d) x += y;
+            }
+            if (u < ntask) s_first[u] = sum + x - c;
+            sum += __shfl_sync(full, x, 31);
+        }
+        __syncwarp();
+        // the walls' slots start a warp
+        const int pw = npp < ntask ? s_first[npp] : sum;
+        const int shift = (32 - (pw & 31)) & 31;
+        __syncwarp();
+        for (int u = npp + lane; u < ntask; u += 32) s_first[u] += shift;
+        if (lane == 0) {
+            s_first[ntask] = sum + shift;
+            s_pw = pw + shift;
+        }
+    }
+    __syncthreads();
+    // the block's slots, a thread each
+    for (int j = threadIdx.x; j < s_first[ntask]; j += blockDim.x) {
+        int lo = 0, hi = ntask;  // the last pair that starts at or before slot j
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (s_first[mid] <= j) lo = mid; else hi = mid;
+        }
+        const bool wall = j >= s_pw;
+        const int t = wall ? SMALL_TASKS + lo - npp : lo;
+        const int2 k = s_task[t], slot = s_slot[t];
+        const ushort2 cnt = s_cnt[t];
+        const int i = j - s_first[lo], At = A0 + k.y % SMALL_BODIES;
+        if (i >= cnt.x) continue;
+        const bool hit =
+            wall ? small_contact<FD_PW, MIXED>(n, a.Lw, a.recw, At, k.x, slot.x + i, slot.y, cnt.y)
+                 : small_contact<FD_PP, MIXED>(n, n.L, n.a.rec, At, k.x, slot.x + i, slot.y, cnt.y);
+        if (hit) atomicAdd(&s_hits[t], 1);
+    }
+    __syncthreads();
+    // the sums of the pairs that hold contacts, as sum_list
+    const int grp = lane >> 3, l = lane & 7;
+    for (int u0 = 4 * wib; u0 < ntask; u0 += 4 * SMALL_WARPS) {
+        const int u = u0 + grp;
+        const bool wall = u >= npp;
+        const int t = u >= ntask ? -1 : wall ? SMALL_TASKS + u - npp : u;
+        const int hits = t >= 0 ? s_hits[t] : 0;
+        const int base = hits ? s_slot[t].x : 0, c = hits ? s_cnt[t].x : 0;
+        const PairListDev& L = wall ? a.Lw : n.L;
+        Real acc = 0, acc8 = 0;
+        const int cmax = __reduce_max_sync(full, c);
+        for (int j0 = 0; j0 < cmax; j0 += 8) {
+            const bool contact = j0 + l < c && L.c_node[base + j0 + l] >= 0;
+            unsigned int m = (__ballot_sync(full, contact) >> (8 * grp)) & 0xffu;
+            for (; m; m &= m - 1u) {
+                const Real* f =
+                    reinterpret_cast<const Real*>(L.c_rec + (long long)CONTACT_REC * (base + j0 + __ffs(m) - 1));
+                acc += f[l];
+                if (l == 0) acc8 += f[8];
+            }
+        }
+        if (!hits) continue;
+        // a pair without a contact sums to zero: nobody reads it
+        const int p = s_task[t].y / SMALL_BODIES;
+        Real* out = reinterpret_cast<Real*>(L.pf) + 9ll * p;
+        out[l] = acc;
+        if (l == 0) {
+            out[8] = acc8;
+            atomicAdd(L.n_hits, hits);
+            if (!wall) L.r_next[p] = atomicExch(&a.r_head[s_task[t].x], p);
+            if (n.a.stats) atomicAdd(&s_stats[3], (unsigned long long)hits);
+        }
     }
     __syncthreads();
     // each particle's own pairs, partners then walls, in order: lane t < 3 sums
@@ -3188,8 +3298,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
         for (int w = 0; w < 2; ++w) {
             const int2 r = s_range[body + w * SMALL_BODIES];
             const Real* pf = reinterpret_cast<const Real*>(w ? a.Lw.pf : n.L.pf);
-            for (int t = r.x; t < r.x + r.y; ++t)
-                if (s_hit[t]) acc += pf[9ll * s_task[t].z + lane];
+            for (int t = r.x + w * SMALL_TASKS; t < r.x + w * SMALL_TASKS + r.y; ++t)
+                if (s_hits[t]) acc += pf[9ll * (s_task[t].y / SMALL_BODIES) + lane];
         }
         reinterpret_cast<Real*>(a.own)[6ll * A + lane] = acc;
     }
@@ -3330,14 +3440,15 @@ __global__ void k_view_gather(PairListDev L, const int* order, long long n, Cont
         const int s = order[i];
         v.master[i] = L.c_node[s];
         v.slave[i] = L.c_slave[s];
+        const double* r = L.c_rec + (long long)CONTACT_REC * s;
         for (int d = 0; d < 3; ++d) {
-            v.point[3 * i + d] = L.c_point[3 * s + d];
-            v.normal[3 * i + d] = L.c_normal[3 * s + d];
+            v.point[3 * i + d] = r[CONTACT_POINT + d];
+            v.normal[3 * i + d] = r[CONTACT_NORMAL + d];
             v.spring[3 * i + d] = L.c_spring[3 * s + d];
         }
-        v.overlap[i] = L.c_overlap[s];
-        v.en[i] = L.c_en[s];
-        v.es[i] = L.c_es[s];
+        v.overlap[i] = r[CONTACT_OVERLAP];
+        v.en[i] = r[CONTACT_EN];
+        v.es[i] = r[CONTACT_ES];
     }
 }
 // the contacts of a list packed field by field (count of them, in no order):
@@ -3351,14 +3462,15 @@ __global__ void k_pack_contacts(PairListDev L, ContactPackDev v, int* at, int co
         const int i = atomicAdd(at, 1);
         if (i >= count) continue;
         v.id[i] = make_int2(node, L.c_slave[s]);
+        const double* r = L.c_rec + (long long)CONTACT_REC * s;
         for (int d = 0; d < 3; ++d) {
-            if (v.point) v.point[3 * i + d] = L.c_point[3 * s + d];
-            if (v.normal) v.normal[3 * i + d] = L.c_normal[3 * s + d];
+            if (v.point) v.point[3 * i + d] = r[CONTACT_POINT + d];
+            if (v.normal) v.normal[3 * i + d] = r[CONTACT_NORMAL + d];
             if (v.spring) v.spring[3 * i + d] = L.c_spring[3 * s + d];
         }
-        if (v.overlap) v.overlap[i] = L.c_overlap[s];
-        if (v.en) v.en[i] = L.c_en[s];
-        if (v.es) v.es[i] = L.c_es[s];
+        if (v.overlap) v.overlap[i] = r[CONTACT_OVERLAP];
+        if (v.en) v.en[i] = r[CONTACT_EN];
+        if (v.es) v.es[i] = r[CONTACT_ES];
     }
 }
 __global__ void k_bond_view(BondDev B, BondViewDev v)
@@ -3410,6 +3522,28 @@ void scan_inclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t
     k_scan_tile<true><<<(unsigned)tiles, SCAN_TPB, 0, s>>>(in, out, n, sums, nullptr); note_launch();
     scan_exclusive(sums, sums, tiles, tmp + tiles, s);
     k_scan_add<<<(unsigned)tiles, SCAN_TPB, 0, s>>>(out, n, sums, nullptr); note_launch();
+}
+
+__global__ void __launch_bounds__(TPB) k_sdf_quads(const double* sdf, const float* sdf32, double4* quad,
+                                                   float4* quad32, int3 size, long long n)
+{
+    const long long sx = size.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        // points of the last column or row start no cell
+        const bool cell = i % sx + 1 < sx && (i / sx) % size.y + 1 < size.y;
+        quad[i] = cell ? make_double4(sdf[i], sdf[i + 1], sdf[i + sx], sdf[i + sx + 1]) : make_double4(0., 0., 0., 0.);
+        quad32[i] =
+            cell ? make_float4(sdf32[i], sdf32[i + 1], sdf32[i + sx], sdf32[i + sx + 1]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+void launch_sdf_quads(const double* sdf, const float* sdf32, double4* quad, float4* quad32, long long off, int3 size,
+                      cudaStream_t s)
+{
+    const long long n = (long long)size.x * size.y * size.z;
+    if (n <= 0) return;
+    k_sdf_quads<<<(int)std::min<long long>((n + TPB - 1) / TPB, 148 * 8), TPB, 0, s>>>(sdf + off, sdf32 + off,
+                                                                                       quad + off, quad32 + off, size, n);
+    note_launch();
 }
 
 void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s, unsigned int* build, int par)
@@ -3567,7 +3701,7 @@ void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream
     else k_contact_lists<false, 1><<<a.block0[n], TPB, 0, s>>>(a);
     note_launch();
     if (!c.with_force) return;
-    share(blocks, shape[3] > 0 ? shape[3] : 4);
+    share(blocks, shape[3] > 0 ? shape[3] : FD_SUM_BLOCKS);
     a = list_set(lists, n, c, blocks);
     if (c.mixed) k_sum_lists<float><<<a.block0[n], TPB, 0, s>>>(a, c.R);
     else k_sum_lists<double><<<a.block0[n], TPB, 0, s>>>(a, c.R);

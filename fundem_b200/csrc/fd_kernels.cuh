@@ -16,6 +16,9 @@
 #define FD_PROBE_MIN_BLOCKS 4
 #endif
 
+#ifndef FD_SUM_BLOCKS
+#define FD_SUM_BLOCKS 8
+#endif
 #ifndef FD_SMALL_MIN_BLOCKS
 #define FD_SMALL_MIN_BLOCKS 2
 #endif
@@ -53,17 +56,16 @@ struct PairListDev {
                        // for the contact-law pass (n_hits of them)
     int* c_k;          // node key of each slot: cluster-order index relative to
                        // the geometry (ascending within a pair)
-    double* c_force;   // 9 per slot: F, torque on A, torque on B (contacts only)
+    // per slot that holds a contact, 20 doubles (five sectors, so that a
+    // contact's result is written whole): [0 .. 8] F, torque on A, torque on B
+    // (of the mode's type), [10 .. 18] with records: contact point, normal,
+    // overlap, normal and tangential energy
+    double* c_rec;
     int4* p_aux;       // per pair: cell of B (x, y, z), first history slot
     int* p_hist_cnt;   // per pair: history slots
     int* r_next;       // per pair: the next pair (code) of its partner's list
     int* p_hit;        // per pair: 1 when a slot of it holds a contact
     double* c_spring;  // 3 per contact
-    double* c_point;   // 3 per contact (records)
-    double* c_normal;  // 3 per contact (records)
-    double* c_overlap; // records
-    double* c_en;      // records
-    double* c_es;      // records
     int* n_slots;      // device counter: slots used
     int* n_hits;       // device counter: contacts (n_slots + 1)
     int cap_contacts;  // slot capacity
@@ -80,6 +82,9 @@ struct PairListDev {
     int* o_c_k;
     double* o_c_spring;
 };
+
+constexpr int CONTACT_REC = 20, CONTACT_POINT = 10, CONTACT_NORMAL = 13, CONTACT_OVERLAP = 16, CONTACT_EN = 17,
+              CONTACT_ES = 18;
 
 // Reverse index over the particle-particle and ghost lists together: for each
 // particle, the pairs in which it is the partner, as codes pair * 8 + kind,
@@ -121,6 +126,10 @@ struct GeoSetDev {
     const FdGeo* geo;
     const double* sdf;
     const float* sdf32;
+    // per grid point the four corner values (x, x + 1) of rows y and y + 1:
+    // what an interpolation reads of one z plane, in one load
+    const double4* sdf_quad;
+    const float4* sdf32_quad;
     const float* dist;
     const float* cellmin;
     const double3* nodes;     // cluster order
@@ -326,6 +335,8 @@ struct BondViewDev {
 // cell hash of each object (-1 outside the grid) and its single-precision
 // rotation rows; build (non-null): the cell table's build numbers, renewed for
 // a step of list generation par
+void launch_sdf_quads(const double* sdf, const float* sdf32, double4* quad, float4* quad32, long long off, int3 size,
+                      cudaStream_t s);
 void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s, unsigned int* build = nullptr, int par = 0);
 // stable sort of n 64-bit keys (key 0 .. num_keys - 1, or negative: last) on
 // the stream: out_idx gets the permutation, out_key the sorted keys (~0 for
