@@ -480,8 +480,9 @@ struct ObjHost {
 };
 
 struct PairGen {
-    DevArray<int> pairA, pairB, seg_off, seg_cnt, c_off, c_cnt, c_node, c_slave, c_k, counters;
-    DevArray<double> pf, c_spring;
+    DevArray<int> pairA, pairB, seg_off, seg_cnt, c_off, c_cnt, c_node, c_at, c_k, counters;
+    DevArray<double> pf;
+    DevArray<double4> c_hist;
 };
 
 struct PairList {
@@ -509,8 +510,8 @@ struct PairList {
         for (PairGen& g : gen) {
             g.pairA.alloc(cap_pairs); g.pairB.alloc(cap_pairs); g.seg_off.alloc(m); g.seg_cnt.alloc(m);
             g.c_off.alloc(cap_pairs); g.c_cnt.alloc(cap_pairs); g.pf.alloc((size_t)cap_pairs * 9);
-            g.c_node.alloc(cap_contacts); g.c_slave.alloc(cap_contacts); g.c_k.alloc(cap_contacts);
-            g.c_spring.alloc((size_t)cap_contacts * 3);
+            g.c_node.alloc(cap_contacts); g.c_at.alloc(cap_contacts); g.c_k.alloc(cap_contacts);
+            g.c_hist.alloc(cap_contacts);
             g.counters.alloc(3);
         }
         c_pair.alloc(cap_contacts); c_hit.alloc(cap_contacts, false); c_rec.alloc((size_t)cap_contacts * fd::CONTACT_REC);
@@ -536,8 +537,8 @@ struct PairList {
         }
         if (capc > cap_contacts) {
             for (PairGen& g : gen) {
-                g.c_node.grow(capc, cap_contacts); g.c_slave.grow(capc, cap_contacts); g.c_k.grow(capc, cap_contacts);
-                g.c_spring.grow((size_t)capc * 3, (size_t)cap_contacts * 3);
+                g.c_node.grow(capc, cap_contacts); g.c_at.grow(capc, cap_contacts); g.c_k.grow(capc, cap_contacts);
+                g.c_hist.grow(capc, cap_contacts);
             }
             c_pair.grow(capc, 0);
             c_hit.grow(capc, 0);
@@ -557,10 +558,10 @@ struct PairList {
         v.o_pairA = o.pairA.p; v.o_counters = o.counters.p;
         v.o_pairB = o.pairB.p; v.o_seg_off = o.seg_off.p; v.o_seg_cnt = o.seg_cnt.p; v.o_c_off = o.c_off.p;
         v.o_c_cnt = o.c_cnt.p;
-        v.c_node = c.c_node.p; v.c_slave = c.c_slave.p; v.c_spring = c.c_spring.p;
+        v.c_node = c.c_node.p; v.c_at = c.c_at.p; v.c_hist = c.c_hist.p;
         v.n_slots = c.counters.p + 1; v.n_hits = c.counters.p + 2; v.cap_contacts = cap_contacts;
         v.c_pair = c_pair.p; v.c_hit = c_hit.p; v.c_k = c.c_k.p; v.o_c_k = o.c_k.p; v.c_rec = c_rec.p; v.p_aux = p_aux.p; v.p_hist_cnt = p_hist_cnt.p; v.r_next = r_next.p; v.p_hit = p_hit.p;
-        v.o_c_node = o.c_node.p; v.o_c_spring = o.c_spring.p;
+        v.o_c_node = o.c_node.p; v.o_c_at = o.c_at.p; v.o_c_hist = o.c_hist.p;
         v.c_phi0 = c_phi0.p;
         v.p_bound = p_bound.p;
         v.c_test = c_test.p;
@@ -2381,8 +2382,8 @@ int fundem_set_contacts(fundem_sim* s, int kind, long long n, const int* node, c
             if (partner[a] != partner[b]) return partner[a] < partner[b];
             return key(node[a]) < key(node[b]);
         });
-        std::vector<int> pairA, pairB, c_off, c_cnt, seg_off(np, 0), seg_cnt(np, 0), cn, cs, ck;
-        std::vector<double> csp;
+        std::vector<int> pairA, pairB, c_off, c_cnt, seg_off(np, 0), seg_cnt(np, 0), cn, cs, ck, at;
+        std::vector<double4> hist;
         for (size_t t = 0; t < order.size(); ++t) {
             const size_t k = order[t];
             const int A = owner(node[k]), B = partner[k];
@@ -2398,7 +2399,9 @@ int fundem_set_contacts(fundem_sim* s, int kind, long long n, const int* node, c
             cn.push_back(node[k]);
             cs.push_back(B);
             ck.push_back(key(node[k]));
-            csp.insert(csp.end(), {spring[3 * k], spring[3 * k + 1], spring[3 * k + 2]});
+            at.push_back((int)t);
+            hist.push_back(make_double4(spring[3 * k], spring[3 * k + 1], spring[3 * k + 2], 0.0));
+            std::memcpy(&hist.back().w, &B, sizeof(B));
         }
         L.grow(std::max<int>(L.cap_pairs, (int)pairA.size() * 2), std::max<int>(L.cap_contacts, (int)cn.size() * 2));
         PairGen& g = L.gen[L.cur];
@@ -2409,11 +2412,11 @@ int fundem_set_contacts(fundem_sim* s, int kind, long long n, const int* node, c
         g.c_off.upload(c_off.data(), c_off.size(), s->stream);
         g.c_cnt.upload(c_cnt.data(), c_cnt.size(), s->stream);
         g.c_node.upload(cn.data(), cn.size(), s->stream);
-        g.c_slave.upload(cs.data(), cs.size(), s->stream);
+        g.c_at.upload(at.data(), at.size(), s->stream);
         g.c_k.upload(ck.data(), ck.size(), s->stream);
         L.up_node = cn;
         L.up_partner = cs;
-        g.c_spring.upload(csp.data(), csp.size(), s->stream);
+        g.c_hist.upload(hist.data(), hist.size(), s->stream);
         const int counters[3] = {(int)pairA.size(), (int)cn.size(), (int)cn.size()};
         g.counters.upload(counters, 3, s->stream);
         FD_CUDA(cudaStreamSynchronize(s->stream));

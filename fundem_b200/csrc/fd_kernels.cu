@@ -1802,29 +1802,38 @@ __device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, int A, int B
     return node_predicate<KIND>(e.gp, bcell, sg, e.cB, e.qB, GB, SB.sdf_quad, rB2, n.a.probe, e.ov, e.fx, e.fy, e.fz, e.pv);
 }
 
-// A contact's results go out in 16-byte stores to five whole sectors.  As seven
-// arrays (force, point, normal, overlap, energies) they were 18 stores to
-// about eleven part-written sectors at as many places.
-__device__ __forceinline__ void store_record(const PairListDev& L, int s, double3 pt, double3 nrm, double ov,
+// A contact's results go out in 16-byte stores to six whole sectors, side by
+// side with the next contact's (at place t of c_hist and c_rec).  As nine
+// arrays with an entry per slot they were 22 stores to some fifteen part-written
+// sectors, spread over 2.5 GB for 262,144 particles, and the sums read them
+// back from there.  That took the contact pass
+// from 112 to 88 us, the sums from 65 to 57.
+__device__ __forceinline__ void store_hist(const PairListDev& L, int t, double3 spring, int B)
+{
+    double2* o = reinterpret_cast<double2*>(L.c_hist + t);
+    o[0] = make_double2(spring.x, spring.y);
+    o[1] = make_double2(spring.z, __hiloint2double(0, B));
+}
+__device__ __forceinline__ void store_record(const PairListDev& L, int t, double3 pt, double3 nrm, double ov,
                                              double en, double es)
 {
-    double2* o = reinterpret_cast<double2*>(L.c_rec + (long long)CONTACT_REC * s + CONTACT_POINT);
+    double2* o = reinterpret_cast<double2*>(L.c_rec + (long long)CONTACT_REC * t + CONTACT_POINT);
     o[0] = make_double2(pt.x, pt.y);
     o[1] = make_double2(pt.z, nrm.x);
     o[2] = make_double2(nrm.y, nrm.z);
     o[3] = make_double2(ov, en);
     reinterpret_cast<double*>(o)[8] = es;
 }
-__device__ __forceinline__ void store_force(const PairListDev& L, int s, const double f[9])
+__device__ __forceinline__ void store_force(const PairListDev& L, int t, const double f[9])
 {
-    double2* o = reinterpret_cast<double2*>(L.c_rec + (long long)CONTACT_REC * s);
+    double2* o = reinterpret_cast<double2*>(L.c_rec + (long long)CONTACT_REC * t);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) o[t] = make_double2(f[2 * t], f[2 * t + 1]);
+    for (int k = 0; k < 4; ++k) o[k] = make_double2(f[2 * k], f[2 * k + 1]);
     reinterpret_cast<double*>(o)[8] = f[8];
 }
-__device__ __forceinline__ void store_force(const PairListDev& L, int s, const float f[9])
+__device__ __forceinline__ void store_force(const PairListDev& L, int t, const float f[9])
 {
-    float4* o = reinterpret_cast<float4*>(L.c_rec + (long long)CONTACT_REC * s);
+    float4* o = reinterpret_cast<float4*>(L.c_rec + (long long)CONTACT_REC * t);
     o[0] = make_float4(f[0], f[1], f[2], f[3]);
     o[1] = make_float4(f[4], f[5], f[6], f[7]);
     reinterpret_cast<float*>(o)[8] = f[8];
@@ -1835,7 +1844,7 @@ __device__ __forceinline__ void store_force(const PairListDev& L, int s, const f
 // records, and with forces the contact law, whose force and torques on A and B
 // go to o.  Returns the global boundary-node id.
 template <int KIND>
-__device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int s, int A,
+__device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int s, int t, int A,
                                            int B, int k, int oc_off, int oc_cnt, const SlotEval& e, double o[9])
 {
     const bool periodic = (KIND == FD_PP || KIND == FD_PW) && (n.a.periodic_x || n.a.periodic_y);
@@ -1863,10 +1872,13 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
             const int mid = (lo + hi) >> 1;
             if (L.o_c_k[mid] < k) lo = mid + 1; else hi = mid;
         }
-        if (lo < oc_end && L.o_c_k[lo] == k && L.o_c_node[lo] == nid) {
-            const double* sp = L.o_c_spring + 3ll * lo;
-            spring = mk3(sp[0], sp[1], sp[2]);
-            hist = lo;
+        if (lo < oc_end && L.o_c_k[lo] == k) {
+            const int at = L.o_c_at[lo];
+            if (L.o_c_node[lo] == nid) {
+                const double4 h = load_quad(L.o_c_hist + at);
+                spring = mk3(h.x, h.y, h.z);
+                hist = lo;
+            }
         }
     }
     if (R.hit && s < R.cap) {
@@ -1948,10 +1960,8 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
         o[3] = TA.x; o[4] = TA.y; o[5] = TA.z;
         o[6] = TB.x; o[7] = TB.y; o[8] = TB.z;
     }
-    L.c_slave[s] = B;
-    L.c_spring[3 * s + 0] = spring.x;
-    L.c_spring[3 * s + 1] = spring.y;
-    L.c_spring[3 * s + 2] = spring.z;
+    L.c_at[s] = t;
+    store_hist(L, t, spring, B);
     if (n.a.records) {
         if (!n.with_force) {
             const int mi = n.P.mat[A];
@@ -1964,7 +1974,7 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
                 ks = (ks > 0. && ksj > 0.) ? ks * ksj / (ks + ksj) : 0.;
             }
         }
-        store_record(L, s, pt, nrm, ov, 0.5 * ov * ov * kn, 0.5 * lengthSq3(spring) * ks);
+        store_record(L, t, pt, nrm, ov, 0.5 * ov * ov * kn, 0.5 * lengthSq3(spring) * ks);
     }
     return nid;
 }
@@ -2036,8 +2046,8 @@ __device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int
             int nid = -1;
             if (PASS == 1 && hit) {
                 double o[9];
-                nid = contact_law<KIND>(n, L, n.a.rec, s, A, B, k, aux.w, hist, e, o);
-                if (n.with_force) store_force(L, s, o);
+                nid = contact_law<KIND>(n, L, n.a.rec, s, t, A, B, k, aux.w, hist, e, o);
+                if (n.with_force) store_force(L, t, o);
             }
             if (PASS == 1) {
                 L.c_node[s] = nid;
@@ -2081,7 +2091,7 @@ __device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int
 // slots and a quarter of a contact per pair), so a warp takes 32 pairs' flags
 // in one load, the next ones' meanwhile, and passes on to those that hold one;
 // with eight lanes looking at each pair the sums took
-// 105 us for 262,144 particles, this way 65.
+// 105 us for 262,144 particles, this way 57.
 // ---------------------------------------------------------------------------
 template <typename Real>
 __device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int block, int nblocks, bool link,
@@ -2125,11 +2135,16 @@ __device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int blo
             // l (lane 0 also the ninth) of the contacts among them in turn
             const int cmax = __reduce_max_sync(full, c);
             for (int j0 = 0; j0 < cmax; j0 += 8) {
-                const bool contact = j0 + l < c && L.c_node[o + j0 + l] >= 0;
+                int at = 0;
+                bool contact = false;
+                if (j0 + l < c) {
+                    at = L.c_at[o + j0 + l];
+                    contact = L.c_node[o + j0 + l] >= 0;
+                }
                 unsigned int m = (__ballot_sync(full, contact) >> (8 * grp)) & 0xffu;
                 for (; m; m &= m - 1u) {
-                    const Real* f =
-                        reinterpret_cast<const Real*>(L.c_rec + (long long)CONTACT_REC * (o + j0 + __ffs(m) - 1));
+                    const int t = __shfl_sync(0xffu << (8 * grp), at, 8 * grp + __ffs(m) - 1);
+                    const Real* f = reinterpret_cast<const Real*>(L.c_rec + (long long)CONTACT_REC * t);
                     acc += f[l];
                     if (l == 0) acc8 += f[8];
                 }
@@ -2296,7 +2311,7 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int
 
 // as contact_law
 template <int KIND>
-__device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int s, int A,
+__device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int s, int t, int A,
                                              int B, int k, int oc_off, int oc_cnt, const SlotEval32& e, float o[9])
 {
     const bool periodic = (KIND == FD_PP || KIND == FD_PW) && (n.a.periodic_x || n.a.periodic_y);
@@ -2331,10 +2346,13 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
             const int mid = (lo2 + hi2) >> 1;
             if (L.o_c_k[mid] < k) lo2 = mid + 1; else hi2 = mid;
         }
-        if (lo2 < oc_end && L.o_c_k[lo2] == k && L.o_c_node[lo2] == nid) {
-            const double* sp = L.o_c_spring + 3ll * lo2;
-            spring = mk3(sp[0], sp[1], sp[2]);
-            hist = lo2;
+        if (lo2 < oc_end && L.o_c_k[lo2] == k) {
+            const int at = L.o_c_at[lo2];
+            if (L.o_c_node[lo2] == nid) {
+                const double4 h = load_quad(L.o_c_hist + at);
+                spring = mk3(h.x, h.y, h.z);
+                hist = lo2;
+            }
         }
     }
     if (R.hit && s < R.cap) {
@@ -2412,12 +2430,10 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
         o[3] = TA.x; o[4] = TA.y; o[5] = TA.z;
         o[6] = TB.x; o[7] = TB.y; o[8] = TB.z;
     }
-    L.c_slave[s] = B;
-    L.c_spring[3 * s + 0] = spring.x;
-    L.c_spring[3 * s + 1] = spring.y;
-    L.c_spring[3 * s + 2] = spring.z;
+    L.c_at[s] = t;
+    store_hist(L, t, spring, B);
     if (n.a.records) {
-        store_record(L, s, mk3(cA.x + arm.x, cA.y + arm.y, cA.z + arm.z), mk3(nrm.x, nrm.y, nrm.z), ov,
+        store_record(L, t, mk3(cA.x + arm.x, cA.y + arm.y, cA.z + arm.z), mk3(nrm.x, nrm.y, nrm.z), ov,
                      0.5 * (double)ov * (double)ov * (double)kn, 0.5 * lengthSq3(spring) * (double)ks);
     }
     return nid;
@@ -2487,8 +2503,8 @@ __device__ __forceinline__ void contact_list32(const NarrowArgs& n, int block, i
             int nid = -1;
             if (PASS == 1 && hit) {
                 float o[9];
-                nid = contact_law32<KIND>(n, L, n.a.rec, s, A, B, k, aux.w, hist, e, o);
-                if (n.with_force) store_force(L, s, o);
+                nid = contact_law32<KIND>(n, L, n.a.rec, s, t, A, B, k, aux.w, hist, e, o);
+                if (n.with_force) store_force(L, t, o);
             }
             if (PASS == 1) {
                 L.c_node[s] = nid;
@@ -3026,11 +3042,11 @@ __device__ __forceinline__ bool small_contact(const NarrowArgs& n, const PairLis
     if constexpr (MIXED) {
         SlotEval32 e;
         hit = slot_predicate32<KIND>(n, A, B, k, bcell, 0.f, e);
-        if (hit) nid = contact_law32<KIND>(n, L, R, s, A, B, k, oc_off, oc_cnt, e, o);
+        if (hit) nid = contact_law32<KIND>(n, L, R, s, s, A, B, k, oc_off, oc_cnt, e, o);
     } else {
         SlotEval e;
         hit = slot_predicate<KIND>(n, A, B, k, bcell, 0., e);
-        if (hit) nid = contact_law<KIND>(n, L, R, s, A, B, k, oc_off, oc_cnt, e, o);
+        if (hit) nid = contact_law<KIND>(n, L, R, s, s, A, B, k, oc_off, oc_cnt, e, o);
     }
     if (hit) store_force(L, s, o);
     L.c_node[s] = nid;
@@ -3431,7 +3447,7 @@ __global__ void k_view_keys(PairListDev L, long long* key)
     const int nslots = min(*L.n_slots, L.cap_contacts);
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < L.cap_contacts; s += gridDim.x * blockDim.x) {
         const int node = s < nslots ? L.c_node[s] : -1;
-        key[s] = node >= 0 ? ((long long)node << 32) | (unsigned int)L.c_slave[s] : -1ll;
+        key[s] = node >= 0 ? ((long long)node << 32) | (unsigned int)__double2loint(L.c_hist[L.c_at[s]].w) : -1ll;
     }
 }
 __global__ void k_view_gather(PairListDev L, const int* order, long long n, ContactViewDev v)
@@ -3439,13 +3455,15 @@ __global__ void k_view_gather(PairListDev L, const int* order, long long n, Cont
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const int s = order[i];
         v.master[i] = L.c_node[s];
-        v.slave[i] = L.c_slave[s];
-        const double* r = L.c_rec + (long long)CONTACT_REC * s;
+        const int t = L.c_at[s];
+        const double4 hist = L.c_hist[t];
+        const double* r = L.c_rec + (long long)CONTACT_REC * t;
         for (int d = 0; d < 3; ++d) {
             v.point[3 * i + d] = r[CONTACT_POINT + d];
             v.normal[3 * i + d] = r[CONTACT_NORMAL + d];
-            v.spring[3 * i + d] = L.c_spring[3 * s + d];
+            v.spring[3 * i + d] = d == 0 ? hist.x : d == 1 ? hist.y : hist.z;
         }
+        v.slave[i] = __double2loint(hist.w);
         v.overlap[i] = r[CONTACT_OVERLAP];
         v.en[i] = r[CONTACT_EN];
         v.es[i] = r[CONTACT_ES];
@@ -3461,13 +3479,15 @@ __global__ void k_pack_contacts(PairListDev L, ContactPackDev v, int* at, int co
         if (node < 0) continue;
         const int i = atomicAdd(at, 1);
         if (i >= count) continue;
-        v.id[i] = make_int2(node, L.c_slave[s]);
-        const double* r = L.c_rec + (long long)CONTACT_REC * s;
+        const int t = L.c_at[s];
+        const double4 hist = L.c_hist[t];
+        const double* r = L.c_rec + (long long)CONTACT_REC * t;
         for (int d = 0; d < 3; ++d) {
             if (v.point) v.point[3 * i + d] = r[CONTACT_POINT + d];
             if (v.normal) v.normal[3 * i + d] = r[CONTACT_NORMAL + d];
-            if (v.spring) v.spring[3 * i + d] = L.c_spring[3 * s + d];
+            if (v.spring) v.spring[3 * i + d] = d == 0 ? hist.x : d == 1 ? hist.y : hist.z;
         }
+        v.id[i] = make_int2(node, __double2loint(hist.w));
         if (v.overlap) v.overlap[i] = r[CONTACT_OVERLAP];
         if (v.en) v.en[i] = r[CONTACT_EN];
         if (v.es) v.es[i] = r[CONTACT_ES];

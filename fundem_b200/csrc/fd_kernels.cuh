@@ -50,22 +50,22 @@ struct PairListDev {
     // single-precision filter, contiguous per pair; c_node is the global
     // boundary-node id of a contact and -1 for a slot that is none
     int* c_node;
-    int* c_slave;
+    int* c_at;         // per slot that holds a contact: its place in c_hist and c_rec
     int* c_pair;       // pair of each slot
     int* c_hit;        // slots holding a contact, listed by the predicate pass
                        // for the contact-law pass (n_hits of them)
     int* c_k;          // node key of each slot: cluster-order index relative to
                        // the geometry (ascending within a pair)
-    // per slot that holds a contact, 20 doubles (five sectors, so that a
-    // contact's result is written whole): [0 .. 8] F, torque on A, torque on B
-    // (of the mode's type), [10 .. 18] with records: contact point, normal,
-    // overlap, normal and tangential energy
+    // The contacts lie side by side, not slot by slot: one slot in eight holds
+    // one.  Per contact 20 doubles (five sectors): [0 .. 8] F, torque on A,
+    // torque on B (of the mode's type), [10 .. 18] with records: contact point,
+    // normal, overlap, normal and tangential energy
     double* c_rec;
+    double4* c_hist;   // per contact: tangential spring, partner (int in w's low half)
     int4* p_aux;       // per pair: cell of B (x, y, z), first history slot
     int* p_hist_cnt;   // per pair: history slots
     int* r_next;       // per pair: the next pair (code) of its partner's list
     int* p_hit;        // per pair: 1 when a slot of it holds a contact
-    double* c_spring;  // 3 per contact
     int* n_slots;      // device counter: slots used
     int* n_hits;       // device counter: contacts (n_slots + 1)
     int cap_contacts;  // slot capacity
@@ -80,7 +80,8 @@ struct PairListDev {
     // previous contacts
     int* o_c_node;
     int* o_c_k;
-    double* o_c_spring;
+    int* o_c_at;
+    double4* o_c_hist;
 };
 
 constexpr int CONTACT_REC = 20, CONTACT_POINT = 10, CONTACT_NORMAL = 13, CONTACT_OVERLAP = 16, CONTACT_EN = 17,
