@@ -257,6 +257,7 @@ struct GeoSetHost {
     std::vector<HostGeo> geos;
     // device
     DevArray<FdGeo> d_geo;
+    DevArray<FdGeo32> d_geo32;
     DevArray<double> d_sdf;
     DevArray<float> d_sdf32;
     DevArray<double4> d_sdf_quad;
@@ -368,6 +369,20 @@ struct GeoSetHost {
         }
         d_geo.alloc(std::max<size_t>(table.size(), 1));
         d_geo.upload(table.data(), table.size(), s);
+        std::vector<FdGeo32> table32;
+        for (const FdGeo& t : table) {
+            FdGeo32 g{};
+            g.ox = (float)t.origin.x; g.oy = (float)t.origin.y; g.oz = (float)t.origin.z;
+            g.is = (float)t.inv_spacing; g.spacing = (float)t.spacing;
+            g.radius = (float)t.radius; g.lip = (float)t.lip;
+            g.tight = t.lip < 4.0;
+            g.size = t.size;
+            g.node_off = t.node_off; g.clus_off = t.clus_off; g.clus_count = t.clus_count;
+            g.sdf_off = t.sdf_off; g.dist_off = t.dist_off; g.cellmin_off = t.cellmin_off;
+            table32.push_back(g);
+        }
+        d_geo32.alloc(std::max<size_t>(table32.size(), 1));
+        d_geo32.upload(table32.data(), table32.size(), s);
         d_sdf.alloc(std::max<size_t>(sdf.size(), 1));
         d_sdf.upload(sdf.data(), sdf.size(), s);
         d_sdf32.alloc(std::max<size_t>(sdf32.size(), 1));
@@ -413,6 +428,7 @@ struct GeoSetHost {
         v.geo = d_geo.p;
         v.sdf = d_sdf.p;
         v.sdf32 = d_sdf32.p;
+        v.geo32 = d_geo32.p;
         v.sdf_quad = d_sdf_quad.p;
         v.sdf32_quad = d_sdf32_quad.p;
         v.dist = d_dist.p;
@@ -509,7 +525,7 @@ struct PairList {
         const size_t m = std::max(nobj, 1);
         for (PairGen& g : gen) {
             g.pairA.alloc(cap_pairs); g.pairB.alloc(cap_pairs); g.seg_off.alloc(m); g.seg_cnt.alloc(m);
-            g.c_off.alloc(cap_pairs); g.c_cnt.alloc(cap_pairs); g.pf.alloc((size_t)cap_pairs * 9);
+            g.c_off.alloc(cap_pairs); g.c_cnt.alloc(cap_pairs); g.pf.alloc((size_t)cap_pairs * fd::RESULT);
             g.c_node.alloc(cap_contacts); g.c_at.alloc(cap_contacts); g.c_k.alloc(cap_contacts);
             g.c_hist.alloc(cap_contacts);
             g.counters.alloc(3);
@@ -526,7 +542,7 @@ struct PairList {
         if (capp > cap_pairs) {
             for (PairGen& g : gen) {
                 g.pairA.grow(capp, cap_pairs); g.pairB.grow(capp, cap_pairs); g.c_off.grow(capp, cap_pairs);
-                g.c_cnt.grow(capp, cap_pairs); g.pf.grow((size_t)capp * 9, (size_t)cap_pairs * 9);
+                g.c_cnt.grow(capp, cap_pairs); g.pf.grow((size_t)capp * fd::RESULT, (size_t)cap_pairs * fd::RESULT);
             }
             p_aux.grow(capp, 0);
             p_hist_cnt.grow(capp, 0);
@@ -1138,7 +1154,7 @@ struct fundem_sim {
         const size_t m = std::max<size_t>(n, 1);
         B.d_master.alloc(m); B.d_slave.alloc(m); B.d_active.alloc(m); B.d_point.alloc(m);
         B.d_B.alloc(4 * m); B.d_radius.alloc(m); B.d_L0.alloc(m); B.d_ts.alloc(m); B.d_coh.alloc(m);
-        B.d_mu.alloc(m); B.d_frames.alloc(8 * m); B.d_energy.alloc(6 * m); B.d_out.alloc(9 * m);
+        B.d_mu.alloc(m); B.d_frames.alloc(8 * m); B.d_energy.alloc(6 * m); B.d_out.alloc(fd::RESULT * m);
         B.d_master.upload(B.master.data(), n, stream); B.d_slave.upload(B.slave.data(), n, stream);
         B.d_active.upload(B.active.data(), n, stream); B.d_point.upload(B.point.data(), n, stream);
         B.d_B.upload(B.B.data(), 4 * n, stream); B.d_radius.upload(B.radius.data(), n, stream);

@@ -62,6 +62,19 @@ struct FdGeo {
     fd_sym inv_inertia;
 };
 
+// what the culling stages read of a geometry, in their precision (FdGeo's
+// values rounded): converted where they are used, each was an instruction of
+// the double-precision unit per node and pair
+struct FdGeo32 {
+    float ox, oy, oz;      // origin
+    float is, spacing;     // 1 / spacing, spacing
+    float radius, lip;
+    int tight;             // lip below 4: a distance-like field
+    int3 size;
+    int node_off, clus_off, clus_count;
+    long long sdf_off, dist_off, cellmin_off;
+};
+
 struct FdCluster {
     double3 centre;  // body frame
     double radius;   // max distance of its nodes from the centre

@@ -735,32 +735,31 @@ constexpr double BOUND_REL = 1e-9;
 //     corner minimum is <= 0, 1-Lipschitz in the position,
 //   * the Lipschitz bound of the trilinear SDF (distance-like fields).
 __device__ __forceinline__ bool sphere_culled(float px, float py, float pz, float radius, bool radius_test,
-                                              const FdGeo& GB, const GeoSetDev& SB, double rB, double probe)
+                                              const FdGeo32& GB, const GeoSetDev& SB, float probe)
 {
-    const float scale = (float)rB + radius + (float)GB.spacing;
+    const float scale = GB.radius + radius + GB.spacing;
     const float margin = 2e-5f * scale;
     const float rho = radius + margin;
     if (radius_test) {
-        const float lim = (float)rB + rho;
+        const float lim = GB.radius + rho;
         if (px * px + py * py + pz * pz > lim * lim) return true;
     }
-    const float is = (float)GB.inv_spacing;
-    const float gx = (px - (float)GB.origin.x) * is, gy = (py - (float)GB.origin.y) * is,
-                gz = (pz - (float)GB.origin.z) * is;
+    const float is = GB.is;
+    const float gx = (px - GB.ox) * is, gy = (py - GB.oy) * is, gz = (pz - GB.oz) * is;
     const float rg = rho * is + 1e-4f;
     if (gx < -rg || gy < -rg || gz < -rg) return true;
     if (gx > GB.size.x - 1 + rg || gy > GB.size.y - 1 + rg || gz > GB.size.z - 1 + rg) return true;
-    if (probe == 0.0) {
+    if (probe == 0.f) {
         const int vx = min(max(__float2int_rn(gx), 0), GB.size.x - 1);
         const int vy = min(max(__float2int_rn(gy), 0), GB.size.y - 1);
         const int vz = min(max(__float2int_rn(gz), 0), GB.size.z - 1);
         const float D = __ldg(SB.dist + GB.dist_off + fd_lin3(vx, vy, vz, GB.size));
-        const float sp = (float)GB.spacing;
+        const float sp = GB.spacing;
         const float dx = (gx - vx) * sp, dy = (gy - vy) * sp, dz = (gz - vz) * sp;
         if (D - sqrtf(dx * dx + dy * dy + dz * dz) > rho) return true;
     }
     // the Lipschitz bound only helps where the field is distance-like
-    if (GB.lip < 4.0 && gx >= 0.f && gy >= 0.f && gz >= 0.f && gx < GB.size.x - 1 && gy < GB.size.y - 1 &&
+    if (GB.tight && gx >= 0.f && gy >= 0.f && gz >= 0.f && gx < GB.size.x - 1 && gy < GB.size.y - 1 &&
         gz < GB.size.z - 1) {
         const int i0 = (int)gx, j0 = (int)gy, k0 = (int)gz;
         const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
@@ -772,8 +771,8 @@ __device__ __forceinline__ bool sphere_culled(float px, float py, float pz, floa
         const float c01 = s1.x * (1.f - fx) + s1.y * fx;
         const float c11 = s1.z * (1.f - fx) + s1.w * fx;
         const float phi = (c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz;
-        const float bound = (float)GB.lip * rho + (float)probe;
-        if (phi - bound > 1e-5f * (fabsf(phi) + bound + (float)GB.spacing)) return true;
+        const float bound = GB.lip * rho + probe;
+        if (phi - bound > 1e-5f * (fabsf(phi) + bound + GB.spacing)) return true;
     }
     return false;
 }
@@ -781,14 +780,14 @@ __device__ __forceinline__ bool sphere_culled(float px, float py, float pz, floa
 // Body-level cull of a candidate pair in single precision: A's bounding
 // sphere (radius rA about cA) against B, through B's rotation rows
 __device__ __forceinline__ bool body_culled32(const double3 cA, double rA, const double3 cB, const float4* RB,
-                                              bool radius_test, const FdGeo& GB, const GeoSetDev& SB, double probe)
+                                              bool radius_test, const FdGeo32& GB, const GeoSetDev& SB, double probe)
 {
     const float4 b0 = RB[0], b1 = RB[1], b2 = RB[2];
     const float dx = (float)(cA.x - cB.x), dy = (float)(cA.y - cB.y), dz = (float)(cA.z - cB.z);
     const float px = fmaf(b0.x, dx, fmaf(b1.x, dy, b2.x * dz));
     const float py = fmaf(b0.y, dx, fmaf(b1.y, dy, b2.y * dz));
     const float pz = fmaf(b0.z, dx, fmaf(b1.z, dy, b2.z * dz));
-    return sphere_culled(px, py, pz, (float)rA, radius_test, GB, SB, GB.radius, probe);
+    return sphere_culled(px, py, pz, (float)rA, radius_test, GB, SB, (float)probe);
 }
 
 // cells that can hold the centre of a partner of a body of radius r centred
@@ -922,7 +921,7 @@ __device__ __forceinline__ void broad_cells(const ObjDev& P, const GeoSetDev& G,
                     const double rs = rA + (GHOST ? GB.grid_radius : GB.radius) + skin;
                     if (lengthSq3(cA - cB) <= rs * rs * (1.0 + 4.0 * BOUND_REL))
                         pass = !body_culled32(cA, rA + skin, cB, (GHOST && grot ? grot : P.rot) + 3ll * B, !GHOST,
-                                              GB, G, probe);
+                                              G.geo32[P.geo[B]], G, probe);
                 }
             }
             const unsigned int gm = (__ballot_sync(full, pass) >> gbase) & ((1u << BROAD_LANES) - 1u);
@@ -1027,7 +1026,7 @@ __global__ void __launch_bounds__(TPB) k_nl_filter(ObjDev P, GeoSetDev G, PairLi
                 const double3 cB = P.pos[B];
                 const double rs = rA + GB.radius;
                 if (lengthSq3(cA - cB) <= rs * rs * (1.0 + 4.0 * BOUND_REL))
-                    pass = !body_culled32(cA, rA, cB, P.rot + 3ll * B, true, GB, G, probe);
+                    pass = !body_culled32(cA, rA, cB, P.rot + 3ll * B, true, G.geo32[P.geo[B]], G, probe);
             }
         }
         const unsigned int gm = (__ballot_sync(full, pass) >> gbase) & ((1u << LN) - 1u);
@@ -1151,7 +1150,7 @@ __device__ __forceinline__ void broad_walls(const ObjDev& P, const GeoSetDev& G,
         const double rs = rA + GB.grid_radius + skin;
         const double3 cW = W.pos[w];
         if (lengthSq3(cA - cW) > rs * rs * (1.0 + 4.0 * BOUND_REL)) continue;
-        if (body_culled32(cA, rA + skin, cW, W.rot + 3ll * w, false, GB, GW, probe)) continue;
+        if (body_culled32(cA, rA + skin, cW, W.rot + 3ll * w, false, GW.geo32[W.geo[w]], GW, probe)) continue;
         if (cnt < MAX_CAND) buf[cnt++] = w;
         ++total;
     }
@@ -1161,21 +1160,52 @@ __device__ __forceinline__ void broad_walls(const ObjDev& P, const GeoSetDev& G,
 // ---------------------------------------------------------------------------
 // contact law, contactKernel.cuh:4-77
 // ---------------------------------------------------------------------------
+// The contact law runs in kernels of several forms and must give each the same
+// bits.  Left plain, its sums of products were contracted one way in one kernel
+// and another way in the next, so they are explicit, in the form nvcc gave the
+// contact pass.
+__device__ __forceinline__ double dot3e(double3 a, double3 b) { return dot3f(a.x, a.y, a.z, b.x, b.y, b.z); }
+__device__ __forceinline__ double length3e(double3 v) { return sqrt(dot3e(v, v)); }
+__device__ __forceinline__ double3 scale3e(double s, double3 a)
+{
+    return mk3(__dmul_rn(s, a.x), __dmul_rn(s, a.y), __dmul_rn(s, a.z));
+}
+// s * a + b
+__device__ __forceinline__ double3 axpy3e(double s, double3 a, double3 b)
+{
+    return mk3(__fma_rn(s, a.x, b.x), __fma_rn(s, a.y, b.y), __fma_rn(s, a.z, b.z));
+}
+// s * a + t * b
+__device__ __forceinline__ double3 sum3e(double s, double3 a, double t, double3 b)
+{
+    return axpy3e(s, a, scale3e(t, b));
+}
+__device__ __forceinline__ double3 cross3e(double3 a, double3 b)
+{
+    return mk3(__fma_rn(a.y, b.z, -__dmul_rn(a.z, b.y)), __fma_rn(a.z, b.x, -__dmul_rn(a.x, b.z)),
+               __fma_rn(a.x, b.y, -__dmul_rn(a.y, b.x)));
+}
+
+// (the recorded tangential energy's)
+__device__ __forceinline__ double spring_sq(double3 v) 
+{
+    return __fma_rn(v.z, v.z, __fma_rn(v.y, v.y, __dmul_rn(v.x, v.x)));
+}
+
 __device__ __forceinline__ double3 sliding_spring(double3 prev, double3 sv, double3 n, double3 fn, double mu,
                                                   double k, double c, double dt)
 {
     double3 spring = mk3(0., 0., 0.);
     if (mu > 0. && k > 0.) {
-        double3 p1 = prev - dot3(prev, n) * n;
-        const double ap1 = length3(p1);
-        if (!fd_is_zero(ap1)) p1 = p1 * (length3(prev) / ap1);
-        spring = p1 + sv * dt;
-        double3 sf = -k * spring - c * sv;
-        const double asf = length3(sf);
-        const double afn = length3(fn);
+        double3 p1 = axpy3e(-dot3e(prev, n), n, prev);
+        const double ap1 = length3e(p1);
+        if (!fd_is_zero(ap1)) p1 = scale3e(length3e(prev) / ap1, p1);
+        spring = axpy3e(dt, sv, p1);
+        double3 sf = sum3e(-k, spring, -c, sv);
+        const double asf = length3e(sf);
+        const double afn = length3e(fn);
         if (!fd_is_zero(asf) && asf > mu * afn) {
-            sf = sf * (mu * afn / asf);
-            spring = -(sf + c * sv) * (1.0 / k);
+            spring = scale3e(-(1.0 / k), sum3e(mu * afn / asf, sf, c, sv));
         }
     }
     return spring;
@@ -1186,15 +1216,16 @@ __device__ __forceinline__ void linear_contact(double3& F, double3& spring, doub
 {
     if (delta > 0.) {
         const double lr = log(res);
-        const double diss = -lr / (double)sqrtf((float)(lr * lr + PI_D * PI_D));
+        const double diss = -lr / (double)sqrtf((float)__fma_rn(lr, lr, PI_D * PI_D));
         const double cn = 2. * diss * (double)sqrtf((float)(m * kn));
-        const double3 vn = dot3(vc, n) * n;
-        const double3 fn = (kn * delta) * n - cn * vn;
+        const double vcn = dot3e(vc, n);
+        const double3 vn = scale3e(vcn, n);
+        const double3 fn = sum3e(kn * delta, n, -cn, vn);
         const double cs = 2. * diss * (double)sqrtf((float)(m * ks));
-        const double3 vs = vc - vn;
+        const double3 vs = mk3(__dsub_rn(vc.x, vn.x), __dsub_rn(vc.y, vn.y), __dsub_rn(vc.z, vn.z));
         spring = sliding_spring(spring, vs, n, fn, mu, ks, cs, dt);
-        const double3 fs = -ks * spring - cs * vs;
-        F = fn + fs;
+        const double3 fs = sum3e(-ks, spring, -cs, vs);
+        F = mk3(__dadd_rn(fn.x, fs.x), __dadd_rn(fn.y, fs.y), __dadd_rn(fn.z, fs.z));
     } else {
         spring = mk3(0., 0., 0.);
     }
@@ -1221,8 +1252,11 @@ struct NarrowArgs {
 // the slave side of a pair, by kind
 template <int KIND> struct Slave;
 template <> struct Slave<FD_PP> {
+    __device__ static const ObjDev& body(const NarrowArgs& n) { return n.P; }
+    __device__ static const double3* pos_of(const NarrowArgs& n) { return n.P.pos; }
+    __device__ static const double3* vel_of(const NarrowArgs& n) { return n.P.vel; }
+    __device__ static const long long* hash_of(const NarrowArgs& n) { return n.P.hash; }
     __device__ static double3 pos(const NarrowArgs& n, int j) { return n.P.pos[j]; }
-    __device__ static double3 vel(const NarrowArgs& n, int j) { return n.P.vel[j]; }
     __device__ static const fd_quat* q(const NarrowArgs& n, int j) { return n.P.q + j; }
     __device__ static const float4* rot(const NarrowArgs& n, int j) { return n.P.rot + 3ll * j; }
     __device__ static const FdGeo& geo(const NarrowArgs& n, int j) { return n.G.geo[n.P.geo[j]]; }
@@ -1232,8 +1266,11 @@ template <> struct Slave<FD_PP> {
     static constexpr bool radius_test = true;
 };
 template <> struct Slave<FD_PW> {
+    __device__ static const ObjDev& body(const NarrowArgs& n) { return n.W; }
+    __device__ static const double3* pos_of(const NarrowArgs& n) { return n.W.pos; }
+    __device__ static const double3* vel_of(const NarrowArgs& n) { return n.W.vel; }
+    __device__ static const long long* hash_of(const NarrowArgs& n) { return n.W.hash; }
     __device__ static double3 pos(const NarrowArgs& n, int j) { return n.W.pos[j]; }
-    __device__ static double3 vel(const NarrowArgs& n, int j) { return n.W.vel[j]; }
     __device__ static const fd_quat* q(const NarrowArgs& n, int j) { return n.W.q + j; }
     __device__ static const float4* rot(const NarrowArgs& n, int j) { return n.W.rot + 3ll * j; }
     __device__ static const FdGeo& geo(const NarrowArgs& n, int j) { return n.GW.geo[n.W.geo[j]]; }
@@ -1247,14 +1284,16 @@ template <> struct Slave<FD_PW> {
 // the body's own, as in addGhostLevelSetParticleContactForceTorqueKernel
 // (contactKernel.cu:262), which does not turn it with the image.
 struct SlaveGhost {
+    __device__ static const ObjDev& body(const NarrowArgs& n) { return n.P; }
+    __device__ static const double3* pos_of(const NarrowArgs& n) { return n.gh.pos; }
+    __device__ static const double3* vel_of(const NarrowArgs& n) { return n.gh.vel ? n.gh.vel : n.P.vel; }
+    __device__ static const long long* hash_of(const NarrowArgs& n) { return n.gh.hash; }
     __device__ static double3 pos(const NarrowArgs& n, int j) { return n.gh.pos[j]; }
-    __device__ static double3 vel(const NarrowArgs& n, int j) { return n.gh.vel ? n.gh.vel[j] : n.P.vel[j]; }
     __device__ static const fd_quat* q(const NarrowArgs& n, int j) { return (n.gh.q ? n.gh.q : n.P.q) + j; }
     __device__ static const float4* rot(const NarrowArgs& n, int j)
     {
         return (n.gh.rot ? n.gh.rot : n.P.rot) + 3ll * j;
     }
-    __device__ static const FdGeo& geo(const NarrowArgs& n, int j) { return n.G.geo[n.P.geo[j]]; }
     __device__ static const GeoSetDev& set(const NarrowArgs& n) { return n.G; }
     __device__ static long long hash(const NarrowArgs& n, int j) { return n.gh.hash[j]; }
     __device__ static const FdGrid& grid(const NarrowArgs& n) { return n.pgrid; }
@@ -1449,14 +1488,14 @@ __device__ __forceinline__ CullXf cull_transform(const float4* RA, const float4*
 //   * the Lipschitz bound of the trilinear SDF (coarse grids such as plane
 //     walls, where it is tight).
 template <int KIND>
-__device__ __forceinline__ bool cluster_culled(const float4 cl, const CullXf& x, const FdGeo& GB,
-                                               const GeoSetDev& SB, double rB, double probe)
+__device__ __forceinline__ bool cluster_culled(const float4 cl, const CullXf& x, const FdGeo32& GB,
+                                               const GeoSetDev& SB, float probe)
 {
     const float cx = cl.x, cy = cl.y, cz = cl.z;
     const float px = fmaf(x.m[0], cx, fmaf(x.m[1], cy, fmaf(x.m[2], cz, x.t[0])));
     const float py = fmaf(x.m[3], cx, fmaf(x.m[4], cy, fmaf(x.m[5], cz, x.t[1])));
     const float pz = fmaf(x.m[6], cx, fmaf(x.m[7], cy, fmaf(x.m[8], cz, x.t[2])));
-    return sphere_culled(px, py, pz, cl.w, Slave<KIND>::radius_test, GB, SB, rB, probe);
+    return sphere_culled(px, py, pz, cl.w, Slave<KIND>::radius_test, GB, SB, probe);
 }
 
 // Node filter: true when a node certainly fails the node predicate.  The
@@ -1470,71 +1509,98 @@ __device__ __forceinline__ bool cluster_culled(const float4 cl, const CullXf& x,
 //     error, whose eight corner values all exceed the probe (the trilinear
 //     value is a convex combination of them).
 // Nodes that pass go to the exact double-precision predicate.
-template <int KIND>
-__device__ __forceinline__ bool node_filtered(const float4 p, const CullXf& x, const FdGeo& GB, const GeoSetDev& SB,
-                                              float rB, float perr, double probe)
+//
+// NODES nodes at a time (on: the node is there; out: dropped): the chains
+// from position to interpolation overlap, and none waits at a branch.
+template <int KIND, int NODES>
+__device__ __forceinline__ void node_filter(const float4 (&p)[NODES], const bool (&on)[NODES], const CullXf& x,
+                                             const FdGeo32& GB, const GeoSetDev& SB, float perr, float probe,
+                                             bool (&out)[NODES])
 {
-    const float cx = p.x, cy = p.y, cz = p.z;
-    const float px = fmaf(x.m[0], cx, fmaf(x.m[1], cy, fmaf(x.m[2], cz, x.t[0])));
-    const float py = fmaf(x.m[3], cx, fmaf(x.m[4], cy, fmaf(x.m[5], cz, x.t[1])));
-    const float pz = fmaf(x.m[6], cx, fmaf(x.m[7], cy, fmaf(x.m[8], cz, x.t[2])));
-    if (Slave<KIND>::radius_test) {
-        const float lim = rB + perr;
-        if (px * px + py * py + pz * pz > lim * lim) return true;
-    }
-    const float is = (float)GB.inv_spacing;
-    const float gx = (px - (float)GB.origin.x) * is, gy = (py - (float)GB.origin.y) * is,
-                gz = (pz - (float)GB.origin.z) * is;
+    const float is = GB.is;
     const float ge = perr * is + 1e-4f;
     const float hx = (float)(GB.size.x - 1), hy = (float)(GB.size.y - 1), hz = (float)(GB.size.z - 1);
-    if (gx < -ge || gy < -ge || gz < -ge || gx > hx + ge || gy > hy + ge || gz > hz + ge) return true;
-    if (gx < ge || gy < ge || gz < ge || gx > hx - ge || gy > hy - ge || gz > hz - ge) return false;
-    const int i0 = (int)gx, j0 = (int)gy, k0 = (int)gz;
-    const float fx = gx - i0, fy = gy - j0, fz = gz - k0;
-    if (GB.lip < 4.0) {
+    const float lim = GB.radius + perr;
+    float gx[NODES], gy[NODES], gz[NODES];
+    bool look[NODES];
+#pragma unroll
+    for (int u = 0; u < NODES; ++u) {
+        const float cx = p[u].x, cy = p[u].y, cz = p[u].z;
+        const float px = fmaf(x.m[0], cx, fmaf(x.m[1], cy, fmaf(x.m[2], cz, x.t[0])));
+        const float py = fmaf(x.m[3], cx, fmaf(x.m[4], cy, fmaf(x.m[5], cz, x.t[1])));
+        const float pz = fmaf(x.m[6], cx, fmaf(x.m[7], cy, fmaf(x.m[8], cz, x.t[2])));
+        gx[u] = (px - GB.ox) * is;
+        gy[u] = (py - GB.oy) * is;
+        gz[u] = (pz - GB.oz) * is;
+        out[u] = !on[u] || (Slave<KIND>::radius_test && px * px + py * py + pz * pz > lim * lim) || gx[u] < -ge ||
+                 gy[u] < -ge || gz[u] < -ge || gx[u] > hx + ge || gy[u] > hy + ge || gz[u] > hz + ge;
+        look[u] = !out[u] && !(gx[u] < ge || gy[u] < ge || gz[u] < ge || gx[u] > hx - ge || gy[u] > hy - ge ||
+                               gz[u] > hz - ge);
+    }
+    if (GB.tight) {
         const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
-        const float4* S = SB.sdf32_quad + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
-        const float4 s0 = __ldg(S), s1 = __ldg(S + sxy);
-        const float c00 = s0.x * (1.f - fx) + s0.y * fx;
-        const float c10 = s0.z * (1.f - fx) + s0.w * fx;
-        const float c01 = s1.x * (1.f - fx) + s1.y * fx;
-        const float c11 = s1.z * (1.f - fx) + s1.w * fx;
-        const float phi = (c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz;
-        const float slack = (float)GB.lip * perr + 1e-5f * (fabsf(phi) + (float)GB.spacing);
-        return phi - (float)probe > slack;
+        float4 s0[NODES], s1[NODES];
+#pragma unroll
+        for (int u = 0; u < NODES; ++u) {
+            // a node that needs no look reads the pool's first point
+            const long long i =
+                look[u] ? GB.sdf_off + (long long)(int)gz[u] * sxy + (long long)(int)gy[u] * sx + (int)gx[u] : 0ll;
+            s0[u] = __ldg(SB.sdf32_quad + i);
+            s1[u] = __ldg(SB.sdf32_quad + i + (look[u] ? sxy : 0ll));
+        }
+#pragma unroll
+        for (int u = 0; u < NODES; ++u) {
+            const float fx = gx[u] - (int)gx[u], fy = gy[u] - (int)gy[u], fz = gz[u] - (int)gz[u];
+            const float c00 = s0[u].x * (1.f - fx) + s0[u].y * fx;
+            const float c10 = s0[u].z * (1.f - fx) + s0[u].w * fx;
+            const float c01 = s1[u].x * (1.f - fx) + s1[u].y * fx;
+            const float c11 = s1[u].z * (1.f - fx) + s1[u].w * fx;
+            const float phi = (c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz;
+            const float slack = GB.lip * perr + 1e-5f * (fabsf(phi) + GB.spacing);
+            if (look[u]) out[u] = phi - probe > slack;
+        }
+        return;
     }
     // the trilinear value anywhere the node can be (within ge of its
     // single-precision position, in grid units) is at least the smallest
     // corner minimum over the cells that box touches (one to a few cells:
     // two per axis where the node is within ge of a cell face)
-    const int ilo = max((int)floorf(gx - ge), 0), ihi = min((int)floorf(gx + ge), GB.size.x - 2);
-    const int jlo = max((int)floorf(gy - ge), 0), jhi = min((int)floorf(gy + ge), GB.size.y - 2);
-    const int klo = max((int)floorf(gz - ge), 0), khi = min((int)floorf(gz + ge), GB.size.z - 2);
-    if (ihi - ilo > 2 || jhi - jlo > 2 || khi - klo > 2) return false;  // a margin of more than a cell: keep
     const long long rx = GB.size.x - 1, rxy = (long long)(GB.size.y - 1) * (GB.size.x - 1);
     const float* CM = SB.cellmin + GB.cellmin_off;
-    for (int k = klo; k <= khi; ++k)
-        for (int j = jlo; j <= jhi; ++j)
-            for (int i = ilo; i <= ihi; ++i)
-                if (__ldg(CM + k * rxy + j * rx + i) <= (float)probe) return false;
-    return true;
+    for (int u = 0; u < NODES; ++u) {
+        if (!look[u]) continue;
+        const int ilo = max((int)floorf(gx[u] - ge), 0), ihi = min((int)floorf(gx[u] + ge), GB.size.x - 2);
+        const int jlo = max((int)floorf(gy[u] - ge), 0), jhi = min((int)floorf(gy[u] + ge), GB.size.y - 2);
+        const int klo = max((int)floorf(gz[u] - ge), 0), khi = min((int)floorf(gz[u] + ge), GB.size.z - 2);
+        if (ihi - ilo > 2 || jhi - jlo > 2 || khi - klo > 2) continue;  // a margin of more than a cell: keep
+        bool above = true;
+        for (int k = klo; k <= khi && above; ++k)
+            for (int j = jlo; j <= jhi && above; ++j)
+                for (int i = ilo; i <= ihi && above; ++i) above = !(__ldg(CM + k * rxy + j * rx + i) <= probe);
+        out[u] = above;
+    }
 }
 
 // The nodes of A that may pass the predicate against B, for one warp:
 // cluster culling with one cluster per lane, then the single-precision filter
 // over the nodes of the surviving clusters.  Their keys go to queue in
-// cluster order; returns how many, and the clusters kept.
-template <int KIND>
+// cluster order; returns how many, and the clusters kept.  NODES: clusters
+// filtered at a time.  One where there are warps enough to hide the waits (two
+// take the registers of a quarter of them: a rebuild's selection 1.5 against
+// 1.4 ms at 262,144 particles), two where a warp has an SM's share to itself
+// (a step of 1,000 particles 38.4 against 39.6 us).
+template <int KIND, int NODES>
 __device__ __forceinline__ int cull_pair(const NarrowArgs& n, int A, int B, double skin, int lane,
                                          unsigned short* queue, int& kept)
 {
     const unsigned int lt_mask = (1u << lane) - 1u;
-    const FdGeo& GA = n.G.geo[n.P.geo[A]];
+    const int gA = n.P.geo[A], gB = Slave<KIND>::body(n).geo[B];
     const double3 cA = n.P.pos[A];
     const double3 cB = Slave<KIND>::pos(n, B);
-    const FdGeo& GB = Slave<KIND>::geo(n, B);
     const GeoSetDev& SB = Slave<KIND>::set(n);
-    const double rB = GB.radius;
+    const FdGeo32& GA = n.G.geo32[gA];
+    const FdGeo32& GB = SB.geo32[gB];
+    const float probe = (float)n.a.probe;
     const int ncl = GA.clus_count;
     if (ncl > MAX_CLUSTERS) set_flag(n.a.flags, FD_FLAG_CLUSTER_OVERFLOW);
     unsigned long long keep = 0ull;
@@ -1545,34 +1611,50 @@ __device__ __forceinline__ int cull_pair(const NarrowArgs& n, int A, int B, doub
         if (c < ncl) {
             float4 cl = n.G.clus_sphere[GA.clus_off + c];
             cl.w += (float)skin;
-            k = !cluster_culled<KIND>(cl, xf, GB, SB, rB, n.a.probe);
+            k = !cluster_culled<KIND>(cl, xf, GB, SB, probe);
         }
         keep |= ((unsigned long long)__ballot_sync(0xffffffffu, k)) << c0;
     }
     kept = __popcll(keep);
-    const float perr = 4e-6f * (float)(length3(cA - cB) + GA.radius + rB + GB.spacing) + (float)skin;
+    const float perr = 4e-6f * (float)(length3(cA - cB) + n.G.geo[gA].radius + SB.geo[gB].radius + SB.geo[gB].spacing) +
+                       (float)skin;
     int ncand = 0;
-    // a cluster's range and nodes are loaded while the one before is filtered:
-    // range, node and cell minimum are three dependent loads a cluster
-    int2 cr = make_int2(0, 0);
-    float4 nd = make_float4(0.f, 0.f, 0.f, 0.f);
+    // the next clusters' ranges and nodes are loaded while these are filtered:
+    // range, node and grid values are three dependent loads a cluster
+    int2 r[NODES];
+    float4 node[NODES];
     auto fetch = [&] {
-        const int c = __ffsll((long long)keep) - 1;
-        keep &= keep - 1ull;
-        cr = n.G.clus_range[GA.clus_off + c];
-        if (lane < cr.y) nd = n.G.nodes32[GA.node_off + cr.x + lane];
+#pragma unroll
+        for (int u = 0; u < NODES; ++u) {
+            r[u] = make_int2(0, 0);
+            if (!keep) continue;
+            const int c = __ffsll((long long)keep) - 1;
+            keep &= keep - 1ull;
+            r[u] = n.G.clus_range[GA.clus_off + c];
+            if (lane < r[u].y) node[u] = n.G.nodes32[GA.node_off + r[u].x + lane];
+        }
     };
-    bool more = keep != 0ull;
-    if (more) fetch();
-    while (more) {
-        const int2 r = cr;
-        const float4 node = nd;
-        more = keep != 0ull;
-        if (more) fetch();
-        const bool cand = lane < r.y && !node_filtered<KIND>(node, xf, GB, SB, (float)rB, perr, n.a.probe);
-        const unsigned int m = __ballot_sync(0xffffffffu, cand);
-        if (cand) queue[ncand + __popc(m & lt_mask)] = (unsigned short)(r.x + lane);
-        ncand += __popc(m);
+#pragma unroll
+    for (int u = 0; u < NODES; ++u) node[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    fetch();
+    for (int left = kept; left > 0; left -= NODES) {
+        int first[NODES];
+        float4 p[NODES];
+        bool on[NODES], out[NODES];
+#pragma unroll
+        for (int u = 0; u < NODES; ++u) {
+            first[u] = r[u].x;
+            p[u] = node[u];
+            on[u] = lane < r[u].y;
+        }
+        if (left > NODES) fetch();
+        node_filter<KIND, NODES>(p, on, xf, GB, SB, perr, probe, out);
+#pragma unroll
+        for (int u = 0; u < NODES; ++u) {
+            const unsigned int m = __ballot_sync(0xffffffffu, !out[u]);
+            if (!out[u]) queue[ncand + __popc(m & lt_mask)] = (unsigned short)(first[u] + lane);
+            ncand += __popc(m);
+        }
     }
     __syncwarp();
     return ncand;
@@ -1620,7 +1702,7 @@ __device__ __forceinline__ void select_list(const NarrowArgs& n, int block, int 
         const int A = L.pairA[p];
         const int B = L.pairB[p];
         int kept;
-        int ncand = cull_pair<KIND>(n, A, B, skin, lane, s_node[wib], kept);
+        int ncand = cull_pair<KIND, 1>(n, A, B, skin, lane, s_node[wib], kept);
         if (n.a.stats && lane == 0) {
             atomicAdd(&s_stats[0], 1ull);
             atomicAdd(&s_stats[1], (unsigned long long)min(n.G.geo[n.P.geo[A]].clus_count, MAX_CLUSTERS));
@@ -1771,6 +1853,81 @@ __global__ void __launch_bounds__(TPB) k_slot_filter(NarrowArgs n)
     }
 }
 
+// What the predicate reads of a slot's two bodies, and with law what the
+// contact law does.  All of it is independent, and the asm keeps it in one
+// place: left to itself the compiler places each load near its use, some
+// thirty waits of a microsecond one after the other in the contact pass.
+struct PairState {
+    double3 xA, xB, vA, vB, wA, wB;
+    fd_quat qA, qB;
+    long long hB;
+    int gA, gB, mA, mB, nodes;
+    int hnode, hat;  // a carried slot: its previous self's node id and place (see contact_list)
+    bool carried;
+};
+__device__ __forceinline__ double load_now(const double* p)
+{
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int load_now(const int* p)
+{
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ long long load_now(const long long* p)
+{
+    long long v;
+    asm volatile("ld.global.s64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double3 load_now(const double3* p)
+{
+    return make_double3(load_now(&p->x), load_now(&p->y), load_now(&p->z));
+}
+__device__ __forceinline__ fd_quat load_now(const fd_quat* p)
+{
+    fd_quat v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.q0), "=d"(v.q1), "=d"(v.q2), "=d"(v.q3) : "l"(p));
+    return v;
+}
+template <int KIND, bool LAW>
+__device__ __forceinline__ PairState load_pair(const NarrowArgs& n, int A, int B)
+{
+    const ObjDev& O = Slave<KIND>::body(n);
+    PairState st;
+    st.carried = false;
+    if (!LAW) {
+        // the predicate pass: more warps hide the waits, and more registers
+        // would cost them
+        st.gA = n.P.geo[A];
+        st.gB = O.geo[B];
+        st.hB = Slave<KIND>::hash_of(n)[B];
+        st.xA = n.P.pos[A];
+        st.qA = load_q(n.P.q + A);
+        st.xB = Slave<KIND>::pos_of(n)[B];
+        st.qB = load_q(Slave<KIND>::q(n, B));
+        return st;
+    }
+    st.gA = load_now(n.P.geo + A);
+    st.gB = load_now(O.geo + B);
+    st.hB = load_now(Slave<KIND>::hash_of(n) + B);
+    st.xA = load_now(n.P.pos + A);
+    st.qA = load_now(n.P.q + A);
+    st.xB = load_now(Slave<KIND>::pos_of(n) + B);
+    st.qB = load_now(Slave<KIND>::q(n, B));
+    st.mA = load_now(n.P.mat + A);
+    st.mB = load_now(O.mat + B);
+    st.nodes = load_now(n.P.node_base + A);
+    st.vA = load_now(n.P.vel + A);
+    st.wA = load_now(n.P.angvel + A);
+    st.vB = load_now(Slave<KIND>::vel_of(n) + B);
+    st.wB = load_now(O.angvel + B);
+    return st;
+}
+
 // one slot's node against its partner
 struct SlotEval {
     double3 cA, cB, r, gp;  // centres, node offset from A's centre, node
@@ -1779,19 +1936,19 @@ struct SlotEval {
     double ov, fx, fy, fz, pv[8];
 };
 
-// the exact predicate of node k (relative to the geometry) of A against B;
+// the exact predicate of node k (relative to the geometry) of A against B (st);
 // e.ov keeps ov0 when the predicate stops before the distance
 template <int KIND>
-__device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, int A, int B, int k, int3 bcell, double ov0,
+__device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, const PairState& st, int k, int3 bcell, double ov0,
                                                SlotEval& e)
 {
-    const FdGeo& GA = n.G.geo[n.P.geo[A]];
-    e.cA = n.P.pos[A];
-    const fd_quat qA = load_q(n.P.q + A);
-    e.cB = Slave<KIND>::pos(n, B);
-    e.qB = load_q(Slave<KIND>::q(n, B));
-    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const FdGeo& GA = n.G.geo[st.gA];
+    e.cA = st.xA;
+    const fd_quat qA = st.qA;
+    e.cB = st.xB;
+    e.qB = st.qB;
     const GeoSetDev& SB = Slave<KIND>::set(n);
+    const FdGeo& GB = SB.geo[st.gB];
     const FdGrid& sg = Slave<KIND>::grid(n);
     const double rB2 = GB.radius * GB.radius;
     e.pool = GA.node_off + k;
@@ -1845,11 +2002,12 @@ __device__ __forceinline__ void store_force(const PairListDev& L, int t, const f
 // go to o.  Returns the global boundary-node id.
 template <int KIND>
 __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int s, int t, int A,
-                                           int B, int k, int oc_off, int oc_cnt, const SlotEval& e, double o[9])
+                                           int B, const PairState& st, int k, int oc_off, int oc_cnt,
+                                           const SlotEval& e, double o[9])
 {
     const bool periodic = (KIND == FD_PP || KIND == FD_PW) && (n.a.periodic_x || n.a.periodic_y);
-    const FdGeo& GA = n.G.geo[n.P.geo[A]];
-    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const FdGeo& GA = n.G.geo[st.gA];
+    const FdGeo& GB = Slave<KIND>::set(n).geo[st.gB];
     const double3 cA = e.cA, cB = e.cB, r = e.r, gp = e.gp;
     const fd_quat qB = e.qB;
     const double ov = e.ov;
@@ -1858,13 +2016,19 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
     nrm = fd_rot(qB, nrm);
     nrm = fd_normalize(nrm);
     const double3 pt = gp + (0.5 * ov) * nrm;
-    const int nid = n.P.node_base[A] + n.G.node_lid[pool];
+    const int nid = st.nodes + n.G.node_lid[pool];
     double3 spring = mk3(0., 0., 0.);
     int hist = -1;
-    {
+    if (st.carried) {
+        // a carried layout keeps each slot's previous self at its index
+        if (st.hnode == nid) hist = s;
+        if (hist >= 0) {
+            const double4 h = load_quad(L.o_c_hist + st.hat);
+            spring = mk3(h.x, h.y, h.z);
+        }
+    } else {
         // the previous slots of the pair are ascending in node
-        // key; a node appears at most once per pair.  A carried
-        // layout keeps each slot's previous self at its index.
+        // key; a node appears at most once per pair.
         const int oc_end = oc_off + oc_cnt;
         int lo = oc_off, hi = oc_end;
         if (s >= oc_off && s < oc_end && L.o_c_k[s] == k) lo = hi = s;
@@ -1913,21 +2077,20 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
             if (n.a.periodic_x) { ri = wrap_x(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_x(rj, n.pgrid); }
             if (n.a.periodic_y) { ri = wrap_y(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_y(rj, n.pgrid); }
         }
-        double3 vi = n.P.vel[A], vjs = Slave<KIND>::vel(n, B);
-        const double3 wi = n.P.angvel[A];
+        double3 vi = st.vA, vjs = st.vB;
+        const double3 wi = st.wA, wj = st.wB;
         if ((KIND == FD_PP || KIND == FD_PW) && n.a.sector) {
             sector_fold(ri, vi, n.pgrid.minb);
             if (KIND == FD_PP) sector_fold(rj, vjs, n.pgrid.minb);
         }
-        const int mi = n.P.mat[A];
+        const int mi = st.mA;
         const double invMi = GA.inv_mass;
         const double kni = n.M.kn[mi], ksi = n.M.ks[mi], mui = n.M.mu[mi], ei = n.M.e[mi];
-        double3 vj, wj;
+        double3 vj;
         double effM = 0., mu, res;
         if (KIND == FD_PW) {
             vj = vjs;
-            wj = n.W.angvel[B];
-            const int mj = n.W.mat[B];
+            const int mj = st.mB;
             mu = fmin(mui, n.MW.mu[mj]);
             res = fmin(ei, n.MW.e[mj]);
             if (invMi > 0.) effM = 1. / invMi;
@@ -1935,9 +2098,8 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
             ks = ksi;
         } else {
             vj = vjs;
-            wj = n.P.angvel[B];
             const double invMj = GB.inv_mass;
-            const int mj = n.P.mat[B];
+            const int mj = st.mB;
             const double knj = n.M.kn[mj], ksj = n.M.ks[mj];
             if (kni > 0. && knj > 0.) kn = kni * knj / (kni + knj);
             if (ksi > 0. && ksj > 0.) ks = ksi * ksj / (ksi + ksj);
@@ -1945,7 +2107,7 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
             res = fmin(ei, n.M.e[mj]);
             mu = fmin(mui, n.M.mu[mj]);
         }
-        const double3 vc = (vi + cross3(wi, pt - ri)) - (vj + cross3(wj, pt - rj));
+        const double3 vc = (vi + cross3e(wi, pt - ri)) - (vj + cross3e(wj, pt - rj));
         if (R.hit && s < R.cap) {
             R.vc[3 * s + 0] = vc.x;
             R.vc[3 * s + 1] = vc.y;
@@ -1954,9 +2116,9 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
         }
         double3 F = mk3(0., 0., 0.);
         linear_contact(F, spring, vc, nrm, ov, n.a.dt, kn, ks, mu, res, effM);
-        const double3 TA = cross3(pt - ri, F);
-        const double3 TB = cross3(pt - rj, -F);
-                            o[0] = F.x; o[1] = F.y; o[2] = F.z;
+        const double3 TA = cross3e(pt - ri, F);
+        const double3 TB = cross3e(F, pt - rj);
+        o[0] = F.x; o[1] = F.y; o[2] = F.z;
         o[3] = TA.x; o[4] = TA.y; o[5] = TA.z;
         o[6] = TB.x; o[7] = TB.y; o[8] = TB.z;
     }
@@ -1964,17 +2126,17 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
     store_hist(L, t, spring, B);
     if (n.a.records) {
         if (!n.with_force) {
-            const int mi = n.P.mat[A];
+            const int mi = st.mA;
             kn = n.M.kn[mi];
             ks = n.M.ks[mi];
             if (KIND != FD_PW) {
-                const int mj = n.P.mat[B];
+                const int mj = st.mB;
                 const double knj = n.M.kn[mj], ksj = n.M.ks[mj];
                 kn = (kn > 0. && knj > 0.) ? kn * knj / (kn + knj) : 0.;
                 ks = (ks > 0. && ksj > 0.) ? ks * ksj / (ks + ksj) : 0.;
             }
         }
-        store_record(L, t, pt, nrm, ov, 0.5 * ov * ov * kn, 0.5 * lengthSq3(spring) * ks);
+        store_record(L, t, pt, nrm, ov, 0.5 * ov * ov * kn, 0.5 * spring_sq(spring) * ks);
     }
     return nid;
 }
@@ -2027,11 +2189,17 @@ __device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int
             const int B = L.pairB[p];
             // a carried slot's history is its previous self, and its partner's
             // cell this step's
+            PairState st = load_pair<KIND, PASS == 1>(n, A, B);
+            if (PASS == 1 && carried) {
+                st.carried = true;
+                st.hnode = load_now(L.o_c_node + s);
+                st.hat = load_now(L.o_c_at + s);
+            }
             int4 aux = make_int4(0, 0, 0, s);
             int hist = 1;
             if (carried) {
                 int3 bc;
-                decode_cell(Slave<KIND>::hash(n, B), Slave<KIND>::grid(n).size, bc);
+                decode_cell(st.hB, Slave<KIND>::grid(n).size, bc);
                 aux.x = bc.x; aux.y = bc.y; aux.z = bc.z;
             } else {
                 aux = L.p_aux[p];
@@ -2040,13 +2208,13 @@ __device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int
             SlotEval e;
             // an overlap the predicate did not reach stays +inf (a slot that
             // is never skipped)
-            hit = slot_predicate<KIND>(n, A, B, k, make_int3(aux.x, aux.y, aux.z),
+            hit = slot_predicate<KIND>(n, st, k, make_int3(aux.x, aux.y, aux.z),
                                        PASS == 0 ? __longlong_as_double(0x7ff0000000000000ll) : 0., e);
             if (phi0_store) L.c_phi0[s] = __double2float_rd(-e.ov);
             int nid = -1;
             if (PASS == 1 && hit) {
                 double o[9];
-                nid = contact_law<KIND>(n, L, n.a.rec, s, t, A, B, k, aux.w, hist, e, o);
+                nid = contact_law<KIND>(n, L, n.a.rec, s, t, A, B, st, k, aux.w, hist, e, o);
                 if (n.with_force) store_force(L, t, o);
             }
             if (PASS == 1) {
@@ -2150,8 +2318,9 @@ __device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int blo
                 }
             }
             if (on) {
-                pf[9ll * q.x + l] = acc;
-                if (l == 0) pf[9ll * q.x + 8] = acc8;
+                Real* out = pf + (long long)RESULT * q.x;
+                out[l / 3 * 4 + l % 3] = acc;
+                if (l == 0) out[10] = acc8;
             }
         }
         __syncwarp();
@@ -2237,21 +2406,21 @@ struct SlotEval32 {
 
 // as slot_predicate
 template <int KIND>
-__device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int B, int k, int3 bcell, float ov0,
+__device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, const PairState& st, int k, int3 bcell, float ov0,
                                                  SlotEval32& e)
 {
-    const FdGeo& GA = n.G.geo[n.P.geo[A]];
-    const double3 cA = n.P.pos[A];
-    const double3 cB = Slave<KIND>::pos(n, B);
-    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const FdGeo& GA = n.G.geo[st.gA];
+    const double3 cA = st.xA;
+    const double3 cB = st.xB;
     const GeoSetDev& SB = Slave<KIND>::set(n);
+    const FdGeo& GB = SB.geo[st.gB];
     const FdGrid& sg = Slave<KIND>::grid(n);
     // the rigid transforms in double precision (as in FP64 mode), the
     // position inside the cell and the SDF interpolation in single
     e.cA = cA;
     e.cB = cB;
     e.pool = GA.node_off + k;
-    e.rd = xm_rot(load_q(n.P.q + A), n.G.nodes[e.pool]);
+    e.rd = xm_rot(st.qA, n.G.nodes[e.pool]);
     const double3 gp = mk3(e.rd.x + cA.x, e.rd.y + cA.y, e.rd.z + cA.z);
     e.gp = gp;
     int3 lo, hi;
@@ -2264,7 +2433,7 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int
     if (bcell.x >= lo.x && bcell.x <= hi.x && bcell.y >= lo.y && bcell.y <= hi.y && bcell.z >= lo.z && bcell.z <= hi.z) {
         const double3 rel = mk3(gp.x - cB.x, gp.y - cB.y, gp.z - cB.z);
         if (!Slave<KIND>::radius_test || xm_len2(rel) <= GB.radius * GB.radius) {
-            const double3 lp = xm_rrot(rel, load_q(Slave<KIND>::q(n, B)));
+            const double3 lp = xm_rrot(rel, st.qB);
             const double gx = (lp.x - GB.origin.x) * GB.inv_spacing;
             const double gy = (lp.y - GB.origin.y) * GB.inv_spacing;
             const double gz = (lp.z - GB.origin.z) * GB.inv_spacing;
@@ -2312,11 +2481,12 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, int A, int
 // as contact_law
 template <int KIND>
 __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairListDev& L, const AdjRec& R, int s, int t, int A,
-                                             int B, int k, int oc_off, int oc_cnt, const SlotEval32& e, float o[9])
+                                             int B, const PairState& st, int k, int oc_off, int oc_cnt,
+                                             const SlotEval32& e, float o[9])
 {
     const bool periodic = (KIND == FD_PP || KIND == FD_PW) && (n.a.periodic_x || n.a.periodic_y);
-    const FdGeo& GA = n.G.geo[n.P.geo[A]];
-    const FdGeo& GB = Slave<KIND>::geo(n, B);
+    const FdGeo& GA = n.G.geo[st.gA];
+    const FdGeo& GB = Slave<KIND>::set(n).geo[st.gB];
     const float4* RB = Slave<KIND>::rot(n, B);
     const float4 b0 = RB[0], b1 = RB[1], b2 = RB[2];
     const double3 cA = e.cA, cB = e.cB, rd = e.rd, gp = e.gp;
@@ -2335,10 +2505,16 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
     const float l2 = dotf(nrm, nrm);
     nrm = l2 > 1e-20f ? rsqrtf(l2) * nrm : mkf(0.f, 0.f, 0.f);
     const v3f arm = r + (0.5f * ov) * nrm;  // contact point relative to A's centre
-    const int nid = n.P.node_base[A] + n.G.node_lid[pool];
+    const int nid = st.nodes + n.G.node_lid[pool];
     double3 spring = mk3(0., 0., 0.);
     int hist = -1;
-    {
+    if (st.carried) {
+        if (st.hnode == nid) hist = s;
+        if (hist >= 0) {
+            const double4 h = load_quad(L.o_c_hist + st.hat);
+            spring = mk3(h.x, h.y, h.z);
+        }
+    } else {
         const int oc_end = oc_off + oc_cnt;
         int lo2 = oc_off, hi2 = oc_end;
         if (s >= oc_off && s < oc_end && L.o_c_k[s] == k) lo2 = hi2 = s;
@@ -2356,7 +2532,7 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
         }
     }
     if (R.hit && s < R.cap) {
-        const fd_quat qB = load_q(Slave<KIND>::q(n, B));
+        const fd_quat qB = st.qB;
         R.A[s] = A;
         R.B[s] = B;
         R.Bp[s] = KIND == FD_PW ? -1 : B;
@@ -2379,20 +2555,20 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
         R.arm[3 * s + 2] = rd.z;
         R.wrap[s] = 13 + 27;  // no shift unless the force side records one
     }
-    const int mi = n.P.mat[A];
+    const int mi = st.mA;
     float kn = 0.f, ks = 0.f;
     float mu, res, effM = 0.f;
     const double kni = n.M.kn[mi], ksi = n.M.ks[mi];
     const double invMi = GA.inv_mass;
     if (KIND == FD_PW) {
-        const int mj = n.W.mat[B];
+        const int mj = st.mB;
         mu = (float)fmin(n.M.mu[mi], n.MW.mu[mj]);
         res = (float)fmin(n.M.e[mi], n.MW.e[mj]);
         if (invMi > 0.) effM = (float)(1. / invMi);
         kn = (float)kni;
         ks = (float)ksi;
     } else {
-        const int mj = n.P.mat[B];
+        const int mj = st.mB;
         const double knj = n.M.kn[mj], ksj = n.M.ks[mj], invMj = GB.inv_mass;
         if (kni > 0. && knj > 0.) kn = (float)(kni * knj / (kni + knj));
         if (ksi > 0. && ksj > 0.) ks = (float)(ksi * ksj / (ksi + ksj));
@@ -2406,16 +2582,16 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
             if (n.a.periodic_x) { ri = wrap_x(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_x(rj, n.pgrid); }
             if (n.a.periodic_y) { ri = wrap_y(ri, n.pgrid); if (KIND == FD_PP) rj = wrap_y(rj, n.pgrid); }
         }
-        double3 vid = n.P.vel[A], vjd = Slave<KIND>::vel(n, B);
+        double3 vid = st.vA, vjd = st.vB;
         if ((KIND == FD_PP || KIND == FD_PW) && n.a.sector) {
             sector_fold(ri, vid, n.pgrid.minb);
             if (KIND == FD_PP) sector_fold(rj, vjd, n.pgrid.minb);
         }
         const v3f armA = tof(cA - ri) + arm;
         const v3f armB = tof(cA - rj) + arm;
-        const v3f vi = tof(vid), wi = tof(n.P.angvel[A]);
+        const v3f vi = tof(vid), wi = tof(st.wA);
         const v3f vj = tof(vjd);
-        const v3f wj = tof(KIND == FD_PW ? n.W.angvel[B] : n.P.angvel[B]);
+        const v3f wj = tof(st.wB);
         const v3f vc = (vi + crossf(wi, armA)) - (vj + crossf(wj, armB));
         if (R.hit && s < R.cap) {
             R.vc[3 * s + 0] = vc.x;
@@ -2434,7 +2610,7 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
     store_hist(L, t, spring, B);
     if (n.a.records) {
         store_record(L, t, mk3(cA.x + arm.x, cA.y + arm.y, cA.z + arm.z), mk3(nrm.x, nrm.y, nrm.z), ov,
-                     0.5 * (double)ov * (double)ov * (double)kn, 0.5 * lengthSq3(spring) * (double)ks);
+                     0.5 * (double)ov * (double)ov * (double)kn, 0.5 * spring_sq(spring) * (double)ks);
     }
     return nid;
 }
@@ -2484,11 +2660,17 @@ __device__ __forceinline__ void contact_list32(const NarrowArgs& n, int block, i
             const int B = L.pairB[p];
             // a carried slot's history is its previous self, and its partner's
             // cell this step's
+            PairState st = load_pair<KIND, PASS == 1>(n, A, B);
+            if (PASS == 1 && carried) {
+                st.carried = true;
+                st.hnode = load_now(L.o_c_node + s);
+                st.hat = load_now(L.o_c_at + s);
+            }
             int4 aux = make_int4(0, 0, 0, s);
             int hist = 1;
             if (carried) {
                 int3 bc;
-                decode_cell(Slave<KIND>::hash(n, B), Slave<KIND>::grid(n).size, bc);
+                decode_cell(st.hB, Slave<KIND>::grid(n).size, bc);
                 aux.x = bc.x; aux.y = bc.y; aux.z = bc.z;
             } else {
                 aux = L.p_aux[p];
@@ -2497,13 +2679,13 @@ __device__ __forceinline__ void contact_list32(const NarrowArgs& n, int block, i
             SlotEval32 e;
             // an overlap the predicate did not reach stays +inf (a slot that
             // is never skipped)
-            hit = slot_predicate32<KIND>(n, A, B, k, make_int3(aux.x, aux.y, aux.z),
+            hit = slot_predicate32<KIND>(n, st, k, make_int3(aux.x, aux.y, aux.z),
                                          PASS == 0 ? __int_as_float(0x7f800000) : 0.f, e);
             if (phi0_store) L.c_phi0[s] = e.phi0;
             int nid = -1;
             if (PASS == 1 && hit) {
                 float o[9];
-                nid = contact_law32<KIND>(n, L, n.a.rec, s, t, A, B, k, aux.w, hist, e, o);
+                nid = contact_law32<KIND>(n, L, n.a.rec, s, t, A, B, st, k, aux.w, hist, e, o);
                 if (n.with_force) store_force(L, t, o);
             }
             if (PASS == 1) {
@@ -2675,6 +2857,33 @@ __global__ void __launch_bounds__(TPB) k_step_end(EndArgs a)
     ctrl[4] = 0;
 }
 
+__device__ __forceinline__ double4 load_vec(const double* p) { return load_quad(reinterpret_cast<const double4*>(p)); }
+__device__ __forceinline__ float4 load_vec(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ void store_vec(double* p, double x, double y, double z)
+{
+    reinterpret_cast<double2*>(p)[0] = make_double2(x, y);
+    reinterpret_cast<double2*>(p)[1] = make_double2(z, 0.);
+}
+__device__ __forceinline__ void store_vec(float* p, float x, float y, float z)
+{
+    *reinterpret_cast<float4*>(p) = make_float4(x, y, z, 0.f);
+}
+// a bond's eight frame vectors, 192 bytes in six loads: with 24 loads at a
+// stride of 192 bytes (and six orientations' and nine results' worth more) the
+// bond kernels spent their time in the L1
+__device__ __forceinline__ void load_frames(const double3* p, double3 (&f)[8])
+{
+    const double4* q = reinterpret_cast<const double4*>(p);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const double4 a = load_quad(q + 3 * h), b = load_quad(q + 3 * h + 1), c = load_quad(q + 3 * h + 2);
+        f[4 * h] = make_double3(a.x, a.y, a.z);
+        f[4 * h + 1] = make_double3(a.w, b.x, b.y);
+        f[4 * h + 2] = make_double3(b.z, b.w, c.x);
+        f[4 * h + 3] = make_double3(c.y, c.z, c.w);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // bonds, contactKernel.cuh:138-199 and contactKernel.cu:293-371
 // ---------------------------------------------------------------------------
@@ -2682,17 +2891,18 @@ __global__ void k_bonds(ObjDev P, BondDev Bd)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= Bd.n) return;
-    double* E = Bd.energy + 6ll * k;
-    double* O = Bd.out + 9ll * k;
+    double2* E2 = reinterpret_cast<double2*>(Bd.energy + 6ll * k);
+    double* O = reinterpret_cast<double*>(Bd.out) + (long long)RESULT * k;
     if (Bd.rec_active) Bd.rec_active[k] = Bd.active[k] != 0;
     if (Bd.active[k] == 0) {
-        for (int t = 0; t < 6; ++t) E[t] = 0.;
-        for (int t = 0; t < 9; ++t) O[t] = 0;
+        for (int t = 0; t < 3; ++t) E2[t] = make_double2(0., 0.);
+        for (int t = 0; t < 3; ++t) store_vec(O + 4 * t, 0, 0, 0);
         return;
     }
     const int i = Bd.master[k], j = Bd.slave[k];
-    const fd_quat qi = P.q[i], qj = P.q[j];
-    const double3* f = Bd.frames + 8ll * k;
+    const fd_quat qi = load_q(P.q + i), qj = load_q(P.q + j);
+    double3 f[8];
+    load_frames(Bd.frames + 8ll * k, f);
     const double3 n1i = fd_rot(qi, f[0]), n2i = fd_rot(qi, f[1]), n3i = fd_rot(qi, f[2]);
     const double3 n1j = fd_rot(qj, f[4]), n2j = fd_rot(qj, f[5]), n3j = fd_rot(qj, f[6]);
     const double3 ri = P.pos[i], rj = P.pos[j];
@@ -2712,7 +2922,9 @@ __global__ void k_bonds(ObjDev P, BondDev Bd)
     }
     const double D = length3(rij);
     if (!fd_is_zero(D)) {
-        const double B1 = Bd.B[4 * k], B2 = Bd.B[4 * k + 1], B3 = Bd.B[4 * k + 2], B4 = Bd.B[4 * k + 3];
+        const double4 b = load_vec(Bd.B + 4ll * k);
+        const double B1 = b.x, B2 = b.y, B3 = b.z, B4 = b.w;
+        double E[6];
         const double R = Bd.radius[k], D0 = Bd.L0[k];
         const double3 nij = fd_normalize(rij);
         const double3 e = -nij;
@@ -2736,13 +2948,14 @@ __global__ void k_bonds(ObjDev P, BondDev Bd)
         E[5] = length3(bsf) / Ab + fabs(btt) / Jb * R;
         if (Bd.ts[k] > 0. && E[4] > Bd.ts[k]) act = 0;
         else if (Bd.coh[k] > 0. && E[5] > Bd.coh[k] - Bd.mu[k] * E[4]) act = 0;
+        for (int t = 0; t < 3; ++t) E2[t] = make_double2(E[2 * t], E[2 * t + 1]);
     }
     Bd.active[k] = act;
     const double3 Ti = Mij + cross3(rbi - ri, F);
     const double3 Tj = Mji + cross3(rbj - rj, -F);
-    O[0] = F.x; O[1] = F.y; O[2] = F.z;
-    O[3] = Ti.x; O[4] = Ti.y; O[5] = Ti.z;
-    O[6] = Tj.x; O[7] = Tj.y; O[8] = Tj.z;
+    store_vec(O, F.x, F.y, F.z);
+    store_vec(O + 4, Ti.x, Ti.y, Ti.z);
+    store_vec(O + 8, Tj.x, Tj.y, Tj.z);
 }
 
 // the V-bond (contactKernel.cuh:138-199) in single precision; the frames are
@@ -2752,18 +2965,19 @@ __global__ void k_bonds32(ObjDev P, BondDev Bd)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= Bd.n) return;
-    double* E = Bd.energy + 6ll * k;
-    float* O = reinterpret_cast<float*>(Bd.out) + 9ll * k;
+    double2* E2 = reinterpret_cast<double2*>(Bd.energy + 6ll * k);
+    float* O = reinterpret_cast<float*>(Bd.out) + (long long)RESULT * k;
     if (Bd.rec_active) Bd.rec_active[k] = Bd.active[k] != 0;
     if (Bd.active[k] == 0) {
-        for (int t = 0; t < 6; ++t) E[t] = 0.;
-        for (int t = 0; t < 9; ++t) O[t] = 0;
+        for (int t = 0; t < 3; ++t) E2[t] = make_double2(0., 0.);
+        for (int t = 0; t < 3; ++t) store_vec(O + 4 * t, 0, 0, 0);
         return;
     }
     const int i = Bd.master[k], j = Bd.slave[k];
     const float4 a0 = P.rot[3ll * i], a1 = P.rot[3ll * i + 1], a2 = P.rot[3ll * i + 2];
     const float4 b0 = P.rot[3ll * j], b1 = P.rot[3ll * j + 1], b2 = P.rot[3ll * j + 2];
-    const double3* f = Bd.frames + 8ll * k;
+    double3 f[8];
+    load_frames(Bd.frames + 8ll * k, f);
     const v3f n1i = rowsf(a0, a1, a2, tof(f[0])), n2i = rowsf(a0, a1, a2, tof(f[1])), n3i = rowsf(a0, a1, a2, tof(f[2]));
     const v3f n1j = rowsf(b0, b1, b2, tof(f[4])), n2j = rowsf(b0, b1, b2, tof(f[5])), n3j = rowsf(b0, b1, b2, tof(f[6]));
     const double3 ri = P.pos[i], rj = P.pos[j];
@@ -2782,8 +2996,9 @@ __global__ void k_bonds32(ObjDev P, BondDev Bd)
     }
     const float D = lenf(rij);
     if (D > 1e-20f) {
-        const float B1 = (float)Bd.B[4 * k], B2 = (float)Bd.B[4 * k + 1], B3 = (float)Bd.B[4 * k + 2],
-                    B4 = (float)Bd.B[4 * k + 3];
+        const double4 b = load_vec(Bd.B + 4ll * k);
+        const float B1 = (float)b.x, B2 = (float)b.y, B3 = (float)b.z, B4 = (float)b.w;
+        double E[6];
         const float R = (float)Bd.radius[k], D0 = (float)Bd.L0[k];
         const v3f nij = rsqrtf(dotf(rij, rij)) * rij;
         const v3f e = -nij;
@@ -2810,13 +3025,14 @@ __global__ void k_bonds32(ObjDev P, BondDev Bd)
         E[5] = ss;
         if (Bd.ts[k] > 0. && sn > (float)Bd.ts[k]) act = 0;
         else if (Bd.coh[k] > 0. && ss > (float)(Bd.coh[k] - Bd.mu[k] * (double)sn)) act = 0;
+        for (int t = 0; t < 3; ++t) E2[t] = make_double2(E[2 * t], E[2 * t + 1]);
     }
     Bd.active[k] = act;
     const v3f Ti = Mij + crossf(oi, F);
     const v3f Tj = Mji + crossf(oj, -F);
-    O[0] = F.x; O[1] = F.y; O[2] = F.z;
-    O[3] = Ti.x; O[4] = Ti.y; O[5] = Ti.z;
-    O[6] = Tj.x; O[7] = Tj.y; O[8] = Tj.z;
+    store_vec(O, F.x, F.y, F.z);
+    store_vec(O + 4, Ti.x, Ti.y, Ti.z);
+    store_vec(O + 8, Tj.x, Tj.y, Tj.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -2835,14 +3051,17 @@ struct ReduceArgs {
 template <typename Real> struct ForceSum {
     Real F[3] = {0, 0, 0}, T[3] = {0, 0, 0};
     // one pair or bond result, as the body's own (F, torque) or as the partner's
-    __device__ __forceinline__ void add(const Real* pf, Real sgn, int torque)
+    // (k: its number; torque 1: on A, 2: on B)
+    __device__ __forceinline__ void add(const Real* results, long long k, Real sgn, int torque)
     {
-        F[0] += sgn * pf[0];
-        F[1] += sgn * pf[1];
-        F[2] += sgn * pf[2];
-        T[0] += pf[torque];
-        T[1] += pf[torque + 1];
-        T[2] += pf[torque + 2];
+        const Real* r = results + RESULT * k;
+        const auto f = load_vec(r), t = load_vec(r + 4 * torque);
+        F[0] += sgn * f.x;
+        F[1] += sgn * f.y;
+        F[2] += sgn * f.z;
+        T[0] += t.x;
+        T[1] += t.y;
+        T[2] += t.z;
     }
     // the pairs the particle owns in one list (s: first, c: count; no contact,
     // no sum kept), four hit flags loaded ahead
@@ -2854,7 +3073,7 @@ template <typename Real> struct ForceSum {
             for (int u = 0; u < 4; ++u) h[u] = k + u < s + c ? L.p_hit[k + u] : 0;
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                if (h[u]) add(reinterpret_cast<const Real*>(L.pf) + 9ll * (k + u), Real(1), 3);
+                if (h[u]) add(reinterpret_cast<const Real*>(L.pf), k + u, Real(1), 1);
         }
     }
     __device__ __forceinline__ void bonds(const BondDev& B, int i)
@@ -2862,9 +3081,8 @@ template <typename Real> struct ForceSum {
         const Real* out = reinterpret_cast<const Real*>(B.out);
         for (int e = B.plist_off[i]; e < B.plist_off[i + 1]; ++e) {
             const int code = B.plist[e];
-            const Real* o = out + 9ll * (code >> 1);
-            if ((code & 1) == 0) add(o, Real(1), 3);
-            else add(o, Real(-1), 6);
+            if ((code & 1) == 0) add(out, code >> 1, Real(1), 1);
+            else add(out, code >> 1, Real(-1), 2);
         }
     }
 };
@@ -2924,7 +3142,7 @@ __global__ void __launch_bounds__(128) k_advance(AdvanceArgs a)
                     const int kind = code[u] & 7, k = code[u] >> 3;
                     const PairListDev& L = r.L[kind];
                     if (kind != FD_PP && L.pairA[k] == i) continue;  // a particle against its own ghost
-                    f.add(reinterpret_cast<const Real*>(L.pf) + 9ll * k, Real(-1), 6);
+                    f.add(reinterpret_cast<const Real*>(L.pf), k, Real(-1), 2);
                 }
             }
             if (r.B.n > 0) f.bonds(r.B, i);
@@ -2996,12 +3214,12 @@ struct SmallArgs {
 
 // one pair of list L, one warp: its slots, written to L.c_k.  Returns the first
 // slot, their count, and the slots of the pair's history.
-template <int KIND>
+template <int KIND, int NODES>
 __device__ __forceinline__ int4 small_slots(const NarrowArgs& n, const PairListDev& L, int p, int A, int B, int lane,
                                             unsigned short* queue, unsigned long long* stats)
 {
     int kept;
-    int ncand = cull_pair<KIND>(n, A, B, 0.0, lane, queue, kept);
+    int ncand = cull_pair<KIND, NODES>(n, A, B, 0.0, lane, queue, kept);
     if (n.a.stats && lane == 0) {
         atomicAdd(&stats[0], 1ull);
         atomicAdd(&stats[1], (unsigned long long)min(n.G.geo[n.P.geo[A]].clus_count, MAX_CLUSTERS));
@@ -3033,20 +3251,21 @@ __device__ __forceinline__ bool small_contact(const NarrowArgs& n, const PairLis
                                               int s, int oc_off, int oc_cnt)
 {
     using Real = typename std::conditional<MIXED, float, double>::type;
+    const int k = load_now(L.c_k + s);
+    const PairState st = load_pair<KIND, true>(n, A, B);
     int3 bcell;
-    decode_cell(Slave<KIND>::hash(n, B), Slave<KIND>::grid(n).size, bcell);
-    const int k = L.c_k[s];
+    decode_cell(st.hB, Slave<KIND>::grid(n).size, bcell);
     int nid = -1;
     bool hit;
     Real o[9];
     if constexpr (MIXED) {
         SlotEval32 e;
-        hit = slot_predicate32<KIND>(n, A, B, k, bcell, 0.f, e);
-        if (hit) nid = contact_law32<KIND>(n, L, R, s, s, A, B, k, oc_off, oc_cnt, e, o);
+        hit = slot_predicate32<KIND>(n, st, k, bcell, 0.f, e);
+        if (hit) nid = contact_law32<KIND>(n, L, R, s, s, A, B, st, k, oc_off, oc_cnt, e, o);
     } else {
         SlotEval e;
-        hit = slot_predicate<KIND>(n, A, B, k, bcell, 0., e);
-        if (hit) nid = contact_law<KIND>(n, L, R, s, s, A, B, k, oc_off, oc_cnt, e, o);
+        hit = slot_predicate<KIND>(n, st, k, bcell, 0., e);
+        if (hit) nid = contact_law<KIND>(n, L, R, s, s, A, B, st, k, oc_off, oc_cnt, e, o);
     }
     if (hit) store_force(L, s, o);
     L.c_node[s] = nid;
@@ -3091,10 +3310,12 @@ __device__ __forceinline__ void small_emit(const PairListDev& L, unsigned int* f
     __syncwarp();
 }
 
-template <bool MIXED>
-__global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small_pairs(SmallArgs a)
+// BLOCKS: resident blocks per SM the registers are cut for
+template <bool MIXED, int BLOCKS>
+__global__ void __launch_bounds__(SMALL_WARPS * 32, BLOCKS) k_small_pairs(SmallArgs a)
 {
     using Real = typename std::conditional<MIXED, float, double>::type;
+    constexpr int NODES = BLOCKS > 2 ? 1 : 2;
     // the candidate lists and the node queues are not in use together
     __shared__ union {
         unsigned short queue[SMALL_WARPS][MAX_NODE_QUEUE];
@@ -3154,7 +3375,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
                         const double3 cB = n.P.pos[B];
                         const double rs = rA + GB.radius;
                         if (lengthSq3(cA - cB) <= rs * rs * (1.0 + 4.0 * BOUND_REL))
-                            pass = !body_culled32(cA, rA, cB, n.P.rot + 3ll * B, true, GB, n.G, n.a.probe);
+                            pass = !body_culled32(cA, rA, cB, n.P.rot + 3ll * B, true, n.G.geo32[n.P.geo[B]], n.G,
+                                                  n.a.probe);
                     }
                     const unsigned int m = __ballot_sync(full, pass);
                     if (pass) {
@@ -3198,7 +3420,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
                         const double rs = rA + GB.grid_radius;
                         const double3 cW = n.W.pos[w];
                         pass = lengthSq3(cA - cW) <= rs * rs * (1.0 + 4.0 * BOUND_REL) &&
-                               !body_culled32(cA, rA, cW, n.W.rot + 3ll * w, false, GB, n.GW, n.a.probe);
+                               !body_culled32(cA, rA, cW, n.W.rot + 3ll * w, false, n.GW.geo32[n.W.geo[w]], n.GW,
+                                              n.a.probe);
                     }
                 }
                 const unsigned int m = __ballot_sync(full, pass);
@@ -3220,8 +3443,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
         const int t = wall ? SMALL_TASKS + u - npp : u;
         const int2 k = s_task[t];
         const int At = A0 + k.y % SMALL_BODIES, p = k.y / SMALL_BODIES;
-        const int4 slot = wall ? small_slots<FD_PW>(n, a.Lw, p, At, k.x, lane, q.queue[wib], s_stats)
-                               : small_slots<FD_PP>(n, n.L, p, At, k.x, lane, q.queue[wib], s_stats);
+        const int4 slot = wall ? small_slots<FD_PW, NODES>(n, a.Lw, p, At, k.x, lane, q.queue[wib], s_stats)
+                               : small_slots<FD_PP, NODES>(n, n.L, p, At, k.x, lane, q.queue[wib], s_stats);
         if (lane == 0) {
             s_slot[t] = make_int2(slot.x, slot.z);
             s_cnt[t] = make_ushort2((unsigned short)slot.y, (unsigned short)slot.w);
@@ -3297,10 +3520,10 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
         if (!hits) continue;
         // a pair without a contact sums to zero: nobody reads it
         const int p = s_task[t].y / SMALL_BODIES;
-        Real* out = reinterpret_cast<Real*>(L.pf) + 9ll * p;
-        out[l] = acc;
+        Real* out = reinterpret_cast<Real*>(L.pf) + (long long)RESULT * p;
+        out[l / 3 * 4 + l % 3] = acc;
         if (l == 0) {
-            out[8] = acc8;
+            out[10] = acc8;
             atomicAdd(L.n_hits, hits);
             if (!wall) L.r_next[p] = atomicExch(&a.r_head[s_task[t].x], p);
             if (n.a.stats) atomicAdd(&s_stats[3], (unsigned long long)hits);
@@ -3315,7 +3538,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, FD_SMALL_MIN_BLOCKS) k_small
             const int2 r = s_range[body + w * SMALL_BODIES];
             const Real* pf = reinterpret_cast<const Real*>(w ? a.Lw.pf : n.L.pf);
             for (int t = r.x + w * SMALL_TASKS; t < r.x + w * SMALL_TASKS + r.y; ++t)
-                if (s_hits[t]) acc += pf[9ll * (s_task[t].y / SMALL_BODIES) + lane];
+                if (s_hits[t]) acc += pf[(long long)RESULT * (s_task[t].y / SMALL_BODIES) + lane / 3 * 4 + lane % 3];
         }
         reinterpret_cast<Real*>(a.own)[6ll * A + lane] = acc;
     }
@@ -3357,7 +3580,8 @@ __device__ __forceinline__ void small_partner_sum(const SmallAdvanceArgs& a, int
     }
     const Real* pf = reinterpret_cast<const Real*>(L.pf);
     if (cnt <= LOCAL) {
-        for (int e = 0; e < cnt; ++e) f.add(pf + 9ll * pair[e], Real(-1), 6);
+#pragma unroll 4
+        for (int e = 0; e < cnt; ++e) f.add(pf, pair[e], Real(-1), 2);
         return;
     }
     // a body with many owners: the next owner in order by a pass over the list
@@ -3369,7 +3593,7 @@ __device__ __forceinline__ void small_partner_sum(const SmallAdvanceArgs& a, int
             if (own > last && own < best) { best = own; at = p; }
         }
         last = best;
-        f.add(pf + 9ll * at, Real(-1), 6);
+        f.add(pf, at, Real(-1), 2);
     }
 }
 
@@ -3381,6 +3605,17 @@ __global__ void __launch_bounds__(64) k_small_advance(SmallAdvanceArgs a)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (FRONT && i < 6) a.zero[i / 3][i % 3] = 0;
     if (i < a.P.n) {
+        // one thread a body and a block or less an SM: the kernel is its chain
+        // of loads, so the state is on its way before the sums start
+        Body b;
+        int gi = 0;
+        if (BACK || FRONT) {
+            gi = load_now(a.P.geo + i);
+            b.x = load_now(a.P.pos + i);
+            b.v = load_now(a.P.vel + i);
+            b.w = load_now(a.P.angvel + i);
+            b.q = load_now(a.P.q + i);
+        }
         double3 F, T;
         if (SUM) {
             ForceSum<Real> f;
@@ -3400,8 +3635,7 @@ __global__ void __launch_bounds__(64) k_small_advance(SmallAdvanceArgs a)
             T = a.P.torque[i];
         }
         if (!BACK && !FRONT) return;
-        Body b{a.P.pos[i], a.P.vel[i], a.P.angvel[i], a.P.q[i]};
-        const FdGeo& geo = a.G.geo[a.P.geo[i]];
+        const FdGeo& geo = a.G.geo[gi];
         if (BACK) kick_body(b, geo, F, T, a.gravity, a.h);
         if (FRONT) {
             kick_body(b, geo, F, T, a.gravity, a.h);
@@ -3796,8 +4030,16 @@ void launch_small_pairs(const ObjDev& P, const GeoSetDev& G, const MatDev& M, co
     k.Lw = Lw; k.recw = recw; k.T = T; k.wall_range = wall_range; k.r_head = r_head;
     k.own = own;
     const int blocks = (P.n + SMALL_BODIES - 1) / SMALL_BODIES;
-    if (mixed) k_small_pairs<true><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
-    else k_small_pairs<false><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
+    // A block is a chain of some 20 us whatever its neighbours do.  While all
+    // blocks are resident at two per SM (1,184 particles) the kernel keeps its
+    // registers; more blocks than that go four to an SM with half as many,
+    // spilled values and all (4,096 particles: 65 us a step against 76; 1,000
+    // particles: 46 against 39).
+    const bool many = blocks > 2 * 148;
+    if (mixed && many) k_small_pairs<true, 4><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
+    else if (mixed) k_small_pairs<true, 2><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
+    else if (many) k_small_pairs<false, 4><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
+    else k_small_pairs<false, 2><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
     note_launch();
 }
 

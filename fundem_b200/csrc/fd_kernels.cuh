@@ -16,11 +16,9 @@
 #define FD_PROBE_MIN_BLOCKS 4
 #endif
 
+// the pair sums: short chains of loads, few registers
 #ifndef FD_SUM_BLOCKS
 #define FD_SUM_BLOCKS 8
-#endif
-#ifndef FD_SMALL_MIN_BLOCKS
-#define FD_SMALL_MIN_BLOCKS 2
 #endif
 
 namespace fd {
@@ -35,7 +33,7 @@ struct PairListDev {
     int* seg_cnt;      // per particle A: number of pairs
     int* c_off;        // per pair: first contact
     int* c_cnt;        // per pair: number of contacts
-    double* pf;        // per pair: F (3), torque on A (3), torque on B (3)
+    double* pf;        // per pair, RESULT: F, torque on A, torque on B
     int* n_pairs;      // device counter
     int cap_pairs;
     // previous step (history source)
@@ -84,6 +82,11 @@ struct PairListDev {
     double4* o_c_hist;
 };
 
+// A pair's or bond's force and two torques: three vectors of four (the last
+// unused), so that a body reads its two in one load each.  As nine numbers
+// they were six loads of eight bytes, each at 32 places a warp.
+constexpr int RESULT = 12;
+
 constexpr int CONTACT_REC = 20, CONTACT_POINT = 10, CONTACT_NORMAL = 13, CONTACT_OVERLAP = 16, CONTACT_EN = 17,
               CONTACT_ES = 18;
 
@@ -125,6 +128,7 @@ struct ObjDev {
 struct GeoSetDev {
     int n;
     const FdGeo* geo;
+    const FdGeo32* geo32;
     const double* sdf;
     const float* sdf32;
     // per grid point the four corner values (x, x + 1) of rows y and y + 1:
@@ -199,7 +203,7 @@ struct BondDev {
     const double* mu;
     const double3* frames; // 8 per bond: mn1 mn2 mn3 mp sn1 sn2 sn3 sp
     double* energy;        // 6 per bond: Un Us Ub Ut sn ss
-    double* out;           // 9 per bond: F, Ti, Tj
+    double* out;           // per bond, RESULT: F, Ti, Tj
     const int* plist_off;  // per particle (n+1): bonds touching it
     const int* plist;      // bond id * 2 + side
     int* rec_active;       // adjoint recording (null when off): bond active at the step

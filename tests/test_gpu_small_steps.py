@@ -72,6 +72,7 @@ def _run(fundem, sc, precision, form):
 
 
 CASES = [("heap", n, t) for n, t in ((1, False), (3, True), (4, False), (5, True), (64, True), (343, False))]
+CASES += [("heap", n, t) for n, t in ((1184, True), (1185, True), (2197, False))]  # two, then four blocks per SM
 CASES += [("crowd", m, False) for m in (15, 16, 17, 40)]
 
 
