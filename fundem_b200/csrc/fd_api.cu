@@ -2123,6 +2123,7 @@ int fundem_step_graph(fundem_sim* s, int nsteps, const double g[3], double dt)
             const unsigned long long epoch = s->alloc_epoch, gepoch = g_alloc_epoch.load();
             s->stream = s->cap_stream;
             s->capturing = true;
+            fd::set_launch_ahead(false);
             const long long launches0 = s->launches, pc_steps0 = s->pc_steps;
             cudaGraph_t graph = nullptr;
             cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
@@ -2139,11 +2140,13 @@ int fundem_step_graph(fundem_sim* s, int nsteps, const double g[3], double dt)
                 if (graph) cudaGraphDestroy(graph);
                 s->stream = own;
                 s->capturing = false;
+                fd::set_launch_ahead(true);
                 throw;
             }
             e = cudaStreamEndCapture(s->stream, &graph);
             s->stream = own;
             s->capturing = false;
+            fd::set_launch_ahead(true);
             FD_CUDA(e);
             if (s->alloc_epoch != epoch || g_alloc_epoch.load() != gepoch) {
                 cudaGraphDestroy(graph);

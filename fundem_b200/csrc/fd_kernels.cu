@@ -1,22 +1,23 @@
 // fd_kernels.cu -- sm_100a kernels of the level-set DEM timestep.
 //
-// Per step (one CUDA stream, no host synchronisation):
-//   kick + drift (+ wall drift)            particleIntegrationKernel.cu:3-48
-//   hash + lists of the objects per cell   mySpatialGrid.cu:4-26, buildHashStartEnd.cu:47-137
-//   broad phase: one thread per particle lists candidate partners (bounding
+// Per step (no host synchronisation; the bonds on a stream of their own):
+//   kick, drift, hash (+ walls)            particleIntegrationKernel.cu:3-48, mySpatialGrid.cu:4-26
+//   lists of the objects per cell          buildHashStartEnd.cu:47-137
+//   broad phase: eight lanes per particle list candidate partners (bounding
 //                spheres, or SDF-grid spheres for walls and ghosts), sorted
 //                by partner id, into an A-major pair list
-//   narrow phase + contact force, fused: one warp per candidate pair streams
-//                A's surface nodes cluster by cluster through B's SDF,
-//                culls whole clusters with exact-conservative bounds, applies
-//                the reference's node predicate bit for bit
-//                (LSParticleContactDetectionKernel.cu:4-607), carries the
-//                sliding spring from the previous step, evaluates the linear
-//                spring-dashpot law (contactKernel.cuh:4-77) and reduces the
-//                pair's force and torques with warp shuffles
-//   reverse index of the pair list (pairs grouped by partner)
+//   selection:   one warp per candidate pair culls A's clusters of surface
+//                nodes, then the nodes, against B with exact-conservative
+//                bounds; the rest become the pair's contact slots
+//   predicate:   one thread per slot, the reference's node predicate bit for
+//                bit (LSParticleContactDetectionKernel.cu:4-607)
+//   contact law: one thread per contact, with the sliding spring of the
+//                previous step (contactKernel.cuh:4-77)
+//   pair sums, and the reverse index (pairs grouped by partner)
 //   bonds (contactKernel.cu:293-371), one thread per bond
-//   per-particle reduction in a fixed order (no atomics on forces)
+//   per-particle sums in a fixed order (no atomics on forces)
+// Each stage is one launch for all contact lists; a small set's step is two
+// launches in all.
 #include "fd_kernels.cuh"
 #include "../../include/fundem_b200.h"
 
@@ -28,6 +29,17 @@
 namespace fd {
 
 namespace {
+
+// The two kernels of a small set's step take turns on one stream.  Each is
+// launched while the other runs (launch_ahead): its blocks move in as the
+// other's leave, and this wait, before anything else, holds them until that
+// has finished and its writes are visible.  Every block waits first, so no
+// kernel overtakes the one before.
+__device__ __forceinline__ void step_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 constexpr int TPB = 256;
 constexpr int MAX_CAND = 64;        // candidate partners per particle and kind
@@ -1308,10 +1320,11 @@ template <> struct Slave<FD_GXY> : SlaveGhost {};
 // most of them reading the rebuild flag and returning), and at one or two
 // microseconds each they were a third of the step at 65,000 particles.  Each
 // list has a range of a launch's blocks.
+constexpr int MAX_LISTS = 5;  // particle pairs, walls, three image lists
 struct ListSet {
-    NarrowArgs l[FD_NKIND];
-    int kind[FD_NKIND];           // FD_PP .. FD_GR270
-    int block0[FD_NKIND + 1];
+    NarrowArgs l[MAX_LISTS];
+    int kind[MAX_LISTS];           // FD_PP .. FD_GR270
+    int block0[MAX_LISTS + 1];
     int n;
     CellTableDev T;               // the particles' cell table
     const int2* wall_range;       // see broad_walls
@@ -1401,11 +1414,17 @@ __device__ __forceinline__ double4 load_quad(const double4* p)
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
     return v;
 }
-// (of arrays the kernel does not write)
+// the same of what a kernel before this one wrote (and this one does not)
+__device__ __forceinline__ double4 load_four(const double4* p)
+{
+    double4 v;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ fd_quat load_q(const fd_quat* p)
 {
     fd_quat v;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.q0), "=d"(v.q1), "=d"(v.q2), "=d"(v.q3) : "l"(p));
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.q0), "=d"(v.q1), "=d"(v.q2), "=d"(v.q3) : "l"(p));
     return v;
 }
 
@@ -2023,7 +2042,7 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
         // a carried layout keeps each slot's previous self at its index
         if (st.hnode == nid) hist = s;
         if (hist >= 0) {
-            const double4 h = load_quad(L.o_c_hist + st.hat);
+            const double4 h = load_four(L.o_c_hist + st.hat);
             spring = mk3(h.x, h.y, h.z);
         }
     } else {
@@ -2039,7 +2058,7 @@ __device__ __forceinline__ int contact_law(const NarrowArgs& n, const PairListDe
         if (lo < oc_end && L.o_c_k[lo] == k) {
             const int at = L.o_c_at[lo];
             if (L.o_c_node[lo] == nid) {
-                const double4 h = load_quad(L.o_c_hist + at);
+                const double4 h = load_four(L.o_c_hist + at);
                 spring = mk3(h.x, h.y, h.z);
                 hist = lo;
             }
@@ -2511,7 +2530,7 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
     if (st.carried) {
         if (st.hnode == nid) hist = s;
         if (hist >= 0) {
-            const double4 h = load_quad(L.o_c_hist + st.hat);
+            const double4 h = load_four(L.o_c_hist + st.hat);
             spring = mk3(h.x, h.y, h.z);
         }
     } else {
@@ -2525,7 +2544,7 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
         if (lo2 < oc_end && L.o_c_k[lo2] == k) {
             const int at = L.o_c_at[lo2];
             if (L.o_c_node[lo2] == nid) {
-                const double4 h = load_quad(L.o_c_hist + at);
+                const double4 h = load_four(L.o_c_hist + at);
                 spring = mk3(h.x, h.y, h.z);
                 hist = lo2;
             }
@@ -2711,7 +2730,11 @@ __device__ __forceinline__ void contact_list32(const NarrowArgs& n, int block, i
     if (PASS == 0 && n.a.stats && lane == 0 && hits) atomicAdd(&n.a.stats[3], (unsigned long long)hits);
 }
 
-// the two contact passes and the pair sums of every list
+// The two contact passes of every list, bound by the waits of their gathers
+// (16-22 stalls for a load per issue).  262,144 bodies on a carried step, 2.4
+// million slots tested, 340,000 contacts: predicate 106 us (111 with 8-byte
+// loads of the corners), law 80 us (126 with a result per slot and each load
+// at its use).
 template <bool MIXED, int PASS>
 __global__ void __launch_bounds__(TPB, PASS == 0 ? FD_PROBE_MIN_BLOCKS : FD_CONTACT_MIN_BLOCKS) k_contact_lists(ListSet a)
 {
@@ -2857,8 +2880,8 @@ __global__ void __launch_bounds__(TPB) k_step_end(EndArgs a)
     ctrl[4] = 0;
 }
 
-__device__ __forceinline__ double4 load_vec(const double* p) { return load_quad(reinterpret_cast<const double4*>(p)); }
-__device__ __forceinline__ float4 load_vec(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ double4 load_vec(const double* p) { return load_four(reinterpret_cast<const double4*>(p)); }
+__device__ __forceinline__ float4 load_vec(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void store_vec(double* p, double x, double y, double z)
 {
     reinterpret_cast<double2*>(p)[0] = make_double2(x, y);
@@ -3091,7 +3114,10 @@ template <typename Real> struct ForceSum {
 // second half kick (BACK), and the next step's first half kick, drift, hash
 // and pair-cache check, walls too (FRONT).  Between two steps all of it is one
 // pass over the bodies; the sums, the copy of the wrapped positions, two
-// kicks, two drifts, two hashes and two checks were a launch each.
+// kicks, two drifts, two hashes and two checks were a launch each.  Bound by
+// the waits of range, flag and result, a thread a body; 262,144 bodies take
+// 54 us (162 MB from and to memory: 25 us at the measured copy rate), 72 with
+// the results as single numbers and no load ahead.
 struct AdvanceArgs {
     ObjDev P, W;
     GeoSetDev G, GW;
@@ -3196,6 +3222,11 @@ __global__ void __launch_bounds__(128) k_advance(AdvanceArgs a)
 // cell lists of the next step.  The sums run in the staged kernels' order, so
 // the results are theirs.  A block's few slots leave most of its threads idle
 // in the contact law, so large sets stay with the staged kernels.
+//
+// Bound by the chain of one block: about 9,400 cycles of search, 13,000 of
+// culling (two pairs a warp), 8,000 of predicate and law, 4,000 of sums.  A
+// step of 1,000 particles takes 38 us (50 with a pair's slots in its own warp),
+// of 4,096 65 us (81; 118 a step in the staged kernels).
 // ---------------------------------------------------------------------------
 constexpr int SMALL_BODIES = 4;               // particles per block
 constexpr int SMALL_WARPS = 2 * SMALL_BODIES;  // a warp for each one's partners, one for its walls
@@ -3314,6 +3345,7 @@ __device__ __forceinline__ void small_emit(const PairListDev& L, unsigned int* f
 template <bool MIXED, int BLOCKS>
 __global__ void __launch_bounds__(SMALL_WARPS * 32, BLOCKS) k_small_pairs(SmallArgs a)
 {
+    step_wait();
     using Real = typename std::conditional<MIXED, float, double>::type;
     constexpr int NODES = BLOCKS > 2 ? 1 : 2;
     // the candidate lists and the node queues are not in use together
@@ -3602,6 +3634,7 @@ __device__ __forceinline__ void small_partner_sum(const SmallAdvanceArgs& a, int
 template <typename Real, bool SUM, bool BACK, bool FRONT>
 __global__ void __launch_bounds__(64) k_small_advance(SmallAdvanceArgs a)
 {
+    step_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (FRONT && i < 6) a.zero[i / 3][i % 3] = 0;
     if (i < a.P.n) {
@@ -3663,6 +3696,8 @@ __global__ void __launch_bounds__(64) k_small_advance(SmallAdvanceArgs a)
 // (fundem_launch_count); none when it set none
 thread_local long long* t_launch_counter = nullptr;
 void set_launch_counter(long long* c) { t_launch_counter = c; }
+thread_local bool t_launch_ahead = true;
+void set_launch_ahead(bool on) { t_launch_ahead = on; }
 void count_launch()
 {
     if (t_launch_counter) ++*t_launch_counter;
@@ -3670,6 +3705,33 @@ void count_launch()
 static inline void note_launch()
 {
     if (t_launch_counter) ++*t_launch_counter;
+}
+// A kernel that begins with step_wait.  Not in recorded graphs, whose launches
+// are a microsecond apart as it is (4,096 particles: 65.8 us a step against
+// 64.8); a plain step of 777 particles went from 52.6 to 44.6 us.  Nor the
+// staged kernels, whose waiting blocks hold registers and shared memory that
+// the bonds and the kernel before could use (16,384 particles, 8 plain steps
+// between uploads: 4.1 ms against 3.8).
+template <typename... P, typename... A>
+static void launch_ahead(void (*kernel)(P...), int blocks, int threads, cudaStream_t s, const A&... args)
+{
+    cudaLaunchAttribute ahead{};
+    ahead.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    ahead.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)blocks);
+    c.blockDim = dim3((unsigned)threads);
+    c.stream = s;
+    c.attrs = &ahead;
+    c.numAttrs = t_launch_ahead ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+    note_launch();
+}
+template <typename... P, typename... A>
+static void launch_step(void (*kernel)(P...), int blocks, int threads, cudaStream_t s, const A&... args)
+{
+    kernel<<<blocks, threads, 0, s>>>(args...);
+    note_launch();
 }
 
 // ---------------------------------------------------------------------------
@@ -3839,7 +3901,7 @@ void launch_images(const ObjDev& P, double3* dst, const GhostDev* gh, const int*
 {
     if (P.n <= 0) return;
     ImageArgs a{P, dst, {gh[0], gh[1], gh[2]}, {on[0], on[1], on[2]}, ext_skin, ctrl};
-    k_images<<<nblocks(P.n), TPB, 0, s>>>(a); note_launch();
+    launch_step(k_images, nblocks(P.n), TPB, s, a);
 }
 void reset_image_box(int* occ, cudaStream_t s)
 {
@@ -3894,7 +3956,7 @@ void launch_broad(const ListArgs* lists, int n, const StepShared& c, NlDev* nl, 
     }
     for (int k = 0; k < n; ++k) blocks[k] = std::min(nblocks(c.n), 148 * 8);
     ListSet a = list_set(lists, n, c, blocks);
-    k_begin_lists<<<a.block0[n], TPB, 0, s>>>(a); note_launch();
+    launch_step(k_begin_lists, a.block0[n], TPB, s, a);
     if (nl) {
         // the particle-particle list comes from the neighbour list
         for (int k = 0; k < n; ++k) {
@@ -3917,7 +3979,7 @@ void launch_broad(const ListArgs* lists, int n, const StepShared& c, NlDev* nl, 
     }
     if (total == 0) return;
     a = list_set(lists, n, c, blocks);
-    k_broad_lists<<<total, TPB, 0, s>>>(a); note_launch();
+    launch_step(k_broad_lists, total, TPB, s, a);
 }
 
 void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream_t s)
@@ -3938,28 +4000,22 @@ void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream
     int blocks[FD_NKIND];
     share(blocks, shape[0] > 0 ? shape[0] : FD_SELECT_MIN_BLOCKS);
     ListSet a = list_set(lists, n, c, blocks);
-    k_select_lists<<<a.block0[n], NARROW_WARPS * 32, 0, s>>>(a); note_launch();
+    launch_step(k_select_lists, a.block0[n], NARROW_WARPS * 32, s, a);
     const int probe = shape[1] > 0 ? shape[1] : FD_PROBE_MIN_BLOCKS;
     for (int k = 0; k < n; ++k) {
         if (lists[k].kind != FD_PP || !lists[k].a.gate) continue;
-        k_slot_filter<<<148 * probe, TPB, 0, s>>>(a.l[k]); note_launch();
+        launch_step(k_slot_filter, 148 * probe, TPB, s, a.l[k]);
     }
     share(blocks, probe);
     a = list_set(lists, n, c, blocks);
-    if (c.mixed) k_contact_lists<true, 0><<<a.block0[n], TPB, 0, s>>>(a);
-    else k_contact_lists<false, 0><<<a.block0[n], TPB, 0, s>>>(a);
-    note_launch();
+    launch_step(c.mixed ? k_contact_lists<true, 0> : k_contact_lists<false, 0>, a.block0[n], TPB, s, a);
     share(blocks, shape[2] > 0 ? shape[2] : 4);
     a = list_set(lists, n, c, blocks);
-    if (c.mixed) k_contact_lists<true, 1><<<a.block0[n], TPB, 0, s>>>(a);
-    else k_contact_lists<false, 1><<<a.block0[n], TPB, 0, s>>>(a);
-    note_launch();
+    launch_step(c.mixed ? k_contact_lists<true, 1> : k_contact_lists<false, 1>, a.block0[n], TPB, s, a);
     if (!c.with_force) return;
     share(blocks, shape[3] > 0 ? shape[3] : FD_SUM_BLOCKS);
     a = list_set(lists, n, c, blocks);
-    if (c.mixed) k_sum_lists<float><<<a.block0[n], TPB, 0, s>>>(a, c.R);
-    else k_sum_lists<double><<<a.block0[n], TPB, 0, s>>>(a, c.R);
-    note_launch();
+    launch_step(c.mixed ? k_sum_lists<float> : k_sum_lists<double>, a.block0[n], TPB, s, a, c.R);
 }
 
 void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists, const int* active, const RevDev& R,
@@ -3975,7 +4031,7 @@ void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists,
     a.cached_ghosts = cached_ghosts;
     if (pc) a.pc = *pc; else memset(&a.pc, 0, sizeof(a.pc));
     a.done = done;
-    k_step_end<<<std::min(nblocks(P.n), 148 * 8), TPB, 0, s>>>(a); note_launch();
+    launch_step(k_step_end, std::min(nblocks(P.n), 148 * 8), TPB, s, a);
 }
 
 void launch_advance(const StepShared& c, const ObjDev& P, const PairListDev* lists, const int* active, const BondDev& B,
@@ -4001,9 +4057,7 @@ void launch_advance(const StepShared& c, const ObjDev& P, const PairListDev* lis
     const int blocks = std::max(1, nblocks(P.n + ((parts & STEP_FRONT) ? c.W.n : 0), tpb));
 #define FD_ADVANCE(S, K, F)                                                                  \
     case (S ? STEP_SUM : 0) | (K ? STEP_BACK : 0) | (F ? STEP_FRONT : 0):                    \
-        if (c.mixed) k_advance<float, S, K, F><<<blocks, tpb, 0, s>>>(a);                    \
-        else k_advance<double, S, K, F><<<blocks, tpb, 0, s>>>(a);                           \
-        note_launch();                                                                       \
+        launch_step(c.mixed ? k_advance<float, S, K, F> : k_advance<double, S, K, F>, blocks, tpb, s, a); \
         break;
     switch (parts) {
         FD_ADVANCE(false, false, true)
@@ -4036,11 +4090,9 @@ void launch_small_pairs(const ObjDev& P, const GeoSetDev& G, const MatDev& M, co
     // spilled values and all (4,096 particles: 65 us a step against 76; 1,000
     // particles: 46 against 39).
     const bool many = blocks > 2 * 148;
-    if (mixed && many) k_small_pairs<true, 4><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
-    else if (mixed) k_small_pairs<true, 2><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
-    else if (many) k_small_pairs<false, 4><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
-    else k_small_pairs<false, 2><<<blocks, SMALL_WARPS * 32, 0, s>>>(k);
-    note_launch();
+    launch_ahead(mixed ? (many ? k_small_pairs<true, 4> : k_small_pairs<true, 2>)
+                       : (many ? k_small_pairs<false, 4> : k_small_pairs<false, 2>),
+                 blocks, SMALL_WARPS * 32, s, k);
 }
 
 void launch_small_advance(const ObjDev& P, const GeoSetDev& G, const ObjDev& W, const FdGrid& pgrid,
@@ -4056,9 +4108,7 @@ void launch_small_advance(const ObjDev& P, const GeoSetDev& G, const ObjDev& W, 
     const int blocks = std::max(1, (P.n + ((parts & STEP_FRONT) ? W.n : 0) + tpb - 1) / tpb);
 #define FD_ADVANCE(S, K, F)                                                                                    \
     case (S ? STEP_SUM : 0) | (K ? STEP_BACK : 0) | (F ? STEP_FRONT : 0):                                   \
-        if (mixed) k_small_advance<float, S, K, F><<<blocks, tpb, 0, s>>>(a);                                  \
-        else k_small_advance<double, S, K, F><<<blocks, tpb, 0, s>>>(a);                                       \
-        note_launch();                                                                                         \
+        launch_ahead(mixed ? k_small_advance<float, S, K, F> : k_small_advance<double, S, K, F>, blocks, tpb, s, a); \
         break;
     switch (parts) {
         FD_ADVANCE(false, false, true)

@@ -443,6 +443,9 @@ void launch_pack_contacts(const PairListDev& L, const ContactPackDev& v, int* at
 // the duration of each call.  count_launch() counts one launch made
 // elsewhere (the adjoint kernels).
 void set_launch_counter(long long* c);
+// whether the calling thread launches a step's kernels ahead of one another's
+// end (default) or not (while it records a graph); see launch_ahead
+void set_launch_ahead(bool on);
 void count_launch();
 
 // exclusive scan of n ints (out may alias in); returns needed tmp ints when tmp == nullptr

@@ -279,7 +279,8 @@ constexpr int MESH_BLOCK = 32 * MESH_WARPS;  // also the triangles staged at a t
 // The distance is the minimum over all triangles and the sign the winding
 // number's (a sum of solid angles), in double precision that was three square
 // roots, an arc tangent and a closest point for every node and triangle: 4.6
-// ms for 48^3 nodes and 2,304 triangles, bound by the double-precision pipe.
+// ms for 48^3 nodes and 2,304 triangles, bound by the double-precision pipe (a
+// call, with its copies, 5.1 ms; now 2.6).
 // Here single precision screens both, and double precision decides:
 //   * pass 1 sums the solid angles in single precision (half_angle32) and finds
 //     the triangle of the nearest centroid; its exact distance bounds the

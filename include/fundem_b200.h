@@ -45,9 +45,8 @@ const char* fundem_status_string(int status);
    activateGPUDevice, LSSolver.h:601-613 (which calls exit(1) on failure;
    this returns FUNDEM_ERR_CUDA).  stream may be NULL (the legacy stream).
    Every call's work is ordered on that stream; inside a step the simulation
-   forks the particle-wall and image detection onto two streams of its own
-   and joins them back before the force sums, so a call's work still ends on
-   the given stream. */
+   forks the bonds onto a stream of its own and joins it back before the force
+   sums, so a call's work still ends on the given stream. */
 int fundem_create(fundem_sim** out, int device, void* stream);
 int fundem_destroy(fundem_sim* sim);
 /* precision of the contact path.  FUNDEM_FP64 reproduces the reference.
@@ -373,7 +372,9 @@ const char* fundem_last_error(fundem_sim* sim);
 int fundem_launch_count(fundem_sim* sim, long long* n);
 /* CUDA-event timing of kernel groups on the simulation's stream (off by
    default).  fundem_kernel_time returns the summed device time and the
-   number of timed intervals since the last query, then resets. */
+   number of timed intervals since the last query, then resets.  Steps hash
+   their bodies with the integration: FUNDEM_T_HASH counts the detections
+   outside steps and the cell lists. */
 enum {
     FUNDEM_T_INTEGRATE = 0, FUNDEM_T_HASH = 1, FUNDEM_T_BROAD = 2, FUNDEM_T_NARROW_PP = 3,
     FUNDEM_T_NARROW_PW = 4, FUNDEM_T_GHOST = 5, FUNDEM_T_REDUCE = 6, FUNDEM_NTIMERS = 7
