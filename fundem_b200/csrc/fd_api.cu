@@ -1205,6 +1205,10 @@ struct fundem_sim {
         pgrid = make_grid(mn, mx, pcell, setup_done ? &pgrid : nullptr);
         wgrid = make_grid(mn, mx, wcell, setup_done ? &wgrid : nullptr);
         ptab.alloc(pgrid, P.n());
+        // the particle table's build numbers start again, and the heads of the
+        // reverse index carry them: none may hold a number of the earlier phase
+        if (rev_head.n) FD_CUDA(after_legacy(cudaMemset(rev_head.p, 0, sizeof(rev_head.p[0]) * rev_head.n)));
+        rev_valid = false;
         configure_nl();
         configure_pc();
         if (!wall_groups.empty()) {
@@ -1440,7 +1444,8 @@ struct fundem_sim {
         PairListDev views[FD_NKIND];
         for (int k = 0; k < FD_NKIND; ++k) views[k] = lists[k].view();
         std::copy(active, active + FD_NKIND, step_active);
-        fd::launch_step_end(Pv, Wv, views, active, c.R, pc ? &pcv : nullptr, pcg, end_done.p, stream);
+        fd::launch_step_end(Pv, Wv, views, active, c.R, pc ? &pcv : nullptr, pcg, end_done.p,
+                            flags.p, stream);
         tend(FUNDEM_T_REDUCE);
         if (forked) FD_CUDA(cudaStreamWaitEvent(stream, br_join, 0));
         sum_pending = true;
@@ -2192,7 +2197,8 @@ int fundem_sync(fundem_sim* s)
         if (s->flags.p) FD_CUDA(cudaMemcpy(&f, s->flags.p, sizeof(unsigned int), cudaMemcpyDeviceToHost));
     });
     if (r) return r;
-    if (f & (FD_FLAG_PAIR_OVERFLOW | FD_FLAG_CONTACT_OVERFLOW | FD_FLAG_NEIGHBOR_OVERFLOW | FD_FLAG_CLUSTER_OVERFLOW))
+    if (f & (FD_FLAG_PAIR_OVERFLOW | FD_FLAG_CONTACT_OVERFLOW | FD_FLAG_NEIGHBOR_OVERFLOW | FD_FLAG_CLUSTER_OVERFLOW |
+             FD_FLAG_INDEX))
         return FUNDEM_ERR_CAPACITY;
     if (f & FD_FLAG_NONFINITE) return FUNDEM_ERR_NUMERIC;
     return FUNDEM_OK;

@@ -2793,6 +2793,7 @@ struct EndArgs {
     int cached;               // the pair cache is on; ghosts: so are the translated image lists
     int cached_ghosts;
     unsigned int* done;       // blocks finished (returns to 0)
+    unsigned int* flags;
 };
 __global__ void __launch_bounds__(TPB) k_step_end(EndArgs a)
 {
@@ -2803,7 +2804,12 @@ __global__ void __launch_bounds__(TPB) k_step_end(EndArgs a)
             const unsigned long long h = a.R.head[i];
             int cnt = 0;
             if ((unsigned int)(h >> 32) == build)
-                for (int code = (int)(unsigned int)h; code >= 0; code = a.L[code & 7].r_next[code >> 3]) ++cnt;
+                for (int code = (int)(unsigned int)h; code >= 0 && cnt <= a.R.cap; code = a.L[code & 7].r_next[code >> 3])
+                    ++cnt;
+            if (cnt > a.R.cap) {  // more links than the lists have pairs: not a list
+                set_flag(a.flags, FD_FLAG_INDEX);
+                cnt = 0;
+            }
             const int o = cnt ? atomicAdd(a.R.total, cnt) : 0;
             cnt = min(cnt, a.R.cap - o);
             a.R.off[i] = o;
@@ -4019,7 +4025,7 @@ void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream
 }
 
 void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists, const int* active, const RevDev& R,
-                     const PairCacheDev* pc, bool cached_ghosts, unsigned int* done, cudaStream_t s)
+                     const PairCacheDev* pc, bool cached_ghosts, unsigned int* done, unsigned int* flags, cudaStream_t s)
 {
     if (P.n <= 0) return;
     EndArgs a;
@@ -4031,6 +4037,7 @@ void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists,
     a.cached_ghosts = cached_ghosts;
     if (pc) a.pc = *pc; else memset(&a.pc, 0, sizeof(a.pc));
     a.done = done;
+    a.flags = flags;
     launch_step(k_step_end, std::min(nblocks(P.n), 148 * 8), TPB, s, a);
 }
 
