@@ -1429,8 +1429,12 @@ struct fundem_sim {
             tend(FUNDEM_T_GHOST);
             bonds();
         }
-        for (int d = 0; d < 6; ++d)
+        // the translated images, then the turned ones: with both, more lists
+        // than a launch takes
+        for (int d = 0; d < 6; ++d) {
+            if (d == 3 && sector && n) run(FUNDEM_T_GHOST, FUNDEM_T_GHOST);
             if (ghosts[d].active) add(FD_GX + d);
+        }
         if (!timed && !sector) add(FD_PP);
         if (n) run(FUNDEM_T_GHOST, FUNDEM_T_GHOST);
         step_wrapped = images && !sector ? img_pos.p : nullptr;

@@ -23,8 +23,9 @@
 
 #include <algorithm>
 #include <cstdio>
-#include <type_traits>
 #include <mutex>
+#include <stdexcept>
+#include <type_traits>
 
 namespace fd {
 
@@ -1320,7 +1321,7 @@ template <> struct Slave<FD_GXY> : SlaveGhost {};
 // most of them reading the rebuild flag and returning), and at one or two
 // microseconds each they were a third of the step at 65,000 particles.  Each
 // list has a range of a launch's blocks.
-constexpr int MAX_LISTS = 5;  // particle pairs, walls, three image lists
+constexpr int MAX_LISTS = 5;  // of a launch: particle pairs, walls, three image lists
 struct ListSet {
     NarrowArgs l[MAX_LISTS];
     int kind[MAX_LISTS];           // FD_PP .. FD_GR270
@@ -3927,6 +3928,7 @@ namespace {
 // kernel arguments of a set of lists, with blocks[k] blocks for list k
 ListSet list_set(const ListArgs* lists, int n, const StepShared& c, const int* blocks)
 {
+    if (n > MAX_LISTS) throw std::logic_error("more contact lists than a launch takes");
     ListSet a;
     a.n = n;
     a.T = c.T;
