@@ -749,6 +749,13 @@ struct fundem_sim {
     CellTable ptab;
     PairList lists[FD_NKIND];
     Ghost ghosts[6];  // X, Y, XY, then the sector images R90, R180, R270
+    // The image sets a step builds and detects.  The flags of periodicity can
+    // change between steps; the sets are those of the last setup, and a set
+    // that is not built in a step must not be detected either (its cell lists
+    // would be linked a second time).
+    bool turned_on() const { return sector && ghosts[3].active; }
+    bool image_on(int d) const { return ghosts[d].active && (d < 3 ? perX || perY || sector : sector); }
+    bool translated_on() const { return image_on(0) || image_on(1); }
     DevArray<unsigned int> flags;
     DevArray<unsigned long long> stats;  // narrow-phase work counters (profiling only)
     std::vector<int> node_base;
@@ -1124,7 +1131,7 @@ struct fundem_sim {
         a.gravity = make_double3(0, 0, 0);
         a.periodic_x = perX;
         a.periodic_y = perY;
-        a.sector = sector;
+        a.sector = turned_on();
         a.records = records;
         a.flags = flags.p;
         a.stats = counters ? stats.p : nullptr;
@@ -1245,7 +1252,7 @@ struct fundem_sim {
         small_head.alloc(std::max(np, 1), false);
         small_own.alloc(6 * (size_t)std::max(np, 1));
         FD_CUDA(after_legacy(cudaMemset(small_head.p, 0xff, sizeof(int) * small_head.n)));
-        if ((perX || perY) && !sector) img_pos.alloc(std::max(np, 1), false);
+        if (perX || perY) img_pos.alloc(std::max(np, 1), false);
         if (!br_stream) FD_CUDA(cudaStreamCreateWithFlags(&br_stream, cudaStreamNonBlocking));
         if (!br_join) FD_CUDA(cudaEventCreateWithFlags(&br_join, cudaEventDisableTiming));
         if (!end_done.p) end_done.alloc(1);
@@ -1311,15 +1318,15 @@ struct fundem_sim {
         // the translated image sets share the pair cache (not with sector
         // periodicity): their pairs and slots are kept with the particle
         // pairs', and a wrap or an image in a clamped cell rebuilds them
-        const bool pcg = pc && !sector;
+        const bool turned = turned_on(), images = translated_on();
+        const bool pcg = pc && !turned;
         int* gctrl = pcg ? pcv.ctrl : nullptr;
-        const bool images = perX || perY;
         fd::StepShared c = step_shared(with_force);
         if (with_force) {
             // the reverse index depends only on the lists' pairs: under the
             // pair cache (without sector images, whose lists are detected
             // afresh every step) a step that keeps them keeps the index
-            if (pc && !sector && rev_valid) {
+            if (pc && !turned && rev_valid) {
                 c.R.gate = pcv.ctrl;
                 c.R.gate2 = images ? pcv.ctrl + 4 : nullptr;
             }
@@ -1329,14 +1336,14 @@ struct fundem_sim {
             fd::launch_hash(Pv, pgrid, stream, c.T.build, c.T.par);
             if (W.n_dev > 0) fd::launch_hash(Wv, wgrid, stream);
             for (int d = 0; d < 6; ++d)
-                if (ghosts[d].active) fd::reset_image_box(ghosts[d].occ.p, stream);
+                if (image_on(d)) fd::reset_image_box(ghosts[d].occ.p, stream);
             tend(FUNDEM_T_HASH);
         }
         // the particles at their wrapped positions: a copy, which replaces the
         // positions in the force sums; in place with sector periodicity, whose
         // images are then detected after the particle and wall lists
         ObjDev Pg = Pv;
-        if (images && !sector) Pg.pos = img_pos.p;
+        if (images && !turned) Pg.pos = img_pos.p;
         int active[FD_NKIND] = {1, 1};
         fd::ListArgs L[FD_NKIND];
         int n = 0;
@@ -1386,7 +1393,7 @@ struct fundem_sim {
             int on[3];
             for (int d = 0; d < 3; ++d) {
                 gh[d] = ghosts[d].view(pcg);
-                on[d] = ghosts[d].active;
+                on[d] = image_on(d);
             }
             fd::launch_images(Pv, Pg.pos, gh, on, pcg ? pcv.skin : 0.0, gctrl, stream);
         };
@@ -1406,7 +1413,7 @@ struct fundem_sim {
             if (forked) FD_CUDA(cudaEventRecord(br_join, br_stream));
         };
         const bool timed = profiling && !capturing;
-        if (!sector) {
+        if (!turned) {
             tbegin(FUNDEM_T_GHOST);
             translated();
             tend(FUNDEM_T_GHOST);
@@ -1414,11 +1421,11 @@ struct fundem_sim {
         }
         add(FD_PW);
         if (timed) run(FUNDEM_T_BROAD, FUNDEM_T_NARROW_PW);
-        if (timed || sector) {
+        if (timed || turned) {
             add(FD_PP);
             if (timed) run(FUNDEM_T_BROAD, FUNDEM_T_NARROW_PP);
         }
-        if (sector) {
+        if (turned) {
             // LSSolver.h:780-784: wraps and images after the other detections
             if (n) run(FUNDEM_T_BROAD, FUNDEM_T_NARROW_PP);
             tbegin(FUNDEM_T_GHOST);
@@ -1432,12 +1439,12 @@ struct fundem_sim {
         // the translated images, then the turned ones: with both, more lists
         // than a launch takes
         for (int d = 0; d < 6; ++d) {
-            if (d == 3 && sector && n) run(FUNDEM_T_GHOST, FUNDEM_T_GHOST);
-            if (ghosts[d].active) add(FD_GX + d);
+            if (d == 3 && turned && n) run(FUNDEM_T_GHOST, FUNDEM_T_GHOST);
+            if (image_on(d)) add(FD_GX + d);
         }
-        if (!timed && !sector) add(FD_PP);
+        if (!timed && !turned) add(FD_PP);
         if (n) run(FUNDEM_T_GHOST, FUNDEM_T_GHOST);
-        step_wrapped = images && !sector ? img_pos.p : nullptr;
+        step_wrapped = images && !turned ? img_pos.p : nullptr;
         if (!with_force) {
             if (step_wrapped && Pv.n > 0)
                 FD_CUDA(cudaMemcpyAsync(Pv.pos, img_pos.p, sizeof(double3) * Pv.n, cudaMemcpyDeviceToDevice, stream));
@@ -2002,6 +2009,7 @@ int fundem_set_periodic(fundem_sim* s, int x, int y)
     if (!s) return FUNDEM_ERR_ARG;
     s->perX = x != 0;
     s->perY = y != 0;
+    s->pc_force = true;  // other image lists: the pair cache and the reverse index are built again
     return FUNDEM_OK;
 }
 
@@ -2009,6 +2017,7 @@ int fundem_set_periodic_sector(fundem_sim* s, int on)
 {
     if (!s) return FUNDEM_ERR_ARG;
     s->sector = on != 0;
+    s->pc_force = true;
     return FUNDEM_OK;
 }
 
