@@ -1428,6 +1428,7 @@ struct fundem_sim {
         if (turned) {
             // LSSolver.h:780-784: wraps and images after the other detections
             if (n) run(FUNDEM_T_BROAD, FUNDEM_T_NARROW_PP);
+            if (pc) fd::launch_cache_refs(Pv, Wv, pcv, stream);
             tbegin(FUNDEM_T_GHOST);
             translated();
             fd::launch_sector_wrap(Pg, pgrid, stream);
@@ -1455,7 +1456,7 @@ struct fundem_sim {
         PairListDev views[FD_NKIND];
         for (int k = 0; k < FD_NKIND; ++k) views[k] = lists[k].view();
         std::copy(active, active + FD_NKIND, step_active);
-        fd::launch_step_end(Pv, Wv, views, active, c.R, pc ? &pcv : nullptr, pcg, end_done.p,
+        fd::launch_step_end(Pv, Wv, views, active, c.R, pc ? &pcv : nullptr, pcg, !turned, end_done.p,
                             flags.p, stream);
         tend(FUNDEM_T_REDUCE);
         if (forked) FD_CUDA(cudaStreamWaitEvent(stream, br_join, 0));

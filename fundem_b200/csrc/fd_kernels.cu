@@ -2785,6 +2785,28 @@ __global__ void __launch_bounds__(TPB) k_sum_lists(ListSet a, RevDev R)
 // too (a carried step then finds it in place), the bodies' state becomes the
 // new reference, and the last block renews the flags: a list that overflowed
 // asks for a rebuild, this step's requests become the next step's.
+// the bodies' state as the pair cache's reference
+__device__ __forceinline__ void cache_refs(const PairCacheDev& pc, const ObjDev& P, const ObjDev& W, int i0, int stride)
+{
+    for (int i = i0; i < P.n; i += stride) {
+        pc.ref_pos[i] = P.pos[i];
+        pc.ref_q[i] = P.q[i];
+        pc.ref_vis[i] = P.hash[i] >= 0;
+    }
+    for (int w = i0; w < W.n; w += stride) {
+        pc.wref_pos[w] = W.pos[w];
+        pc.wref_q[w] = W.q[w];
+        pc.wref_hash[w] = W.hash[w];
+    }
+}
+// where the wraps that follow the detection of particles and walls move bodies
+// in place, the references are taken before them: a body moved since its pairs
+// were listed has drifted
+__global__ void __launch_bounds__(TPB) k_cache_refs(PairCacheDev pc, ObjDev P, ObjDev W)
+{
+    if (pc.ctrl[0] != 0) cache_refs(pc, P, W, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
 struct EndArgs {
     ObjDev P, W;
     PairListDev L[FD_NKIND];  // by kind
@@ -2793,6 +2815,7 @@ struct EndArgs {
     PairCacheDev pc;
     int cached;               // the pair cache is on; ghosts: so are the translated image lists
     int cached_ghosts;
+    int refs;                 // the bodies' state is the reference of a build (see k_cache_refs)
     unsigned int* done;       // blocks finished (returns to 0)
     unsigned int* flags;
 };
@@ -2851,18 +2874,7 @@ __global__ void __launch_bounds__(TPB) k_step_end(EndArgs a)
         }
         for (int s = i0; s < ns; s += stride) L.o_c_k[s] = L.c_k[s];
     }
-    if (built) {
-        for (int i = i0; i < a.P.n; i += stride) {
-            a.pc.ref_pos[i] = a.P.pos[i];
-            a.pc.ref_q[i] = a.P.q[i];
-            a.pc.ref_vis[i] = a.P.hash[i] >= 0;
-        }
-        for (int w = i0; w < a.W.n; w += stride) {
-            a.pc.wref_pos[w] = a.W.pos[w];
-            a.pc.wref_q[w] = a.W.q[w];
-            a.pc.wref_hash[w] = a.W.hash[w];
-        }
-    }
+    if (built && a.refs) cache_refs(a.pc, a.P, a.W, i0, stride);
     __syncthreads();
     if (threadIdx.x != 0) return;
     __threadfence();
@@ -4026,8 +4038,14 @@ void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream
     launch_step(c.mixed ? k_sum_lists<float> : k_sum_lists<double>, a.block0[n], TPB, s, a, c.R);
 }
 
+void launch_cache_refs(const ObjDev& P, const ObjDev& W, const PairCacheDev& pc, cudaStream_t s)
+{
+    if (P.n > 0) launch_step(k_cache_refs, std::min(nblocks(P.n), 148 * 8), TPB, s, pc, P, W);
+}
+
 void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists, const int* active, const RevDev& R,
-                     const PairCacheDev* pc, bool cached_ghosts, unsigned int* done, unsigned int* flags, cudaStream_t s)
+                     const PairCacheDev* pc, bool cached_ghosts, bool refs, unsigned int* done, unsigned int* flags,
+                     cudaStream_t s)
 {
     if (P.n <= 0) return;
     EndArgs a;
@@ -4037,6 +4055,7 @@ void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists,
     a.R = R;
     a.cached = pc != nullptr;
     a.cached_ghosts = cached_ghosts;
+    a.refs = refs;
     if (pc) a.pc = *pc; else memset(&a.pc, 0, sizeof(a.pc));
     a.done = done;
     a.flags = flags;

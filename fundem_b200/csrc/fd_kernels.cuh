@@ -398,10 +398,13 @@ struct ListArgs {
 void launch_broad(const ListArgs* lists, int n, const StepShared& c, NlDev* nl, cudaStream_t s);
 void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream_t s);
 // end of a step's detection: the reverse index, and the pair cache's (pc
-// non-null) layouts, references and flags; done: a zeroed counter; flags: the
-// error flags
+// non-null) layouts, references (refs: not yet taken by launch_cache_refs) and
+// flags; done: a zeroed counter; flags: the error flags
 void launch_step_end(const ObjDev& P, const ObjDev& W, const PairListDev* lists, const int* active, const RevDev& R,
-                     const PairCacheDev* pc, bool cached_ghosts, unsigned int* done, unsigned int* flags, cudaStream_t s);
+                     const PairCacheDev* pc, bool cached_ghosts, bool refs, unsigned int* done, unsigned int* flags,
+                     cudaStream_t s);
+// the references of the pair cache, on a step that builds its lists
+void launch_cache_refs(const ObjDev& P, const ObjDev& W, const PairCacheDev& pc, cudaStream_t s);
 // parts of launch_advance and launch_small_advance: a step's force sums over
 // its lists and bonds; its second half kick; the next step's first half kick,
 // drift (walls too), hashes and, with pc, pair-cache checks, for a step of list
