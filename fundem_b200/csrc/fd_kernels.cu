@@ -4066,7 +4066,8 @@ void launch_advance(const StepShared& c, const ObjDev& P, const PairListDev* lis
                     const double3* wrapped, double3 gravity, double dt, const PairCacheDev* pc, int* const* occ,
                     int par, int parts, cudaStream_t s)
 {
-    if (P.n <= 0) return;
+    // without particles there are still walls to move
+    if (P.n <= 0 && (!(parts & STEP_FRONT) || c.W.n <= 0)) return;
     AdvanceArgs a;
     a.P = P; a.W = c.W; a.G = c.G; a.GW = c.GW; a.pgrid = c.pgrid; a.wgrid = c.wgrid;
     a.r.R = c.R;
