@@ -2274,13 +2274,45 @@ __device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int
 // lanes per pair.  The order is the contacts' own: slots without one, of which
 // a cached list holds more, do not change the sum.
 //
-// Bound by the latency of pair, slots, node ids and forces, four loads that
-// wait for one another.  Three pairs in four hold no contact (a settled bed: 8
-// slots and a quarter of a contact per pair), so a warp takes 32 pairs' flags
-// in one load, the next ones' meanwhile, and passes on to those that hold one;
-// with eight lanes looking at each pair the sums took
-// 105 us for 262,144 particles, this way 57.
+// Bound by the latency of pair, slots, node ids and forces, loads that wait for
+// one another.  Three pairs in four hold no contact (a settled bed: 8 slots and
+// a quarter of a contact per pair), so a warp takes several pairs' flags in one
+// load, the next ones' meanwhile, and passes on to those that hold one; with
+// eight lanes looking at each pair the sums took 105 us for 262,144 particles,
+// this way 57 (cold caches; 30 in a run of steps).  A pair of bodies pressed into
+// one another holds hundreds of contacts: their forces are loaded four at a
+// time, the next slots' ids meanwhile, and a short list is shared out over all
+// warps.  With a load per contact and 32 pairs a warp whatever their number,
+// 40,000 pairs of such bodies took 2,660 us, this way 145; eight at a time
+// take 127, but 40 instead of 30 us for the settled bed.
 // ---------------------------------------------------------------------------
+// the forces of the contacts among eight slots, in slot order (m: bit u for
+// slot u of the lane's group of eight; at: the place of the lane's own slot):
+// component l of each onto acc, the ninth onto lane 0's acc8.  For whole warps.
+template <typename Real>
+__device__ __forceinline__ void add_contacts(const double* rec, unsigned int m, int at, int l, Real& acc, Real& acc8)
+{
+    while (__any_sync(0xffffffffu, m != 0u)) {
+        Real v[4], v8[4];
+        bool on[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            on[u] = m != 0u;
+            const int t = __shfl_sync(0xffffffffu, at, on[u] ? __ffs(m) - 1 : 0, 8);
+            m &= m - 1u;
+            const Real* f = reinterpret_cast<const Real*>(rec + (long long)CONTACT_REC * t);
+            v[u] = on[u] ? f[l] : Real(0);
+            v8[u] = on[u] && l == 0 ? f[8] : Real(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (on[u]) {
+                acc += v[u];
+                acc8 += v8[u];
+            }
+    }
+}
+
 template <typename Real>
 __device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int block, int nblocks, bool link,
                                          const RevDev& R, int n_obj, int3* list)
@@ -2303,39 +2335,37 @@ __device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int blo
             L.r_next[p] = (unsigned int)(old >> 32) == build ? (int)(unsigned int)old : -1;
         }
     }
-    const int stride = nthreads >> 5 << 5;
-    int p = thread;
-    bool next = p < npairs && L.p_hit[p] != 0;
-    for (int p0 = thread & ~31; p0 < npairs; p0 += stride) {
+    // a warp takes `take` pairs at a time: as many as it has lanes, or what
+    // gives every warp its share of a short list, four for its four groups at
+    // least
+    const int warp = thread >> 5, nwarps = nthreads >> 5;
+    const int take = min(max((npairs + 4 * nwarps - 1) / (4 * nwarps) * 4, 4), 32);
+    auto flag = [&](int p0) { return lane < take && p0 + lane < npairs && L.p_hit[p0 + lane] != 0; };
+    bool next = flag(warp * take);
+    for (int p0 = warp * take; p0 < npairs; p0 += nwarps * take) {
         const bool hit = next;
         const unsigned int m = __ballot_sync(full, hit);
+        const int p = p0 + lane;
         if (hit) list[__popc(m & ((1u << lane) - 1u))] = make_int3(p, L.c_off[p], L.c_cnt[p]);
         const int count = __popc(m);
-        p += stride;
-        next = p < npairs && L.p_hit[p] != 0;  // the next pairs' flags, meanwhile
+        next = flag(p0 + nwarps * take);  // the next pairs' flags, meanwhile
         __syncwarp();
         for (int i0 = 0; i0 < count; i0 += 4) {
             const bool on = i0 + grp < count;
             const int3 q = on ? list[i0 + grp] : make_int3(0, 0, 0);
             const int o = q.y, c = q.z;
             Real acc = 0, acc8 = 0;
-            // eight slots at a time: lane l looks at slot l, then adds component
-            // l (lane 0 also the ninth) of the contacts among them in turn
+            // eight slots at a time: lane l looks at slot l of the next ones
+            // while the forces of these are added
             const int cmax = __reduce_max_sync(full, c);
+            int at = l < c ? L.c_at[o + l] : 0;
+            int node = l < c ? L.c_node[o + l] : -1;
             for (int j0 = 0; j0 < cmax; j0 += 8) {
-                int at = 0;
-                bool contact = false;
-                if (j0 + l < c) {
-                    at = L.c_at[o + j0 + l];
-                    contact = L.c_node[o + j0 + l] >= 0;
-                }
-                unsigned int m = (__ballot_sync(full, contact) >> (8 * grp)) & 0xffu;
-                for (; m; m &= m - 1u) {
-                    const int t = __shfl_sync(0xffu << (8 * grp), at, 8 * grp + __ffs(m) - 1);
-                    const Real* f = reinterpret_cast<const Real*>(L.c_rec + (long long)CONTACT_REC * t);
-                    acc += f[l];
-                    if (l == 0) acc8 += f[8];
-                }
+                const unsigned int any = __ballot_sync(full, node >= 0);
+                const int here = at, j = j0 + 8 + l;
+                at = j < c ? L.c_at[o + j] : 0;
+                node = j < c ? L.c_node[o + j] : -1;
+                if (any) add_contacts(L.c_rec, (any >> (8 * grp)) & 0xffu, here, l, acc, acc8);
             }
             if (on) {
                 Real* out = pf + (long long)RESULT * q.x;
@@ -2770,7 +2800,7 @@ __device__ __forceinline__ bool rev_built(const RevDev& R)
 }
 
 template <typename Real>
-__global__ void __launch_bounds__(TPB) k_sum_lists(ListSet a, RevDev R)
+__global__ void __launch_bounds__(TPB, 6) k_sum_lists(ListSet a, RevDev R)
 {
     int block, nblocks;
     const int li = list_of(a, block, nblocks);
@@ -3558,15 +3588,11 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, BLOCKS) k_small_pairs(SmallA
         const PairListDev& L = wall ? a.Lw : n.L;
         Real acc = 0, acc8 = 0;
         const int cmax = __reduce_max_sync(full, c);
+        int node = l < c ? L.c_node[base + l] : -1;
         for (int j0 = 0; j0 < cmax; j0 += 8) {
-            const bool contact = j0 + l < c && L.c_node[base + j0 + l] >= 0;
-            unsigned int m = (__ballot_sync(full, contact) >> (8 * grp)) & 0xffu;
-            for (; m; m &= m - 1u) {
-                const Real* f =
-                    reinterpret_cast<const Real*>(L.c_rec + (long long)CONTACT_REC * (base + j0 + __ffs(m) - 1));
-                acc += f[l];
-                if (l == 0) acc8 += f[8];
-            }
+            const unsigned int any = __ballot_sync(full, node >= 0);
+            node = j0 + 8 + l < c ? L.c_node[base + j0 + 8 + l] : -1;
+            if (any) add_contacts(L.c_rec, (any >> (8 * grp)) & 0xffu, base + j0 + l, l, acc, acc8);
         }
         if (!hits) continue;
         // a pair without a contact sums to zero: nobody reads it
