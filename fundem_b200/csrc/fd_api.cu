@@ -2635,8 +2635,7 @@ int fundem_set_launch_shape(fundem_sim* s, const int blocks_per_sm[4])
 int fundem_get_launch_shape(fundem_sim* s, int blocks_per_sm[4])
 {
     if (!s || !blocks_per_sm) return FUNDEM_ERR_ARG;
-    const int def[4] = {FD_SELECT_MIN_BLOCKS, FD_PROBE_MIN_BLOCKS, 4, 4};
-    for (int k = 0; k < 4; ++k) blocks_per_sm[k] = s->launch_shape[k] > 0 ? s->launch_shape[k] : def[k];
+    for (int k = 0; k < 4; ++k) blocks_per_sm[k] = s->launch_shape[k] > 0 ? s->launch_shape[k] : fd::DEFAULT_SHAPE[k];
     return FUNDEM_OK;
 }
 

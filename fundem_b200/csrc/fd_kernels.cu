@@ -2313,6 +2313,8 @@ __device__ __forceinline__ void add_contacts(const double* rec, unsigned int m, 
     }
 }
 
+constexpr int SUM_TPB = 384;  // four such blocks an SM take the registers of 48 warps
+
 template <typename Real>
 __device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int block, int nblocks, bool link,
                                          const RevDev& R, int n_obj, int3* list)
@@ -2800,12 +2802,12 @@ __device__ __forceinline__ bool rev_built(const RevDev& R)
 }
 
 template <typename Real>
-__global__ void __launch_bounds__(TPB, 6) k_sum_lists(ListSet a, RevDev R)
+__global__ void __launch_bounds__(SUM_TPB, FD_SUM_MIN_BLOCKS) k_sum_lists(ListSet a, RevDev R)
 {
     int block, nblocks;
     const int li = list_of(a, block, nblocks);
     const NarrowArgs& n = a.l[li];
-    __shared__ int3 s_list[TPB / 32][32];
+    __shared__ int3 s_list[SUM_TPB / 32][32];
     sum_list<Real>(n.L, a.kind[li], block, nblocks, a.kind[li] != FD_PW && rev_built(R), R, n.P.n,
                    s_list[threadIdx.x >> 5]);
 }
@@ -4035,7 +4037,8 @@ void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream
     // known only on the device): the particle-particle list's defaults fill
     // one resident wave; the short wall and image lists come first and get a
     // quarter of it each, so that they end before the long list does
-    const int* shape = lists[0].a.shape;
+    int shape[4];
+    for (int k = 0; k < 4; ++k) shape[k] = lists[0].a.shape[k] > 0 ? lists[0].a.shape[k] : DEFAULT_SHAPE[k];
     auto share = [&](int* blocks, int per_sm) {
         for (int k = 0; k < n; ++k) {
             const long long need = ((long long)lists[k].L.cap_pairs + NARROW_WARPS - 1) / NARROW_WARPS;
@@ -4044,24 +4047,23 @@ void launch_narrow(const ListArgs* lists, int n, const StepShared& c, cudaStream
         }
     };
     int blocks[FD_NKIND];
-    share(blocks, shape[0] > 0 ? shape[0] : FD_SELECT_MIN_BLOCKS);
+    share(blocks, shape[0]);
     ListSet a = list_set(lists, n, c, blocks);
     launch_step(k_select_lists, a.block0[n], NARROW_WARPS * 32, s, a);
-    const int probe = shape[1] > 0 ? shape[1] : FD_PROBE_MIN_BLOCKS;
     for (int k = 0; k < n; ++k) {
         if (lists[k].kind != FD_PP || !lists[k].a.gate) continue;
-        launch_step(k_slot_filter, 148 * probe, TPB, s, a.l[k]);
+        launch_step(k_slot_filter, 148 * shape[1], TPB, s, a.l[k]);
     }
-    share(blocks, probe);
+    share(blocks, shape[1]);
     a = list_set(lists, n, c, blocks);
     launch_step(c.mixed ? k_contact_lists<true, 0> : k_contact_lists<false, 0>, a.block0[n], TPB, s, a);
-    share(blocks, shape[2] > 0 ? shape[2] : 4);
+    share(blocks, shape[2]);
     a = list_set(lists, n, c, blocks);
     launch_step(c.mixed ? k_contact_lists<true, 1> : k_contact_lists<false, 1>, a.block0[n], TPB, s, a);
     if (!c.with_force) return;
-    share(blocks, shape[3] > 0 ? shape[3] : FD_SUM_BLOCKS);
+    share(blocks, shape[3]);
     a = list_set(lists, n, c, blocks);
-    launch_step(c.mixed ? k_sum_lists<float> : k_sum_lists<double>, a.block0[n], TPB, s, a, c.R);
+    launch_step(c.mixed ? k_sum_lists<float> : k_sum_lists<double>, a.block0[n], SUM_TPB, s, a, c.R);
 }
 
 void launch_cache_refs(const ObjDev& P, const ObjDev& W, const PairCacheDev& pc, cudaStream_t s)

@@ -2,26 +2,30 @@
 #pragma once
 #include "fd_internal.cuh"
 
-// resident blocks per SM the narrow-phase kernels are compiled for (their
-// default grids fill one wave of them)
+// resident blocks per SM the narrow-phase kernels' registers are cut for.  The
+// selection and the predicate pass: latency-bound gathers, so as many resident
+// warps as fit without spilling; the contact law: its loads are kept together,
+// which takes 128 registers.
 #ifndef FD_SELECT_MIN_BLOCKS
 #define FD_SELECT_MIN_BLOCKS 4
 #endif
 #ifndef FD_CONTACT_MIN_BLOCKS
 #define FD_CONTACT_MIN_BLOCKS 2
 #endif
-// the predicate pass of the contact kernels: latency-bound gathers, so as
-// many resident warps as fit without spilling
 #ifndef FD_PROBE_MIN_BLOCKS
 #define FD_PROBE_MIN_BLOCKS 4
 #endif
-
-// the pair sums: short chains of loads, few registers
-#ifndef FD_SUM_BLOCKS
-#define FD_SUM_BLOCKS 8
+#ifndef FD_SUM_MIN_BLOCKS
+#define FD_SUM_MIN_BLOCKS 4
 #endif
 
 namespace fd {
+
+// default launch shape of the narrow phase, blocks per SM: selection, predicate
+// pass, contact law, pair sums.  One resident wave, but two for the law: the
+// first wave's early blocks make room for the rest (262,144 bodies: 44.9 us,
+// 48.3 with one wave, 46.1 with four; 65,003: 16.6, 16.6, 18.8).
+constexpr int DEFAULT_SHAPE[4] = {FD_SELECT_MIN_BLOCKS, FD_PROBE_MIN_BLOCKS, 4, FD_SUM_MIN_BLOCKS};
 
 // Everything one simulation keeps on the device.  Plain pointers; ownership
 // and sizes live in the host-side Sim object (fd_api.cu).
