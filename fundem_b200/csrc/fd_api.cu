@@ -276,7 +276,8 @@ struct GeoSetHost {
     double rmax = 0.0, grid_rmax = 0.0;
     bool built = false;
 
-    void build(bool wall, int inertia_mode, cudaStream_t s)
+    // fp64: the contact path reads the set in double precision
+    void build(bool wall, int inertia_mode, bool fp64, cudaStream_t s)
     {
         table.clear();
         key_of.clear();
@@ -387,10 +388,6 @@ struct GeoSetHost {
         d_sdf.upload(sdf.data(), sdf.size(), s);
         d_sdf32.alloc(std::max<size_t>(sdf32.size(), 1));
         d_sdf32.upload(sdf32.data(), sdf32.size(), s);
-        d_sdf_quad.alloc(std::max<size_t>(sdf.size(), 1), false);
-        d_sdf32_quad.alloc(std::max<size_t>(sdf.size(), 1), false);
-        for (const FdGeo& t : table)
-            fd::launch_sdf_quads(d_sdf.p, d_sdf32.p, d_sdf_quad.p, d_sdf32_quad.p, t.sdf_off, t.size, s);
         d_dist.alloc(std::max<size_t>(dist.size(), 1));
         d_dist.upload(dist.data(), dist.size(), s);
         d_cellmin.alloc(std::max<size_t>(cellmin.size(), 1));
@@ -417,8 +414,28 @@ struct GeoSetHost {
         d_clus_sphere.upload(cs32.data(), cs32.size(), s);
         d_clus_range.alloc(std::max<size_t>(cr.size(), 1));
         d_clus_range.upload(cr.data(), cr.size(), s);
+        faces(sdf.size(), fp64, s);
         FD_CUDA(cudaStreamSynchronize(s));
         built = true;
+    }
+
+    // The tables of cell faces (see load_corners), 16 bytes a grid point in
+    // single precision and, with fp64, 32 in double.  They are a copy of the
+    // grids that saves loads, so they may not cost a run its memory: a set
+    // whose tables would take more than an eighth of what is free goes without
+    // (on an empty 180 GB device, above 470 million points).
+    void faces(size_t points, bool fp64, cudaStream_t s)
+    {
+        d_sdf_quad.release();
+        d_sdf32_quad.release();
+        const size_t bytes = points * (sizeof(float4) + (fp64 ? sizeof(double4) : 0));
+        size_t free = 0, all = 0;
+        FD_CUDA(cudaMemGetInfo(&free, &all));
+        if (points == 0 || bytes > free / 8) return;
+        d_sdf32_quad.alloc(points, false);
+        if (fp64) d_sdf_quad.alloc(points, false);
+        for (const FdGeo& t : table)
+            fd::launch_sdf_quads(d_sdf.p, d_sdf32.p, d_sdf_quad.p, d_sdf32_quad.p, t.sdf_off, t.size, s);
     }
 
     GeoSetDev view() const
@@ -1191,8 +1208,8 @@ struct fundem_sim {
     {
         FD_CUDA(cudaSetDevice(device));
         if (geo_dirty) {
-            pgeo.build(false, inertia_mode, stream);
-            wgeo.build(true, inertia_mode, stream);
+            pgeo.build(false, inertia_mode, !mixed(), stream);
+            wgeo.build(true, inertia_mode, true, stream);  // mixed precision too interpolates walls in double
             pmat.upload(stream);
             wmat.upload(stream);
             geo_dirty = false;
@@ -1660,6 +1677,8 @@ int fundem_set_precision(fundem_sim* s, int mode)
 {
     if (!s || (mode != FUNDEM_FP64 && mode != FUNDEM_FP32_MIXED)) return FUNDEM_ERR_ARG;
     s->precision = mode;
+    // the next setup adds the tables that this precision reads
+    if (s->setup_done && !s->mixed() && !s->pgeo.d_sdf_quad.p) s->geo_dirty = true;
     return FUNDEM_OK;
 }
 

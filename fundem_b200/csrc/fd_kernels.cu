@@ -737,6 +737,44 @@ __device__ void emit_pairs(int A, int* buf, int cnt, int total, const PairListDe
 
 constexpr double BOUND_REL = 1e-9;
 
+// The predicate and contact passes read about 27 numbers a slot at addresses
+// that differ from lane to lane, and the L1 serves a warp's addresses one line
+// at a time: 79% of its rate at 65,003 particles.  Orientations and the
+// interpolation's corners come in 32-byte loads instead (4 to 1 and 8 to 2).
+__device__ __forceinline__ double4 load_quad(const double4* p)
+{
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+// The corner values of the cell at point i of a set's grids, of the planes z
+// (s0) and z + 1 (s1): from the table of faces, or one by one where the set's
+// table would take too much memory (see GeoSetHost::faces).
+__device__ __forceinline__ void load_corners(const GeoSetDev& S, long long i, long long sx, long long sxy, double4& s0,
+                                             double4& s1)
+{
+    if (S.sdf_quad) {
+        s0 = load_quad(S.sdf_quad + i);
+        s1 = load_quad(S.sdf_quad + i + sxy);
+        return;
+    }
+    const double *g = S.sdf + i, *h = g + sxy;
+    s0 = make_double4(__ldg(g), __ldg(g + 1), __ldg(g + sx), __ldg(g + sx + 1));
+    s1 = make_double4(__ldg(h), __ldg(h + 1), __ldg(h + sx), __ldg(h + sx + 1));
+}
+__device__ __forceinline__ void load_corners(const GeoSetDev& S, long long i, long long sx, long long sxy, float4& s0,
+                                             float4& s1)
+{
+    if (S.sdf32_quad) {
+        s0 = __ldg(S.sdf32_quad + i);
+        s1 = __ldg(S.sdf32_quad + i + sxy);
+        return;
+    }
+    const float *g = S.sdf32 + i, *h = g + sxy;
+    s0 = make_float4(__ldg(g), __ldg(g + 1), __ldg(g + sx), __ldg(g + sx + 1));
+    s1 = make_float4(__ldg(h), __ldg(h + 1), __ldg(h + sx), __ldg(h + sx + 1));
+}
+
 // True when no point within `radius` of p (a position in B's body frame, in
 // single precision) can pass the node predicate against B (or, with probe >
 // 0, come within `probe` of B).  Conservative: single-precision evaluation
@@ -776,8 +814,8 @@ __device__ __forceinline__ bool sphere_culled(float px, float py, float pz, floa
         gz < GB.size.z - 1) {
         const int i0 = (int)gx, j0 = (int)gy, k0 = (int)gz;
         const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
-        const float4* S = SB.sdf32_quad + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
-        const float4 s0 = __ldg(S), s1 = __ldg(S + sxy);
+        float4 s0, s1;
+        load_corners(SB, GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0, sx, sxy, s0, s1);
         const float fx = gx - i0, fy = gy - j0, fz = gz - k0;
         const float c00 = s0.x * (1.f - fx) + s0.y * fx;
         const float c10 = s0.z * (1.f - fx) + s0.w * fx;
@@ -1405,17 +1443,7 @@ __global__ void __launch_bounds__(TPB) k_broad_lists(ListSet a)
     }
 }
 
-// The predicate and contact passes read about 27 numbers a slot at addresses
-// that differ from lane to lane, and the L1 serves a warp's addresses one line
-// at a time: 79% of its rate at 65,003 particles.  Orientations and the
-// interpolation's corners come in 32-byte loads instead (4 to 1 and 8 to 2).
-__device__ __forceinline__ double4 load_quad(const double4* p)
-{
-    double4 v;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
-    return v;
-}
-// the same of what a kernel before this one wrote (and this one does not)
+// load_quad of what a kernel before this one wrote (and this one does not)
 __device__ __forceinline__ double4 load_four(const double4* p)
 {
     double4 v;
@@ -1433,7 +1461,7 @@ __device__ __forceinline__ fd_quat load_q(const fd_quat* p)
 // fills the grid fraction and the eight corner values.
 template <int KIND>
 __device__ __forceinline__ bool node_predicate(const double3 gp, const int3 bcell, const FdGrid& sg, const double3 cB,
-                                               const fd_quat qB, const FdGeo& GB, const double4* quads, double rB2,
+                                               const fd_quat qB, const FdGeo& GB, const GeoSetDev& SB, double rB2,
                                                double probe, double& overlap, double& fx, double& fy, double& fz,
                                                double p[8])
 {
@@ -1456,8 +1484,8 @@ __device__ __forceinline__ bool node_predicate(const double3 gp, const int3 bcel
     fy = gy - (double)j0;
     fz = gz - (double)k0;
     const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
-    const double4* S = quads + GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0;
-    const double4 s0 = load_quad(S), s1 = load_quad(S + sxy);
+    double4 s0, s1;
+    load_corners(SB, GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0, sx, sxy, s0, s1);
     p[0] = s0.x; p[1] = s0.y; p[2] = s0.z; p[3] = s0.w;
     p[4] = s1.x; p[5] = s1.y; p[6] = s1.z; p[7] = s1.w;
     overlap = -xm_trilinear(fx, fy, fz, p);
@@ -1565,8 +1593,7 @@ __device__ __forceinline__ void node_filter(const float4 (&p)[NODES], const bool
             // a node that needs no look reads the pool's first point
             const long long i =
                 look[u] ? GB.sdf_off + (long long)(int)gz[u] * sxy + (long long)(int)gy[u] * sx + (int)gx[u] : 0ll;
-            s0[u] = __ldg(SB.sdf32_quad + i);
-            s1[u] = __ldg(SB.sdf32_quad + i + (look[u] ? sxy : 0ll));
+            load_corners(SB, i, look[u] ? sx : 0ll, look[u] ? sxy : 0ll, s0[u], s1[u]);
         }
 #pragma unroll
         for (int u = 0; u < NODES; ++u) {
@@ -1976,7 +2003,7 @@ __device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, const PairSt
     e.r = xm_rot(qA, node);
     e.gp = mk3(e.r.x + e.cA.x, e.r.y + e.cA.y, e.r.z + e.cA.z);
     e.ov = ov0;
-    return node_predicate<KIND>(e.gp, bcell, sg, e.cB, e.qB, GB, SB.sdf_quad, rB2, n.a.probe, e.ov, e.fx, e.fy, e.fz, e.pv);
+    return node_predicate<KIND>(e.gp, bcell, sg, e.cB, e.qB, GB, SB, rB2, n.a.probe, e.ov, e.fx, e.fy, e.fz, e.pv);
 }
 
 // A contact's results go out in 16-byte stores to six whole sectors, side by
@@ -2503,7 +2530,8 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, const Pair
                     // of a metre): single-precision interpolation
                     // there would carry errors of 1e-8 m, so the
                     // (few) wall contacts interpolate in double
-                    const double4 s0 = load_quad(SB.sdf_quad + c0), s1 = load_quad(SB.sdf_quad + c0 + sxy);
+                    double4 s0, s1;
+                    load_corners(SB, c0, sx, sxy, s0, s1);
                     double pd[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
                     const double ovd = -xm_trilinear(gx - (double)i0, gy - (double)j0, gz - (double)k0, pd);
 #pragma unroll
@@ -2512,7 +2540,8 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, const Pair
                     e.phi0 = __double2float_rd(-ovd);
                     hit = ovd >= -n.a.probe;
                 } else {
-                    const float4 s0 = __ldg(SB.sdf32_quad + c0), s1 = __ldg(SB.sdf32_quad + c0 + sxy);
+                    float4 s0, s1;
+                    load_corners(SB, c0, sx, sxy, s0, s1);
                     pv[0] = s0.x; pv[1] = s0.y; pv[2] = s0.z; pv[3] = s0.w;
                     pv[4] = s1.x; pv[5] = s1.y; pv[6] = s1.z; pv[7] = s1.w;
                     const float c00 = pv[0] * (1.f - fx) + pv[1] * fx, c10 = pv[2] * (1.f - fx) + pv[3] * fx;
@@ -3894,7 +3923,8 @@ __global__ void __launch_bounds__(TPB) k_sdf_quads(const double* sdf, const floa
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         // points of the last column or row start no cell
         const bool cell = i % sx + 1 < sx && (i / sx) % size.y + 1 < size.y;
-        quad[i] = cell ? make_double4(sdf[i], sdf[i + 1], sdf[i + sx], sdf[i + sx + 1]) : make_double4(0., 0., 0., 0.);
+        if (quad)
+            quad[i] = cell ? make_double4(sdf[i], sdf[i + 1], sdf[i + sx], sdf[i + sx + 1]) : make_double4(0., 0., 0., 0.);
         quad32[i] =
             cell ? make_float4(sdf32[i], sdf32[i + 1], sdf32[i + sx], sdf32[i + sx + 1]) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -3905,7 +3935,7 @@ void launch_sdf_quads(const double* sdf, const float* sdf32, double4* quad, floa
     const long long n = (long long)size.x * size.y * size.z;
     if (n <= 0) return;
     k_sdf_quads<<<(int)std::min<long long>((n + TPB - 1) / TPB, 148 * 8), TPB, 0, s>>>(sdf + off, sdf32 + off,
-                                                                                       quad + off, quad32 + off, size, n);
+                                                                                       quad ? quad + off : nullptr, quad32 + off, size, n);
     note_launch();
 }
 

@@ -136,7 +136,7 @@ struct GeoSetDev {
     const double* sdf;
     const float* sdf32;
     // per grid point the four corner values (x, x + 1) of rows y and y + 1:
-    // what an interpolation reads of one z plane, in one load
+    // what an interpolation reads of one z plane, in one load (null: not kept)
     const double4* sdf_quad;
     const float4* sdf32_quad;
     const float* dist;
@@ -341,11 +341,12 @@ struct BondViewDev {
     double3* frames[8]; // master n1 n2 n3 point, slave n1 n2 n3 point (body frames)
 };
 
+// the tables of cell faces of one grid at off in the pools (quad may be null)
+void launch_sdf_quads(const double* sdf, const float* sdf32, double4* quad, float4* quad32, long long off, int3 size,
+                      cudaStream_t s);
 // cell hash of each object (-1 outside the grid) and its single-precision
 // rotation rows; build (non-null): the cell table's build numbers, renewed for
 // a step of list generation par
-void launch_sdf_quads(const double* sdf, const float* sdf32, double4* quad, float4* quad32, long long off, int3 size,
-                      cudaStream_t s);
 void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s, unsigned int* build = nullptr, int par = 0);
 // stable sort of n 64-bit keys (key 0 .. num_keys - 1, or negative: last) on
 // the stream: out_idx gets the permutation, out_key the sorted keys (~0 for
