@@ -2476,6 +2476,16 @@ __device__ __forceinline__ v3f linear_contact32(double3& spring, v3f vc, v3f n, 
     return fn + (-ks * tof(spring) - cs * vs);
 }
 
+// explicit fused multiply-adds, as in the contact law: the predicate pass, the
+// law pass, the image lists' and the small steps must give a node the same
+// overlap
+__device__ __forceinline__ float lerp32(float a, float b, float t) { return fmaf(a, 1.f - t, __fmul_rn(b, t)); }
+__device__ __forceinline__ float trilinear32(const float* p, float x, float y, float z)
+{
+    return lerp32(lerp32(lerp32(p[0], p[1], x), lerp32(p[2], p[3], x), y),
+                  lerp32(lerp32(p[4], p[5], x), lerp32(p[6], p[7], x), y), z);
+}
+
 // one slot's node against its partner, single-precision SDF
 struct SlotEval32 {
     double3 cA, cB, rd, gp;  // centres, node offset from A's centre, node
@@ -2544,9 +2554,7 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, const Pair
                     load_corners(SB, c0, sx, sxy, s0, s1);
                     pv[0] = s0.x; pv[1] = s0.y; pv[2] = s0.z; pv[3] = s0.w;
                     pv[4] = s1.x; pv[5] = s1.y; pv[6] = s1.z; pv[7] = s1.w;
-                    const float c00 = pv[0] * (1.f - fx) + pv[1] * fx, c10 = pv[2] * (1.f - fx) + pv[3] * fx;
-                    const float c01 = pv[4] * (1.f - fx) + pv[5] * fx, c11 = pv[6] * (1.f - fx) + pv[7] * fx;
-                    e.ov = -((c00 * (1.f - fy) + c10 * fy) * (1.f - fz) + (c01 * (1.f - fy) + c11 * fy) * fz);
+                    e.ov = -trilinear32(pv, fx, fy, fz);
                     e.phi0 = -e.ov;
                     hit = e.ov >= -(float)n.a.probe;
                 }
@@ -2578,10 +2586,12 @@ __device__ __forceinline__ int contact_law32(const NarrowArgs& n, const PairList
     // gradient with the x weight truncated as the reference does
     // (LSParticleContactDetectionKernel.cuh:34)
     const float wy0 = 1.f - fy, wy1 = fy, wz0 = 1.f - fz, wz1 = fz;
-    const v3f gB = mkf((pv[1] - pv[0]) * wy0 * wz0 + (pv[3] - pv[2]) * wy1 * wz0 +
-                           (pv[5] - pv[4]) * wy0 * wz1 + (pv[7] - pv[6]) * wy1 * wz1,
-                       (pv[2] - pv[0]) * wz0 + (pv[6] - pv[4]) * wz1,
-                       (pv[4] - pv[0]) * wy0 + (pv[6] - pv[2]) * wy1);
+    const v3f gB =
+        mkf(fmaf(__fmul_rn(pv[7] - pv[6], wy1), wz1,
+                 fmaf(__fmul_rn(pv[5] - pv[4], wy0), wz1,
+                      fmaf(__fmul_rn(pv[1] - pv[0], wy0), wz0, __fmul_rn(__fmul_rn(pv[3] - pv[2], wy1), wz0)))),
+            fmaf(pv[2] - pv[0], wz0, __fmul_rn(pv[6] - pv[4], wz1)),
+            fmaf(pv[4] - pv[0], wy0, __fmul_rn(pv[6] - pv[2], wy1)));
     v3f nrm = rowsf(b0, b1, b2, gB);
     const float l2 = dotf(nrm, nrm);
     nrm = l2 > 1e-20f ? rsqrtf(l2) * nrm : mkf(0.f, 0.f, 0.f);
