@@ -931,6 +931,20 @@ struct fundem_sim {
             pc_force = true;
         }
     }
+    // before a step's first launch: list capacities follow the counts every
+    // CAPACITY_CHECK steps, counted across calls, and the pair cache's checks
+    void host_checks()
+    {
+        if (hook_steps % CAPACITY_CHECK == 0) ensure_capacity();
+        pc_check_overflow();
+        pc_reserve();
+        pc_prepare();
+    }
+    // whether they do anything before step number n
+    bool host_check_due(long long n) const
+    {
+        return n % CAPACITY_CHECK == 0 || (pc_active() && (pc_verify || pc_force));
+    }
     // reverse index over the particle and ghost lists (capacity: their pair
     // capacities together)
     DevArray<int> rev_cnt, rev_off, rev_code, rev_total;
@@ -2084,10 +2098,8 @@ int fundem_step_begin(fundem_sim* s, const double g[3], double dt)
     if (!s || !g) return FUNDEM_ERR_ARG;
     if (!s->setup_done) return FUNDEM_ERR_STATE;
     return guard(s, [&] {
-        if (++s->hook_steps % CAPACITY_CHECK == 0) s->ensure_capacity();
-        s->pc_check_overflow();
-        s->pc_reserve();
-        s->pc_prepare();
+        ++s->hook_steps;
+        s->host_checks();
         s->front(d3(g), dt);
         s->detect_all(true, dt);
         s->finish_forces();
@@ -2107,19 +2119,20 @@ int fundem_step(fundem_sim* s, int nsteps, const double g[3], double dt)
     if (!s->setup_done) return FUNDEM_ERR_STATE;
     return guard(s, [&] {
         FD_CUDA(cudaSetDevice(s->device));
+        // a step's first half kick and drift run with the step before's second
+        // half kick, but not across the checks: those can fail (a list that
+        // grows needs memory), and between its drift, which fills the cell
+        // lists, and its detection, which uses them up, a step is not left
+        bool open = false;  // the step's first half has run
         for (int k = 0; k < nsteps; ++k) {
-            // list capacities follow the counts every CAPACITY_CHECK steps,
-            // counted across calls
-            if (++s->hook_steps % CAPACITY_CHECK == 0) s->ensure_capacity();
-            s->pc_check_overflow();
-            s->pc_reserve();
-            s->pc_prepare();
-            // the host checks above touch no particle state: a step's first
-            // half kick and drift run with the previous step's second half
-            // kick (back_front), ahead of them
-            if (k == 0) s->front(d3(g), dt);
+            ++s->hook_steps;
+            if (!open) {
+                s->host_checks();
+                s->front(d3(g), dt);
+            }
             s->detect_all(true, dt);
-            if (k + 1 < nsteps) s->back_front(d3(g), dt);
+            open = k + 1 < nsteps && !s->host_check_due(s->hook_steps + 1);
+            if (open) s->back_front(d3(g), dt);
             else s->back(d3(g), dt);
         }
         FD_CUDA(cudaGetLastError());
