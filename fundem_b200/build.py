@@ -19,7 +19,7 @@ LIB = os.path.join(LIBDIR, "libfundem_b200.so")
 SOURCES = ["fd_kernels.cu", "fd_adjoint.cu", "fd_api.cu", "fd_levelset.cu"]
 # per-source flags: the grid generator rounds every add and multiply on its own
 SOURCE_FLAGS = {"fd_levelset.cu": ["-fmad=false"]}
-HEADERS = ["fd_internal.cuh", "fd_kernels.cuh", "fd_adjoint.cuh"]
+HEADERS = ["fd_internal.cuh", "fd_kernels.cuh", "fd_adjoint.cuh", "fd_build.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC = os.environ.get("NVCC", "nvcc")
 # extra compiler definitions, e.g. FUNDEM_NVCC_DEFS="-DFD_NARROW_MIN_BLOCKS=1"

@@ -2,6 +2,7 @@
 // memory, step orchestration and the C ABI declared in include/fundem_b200.h.
 #include "../../include/fundem_b200.h"
 #include "fd_adjoint.cuh"
+#include "fd_build.h"
 #include "fd_kernels.cuh"
 
 #include <algorithm>
@@ -633,8 +634,15 @@ struct CellTable {
         next.alloc(m, false);
         // with the zeroed heads: no head holds a number from these on
         build.alloc(2, false);
-        const unsigned int first[2] = {1u, 1u};
-        FD_CUDA(after_legacy(cudaMemcpy(build.p, first, sizeof(first), cudaMemcpyHostToDevice)));
+        FD_CUDA(after_legacy(cudaMemcpy(build.p, FIRST, sizeof(FIRST), cudaMemcpyHostToDevice)));
+    }
+    static constexpr unsigned int FIRST[2] = {1u, 1u};
+    // empty heads, the first build numbers again
+    void restart(cudaStream_t s)
+    {
+        if (!head.n) return;
+        FD_CUDA(cudaMemsetAsync(head.p, 0, sizeof(head.p[0]) * head.n, s));
+        FD_CUDA(cudaMemcpyAsync(build.p, FIRST, sizeof(FIRST), cudaMemcpyHostToDevice, s));
     }
     CellTableDev view(int par)
     {
@@ -931,11 +939,24 @@ struct fundem_sim {
             pc_force = true;
         }
     }
+    // Before `steps` steps or detections are launched, outside any capture: when
+    // the build numbers could come round, every head that carries one is
+    // cleared and they start again.
+    fd::BuildClock clock;
+    void build_room(long long steps)
+    {
+        if (!clock.due((uint64_t)steps)) return;
+        ptab.restart(stream);
+        for (Ghost& g : ghosts) g.cells.restart(stream);
+        if (rev_head.n) FD_CUDA(cudaMemsetAsync(rev_head.p, 0, sizeof(rev_head.p[0]) * rev_head.n, stream));
+        clock.restart();
+    }
     // before a step's first launch: list capacities follow the counts every
     // CAPACITY_CHECK steps, counted across calls, and the pair cache's checks
     void host_checks()
     {
         if (hook_steps % CAPACITY_CHECK == 0) ensure_capacity();
+        build_room(CAPACITY_CHECK);
         pc_check_overflow();
         pc_reserve();
         pc_prepare();
@@ -1247,6 +1268,7 @@ struct fundem_sim {
         // reverse index carry them: none may hold a number of the earlier phase
         if (rev_head.n) FD_CUDA(after_legacy(cudaMemset(rev_head.p, 0, sizeof(rev_head.p[0]) * rev_head.n)));
         rev_valid = false;
+        clock.restart();
         configure_nl();
         configure_pc();
         if (!wall_groups.empty()) {
@@ -1540,6 +1562,9 @@ struct fundem_sim {
     void detect_fit(double probe)
     {
         const unsigned int grow_bits = FD_FLAG_PAIR_OVERFLOW | FD_FLAG_CONTACT_OVERFLOW;
+        constexpr int ATTEMPTS = 4;
+        build_room(ATTEMPTS);
+        note_builds(ATTEMPTS);
         unsigned int f0 = 0;
         FD_CUDA(cudaStreamSynchronize(stream));
         FD_CUDA(cudaMemcpy(&f0, flags.p, sizeof(f0), cudaMemcpyDeviceToHost));
@@ -1569,7 +1594,7 @@ struct fundem_sim {
             ensure_capacity();
             unsigned int f = 0;
             FD_CUDA(cudaMemcpy(&f, flags.p, sizeof(f), cudaMemcpyDeviceToHost));
-            if (!(f & grow_bits) || attempt == 3) {
+            if (!(f & grow_bits) || attempt == ATTEMPTS - 1) {
                 const unsigned int keep = f | f0;
                 FD_CUDA(cudaMemcpyAsync(flags.p, &keep, sizeof(keep), cudaMemcpyHostToDevice, stream));
                 break;
@@ -1577,8 +1602,15 @@ struct fundem_sim {
         }
     }
 
+    // fronts and detections outside steps take build numbers; a capture takes
+    // them when it is replayed
+    void note_builds(long long steps)
+    {
+        if (!capturing) clock.note((uint64_t)steps);
+    }
     void front(double3 g, double dt)
     {
+        note_builds(1);
         small = small_on();
         sum_pending = false;
         step_wrapped = nullptr;
@@ -1586,7 +1618,11 @@ struct fundem_sim {
     }
     void back(double3 g, double dt) { advance(g, dt, fd::STEP_BACK); }
     // back() of one step and front() of the next, the bodies in one pass
-    void back_front(double3 g, double dt) { advance(g, dt, fd::STEP_BACK | fd::STEP_FRONT); }
+    void back_front(double3 g, double dt)
+    {
+        note_builds(1);
+        advance(g, dt, fd::STEP_BACK | fd::STEP_FRONT);
+    }
 };
 
 namespace {
@@ -2222,6 +2258,8 @@ int fundem_step_graph(fundem_sim* s, int nsteps, const double g[3], double dt)
             if (nsteps & 1)
                 for (int k = 0; k < FD_NKIND; ++k) s->lists[k].cur ^= 1;
         }
+        s->build_room(nsteps);
+        s->note_builds(nsteps);
         s->pc_prepare();
         FD_CUDA(cudaGraphLaunch(G.exec, s->stream));
         s->launches += G.kernels;
@@ -2804,6 +2842,7 @@ int fundem_adjoint_forward(fundem_sim* s, int nsteps, const double g[3], double 
                 A.seg_steps.push_back(0);
             }
             if (A.steps % CAPACITY_CHECK == 0) s->ensure_capacity();
+            s->build_room(1);
             s->front(gg, dt);
             s->detect_all(true, dt);
             s->back(gg, dt);
@@ -2897,6 +2936,7 @@ int fundem_adjoint_backward_rot(fundem_sim* s, const double* dl_dpos, const doub
             if (rot) fd::adj_record_rot(s->P.view(), T.prot.p, fd::ADJ_REC_QW | fd::ADJ_REC_T, s->stream);
             for (int t = 0; t < ns; ++t) {
                 s->record_step = t;
+                s->build_room(1);
                 s->front(A.g, A.dt);
                 if (rot) fd::adj_record_rot(s->P.view(), T.prot.p + prs * (t + 1), fd::ADJ_REC_QW, s->stream);
                 s->detect_all(true, A.dt);

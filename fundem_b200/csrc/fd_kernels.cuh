@@ -164,7 +164,8 @@ struct MatDev {
 // keeps an open-addressing hash table of its occupied cells instead.  A head
 // holds (build number << 32 | first object): a head of another build is
 // empty.  There is one build number per list generation; each is newer than
-// every number a head can hold when its step begins.
+// every number a head can hold when its step begins (fd_build.h keeps them from
+// coming round).
 struct CellTableDev {
     FdGrid g;
     int hashed;                 // 0: a head per cell, 1: hash table of occupied cells
