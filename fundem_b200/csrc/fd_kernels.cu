@@ -1443,17 +1443,19 @@ __global__ void __launch_bounds__(TPB) k_broad_lists(ListSet a)
     }
 }
 
-// load_quad of what a kernel before this one wrote (and this one does not)
+// load_quad of what kernels write.  Volatile: without it the asm is a function of
+// its address to the compiler, which may then merge two of them or move one
+// ahead of a barrier or of step_wait
 __device__ __forceinline__ double4 load_four(const double4* p)
 {
     double4 v;
-    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ fd_quat load_q(const fd_quat* p)
 {
     fd_quat v;
-    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.q0), "=d"(v.q1), "=d"(v.q2), "=d"(v.q3) : "l"(p));
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.q0), "=d"(v.q1), "=d"(v.q2), "=d"(v.q3) : "l"(p));
     return v;
 }
 
