@@ -271,6 +271,7 @@ __device__ __forceinline__ float half_angle32(float px, float py, float pz, cons
     return atan2f(num, den);
 }
 
+constexpr int MESH_SCREENED = 1 << 22;  // see k_levelset_mesh
 constexpr int MESH_WARPS = 4;
 constexpr int MESH_BLOCK = 32 * MESH_WARPS;  // also the triangles staged at a time
 
@@ -291,6 +292,21 @@ constexpr int MESH_BLOCK = 32 * MESH_WARPS;  // also the triangles staged at a t
 //     closed mesh gives one) is summed again in double precision, in
 //     triangle order.
 // So every value is the one the double-precision scan gives.
+//
+// Why a quarter of a turn is enough.  Rounding the coordinates moves each
+// vertex and the node by at most 6e-8 of the extent, the same way for all
+// triangles: a closed mesh stays closed, and its winding number about the moved
+// node differs only where the node changes sides, that is within 2e-7 of the
+// surface.  There the triangle it would cross, and those next to an edge or a
+// corner it is that close to, fail half_angle32's tests (their angle is near
+// pi, or a corner is within 1e-4) and are evaluated exactly.  Of the other
+// triangles each term is off by the products' roundings, some 4e-7 of lll,
+// against a num or den of at least 0.02 lll: at most 2e-5 for the few that
+// subtend a large angle, and some 1e-7 for a triangle whose corners lie close
+// together seen from the node (den is about 4 lll there), as all but a few are
+// in a mesh of many.  A quarter of a turn is 1.6 in half angles: sixteen
+// million such triangles all off the same way.  A mesh of more than
+// MESH_SCREENED triangles is summed in double precision.
 __global__ void __launch_bounds__(MESH_BLOCK) k_levelset_mesh(const double* __restrict__ tri,
                                                               const MeshTri* __restrict__ mesh, int ntri, int flip,
                                                               double3 o, double h, int3 n, double3 centre, double unit,
@@ -392,7 +408,7 @@ __global__ void __launch_bounds__(MESH_BLOCK) k_levelset_mesh(const double* __re
     wsum *= 2.0;
     const double turns = fabs(wsum / (4.0 * 3.14159265358979323846));
     bool inside = turns > 0.5;
-    if (!(turns < 0.25 || turns > 0.75)) {
+    if (!(turns < 0.25 || turns > 0.75) || ntri > MESH_SCREENED) {
         wsum = 0.0;
         for (int t = 0; t < ntri; ++t) {
             const double* T = tri + 9ll * t;
