@@ -1180,7 +1180,6 @@ struct fundem_sim {
         fd::StepArgs a{};
         a.dt = dt;
         a.probe = probe;
-        a.gravity = make_double3(0, 0, 0);
         a.periodic_x = perX;
         a.periodic_y = perY;
         a.sector = turned_on();

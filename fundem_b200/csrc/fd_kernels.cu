@@ -93,9 +93,8 @@ __device__ __forceinline__ int block_excl_scan(int v, int* total)
 }
 
 template <bool INCLUSIVE>
-__global__ void k_scan_tile(const int* in, int* out, long long n, int* tile_sums, const int* gate)
+__global__ void k_scan_tile(const int* in, int* out, long long n, int* tile_sums)
 {
-    if (gate && *gate == 0) return;
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
     int s = 0;
@@ -117,9 +116,8 @@ __global__ void k_scan_tile(const int* in, int* out, long long n, int* tile_sums
     if (tile_sums && threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-__global__ void k_scan_add(int* out, long long n, const int* tile_off, const int* gate)
+__global__ void k_scan_add(int* out, long long n, const int* tile_off)
 {
-    if (gate && *gate == 0) return;
     const long long i = (long long)blockIdx.x * SCAN_TILE + threadIdx.x;
     const int add = tile_off[blockIdx.x];
 #pragma unroll
@@ -266,20 +264,18 @@ constexpr int RS_TPB = 256;
 constexpr int RS_RADIX = 256;
 constexpr unsigned long long RS_NONE = ~0ull;  // key of an object in no cell
 
-__global__ void k_rs_keys(const long long* hash, int n, long long num, unsigned long long* key, int* idx,
-                          const int* gate)
+__global__ void k_rs_keys(const long long* hash, int n, long long num, unsigned long long* key, int* idx)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (gate && *gate == 0)) return;
+    if (i >= n) return;
     const long long h = hash[i];
     key[i] = (h >= 0 && h < num) ? (unsigned long long)h : RS_NONE;
     idx[i] = i;
 }
 
 __global__ void __launch_bounds__(RS_TPB) k_rs_hist(const unsigned long long* key, int n, int shift, int* bcount,
-                                                   int nblk, const int* gate)
+                                                   int nblk)
 {
-    if (gate && *gate == 0) return;
     __shared__ int h[RS_RADIX];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -290,10 +286,8 @@ __global__ void __launch_bounds__(RS_TPB) k_rs_hist(const unsigned long long* ke
 }
 
 __global__ void __launch_bounds__(RS_TPB) k_rs_scatter(const unsigned long long* key, const int* idx, int n, int shift,
-                                                      const int* boff, int nblk, unsigned long long* okey, int* oidx,
-                                                      const int* gate)
+                                                      const int* boff, int nblk, unsigned long long* okey, int* oidx)
 {
-    if (gate && *gate == 0) return;
     constexpr int NW = RS_TPB / 32;
     __shared__ int wcnt[NW][RS_RADIX];
     for (int d = threadIdx.x; d < NW * RS_RADIX; d += RS_TPB) (&wcnt[0][0])[d] = 0;
@@ -1820,15 +1814,6 @@ __global__ void __launch_bounds__(NARROW_WARPS * 32, FD_SELECT_MIN_BLOCKS) k_sel
 }
 
 // ---------------------------------------------------------------------------
-// narrow phase, stage 2: one thread per contact slot.  The exact
-// double-precision node predicate (LSParticleContactDetectionKernel.cu:37-119);
-// for a contact, the normal, the contact point and the history carried over
-// from the previous step (first match on the node, :288-297), then the
-// contact law (contactKernel.cu:46-291).  A slot whose node is not in contact
-// keeps node id -1.  Force and torques go to the slot; stage 3 sums them per
-// pair.
-// ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // pair cache, particle-particle list, carried steps: the slots the predicate
 // pass must test.  A slot is skipped when its node was outside B at the
 // rebuild by more than the SDF can change under the pair's relative motion
@@ -1902,6 +1887,15 @@ __global__ void __launch_bounds__(TPB) k_slot_filter(NarrowArgs n)
     }
 }
 
+// ---------------------------------------------------------------------------
+// narrow phase, stage 2, in two passes: one thread per contact slot runs the
+// exact double-precision node predicate (LSParticleContactDetectionKernel.cu:
+// 37-119); one thread per contact the normal, the contact point, the history
+// carried over from the previous step (first match on the node, :288-297) and
+// the contact law (contactKernel.cu:46-291).  A slot whose node is not in
+// contact keeps node id -1.  Force and torques go to the contact's record;
+// stage 3 sums them per pair.
+// ---------------------------------------------------------------------------
 // What the predicate reads of a slot's two bodies, and with law what the
 // contact law does.  All of it is independent, and the asm keeps it in one
 // place: left to itself the compiler places each load near its use, some
@@ -3900,32 +3894,32 @@ size_t scan_tmp_size(long long n)
     return total + 1;
 }
 
-void scan_exclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t s, const int* gate)
+void scan_exclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t s)
 {
     if (n <= 0) return;
     if (n <= SCAN_TILE) {
-        k_scan_tile<false><<<1, SCAN_TPB, 0, s>>>(in, out, n, nullptr, gate); note_launch();
+        k_scan_tile<false><<<1, SCAN_TPB, 0, s>>>(in, out, n, nullptr); note_launch();
         return;
     }
     const long long tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     int* sums = tmp;
-    k_scan_tile<false><<<(unsigned)tiles, SCAN_TPB, 0, s>>>(in, out, n, sums, gate); note_launch();
-    scan_exclusive(sums, sums, tiles, tmp + tiles, s, gate);
-    k_scan_add<<<(unsigned)tiles, SCAN_TPB, 0, s>>>(out, n, sums, gate); note_launch();
+    k_scan_tile<false><<<(unsigned)tiles, SCAN_TPB, 0, s>>>(in, out, n, sums); note_launch();
+    scan_exclusive(sums, sums, tiles, tmp + tiles, s);
+    k_scan_add<<<(unsigned)tiles, SCAN_TPB, 0, s>>>(out, n, sums); note_launch();
 }
 
 void scan_inclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t s)
 {
     if (n <= 0) return;
     if (n <= SCAN_TILE) {
-        k_scan_tile<true><<<1, SCAN_TPB, 0, s>>>(in, out, n, nullptr, nullptr); note_launch();
+        k_scan_tile<true><<<1, SCAN_TPB, 0, s>>>(in, out, n, nullptr); note_launch();
         return;
     }
     const long long tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     int* sums = tmp;
-    k_scan_tile<true><<<(unsigned)tiles, SCAN_TPB, 0, s>>>(in, out, n, sums, nullptr); note_launch();
+    k_scan_tile<true><<<(unsigned)tiles, SCAN_TPB, 0, s>>>(in, out, n, sums); note_launch();
     scan_exclusive(sums, sums, tiles, tmp + tiles, s);
-    k_scan_add<<<(unsigned)tiles, SCAN_TPB, 0, s>>>(out, n, sums, nullptr); note_launch();
+    k_scan_add<<<(unsigned)tiles, SCAN_TPB, 0, s>>>(out, n, sums); note_launch();
 }
 
 __global__ void __launch_bounds__(TPB) k_sdf_quads(const double* sdf, const float* sdf32, double4* quad,
@@ -3962,8 +3956,7 @@ void radix_sort_scratch(int n, size_t& bcount_ints, size_t& bscan_ints)
     bscan_ints = scan_tmp_size((long long)bcount_ints);
 }
 void radix_sort_keys(const long long* keys, int n, long long num_keys, unsigned long long* out_key, int* out_idx,
-                     unsigned long long* key_b, int* idx_b, int* bcount, int* bscan_tmp, cudaStream_t s,
-                     const int* gate)
+                     unsigned long long* key_b, int* idx_b, int* bcount, int* bscan_tmp, cudaStream_t s)
 {
     if (n <= 0) return;
     // bits a key can use; keys of objects in no cell sort after every cell
@@ -3975,12 +3968,12 @@ void radix_sort_keys(const long long* keys, int n, long long num_keys, unsigned 
     unsigned long long* kb[2] = {out_key, key_b};
     int* ib[2] = {out_idx, idx_b};
     int src = passes & 1;
-    k_rs_keys<<<nblocks(n), TPB, 0, s>>>(keys, n, num_keys, kb[src], ib[src], gate); note_launch();
+    k_rs_keys<<<nblocks(n), TPB, 0, s>>>(keys, n, num_keys, kb[src], ib[src]); note_launch();
     for (int p = 0; p < passes; ++p) {
         const int shift = 8 * p;
-        k_rs_hist<<<nblk, RS_TPB, 0, s>>>(kb[src], n, shift, bcount, nblk, gate); note_launch();
-        scan_exclusive(bcount, bcount, (long long)RS_RADIX * nblk, bscan_tmp, s, gate);
-        k_rs_scatter<<<nblk, RS_TPB, 0, s>>>(kb[src], ib[src], n, shift, bcount, nblk, kb[src ^ 1], ib[src ^ 1], gate);
+        k_rs_hist<<<nblk, RS_TPB, 0, s>>>(kb[src], n, shift, bcount, nblk); note_launch();
+        scan_exclusive(bcount, bcount, (long long)RS_RADIX * nblk, bscan_tmp, s);
+        k_rs_scatter<<<nblk, RS_TPB, 0, s>>>(kb[src], ib[src], n, shift, bcount, nblk, kb[src ^ 1], ib[src ^ 1]);
         note_launch();
         src ^= 1;
     }

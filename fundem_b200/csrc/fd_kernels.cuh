@@ -299,7 +299,6 @@ struct StepArgs {
     AdjRec rec;      // recording of the list being launched (rec.hit null: off)
     double dt;
     double probe;      // contact when overlap >= -probe (0 in a timestep)
-    double3 gravity;
     int periodic_x, periodic_y;
     int sector;      // sector periodicity (the force side of particle and wall contacts folds bodies)
     int records;
@@ -354,8 +353,7 @@ void launch_hash(const ObjDev& O, const FdGrid& g, cudaStream_t s, unsigned int*
 // the negative ones).  Scratch: key_b (n), idx_b (n), bcount and bscan_tmp
 // sized by radix_sort_scratch.
 void radix_sort_keys(const long long* keys, int n, long long num_keys, unsigned long long* out_key, int* out_idx,
-                     unsigned long long* key_b, int* idx_b, int* bcount, int* bscan_tmp, cudaStream_t s,
-                     const int* gate = nullptr);
+                     unsigned long long* key_b, int* idx_b, int* bcount, int* bscan_tmp, cudaStream_t s);
 // ints needed for bcount and bscan_tmp for n keys
 void radix_sort_scratch(int n, size_t& bcount_ints, size_t& bscan_ints);
 // The periodic wraps (positions into dst, which may be P.pos) and the
@@ -460,7 +458,7 @@ void count_launch();
 
 // exclusive scan of n ints (out may alias in); returns needed tmp ints when tmp == nullptr
 size_t scan_tmp_size(long long n);
-void scan_exclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t s, const int* gate = nullptr);
+void scan_exclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t s);
 // inclusive scan of n ints; tmp as for scan_exclusive
 void scan_inclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t s);
 
