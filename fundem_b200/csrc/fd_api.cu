@@ -993,14 +993,18 @@ struct fundem_sim {
     }
     // Small sets step with two launches (launch_small_pairs,
     // launch_small_advance).  The rule: no images, no pair cache or neighbour
-    // list (so fewer particles than either starts at), a dense cell table,
-    // and not under the stage timers, which see the stages one by one.
-    // Measured per step of a pour (graph replay): see k_small_pairs.
+    // list, a dense cell table, not under the stage timers, which see the
+    // stages one by one, and no more particles than the block of a small step
+    // pays for: its threads idle through most of the contact law.  Ten steps of
+    // a pour, small against staged, us: 4,096 particles 906 against 1,140 (graph
+    // 876, 967), 5,000 1,045 and 1,139 (979, 959), 6,500 1,274 and 1,241 (1,196,
+    // 1,058), 8,191 1,553 and 1,324 (1,430, 1,154).
+    static constexpr int SMALL_PARTICLES = 5120;
     DevArray<int> small_head;
     DevArray<double> small_own;
     bool small_on() const
     {
-        return P.n_dev > 0 && P.n_dev < NL_MIN_PARTICLES && !use_nl && !pc_active() && !perX && !perY && !sector &&
+        return P.n_dev > 0 && P.n_dev <= SMALL_PARTICLES && !use_nl && !pc_active() && !perX && !perY && !sector &&
                !ptab.hashed && (!profiling || capturing);
     }
     // the current step (set by front): small, with the pair cache; whether its

@@ -3298,9 +3298,9 @@ __global__ void __launch_bounds__(128) k_advance(AdvanceArgs a)
 
 // ---------------------------------------------------------------------------
 // Small sets (no neighbour list, no pair cache, no images).  A step of the
-// staged kernels is 24 dependent launches, each a few microseconds of latency
-// and next to no work at these sizes: 102 us a step for 1,000 particles in a
-// graph replay.  Here a step is two launches.  k_small_pairs takes each
+// staged kernels is a dozen dependent launches, each a few microseconds of
+// latency and next to no work at these sizes: 73 us a step for 1,000 particles
+// in a graph replay.  Here a step is two launches.  k_small_pairs takes each
 // particle's partners and walls from the cell lists, culls each candidate pair
 // in one warp, takes the block's slots through predicate and contact law one
 // thread each, and sums its pairs with eight lanes each; k_small_advance sums
@@ -3312,7 +3312,7 @@ __global__ void __launch_bounds__(128) k_advance(AdvanceArgs a)
 // Bound by the chain of one block: about 9,400 cycles of search, 13,000 of
 // culling (two pairs a warp), 8,000 of predicate and law, 4,000 of sums.  A
 // step of 1,000 particles takes 38 us (50 with a pair's slots in its own warp),
-// of 4,096 65 us (81; 118 a step in the staged kernels).
+// of 4,096 65 us (81).  Where the staged kernels take over: SMALL_PARTICLES.
 // ---------------------------------------------------------------------------
 constexpr int SMALL_BODIES = 4;               // particles per block
 constexpr int SMALL_WARPS = 2 * SMALL_BODIES;  // a warp for each one's partners, one for its walls
@@ -3788,12 +3788,11 @@ static inline void note_launch()
 {
     if (t_launch_counter) ++*t_launch_counter;
 }
-// A kernel that begins with step_wait.  Not in recorded graphs, whose launches
-// are a microsecond apart as it is (4,096 particles: 65.8 us a step against
-// 64.8); a plain step of 777 particles went from 52.6 to 44.6 us.  Nor the
-// staged kernels, whose waiting blocks hold registers and shared memory that
-// the bonds and the kernel before could use (16,384 particles, 8 plain steps
-// between uploads: 4.1 ms against 3.8).
+// For kernels that begin with step_wait: the two of a small set's step, plain
+// launches.  Not in recorded graphs, whose launches are a microsecond apart as
+// it is (4,096 particles: 65.8 us a step against 64.8); a plain step of 777
+// particles went from 52.6 to 44.6 us.  The staged kernels have no such wait and
+// are launched one after the other; whether they would gain was not measured.
 template <typename... P, typename... A>
 static void launch_ahead(void (*kernel)(P...), int blocks, int threads, cudaStream_t s, const A&... args)
 {
