@@ -2496,6 +2496,8 @@ int fundem_set_contacts(fundem_sim* s, int kind, long long n, const int* node, c
         });
         std::vector<int> pairA, pairB, c_off, c_cnt, seg_off(np, 0), seg_cnt(np, 0), cn, cs, ck, at;
         std::vector<double4> hist;
+        for (auto* v : {&cn, &cs, &ck, &at}) v->reserve(order.size());
+        hist.reserve(order.size());
         for (size_t t = 0; t < order.size(); ++t) {
             const size_t k = order[t];
             const int A = owner(node[k]), B = partner[k];
