@@ -72,19 +72,28 @@ template <typename T> struct DevArray {
     void alloc(size_t count, bool zero = true)
     {
         release();
-        n = count;
         if (count == 0) return;
         bump_alloc_epoch();
-        FD_CUDA(cudaMalloc((void**)&p, sizeof(T) * count));
+        p = take(count);
+        n = count;  // with the memory: a failed allocation leaves an empty array
         if (zero) FD_CUDA(after_legacy(cudaMemset(p, 0, sizeof(T) * count)));
+    }
+    // memory for count elements; a failure is this call's only, not the next
+    // call's last error
+    static T* take(size_t count)
+    {
+        T* q = nullptr;
+        const cudaError_t e = cudaMalloc((void**)&q, sizeof(T) * count);
+        if (e != cudaSuccess) cudaGetLastError();
+        FD_CUDA(e);
+        return q;
     }
     // grow keeping the first `keep` elements
     void grow(size_t count, size_t keep)
     {
         if (count <= n) return;
         bump_alloc_epoch();
-        T* q = nullptr;
-        FD_CUDA(cudaMalloc((void**)&q, sizeof(T) * count));
+        T* q = take(count);
         FD_CUDA(after_legacy(cudaMemset(q, 0, sizeof(T) * count)));
         if (p && keep) FD_CUDA(after_legacy(cudaMemcpy(q, p, sizeof(T) * std::min(keep, n), cudaMemcpyDeviceToDevice)));
         if (p) cudaFree(p);
@@ -977,7 +986,8 @@ struct fundem_sim {
     {
         const int np = std::max(P.n(), 1);
         if (rev_cnt.n < (size_t)np) {
-            rev_cnt.alloc(np); rev_off.alloc(np); rev_head.alloc(np); rev_total.alloc(1);
+            rev_off.alloc(np); rev_head.alloc(np); rev_total.alloc(1);
+            rev_cnt.alloc(np);  // last: its size says that all are there
             rev_valid = false;
         }
         long long cap = 0;
@@ -1575,9 +1585,9 @@ struct fundem_sim {
         const bool wraps = (perX || perY || sector) && np > 0 && P.n_dev == (int)np;
         if (wraps) {
             if (keep_pos.n < np) {
-                keep_pos.alloc(np, false);
                 keep_vel.alloc(np, false);
                 keep_q.alloc(np, false);
+                keep_pos.alloc(np, false);
             }
             FD_CUDA(cudaMemcpyAsync(keep_pos.p, P.d_pos.p, np * sizeof(double3), cudaMemcpyDeviceToDevice, stream));
             FD_CUDA(cudaMemcpyAsync(keep_vel.p, P.d_vel.p, np * sizeof(double3), cudaMemcpyDeviceToDevice, stream));
@@ -1811,7 +1821,7 @@ int fundem_contact_view_get(fundem_sim* s, int kind, fundem_contact_view* out)
         const size_t cap = (size_t)std::max(L.cap_contacts, 1);
         auto& V = s->cviews[kind];
         if (V.keys.n < cap) {
-            V.keys.alloc(cap, false); V.order.alloc(cap, false); V.idx_b.alloc(cap, false);
+            V.order.alloc(cap, false); V.idx_b.alloc(cap, false);
             V.skey.alloc(cap, false); V.key_b.alloc(cap, false);
             size_t bc = 0, bs = 0;
             fd::radix_sort_scratch((int)cap, bc, bs);
@@ -1819,6 +1829,7 @@ int fundem_contact_view_get(fundem_sim* s, int kind, fundem_contact_view* out)
             V.master.alloc(cap, false); V.slave.alloc(cap, false); V.overlap.alloc(cap, false);
             V.en.alloc(cap, false); V.es.alloc(cap, false);
             V.point.alloc(3 * cap, false); V.normal.alloc(3 * cap, false); V.spring.alloc(3 * cap, false);
+            V.keys.alloc(cap, false);
         }
         fd::ContactViewDev v{V.point.p, V.normal.p, V.overlap.p, V.en.p, V.es.p, V.spring.p, V.master.p, V.slave.p};
         const long long max_key = (s->n_nodes + 1) << 32;
@@ -1841,9 +1852,9 @@ int fundem_bond_view_get(fundem_sim* s, fundem_bond_view* out)
         fd::BondDev bd = s->bond_view();
         const size_t m = (size_t)std::max(bd.n, 1);
         if (s->bview_B.n < 4 * m) {
-            s->bview_B.alloc(4 * m, false);
             s->bview_energy.alloc(6 * m, false);
             s->bview_frames.alloc(8 * m, false);
+            s->bview_B.alloc(4 * m, false);
         }
         fd::BondViewDev v{};
         for (int t = 0; t < 4; ++t) v.B[t] = s->bview_B.p + t * m;
@@ -2426,8 +2437,8 @@ int fundem_get_contacts(fundem_sim* s, int kind, int* node, int* partner, double
         if (s->pack_buf.n < words) {
             // no captured step reads these: its graphs stay valid
             const unsigned long long epoch = s->alloc_epoch;
-            s->pack_buf.alloc(words + words / 2, false);
             if (!s->pack_at.p) s->pack_at.alloc(1);
+            s->pack_buf.alloc(words + words / 2, false);
             s->alloc_epoch = epoch;
         }
         size_t off[6] = {0, 0, 0, 0, 0, 0}, at = n;
