@@ -2302,41 +2302,50 @@ __device__ __forceinline__ void contact_list(const NarrowArgs& n, int block, int
 // a quarter of a contact per pair), so a warp takes several pairs' flags in one
 // load, the next ones' meanwhile, and passes on to those that hold one; with
 // eight lanes looking at each pair the sums took 105 us for 262,144 particles,
-// this way 57 (cold caches; 30 in a run of steps).  A pair of bodies pressed into
-// one another holds hundreds of contacts: their forces are loaded four at a
-// time, the next slots' ids meanwhile, and a short list is shared out over all
-// warps.  With a load per contact and 32 pairs a warp whatever their number,
-// 40,000 pairs of such bodies took 2,660 us, this way 145; eight at a time
-// take 127, but 40 instead of 30 us for the settled bed.
+// this way 57 (cold caches; 28 to 38 in a run of steps).  A pair of bodies
+// pressed into one another holds hundreds of contacts: their forces are loaded
+// three at a time, the next slots' ids meanwhile, and a short list is shared out
+// over all warps.  With a load per contact and 32 pairs a warp whatever their
+// number, 40,000 pairs of such bodies took 2,660 us, this way 195.  Four or eight
+// at a time take 150 and 127, but registers of the other warps: a settled bed
+// of 262,144 then 40 and 48 us, not 38.
 // ---------------------------------------------------------------------------
-// the forces of the contacts among eight slots, in slot order (m: bit u for
-// slot u of the lane's group of eight; at: the place of the lane's own slot):
-// component l of each onto acc, the ninth onto lane 0's acc8.  For whole warps.
+// the forces of the first COUNT contacts that m still names (bit u: slot u of
+// the lane's group of eight; at: the place of the lane's own slot), in slot
+// order: component l of each onto acc, the ninth onto lane 0's acc8.  For whole
+// warps.
+template <int COUNT, typename Real>
+__device__ __forceinline__ void add_some(const double* rec, unsigned int& m, int at, int l, Real& acc, Real& acc8)
+{
+    Real v[COUNT], v8[COUNT];
+    bool on[COUNT];
+#pragma unroll
+    for (int u = 0; u < COUNT; ++u) {
+        on[u] = m != 0u;
+        const int t = __shfl_sync(0xffffffffu, at, on[u] ? __ffs(m) - 1 : 0, 8);
+        m &= m - 1u;
+        const Real* f = reinterpret_cast<const Real*>(rec + (long long)CONTACT_REC * t);
+        v[u] = on[u] ? f[l] : Real(0);
+        v8[u] = on[u] && l == 0 ? f[8] : Real(0);
+    }
+#pragma unroll
+    for (int u = 0; u < COUNT; ++u)
+        if (on[u]) {
+            acc += v[u];
+            acc8 += v8[u];
+        }
+}
 template <typename Real>
 __device__ __forceinline__ void add_contacts(const double* rec, unsigned int m, int at, int l, Real& acc, Real& acc8)
 {
-    while (__any_sync(0xffffffffu, m != 0u)) {
-        Real v[4], v8[4];
-        bool on[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            on[u] = m != 0u;
-            const int t = __shfl_sync(0xffffffffu, at, on[u] ? __ffs(m) - 1 : 0, 8);
-            m &= m - 1u;
-            const Real* f = reinterpret_cast<const Real*>(rec + (long long)CONTACT_REC * t);
-            v[u] = on[u] ? f[l] : Real(0);
-            v8[u] = on[u] && l == 0 ? f[8] : Real(0);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (on[u]) {
-                acc += v[u];
-                acc8 += v8[u];
-            }
+    if (!__any_sync(0xffffffffu, __popc(m) > 1)) {
+        add_some<1>(rec, m, at, l, acc, acc8);
+        return;
     }
+    while (__any_sync(0xffffffffu, m != 0u)) add_some<3>(rec, m, at, l, acc, acc8);
 }
 
-constexpr int SUM_TPB = 384;  // four such blocks an SM take the registers of 48 warps
+constexpr int SUM_TPB = 512;  // four such blocks fill an SM's warps
 
 template <typename Real>
 __device__ __forceinline__ void sum_list(const PairListDev& L, int kind, int block, int nblocks, bool link,
