@@ -56,8 +56,9 @@ def log(*a):
 
 class ClockSampler:
     """SM clock, power and clock-event reasons sampled during the timed
-    region: NVML in a thread every 5 ms (the region can be a few tens of
-    milliseconds), or nvidia-smi every 200 ms where NVML is missing."""
+    region: NVML in a thread every millisecond (the region can be less than
+    ten), or nvidia-smi every 200 ms where NVML is missing.  start() returns
+    after the first reading, so that the region has one just before it."""
 
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -66,13 +67,15 @@ class ClockSampler:
     REASONS = {0x4: "sw_power_cap", 0x8: "hw_slowdown", 0x20: "sw_thermal_slowdown",
                0x40: "hw_thermal_slowdown", 0x80: "hw_power_brake_slowdown"}
 
-    def __init__(self, index, period_s=0.005):
+    def __init__(self, index, period_s=0.001):
         self.index = index
         self.period = period_s
         self.samples = []   # (sm_mhz, max_mhz, power_w, reason bits)
         self.proc = None
         self.nvml = None
         self._stop = threading.Event()
+        self._first = threading.Event()
+        self._before = 0    # readings before the region
 
     def _nvml_handle(self):
         """The NVML handle of CUDA device `index`, matched by UUID (NVML and
@@ -99,6 +102,8 @@ class ClockSampler:
             self.nvml, h = self._nvml_handle()
             self.thread = threading.Thread(target=self._poll_nvml, args=(h,), daemon=True)
             self.thread.start()
+            self._first.wait(2.0)
+            self._before = len(self.samples)
             return
         except Exception:
             self.nvml = None
@@ -120,6 +125,7 @@ class ClockSampler:
             try:
                 self.samples.append((float(N.nvmlDeviceGetClockInfo(h, N.NVML_CLOCK_SM)), float(mx),
                                      N.nvmlDeviceGetPowerUsage(h) / 1e3, int(get_reasons(h))))
+                self._first.set()
             except Exception:
                 pass
             time.sleep(self.period)
@@ -150,6 +156,8 @@ class ClockSampler:
         if not self.samples:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": [], "samples": 0,
                     "source": "nvml" if self.nvml else ("nvidia-smi" if self.proc else "unavailable")}
+        # the readings of the region; the one before it where it was too short for any
+        self.samples = self.samples[self._before:] or self.samples
         sm = [x[0] for x in self.samples]
         reasons = set()
         for x in self.samples:
@@ -278,7 +286,6 @@ def run_fundem(args, rank, world, dist):
         dist.barrier()
     torch.cuda.synchronize()
     clocks.start()
-    time.sleep(0.02)  # the sampler's first reading precedes the region
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     if args.profile:
         torch.cuda.profiler.start()
@@ -452,7 +459,8 @@ def run_fundem(args, rank, world, dist):
                      "traffic": (traffic_per_pair * pairs) if traffic_per_pair else None,
                      "traffic_source": TRAFFIC_PROFILE + " (ncu DRAM bytes per candidate pair x pairs)"
                      if traffic_per_pair else None,
-                     "kernel": "k_narrow<PP> (narrow phase + contact law)", "peak_source": pk_kind,
+                     "kernel": "particle-particle narrow phase: k_select_lists, k_slot_filter, both "
+                               "k_contact_lists passes, k_sum_lists", "peak_source": pk_kind,
                      "kernel_ms": nar_avg, "algorithmic_bytes": nar_bytes,
                      "step_achieved_gbs": step_bytes / (t_max / args.steps / 1e3) / 1e9},
         "roofline_fp64": fp64_roofline(wc, wc_steps, nar_avg),
@@ -467,9 +475,8 @@ def run_fundem(args, rank, world, dist):
         "launch_shape": shape,
         "kernel_timing": "a second pass of K steps right after the headline, with CUDA-event timers on the "
                          "simulation's stream around each kernel group (all stages on that one stream)",
-        "streams": "headline and plain launches: the particle-particle list on the simulation's stream; the "
-                   "particle-wall list and the image lists (with the bonds at the end of one of them) on two "
-                   "more streams, forked after the hash stage and joined before the force sums",
+        "streams": "headline and plain launches: every stage once for all contact lists on the simulation's "
+                   "stream; the bonds on a stream of their own beside the detection, joined before the force sums",
         "reference_gpu": ref_gpu,
         "narrow_work_per_step": {"pairs": wc[0] / wc_steps, "clusters": wc[1] / wc_steps,
                                  "clusters_kept": wc[2] / wc_steps, "node_contacts": wc[3] / wc_steps,
