@@ -1115,6 +1115,22 @@ struct fundem_sim {
     // outside a step starts again from (detect_fit)
     DevArray<double> pack_buf;
     DevArray<int> pack_at;
+    // room for `words` (`want`: with some to spare); false without the memory.  No
+    // captured step reads these: its graphs stay valid
+    bool pack_reserve(size_t want, size_t words)
+    {
+        if (pack_at.p && pack_buf.n >= words) return true;
+        const unsigned long long epoch = alloc_epoch;
+        bool ok = true;
+        try {
+            if (!pack_at.p) pack_at.alloc(1);
+            if (pack_buf.n < words) pack_buf.alloc(want, false);
+        } catch (const CudaError&) {
+            ok = false;
+        }
+        alloc_epoch = epoch;
+        return ok;
+    }
     DevArray<double3> keep_pos, keep_vel;
     DevArray<fd_quat> keep_q;
     ~fundem_sim()
@@ -2434,32 +2450,58 @@ int fundem_get_contacts(fundem_sim* s, int kind, int* node, int* partner, double
         size_t words = n;  // ids: one word each
         for (int f = 0; f < 6; ++f)
             if (dst[f]) words += width[f] * n;
-        if (s->pack_buf.n < words) {
-            // no captured step reads these: its graphs stay valid
-            const unsigned long long epoch = s->alloc_epoch;
-            if (!s->pack_at.p) s->pack_at.alloc(1);
-            s->pack_buf.alloc(words + words / 2, false);
-            s->alloc_epoch = epoch;
-        }
         size_t off[6] = {0, 0, 0, 0, 0, 0}, at = n;
-        double* dev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
         for (int f = 0; f < 6; ++f) {
             if (!dst[f]) continue;
             off[f] = at;
-            dev[f] = s->pack_buf.p + at;
             at += width[f] * n;
         }
-        const fd::ContactPackDev v{reinterpret_cast<int2*>(s->pack_buf.p), dev[0], dev[1], dev[2], dev[3], dev[4], dev[5]};
-        fd::launch_pack_contacts(L.view(), v, s->pack_at.p, (int)n, s->stream);
-        int found = 0;
         std::vector<double> h(words);
-        FD_CUDA(cudaMemcpyAsync(&found, s->pack_at.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-        FD_CUDA(cudaMemcpyAsync(h.data(), s->pack_buf.p, sizeof(double) * words, cudaMemcpyDeviceToHost, s->stream));
-        FD_CUDA(cudaStreamSynchronize(s->stream));
-        // the caller sized its arrays with fundem_num_contacts
-        if ((size_t)found != n)
-            throw std::runtime_error("contact list inconsistent: " + std::to_string(found) + " contacts, counter " +
-                                     std::to_string(n));
+        // the buffer is kept for the next call up to 64 MB; without memory for
+        // it the list is read as it is
+        constexpr size_t KEPT = (64u << 20) / sizeof(double);
+        if (s->pack_reserve(words + words / 2 <= KEPT ? words + words / 2 : words, words)) {
+            double* dev[6];
+            for (int f = 0; f < 6; ++f) dev[f] = dst[f] ? s->pack_buf.p + off[f] : nullptr;
+            const fd::ContactPackDev v{reinterpret_cast<int2*>(s->pack_buf.p), dev[0], dev[1], dev[2], dev[3], dev[4], dev[5]};
+            fd::launch_pack_contacts(L.view(), v, s->pack_at.p, (int)n, s->stream);
+            int found = 0;
+            FD_CUDA(cudaMemcpyAsync(&found, s->pack_at.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+            FD_CUDA(cudaMemcpyAsync(h.data(), s->pack_buf.p, sizeof(double) * words, cudaMemcpyDeviceToHost, s->stream));
+            FD_CUDA(cudaStreamSynchronize(s->stream));
+            if (s->pack_buf.n > KEPT) s->pack_buf.release();
+            // the caller sized its arrays with fundem_num_contacts
+            if ((size_t)found != n)
+                throw std::runtime_error("contact list inconsistent: " + std::to_string(found) + " contacts, counter " +
+                                         std::to_string(n));
+        } else {
+            // slots, and the contacts' places that they name
+            const size_t m = (size_t)c[1];
+            std::vector<int> hn(m), place(m);
+            std::vector<double4> hist(m);
+            std::vector<double> rec((size_t)fd::CONTACT_REC * m);
+            FD_CUDA(cudaMemcpy(hn.data(), g.c_node.p, sizeof(int) * m, cudaMemcpyDeviceToHost));
+            FD_CUDA(cudaMemcpy(place.data(), g.c_at.p, sizeof(int) * m, cudaMemcpyDeviceToHost));
+            FD_CUDA(cudaMemcpy(hist.data(), g.c_hist.p, sizeof(double4) * m, cudaMemcpyDeviceToHost));
+            FD_CUDA(cudaMemcpy(rec.data(), L.c_rec.p, sizeof(double) * rec.size(), cudaMemcpyDeviceToHost));
+            const int from[6] = {fd::CONTACT_POINT, fd::CONTACT_NORMAL, fd::CONTACT_OVERLAP, -1, fd::CONTACT_EN, fd::CONTACT_ES};
+            size_t k = 0;
+            for (size_t sl = 0; sl < m; ++sl) {
+                if (hn[sl] < 0) continue;
+                if (k == n) throw std::runtime_error("contact list inconsistent: more contacts than its counter");
+                const double4 t = hist[place[sl]];
+                const double* r = rec.data() + (size_t)fd::CONTACT_REC * place[sl];
+                const double spr[3] = {t.x, t.y, t.z};
+                int2 ids = make_int2(hn[sl], 0);
+                std::memcpy(&ids.y, &t.w, sizeof(ids.y));
+                std::memcpy(&h[k], &ids, sizeof(ids));
+                for (int f = 0; f < 6; ++f)
+                    for (size_t d = 0; dst[f] && d < width[f]; ++d)
+                        h[off[f] + width[f] * k + d] = from[f] < 0 ? spr[d] : r[from[f] + d];
+                ++k;
+            }
+            if (k != n) throw std::runtime_error("contact list inconsistent: fewer contacts than its counter");
+        }
         const int2* id = reinterpret_cast<const int2*>(h.data());
         std::vector<std::pair<uint64_t, uint32_t>> order(n);
         for (size_t k = 0; k < n; ++k)

@@ -141,7 +141,10 @@ int fundem_move(fundem_sim* sim, int wall, int index, const double offset[3]);
 int fundem_add_bonds(fundem_sim* sim, int n, const int* master, const int* slave, const double* point,
                      const double* normal, const double* radius, const double* length, const double* young,
                      const double* poisson, const double* tensile, const double* cohesion, const double* friction);
-/* addPeriodicBoundaryXD / YD / removePeriodicBoundary, LSSolver.h:384-414 */
+/* addPeriodicBoundaryXD / YD / removePeriodicBoundary, LSSolver.h:384-414.
+   The image sets are those of the last fundem_setup: a direction switched
+   off has no images from the next step on, one switched on has them after
+   the next setup. */
 int fundem_set_periodic(fundem_sim* sim, int x, int y);
 /* addPeriodicBoundarySector / removePeriodicBoundary, LSSolver.h:410-424
    (PeriodicBoundary.h:319-425): the quarter sector x >= min.x, y >= min.y
