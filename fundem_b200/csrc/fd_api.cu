@@ -448,6 +448,8 @@ struct GeoSetHost {
             fd::launch_sdf_quads(d_sdf.p, d_sdf32.p, d_sdf_quad.p, d_sdf32_quad.p, t.sdf_off, t.size, s);
     }
 
+    bool has_faces(bool fp64) const { return d_sdf32_quad.p && (!fp64 || d_sdf_quad.p); }
+
     GeoSetDev view() const
     {
         GeoSetDev v;
@@ -1004,7 +1006,7 @@ struct fundem_sim {
     // Small sets step with two launches (launch_small_pairs,
     // launch_small_advance).  The rule: no images, no pair cache or neighbour
     // list, a dense cell table, not under the stage timers, which see the
-    // stages one by one, and no more particles than the block of a small step
+    // stages one by one, with the tables of cell faces, and no more particles than the block of a small step
     // pays for: its threads idle through most of the contact law.  Ten steps of
     // a pour, small against staged, us: 4,096 particles 906 against 1,140 (graph
     // 876, 967), 5,000 1,045 and 1,139 (979, 959), 6,500 1,274 and 1,241 (1,196,
@@ -1015,7 +1017,8 @@ struct fundem_sim {
     bool small_on() const
     {
         return P.n_dev > 0 && P.n_dev <= SMALL_PARTICLES && !use_nl && !pc_active() && !perX && !perY && !sector &&
-               !ptab.hashed && (!profiling || capturing);
+               !ptab.hashed && (!profiling || capturing) && pgeo.has_faces(!mixed()) &&
+               (W.n_dev == 0 || wgeo.has_faces(true));
     }
     // the current step (set by front): small, with the pair cache; whether its
     // force sums are still to run, and the wrapped positions they take over

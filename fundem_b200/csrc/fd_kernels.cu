@@ -743,11 +743,14 @@ __device__ __forceinline__ double4 load_quad(const double4* p)
 }
 // The corner values of the cell at point i of a set's grids, of the planes z
 // (s0) and z + 1 (s1): from the table of faces, or one by one where the set's
-// table would take too much memory (see GeoSetHost::faces).
+// table would take too much memory (see GeoSetHost::faces).  FACES: the table is
+// there; the way without it costs the small steps' pair kernel registers that it
+// has not got (ten steps of 4,096 particles 639 us with it, 625 without).
+template <bool FACES>
 __device__ __forceinline__ void load_corners(const GeoSetDev& S, long long i, long long sx, long long sxy, double4& s0,
                                              double4& s1)
 {
-    if (S.sdf_quad) {
+    if (FACES || S.sdf_quad) {
         s0 = load_quad(S.sdf_quad + i);
         s1 = load_quad(S.sdf_quad + i + sxy);
         return;
@@ -756,10 +759,11 @@ __device__ __forceinline__ void load_corners(const GeoSetDev& S, long long i, lo
     s0 = make_double4(__ldg(g), __ldg(g + 1), __ldg(g + sx), __ldg(g + sx + 1));
     s1 = make_double4(__ldg(h), __ldg(h + 1), __ldg(h + sx), __ldg(h + sx + 1));
 }
+template <bool FACES>
 __device__ __forceinline__ void load_corners(const GeoSetDev& S, long long i, long long sx, long long sxy, float4& s0,
                                              float4& s1)
 {
-    if (S.sdf32_quad) {
+    if (FACES || S.sdf32_quad) {
         s0 = __ldg(S.sdf32_quad + i);
         s1 = __ldg(S.sdf32_quad + i + sxy);
         return;
@@ -779,6 +783,7 @@ __device__ __forceinline__ void load_corners(const GeoSetDev& S, long long i, lo
 //   * D(v): lower bound on the distance from grid node v to any cell whose
 //     corner minimum is <= 0, 1-Lipschitz in the position,
 //   * the Lipschitz bound of the trilinear SDF (distance-like fields).
+template <bool FACES = false>
 __device__ __forceinline__ bool sphere_culled(float px, float py, float pz, float radius, bool radius_test,
                                               const FdGeo32& GB, const GeoSetDev& SB, float probe)
 {
@@ -809,7 +814,7 @@ __device__ __forceinline__ bool sphere_culled(float px, float py, float pz, floa
         const int i0 = (int)gx, j0 = (int)gy, k0 = (int)gz;
         const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
         float4 s0, s1;
-        load_corners(SB, GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0, sx, sxy, s0, s1);
+        load_corners<FACES>(SB, GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0, sx, sxy, s0, s1);
         const float fx = gx - i0, fy = gy - j0, fz = gz - k0;
         const float c00 = s0.x * (1.f - fx) + s0.y * fx;
         const float c10 = s0.z * (1.f - fx) + s0.w * fx;
@@ -824,6 +829,7 @@ __device__ __forceinline__ bool sphere_culled(float px, float py, float pz, floa
 
 // Body-level cull of a candidate pair in single precision: A's bounding
 // sphere (radius rA about cA) against B, through B's rotation rows
+template <bool FACES = false>
 __device__ __forceinline__ bool body_culled32(const double3 cA, double rA, const double3 cB, const float4* RB,
                                               bool radius_test, const FdGeo32& GB, const GeoSetDev& SB, double probe)
 {
@@ -832,7 +838,7 @@ __device__ __forceinline__ bool body_culled32(const double3 cA, double rA, const
     const float px = fmaf(b0.x, dx, fmaf(b1.x, dy, b2.x * dz));
     const float py = fmaf(b0.y, dx, fmaf(b1.y, dy, b2.y * dz));
     const float pz = fmaf(b0.z, dx, fmaf(b1.z, dy, b2.z * dz));
-    return sphere_culled(px, py, pz, (float)rA, radius_test, GB, SB, (float)probe);
+    return sphere_culled<FACES>(px, py, pz, (float)rA, radius_test, GB, SB, (float)probe);
 }
 
 // cells that can hold the centre of a partner of a body of radius r centred
@@ -1455,7 +1461,7 @@ __device__ __forceinline__ fd_quat load_q(const fd_quat* p)
 
 // Evaluate node predicate for one node.  Returns true when overlap >= 0 and
 // fills the grid fraction and the eight corner values.
-template <int KIND>
+template <int KIND, bool FACES>
 __device__ __forceinline__ bool node_predicate(const double3 gp, const int3 bcell, const FdGrid& sg, const double3 cB,
                                                const fd_quat qB, const FdGeo& GB, const GeoSetDev& SB, double rB2,
                                                double probe, double& overlap, double& fx, double& fy, double& fz,
@@ -1481,7 +1487,7 @@ __device__ __forceinline__ bool node_predicate(const double3 gp, const int3 bcel
     fz = gz - (double)k0;
     const long long sx = GB.size.x, sxy = (long long)GB.size.x * GB.size.y;
     double4 s0, s1;
-    load_corners(SB, GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0, sx, sxy, s0, s1);
+    load_corners<FACES>(SB, GB.sdf_off + (long long)k0 * sxy + (long long)j0 * sx + i0, sx, sxy, s0, s1);
     p[0] = s0.x; p[1] = s0.y; p[2] = s0.z; p[3] = s0.w;
     p[4] = s1.x; p[5] = s1.y; p[6] = s1.z; p[7] = s1.w;
     overlap = -xm_trilinear(fx, fy, fz, p);
@@ -1531,7 +1537,7 @@ __device__ __forceinline__ CullXf cull_transform(const float4* RA, const float4*
 //     corner minimum is <= 0, 1-Lipschitz in the position,
 //   * the Lipschitz bound of the trilinear SDF (coarse grids such as plane
 //     walls, where it is tight).
-template <int KIND>
+template <int KIND, bool FACES>
 __device__ __forceinline__ bool cluster_culled(const float4 cl, const CullXf& x, const FdGeo32& GB,
                                                const GeoSetDev& SB, float probe)
 {
@@ -1539,7 +1545,7 @@ __device__ __forceinline__ bool cluster_culled(const float4 cl, const CullXf& x,
     const float px = fmaf(x.m[0], cx, fmaf(x.m[1], cy, fmaf(x.m[2], cz, x.t[0])));
     const float py = fmaf(x.m[3], cx, fmaf(x.m[4], cy, fmaf(x.m[5], cz, x.t[1])));
     const float pz = fmaf(x.m[6], cx, fmaf(x.m[7], cy, fmaf(x.m[8], cz, x.t[2])));
-    return sphere_culled(px, py, pz, cl.w, Slave<KIND>::radius_test, GB, SB, probe);
+    return sphere_culled<FACES>(px, py, pz, cl.w, Slave<KIND>::radius_test, GB, SB, probe);
 }
 
 // Node filter: true when a node certainly fails the node predicate.  The
@@ -1556,7 +1562,7 @@ __device__ __forceinline__ bool cluster_culled(const float4 cl, const CullXf& x,
 //
 // NODES nodes at a time (on: the node is there; out: dropped): the chains
 // from position to interpolation overlap, and none waits at a branch.
-template <int KIND, int NODES>
+template <int KIND, int NODES, bool FACES>
 __device__ __forceinline__ void node_filter(const float4 (&p)[NODES], const bool (&on)[NODES], const CullXf& x,
                                              const FdGeo32& GB, const GeoSetDev& SB, float perr, float probe,
                                              bool (&out)[NODES])
@@ -1589,7 +1595,7 @@ __device__ __forceinline__ void node_filter(const float4 (&p)[NODES], const bool
             // a node that needs no look reads the pool's first point
             const long long i =
                 look[u] ? GB.sdf_off + (long long)(int)gz[u] * sxy + (long long)(int)gy[u] * sx + (int)gx[u] : 0ll;
-            load_corners(SB, i, look[u] ? sx : 0ll, look[u] ? sxy : 0ll, s0[u], s1[u]);
+            load_corners<FACES>(SB, i, look[u] ? sx : 0ll, look[u] ? sxy : 0ll, s0[u], s1[u]);
         }
 #pragma unroll
         for (int u = 0; u < NODES; ++u) {
@@ -1632,7 +1638,7 @@ __device__ __forceinline__ void node_filter(const float4 (&p)[NODES], const bool
 // take the registers of a quarter of them: a rebuild's selection 1.5 against
 // 1.4 ms at 262,144 particles), two where a warp has an SM's share to itself
 // (a step of 1,000 particles 38.4 against 39.6 us).
-template <int KIND, int NODES>
+template <int KIND, int NODES, bool FACES = false>
 __device__ __forceinline__ int cull_pair(const NarrowArgs& n, int A, int B, double skin, int lane,
                                          unsigned short* queue, int& kept)
 {
@@ -1654,7 +1660,7 @@ __device__ __forceinline__ int cull_pair(const NarrowArgs& n, int A, int B, doub
         if (c < ncl) {
             float4 cl = n.G.clus_sphere[GA.clus_off + c];
             cl.w += (float)skin;
-            k = !cluster_culled<KIND>(cl, xf, GB, SB, probe);
+            k = !cluster_culled<KIND, FACES>(cl, xf, GB, SB, probe);
         }
         keep |= ((unsigned long long)__ballot_sync(0xffffffffu, k)) << c0;
     }
@@ -1691,7 +1697,7 @@ __device__ __forceinline__ int cull_pair(const NarrowArgs& n, int A, int B, doub
             on[u] = lane < r[u].y;
         }
         if (left > NODES) fetch();
-        node_filter<KIND, NODES>(p, on, xf, GB, SB, perr, probe, out);
+        node_filter<KIND, NODES, FACES>(p, on, xf, GB, SB, perr, probe, out);
 #pragma unroll
         for (int u = 0; u < NODES; ++u) {
             const unsigned int m = __ballot_sync(0xffffffffu, !out[u]);
@@ -1981,7 +1987,7 @@ struct SlotEval {
 
 // the exact predicate of node k (relative to the geometry) of A against B (st);
 // e.ov keeps ov0 when the predicate stops before the distance
-template <int KIND>
+template <int KIND, bool FACES = false>
 __device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, const PairState& st, int k, int3 bcell, double ov0,
                                                SlotEval& e)
 {
@@ -1999,7 +2005,7 @@ __device__ __forceinline__ bool slot_predicate(const NarrowArgs& n, const PairSt
     e.r = xm_rot(qA, node);
     e.gp = mk3(e.r.x + e.cA.x, e.r.y + e.cA.y, e.r.z + e.cA.z);
     e.ov = ov0;
-    return node_predicate<KIND>(e.gp, bcell, sg, e.cB, e.qB, GB, SB, rB2, n.a.probe, e.ov, e.fx, e.fy, e.fz, e.pv);
+    return node_predicate<KIND, FACES>(e.gp, bcell, sg, e.cB, e.qB, GB, SB, rB2, n.a.probe, e.ov, e.fx, e.fy, e.fz, e.pv);
 }
 
 // A contact's results go out in 16-byte stores to six whole sectors, side by
@@ -2499,7 +2505,7 @@ struct SlotEval32 {
 };
 
 // as slot_predicate
-template <int KIND>
+template <int KIND, bool FACES = false>
 __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, const PairState& st, int k, int3 bcell, float ov0,
                                                  SlotEval32& e)
 {
@@ -2546,7 +2552,7 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, const Pair
                     // there would carry errors of 1e-8 m, so the
                     // (few) wall contacts interpolate in double
                     double4 s0, s1;
-                    load_corners(SB, c0, sx, sxy, s0, s1);
+                    load_corners<FACES>(SB, c0, sx, sxy, s0, s1);
                     double pd[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
                     const double ovd = -xm_trilinear(gx - (double)i0, gy - (double)j0, gz - (double)k0, pd);
 #pragma unroll
@@ -2556,7 +2562,7 @@ __device__ __forceinline__ bool slot_predicate32(const NarrowArgs& n, const Pair
                     hit = ovd >= -n.a.probe;
                 } else {
                     float4 s0, s1;
-                    load_corners(SB, c0, sx, sxy, s0, s1);
+                    load_corners<FACES>(SB, c0, sx, sxy, s0, s1);
                     pv[0] = s0.x; pv[1] = s0.y; pv[2] = s0.z; pv[3] = s0.w;
                     pv[4] = s1.x; pv[5] = s1.y; pv[6] = s1.z; pv[7] = s1.w;
                     e.ov = -trilinear32(pv, fx, fy, fz);
@@ -3345,7 +3351,7 @@ __device__ __forceinline__ int4 small_slots(const NarrowArgs& n, const PairListD
                                             unsigned short* queue, unsigned long long* stats)
 {
     int kept;
-    int ncand = cull_pair<KIND, NODES>(n, A, B, 0.0, lane, queue, kept);
+    int ncand = cull_pair<KIND, NODES, true>(n, A, B, 0.0, lane, queue, kept);
     if (n.a.stats && lane == 0) {
         atomicAdd(&stats[0], 1ull);
         atomicAdd(&stats[1], (unsigned long long)min(n.G.geo[n.P.geo[A]].clus_count, MAX_CLUSTERS));
@@ -3386,11 +3392,11 @@ __device__ __forceinline__ bool small_contact(const NarrowArgs& n, const PairLis
     Real o[9];
     if constexpr (MIXED) {
         SlotEval32 e;
-        hit = slot_predicate32<KIND>(n, st, k, bcell, 0.f, e);
+        hit = slot_predicate32<KIND, true>(n, st, k, bcell, 0.f, e);
         if (hit) nid = contact_law32<KIND>(n, L, R, s, s, A, B, st, k, oc_off, oc_cnt, e, o);
     } else {
         SlotEval e;
-        hit = slot_predicate<KIND>(n, st, k, bcell, 0., e);
+        hit = slot_predicate<KIND, true>(n, st, k, bcell, 0., e);
         if (hit) nid = contact_law<KIND>(n, L, R, s, s, A, B, st, k, oc_off, oc_cnt, e, o);
     }
     if (hit) store_force(L, s, o);
@@ -3502,7 +3508,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, BLOCKS) k_small_pairs(SmallA
                         const double3 cB = n.P.pos[B];
                         const double rs = rA + GB.radius;
                         if (lengthSq3(cA - cB) <= rs * rs * (1.0 + 4.0 * BOUND_REL))
-                            pass = !body_culled32(cA, rA, cB, n.P.rot + 3ll * B, true, n.G.geo32[n.P.geo[B]], n.G,
+                            pass = !body_culled32<true>(cA, rA, cB, n.P.rot + 3ll * B, true, n.G.geo32[n.P.geo[B]], n.G,
                                                   n.a.probe);
                     }
                     const unsigned int m = __ballot_sync(full, pass);
@@ -3547,7 +3553,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, BLOCKS) k_small_pairs(SmallA
                         const double rs = rA + GB.grid_radius;
                         const double3 cW = n.W.pos[w];
                         pass = lengthSq3(cA - cW) <= rs * rs * (1.0 + 4.0 * BOUND_REL) &&
-                               !body_culled32(cA, rA, cW, n.W.rot + 3ll * w, false, n.GW.geo32[n.W.geo[w]], n.GW,
+                               !body_culled32<true>(cA, rA, cW, n.W.rot + 3ll * w, false, n.GW.geo32[n.W.geo[w]], n.GW,
                                               n.a.probe);
                     }
                 }
@@ -3696,28 +3702,34 @@ __device__ __forceinline__ void small_partner_sum(const SmallAdvanceArgs& a, int
     const int head = a.r_head[i];
     if (head < 0) return;
     a.r_head[i] = -1;
+    int pair[LOCAL], owner[LOCAL], cnt = 0;
+    for (int p = head; p >= 0; p = L.r_next[p], ++cnt) {
+        if (cnt >= LOCAL) continue;
+        const int own = L.pairA[p];
+        int b = cnt - 1;
+        while (b >= 0 && owner[b] > own) { owner[b + 1] = owner[b]; pair[b + 1] = pair[b]; --b; }
+        owner[b + 1] = own;
+        pair[b + 1] = p;
+    }
     const Real* pf = reinterpret_cast<const Real*>(L.pf);
-    int pair[LOCAL], owner[LOCAL], last = -1;
-    for (bool more = true; more;) {
-        int cnt = 0;
-        more = false;
+    if (cnt <= LOCAL) {
+#pragma unroll 4
+        for (int e = 0; e < cnt; ++e) f.add(pf, pair[e], Real(-1), 2);
+        return;
+    }
+    int last = -1;
+    for (int left = cnt; left > 0; left -= LOCAL) {
+        int kept = 0;
         for (int p = head; p >= 0; p = L.r_next[p]) {
             const int own = L.pairA[p];
-            if (own <= last) continue;
-            if (cnt == LOCAL) {
-                more = true;
-                if (own > owner[LOCAL - 1]) continue;
-                --cnt;
-            }
-            int b = cnt - 1;
+            if (own <= last || (kept == LOCAL && own > owner[LOCAL - 1])) continue;
+            int b = (kept < LOCAL ? kept++ : LOCAL - 1) - 1;
             while (b >= 0 && owner[b] > own) { owner[b + 1] = owner[b]; pair[b + 1] = pair[b]; --b; }
             owner[b + 1] = own;
             pair[b + 1] = p;
-            ++cnt;
         }
-#pragma unroll 4
-        for (int e = 0; e < cnt; ++e) f.add(pf, pair[e], Real(-1), 2);
-        if (cnt) last = owner[cnt - 1];
+        for (int e = 0; e < kept; ++e) f.add(pf, pair[e], Real(-1), 2);
+        last = owner[LOCAL - 1];
     }
 }
 
