@@ -1006,11 +1006,12 @@ struct fundem_sim {
     // Small sets step with two launches (launch_small_pairs,
     // launch_small_advance).  The rule: no images, no pair cache or neighbour
     // list, a dense cell table, not under the stage timers, which see the
-    // stages one by one, with the tables of cell faces, and no more particles than the block of a small step
-    // pays for: its threads idle through most of the contact law.  Ten steps of
-    // a pour, small against staged, us: 4,096 particles 906 against 1,140 (graph
-    // 876, 967), 5,000 1,045 and 1,139 (979, 959), 6,500 1,274 and 1,241 (1,196,
-    // 1,058), 8,191 1,553 and 1,324 (1,430, 1,154).
+    // stages one by one, with the tables of cell faces, and no more particles
+    // than the block of a small step pays for: its threads idle through most of
+    // the contact law.  Ten steps of a pour, small against staged, us: 4,096
+    // particles 906 against 1,140 (graph 876, 967), 5,000 1,045 and 1,139 (979,
+    // 959), 6,500 1,274 and 1,241 (1,196, 1,058), 8,191 1,553 and 1,324 (1,430,
+    // 1,154).
     static constexpr int SMALL_PARTICLES = 5120;
     DevArray<int> small_head;
     DevArray<double> small_own;
